@@ -22,6 +22,15 @@ struct pt_batch {
   };
   std::vector<Cls> classes;
   int64_t tiles;
+  // problems on layer tiles: their (problem, tile) and (problem, first node)
+  // lists, and the scratch that an apply takes from `lay_pool` on its stream
+  // (applies on several streams each get their own)
+  int2 *d_lay;
+  int64_t lay_tiles, lay_nodes, lay_values;
+  std::vector<int2> hlay;
+  int coloured;             // problems on coloured tiles
+  cudaMemPool_t lay_pool;
+  bool own_lay_pool;
   // pooled (server) batches: stream-ordered buffers; host copies kept until destroy
   cudaMemPool_t pool;
   cudaStream_t stream;
@@ -66,20 +75,54 @@ __global__ void batch_bc_kernel(const ptk::BatchProb *__restrict__ probs, const 
                                 T *const *__restrict__ yptr)
 {
   const ptk::BatchProb &p = probs[blockIdx.y];
-  if (!p.mask) return;
+  if (!p.mask || p.layer) return;
   const T *x = uptr[blockIdx.y];
   T *y = yptr[blockIdx.y];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.nvel; i += (int64_t)gridDim.x * blockDim.x)
     if (p.mask[i]) y[i] = x[i];
 }
 
+// The problems on layer tiles: every tile in one launch, every node in a second.
+template <typename T, bool MASKED>
+pt_status batch_apply_layers(pt_batch *b, const T *const *u, T *const *y, cudaStream_t st)
+{
+  constexpr size_t smem = ptk::layer_smem_bytes<T, LNT>();
+  pt_status as = kernel_attrs((const void *)ptk::a11_layer_batch_kernel<T, LNT, MASKED>, smem);
+  if (as != PT_OK) return as;
+  const ptk::BatchProb *probs = std::is_same<T, double>::value ? b->d_probs64 : b->d_probs32;
+  T *scratch = nullptr;
+  PT_CUDA(cudaMallocFromPoolAsync((void **)&scratch, sizeof(T) * (size_t)b->lay_values, b->lay_pool, st));
+  ptk::a11_layer_batch_kernel<T, LNT, MASKED><<<(unsigned)b->lay_tiles, LNT, smem, st>>>(probs, b->d_lay, u, scratch);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) {
+    cudaLaunchAttribute pdl[1];
+    pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)b->lay_nodes);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = pdl;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, ptk::layer_gather_batch_kernel<T, LNT, MASKED>, probs,
+                           (const int2 *)(b->d_lay + b->lay_tiles), u, (const T *)scratch, y);
+  }
+  cudaFreeAsync(scratch, st);
+  if (e != cudaSuccess) return fail(PT_ERR_CUDA, "batched layer tiles: %s", cudaGetErrorString(e));
+  return PT_OK;
+}
+
 // MASKED: the MatShell apply of every problem with a mask (columns inside the
-// kernel, rows by one more launch).
+// kernel, rows by one more launch; layer tiles set both).
 template <typename T, bool MASKED>
 pt_status batch_apply(pt_batch *b, const T *const *u, T *const *y, void *stream)
 {
   if (!b || !u || !y) return fail(PT_ERR_BAD_ARG, "NULL argument");
   const cudaStream_t st = (cudaStream_t)stream;
+  if (b->lay_tiles) {
+    pt_status s = batch_apply_layers<T, MASKED>(b, u, y, st);
+    if (s != PT_OK) return s;
+  }
   bool first = true;
   for (const pt_batch::Cls &c : b->classes) {
     pt_status s;
@@ -89,7 +132,7 @@ pt_status batch_apply(pt_batch *b, const T *const *u, T *const *y, void *stream)
     if (s != PT_OK) return s;
     first = false;
   }
-  if (MASKED) {
+  if (MASKED && b->coloured) {
     const ptk::BatchProb *probs = std::is_same<T, double>::value ? b->d_probs64 : b->d_probs32;
     batch_bc_kernel<T><<<dim3(32, (unsigned)b->n), 256, 0, st>>>(probs, u, y);
     cudaError_t e = cudaGetLastError();
@@ -114,7 +157,9 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
   std::vector<ptk::BatchProb> p64(n), p32(n);
   // class key: (pass, TX) -> items
   std::map<std::pair<int, int>, std::vector<int4>> cls;
-  int64_t tiles = 0;
+  int64_t tiles = 0, lay_values = 0;
+  int coloured = 0;
+  std::vector<int2> lay, lay_nodes;
   for (int i = 0; i < n; i++) {
     pt_op *op = ops[i];
     pt_status s = check_ready(op, true);
@@ -122,12 +167,10 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
     if (!op->full_box) return fail(PT_ERR_UNSUPPORTED, "batch problem %d: one-rank boxes only", i);
     if ((s = ensure_geometry(op)) != PT_OK) return s;
     if (!op->geom_ok) return fail(PT_ERR_BAD_ARG, "batch problem %d has w*eta/detJ <= 0 somewhere", i);
-    // any tile width covers the box: tiles read K columns ex < mx <= MXP
     const int TX = tile_x ? tile_x : op->TX;
     ptk::BatchProb d;
     d.b = op->box;
     d.ntx = (op->mx + TX - 1) / TX;
-    d.MXP = op->MXP;
     int L = (lz && lz[i] > 0) ? lz[i] : op->LZ;
     if (L > op->mz) L = op->mz;
     d.LZ = L;
@@ -136,10 +179,24 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
     d.mask = op->has_mask ? op->d_mask : nullptr;
     d.mbits = op->has_mask ? op->d_mbits : nullptr;
     d.nvel = op->nvel;
+    // layer tiles unless the caller asks for a z-chunk depth (a box whose own
+    // applies use element matrices too: they are not batched)
+    d.layer = (op->a11_kernel == A11_LAYER || op->a11_kernel == A11_EBE) && !(lz && lz[i] > 0);
+    d.lg = op->lg;
+    d.lay_off = lay_values;
     d.K = op->d_K;
     p64[i] = d;
     d.K = op->d_K32;
     p32[i] = d;
+    if (d.layer) {
+      const int64_t nt = op->lg.tiles;
+      lay_values += nt * ptk::LayerLayout<LNT>::TILE;
+      tiles += nt;
+      for (int64_t k = 0; k < nt; k++) lay.push_back(make_int2(i, (int)k));
+      for (int64_t k = 0; k < (int64_t)op->lg.nodes(); k += ptk::LAYER_GATHER_NODES) lay_nodes.push_back(make_int2(i, (int)k));
+      continue;
+    }
+    coloured++;
     for (int zc = 0; zc < d.nzc; zc++)
       for (int ej = 0; ej < op->my; ej++)
         for (int tx = 0; tx < d.ntx; tx++) {
@@ -153,6 +210,12 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
   b->n = n;
   b->ops.assign(ops, ops + n);
   b->tiles = tiles;
+  b->coloured = coloured;
+  b->lay_tiles = (int64_t)lay.size();
+  b->lay_nodes = (int64_t)lay_nodes.size();
+  b->lay_values = lay_values;
+  b->hlay = std::move(lay);
+  b->hlay.insert(b->hlay.end(), lay_nodes.begin(), lay_nodes.end());
   b->pool = pool;
   b->stream = stream;
   std::vector<int4> &all = b->hitems;
@@ -168,21 +231,39 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
   b->h64 = p64;
   b->h32 = p32;
   cudaError_t e;
-  const size_t bp = sizeof(ptk::BatchProb) * n, bi = sizeof(int4) * all.size();
+  const size_t bp = sizeof(ptk::BatchProb) * n, bi = sizeof(int4) * (all.size() + 1);
+  const size_t bl = sizeof(int2) * (b->hlay.size() + 1), bic = bi - sizeof(int4), blc = bl - sizeof(int2);
   if (pool) {
     e = cudaMallocFromPoolAsync((void **)&b->d_probs64, bp, pool, stream);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&b->d_probs32, bp, pool, stream);
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&b->d_items, bi, pool, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_probs64, b->h64.data(), bp, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_probs32, b->h32.data(), bp, cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_items, all.data(), bi, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_items, all.data(), bic, cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync((void **)&b->d_lay, bl, pool, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(b->d_lay, b->hlay.data(), blc, cudaMemcpyHostToDevice, stream);
+    b->lay_pool = pool;
   } else {
     e = cudaMalloc(&b->d_probs64, bp);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_probs32, bp);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_items, bi);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_probs64, p64.data(), bp, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_probs32, p32.data(), bp, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_items, all.data(), bi, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_items, all.data(), bic, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_lay, bl);
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_lay, b->hlay.data(), blc, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && b->lay_tiles) {
+      cudaMemPoolProps pp{};
+      pp.allocType = cudaMemAllocationTypePinned;
+      pp.location.type = cudaMemLocationTypeDevice;
+      e = cudaGetDevice(&pp.location.id);
+      if (e == cudaSuccess) e = cudaMemPoolCreate(&b->lay_pool, &pp);
+      if (e == cudaSuccess) {
+        b->own_lay_pool = true;
+        uint64_t keep = UINT64_MAX;  // kept from apply to apply, given back with the batch
+        e = cudaMemPoolSetAttribute(b->lay_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      }
+    }
   }
   if (e != cudaSuccess) {
     pt_status s = fail(e == cudaErrorMemoryAllocation ? PT_ERR_OOM : PT_ERR_CUDA, "pt_batch_create: %s",
@@ -207,17 +288,21 @@ pt_status pt_batch_create(int n, pt_op *const *ops, const int32_t *lz, pt_batch 
 pt_status pt_batch_destroy(pt_batch *b)
 {
   if (!b) return PT_OK;
-  void *bufs[] = {b->d_probs64, b->d_probs32, b->d_items};
+  void *bufs[] = {b->d_probs64, b->d_probs32, b->d_items, b->d_lay};
   for (void *p : bufs) {
     if (!p) continue;
     if (b->pool) cudaFreeAsync(p, b->stream);
     else cudaFree(p);
   }
+  if (b->own_lay_pool) cudaMemPoolDestroy(b->lay_pool);
   delete b;
   return PT_OK;
 }
 
-int64_t pt_batch_launches_per_apply(const pt_batch *b) { return b ? (int64_t)b->classes.size() : 0; }
+int64_t pt_batch_launches_per_apply(const pt_batch *b)
+{
+  return b ? (int64_t)b->classes.size() + (b->lay_tiles ? 2 : 0) : 0;
+}
 int64_t pt_batch_tiles(const pt_batch *b) { return b ? b->tiles : 0; }
 
 pt_status pt_batch_a11_apply_d(pt_batch *b, const double *const *u, double *const *y, int masked, void *stream)

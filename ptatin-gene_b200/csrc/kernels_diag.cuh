@@ -41,25 +41,23 @@ constexpr size_t diag_smem_bytes()
 }
 
 // One element (thread t), quadrature plane A: Q_m for m = 0..2 into the
-// tile, then S.  Ke points at K(row, q = 0, r = 0, ex).
-template <int TX, bool KTX>
+// tile, then S.  Ke points at the element's entry (0, 0) of K.
+template <int TX>
 __device__ __forceinline__ void diag_element_plane(int A, double *yt, double *side, const int sl[3], int t, int warp,
-                                                   bool to_side, unsigned amask, const double *__restrict__ Ke,
-                                                   int64_t MXP_)
+                                                   bool to_side, unsigned amask, const double *__restrict__ Ke)
 {
-  const int64_t MXP = KTX ? (int64_t)TX : MXP_;
   double z[3][3];
 #pragma unroll
   for (int s = 0; s < 3; s++)
 #pragma unroll
     for (int k = 0; k < 3; k++) z[s][k] = c_zdiag[A][s][k];
-  const double *kp = Ke + (int64_t)(9 * A) * 9 * MXP;
+  const double *kp = Ke + koff(9 * A, 0);
   double S[27];
 #pragma unroll 1
   for (int m = 0; m < 3; m++) {
-    const double *km = kp + (int64_t)(3 * m) * MXP;
+    const double *km = kp + koff(0, 3 * m);
     double Q[27];
-    q2::diag_form_plane<double>([&](int p, int d) { return ldk(km + (int64_t)(9 * p + d) * MXP); }, z, Q);
+    q2::diag_form_plane<double>([&](int p, int d) { return ldk(km + koff(p, d)); }, z, Q);
     if (m == 0) {
 #pragma unroll
       for (int n = 0; n < 27; n++) S[n] = Q[n];
@@ -74,11 +72,10 @@ __device__ __forceinline__ void diag_element_plane(int A, double *yt, double *si
 }
 
 // One tile (x-tile tx, row ej, z-chunk zc); the whole CTA.
-template <int TX, bool KTX>
+template <int TX>
 __device__ __forceinline__ void diag_tile(const StreamGrid &g, int tx, int ej, int zc, const double *__restrict__ K,
                                           double *__restrict__ y)
 {
-  const int64_t MXP = KTX ? (int64_t)TX : g.MXP;
   using L = TileLayout<TX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *yt = reinterpret_cast<double *>(smem_raw);
@@ -98,22 +95,23 @@ __device__ __forceinline__ void diag_tile(const StreamGrid &g, int tx, int ej, i
 
   const bool to_side = (lane == 31) && (warp < L::NW - 1);
   const unsigned amask = __ballot_sync(0xffffffffu, active);
-  if (t == 0) prefetch_k_plane(K + kidx(ej + (int64_t)g.b.my * ek0, 0, 0, MXP, 0), (uint32_t)(sizeof(double) * 81 * MXP));
+  const int64_t e0 = ex0 + (int64_t)g.b.mx * ej, el = (int64_t)g.b.mx * g.b.my;
+  const int ne = min(TX, g.b.mx - ex0);
+  prefetch_k(K, 0, e0 + el * ek0, e0 + el * ek0 + ne);
 
 #pragma unroll 1
   for (int ek = ek0; ek < ek1; ek++) {
-    const int64_t row = ej + (int64_t)g.b.my * ek;
     const int s0 = (int)((2 * (int64_t)ek) % 3), s1 = (s0 + 1) % 3, s2 = (s0 + 2) % 3;
     const int sl[3] = {s0, s1, s2};
     const bool more = ek + 1 < ek1;
     if (active) {
-      const int64_t krow = kidx(row, 0, 0, MXP, ex);
-      const uint32_t kb = (uint32_t)(sizeof(double) * 81 * MXP);
+      const int64_t e = e0 + el * ek;
+      const double *Ke = K + kelem(e + t);
 #pragma unroll 1
       for (int A = 0; A < 3; A++) {
-        if (t == 0 && (A < 2 || more))
-          prefetch_k_plane(A < 2 ? K + kidx(row, 9 * (A + 1), 0, MXP, 0) : K + kidx(row + g.b.my, 0, 0, MXP, 0), kb);
-        diag_element_plane<TX, KTX>(A, yt, side, sl, t, warp, to_side, amask, K + krow, MXP);
+        if (A < 2) prefetch_k(K, A + 1, e, e + ne);
+        else if (more) prefetch_k(K, 0, e + el, e + el + ne);
+        diag_element_plane<TX>(A, yt, side, sl, t, warp, to_side, amask, Ke);
       }
     }
     __syncthreads();
@@ -138,13 +136,13 @@ constexpr int diag_min_blocks()
   return 256 / TX;
 }
 
-template <int TX, bool KTX>
+template <int TX>
 __global__ void __launch_bounds__(TX, diag_min_blocks<TX>()) diag_stream_kernel(StreamGrid g, const double *__restrict__ K,
                                                                                double *__restrict__ y)
 {
   const int bid = blockIdx.x;
   const int ixc = bid % g.nxc, iyc = (bid / g.nxc) % g.nyc, izc = bid / (g.nxc * g.nyc);
-  diag_tile<TX, KTX>(g, g.px + 2 * ixc, g.py + 2 * iyc, g.zc0 + 2 * izc, K, y);
+  diag_tile<TX>(g, g.px + 2 * ixc, g.py + 2 * iyc, g.zc0 + 2 * izc, K, y);
 }
 
 }  // namespace ptk

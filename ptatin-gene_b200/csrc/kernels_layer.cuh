@@ -1,0 +1,449 @@
+// Layer tiles ("b200_layer"): the streaming A11 kernel's arithmetic on
+// single-layer tiles, for boxes too small to hide a z-march.
+//
+// What bounds a small box is latency, not bandwidth: one element takes a
+// thread about 20 us (4,700 dependent FP64 operations at two warps per
+// scheduler), and the coloured z-march puts a chunk's layers and four colour
+// launches one behind the other (41x37x29: 115 us for 1,375 warps of work, on
+// a chip that holds 1,184).  Here every element runs at once: each tile
+// writes its node sums to scratch, and one gather adds the (at most 4 per
+// row, 8 at an x-tile edge) sums of a node in a fixed order, with the
+// Dirichlet rows in the same pass.  Two launches, deterministic, no colours.
+// The price is the scratch, about 450 B written and read per element next to
+// 1.9 KB of K, which is why large boxes keep the z-march.
+//
+// A tile is E consecutive elements whatever the row length (layer_grid.cuh),
+// so rows that do not divide it leave no thread idle.
+#pragma once
+
+#include <cstdint>
+
+#include "kernels_diag.cuh"
+#include "layer_grid.cuh"
+
+namespace ptk {
+
+constexpr int LAYER_NT = 128;
+
+template <typename T, int NT>
+constexpr size_t layer_smem_bytes()
+{
+  return sizeof(T) * (2 * (size_t)LayerLayout<NT>::TILE + LayerLayout<NT>::SIDE);
+}
+
+template <typename T, int NT>
+constexpr size_t layer_diag_smem_bytes()
+{
+  return sizeof(T) * ((size_t)LayerLayout<NT>::TILE + LayerLayout<NT>::SIDE);
+}
+
+// The thread's element and its entries of a tile's node row.
+struct LayerThread {
+  int e;         // element
+  bool active;
+  int od, en;    // 2t+1, and 2t+2: tid + 1 or the segment's end entry
+  bool to_side;  // 2t+2 is the next warp's first column: kept in the side buffer
+};
+
+template <int NT>
+__device__ __forceinline__ LayerThread layer_thread(const LayerGrid &g, int tile)
+{
+  LayerThread a;
+  const int tid = threadIdx.x, e0 = tile * g.E;
+  a.e = e0 + tid;
+  a.active = tid < g.E && a.e < g.nel;
+  const int row = (int)g.dmx.div((uint32_t)a.e), row0 = (int)g.dmx.div((uint32_t)e0);
+  const bool last = a.e + 1 == (row + 1) * g.mx || tid + 1 == g.E;  // of its segment
+  a.od = g.odd + tid;
+  a.en = last ? 2 * g.odd + (row - row0) : tid + 1;
+  a.to_side = (tid & 31) == 31 && !last;
+  return a;
+}
+
+// A segment's first dof (node row 0 of node plane 0), first thread and length.
+struct LayerSeg {
+  int64_t k0;
+  int t0, len;
+};
+
+// Fetches the tile's node values of u (Dirichlet entries as zeros where mbits
+// is given) with asynchronous copies, every copy of the tile in flight at
+// once, a warp to a line (one of a segment's 9 node rows).  The mask words of
+// all lines are staged first (`stage`: shared memory that nothing else uses
+// yet, the size of a tile), so the copies wait for one round trip and not for
+// one each.  Ends with the copies committed; `stage` is free after the next
+// barrier.
+template <typename T, int NT>
+__device__ __forceinline__ void layer_fetch(T *ut, void *stage, const LayerGrid &g, int tile, const T *__restrict__ u,
+                                            const uint32_t *__restrict__ mbits)
+{
+  using L = LayerLayout<NT>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e0 = tile * g.E, n = min(g.E, g.nel - e0);
+  const int row0 = (int)g.dmx.div((uint32_t)e0);
+  const int segs = (int)g.dmx.div((uint32_t)(e0 + n - 1)) - row0 + 1, lines = 9 * segs;
+  LayerSeg *seg = reinterpret_cast<LayerSeg *>(stage);
+  uint32_t *words = reinterpret_cast<uint32_t *>(seg + segs);
+  const int mw = (3 * (2 * min(g.mx, n) + 1) + 31) / 32 + 1;  // words that cover a line, wherever it starts
+  if ((int)threadIdx.x < segs) {
+    LayerSeg s;
+    const int row = row0 + threadIdx.x;
+    const int ek = (int)g.dmy.div((uint32_t)row), ej = row - ek * g.my;
+    layer_segment(g, e0, row0, n, threadIdx.x, s.t0, s.len);
+    s.k0 = 3 * (g.off + 2 * (int64_t)(e0 + s.t0 - row * g.mx) + 2 * (int64_t)ej * g.X + 2 * (int64_t)ek * g.XY);
+    seg[threadIdx.x] = s;
+  }
+  __syncthreads();
+  if (mbits) {
+    for (int line = warp; line < lines; line += L::NW) {
+      const int sg = line / 9, kj = line - 9 * sg, k = kj / 3, j = kj - 3 * k;
+      const LayerSeg s = seg[sg];
+      const int64_t k0 = s.k0 + 3 * (j * g.X + k * g.XY);
+      const int64_t w0 = k0 >> 5;
+      const int nw = (int)(((k0 + 3 * (2 * s.len + 1) - 1) >> 5) - w0 + 1);
+      if (lane < nw) words[line * mw + lane] = mbits[w0 + lane];
+    }
+    __syncthreads();
+  }
+  for (int line = warp; line < lines; line += L::NW) {
+    const int sg = line / 9, kj = line - 9 * sg, k = kj / 3, j = kj - 3 * k;
+    const LayerSeg s = seg[sg];
+    const int64_t k0 = s.k0 + 3 * (j * g.X + k * g.XY);
+    const int nd = 3 * (2 * s.len + 1);
+    const T *src = u + k0;
+    T *row = ut + k * L::PLANE + j * L::ROW + s.t0;
+    const int end = 2 * g.odd + sg - s.t0;  // the end entry, from `row`
+    const uint32_t *w = words + line * mw;
+    const int b0 = (int)(k0 & 31);
+#pragma unroll 4
+    for (int d = lane; d < nd; d += 32) {
+      const int m = (d * 43691) >> 17, c = d - 3 * m;  // d / 3 for d < 2^16
+      const int h = m >> 1;
+      T *dst = row + c * L::COMP + ((m & 1) ? g.odd + h : (h == s.len ? end : h));
+      uint32_t bytes = sizeof(T);
+      if (mbits) {
+        const int pos = b0 + d;
+        if ((w[pos >> 5] >> (pos & 31)) & 1u) bytes = 0;  // zero-filled
+      }
+      const uint32_t sd = (uint32_t)__cvta_generic_to_shared(dst);
+      if (sizeof(T) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sd), "l"(src + d), "r"(bytes) : "memory");
+      else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sd), "l"(src + d), "r"(bytes) : "memory");
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <typename T, int NT>
+__device__ __forceinline__ void layer_zero(T *yt)
+{
+  using L = LayerLayout<NT>;
+  // the tile and the side buffer behind it
+  constexpr int N16 = (int)(sizeof(T) * (L::TILE + L::SIDE) / 16);
+  static_assert(sizeof(T) * (L::TILE + L::SIDE) % 16 == 0, "16-byte stores");
+  for (int i = threadIdx.x; i < N16; i += NT) reinterpret_cast<uint4 *>(yt)[i] = make_uint4(0, 0, 0, 0);
+}
+
+// Adds V (27 node values [k*9 + j*3 + i]) to component l of the thread's
+// nodes, columns 2t and 2t+1 first, then (after the warp's other lanes) 2t+2:
+// the order in which a column shared by two elements is summed is fixed.  A
+// group's entries are all read before any is written (tile_add_nodes).
+template <typename T, int NT>
+__device__ __forceinline__ void layer_add(T *yt, T *side, const LayerThread &a, unsigned amask, int l, const T V[27])
+{
+  using L = LayerLayout<NT>;
+  {
+    T *b0 = yt + l * L::COMP + threadIdx.x, *b1 = yt + l * L::COMP + a.od;
+    T c[18];
+#pragma unroll
+    for (int kj = 0; kj < 9; kj++) {
+      c[2 * kj] = b0[kj * L::ROW];
+      c[2 * kj + 1] = b1[kj * L::ROW];
+    }
+#pragma unroll
+    for (int kj = 0; kj < 9; kj++) {
+      b0[kj * L::ROW] = c[2 * kj] + V[3 * kj];
+      b1[kj * L::ROW] = c[2 * kj + 1] + V[3 * kj + 1];
+    }
+  }
+  __syncwarp(amask);
+  {
+    T *b2 = a.to_side ? side + (threadIdx.x >> 5) * 27 + l : yt + l * L::COMP + a.en;
+    const int s = a.to_side ? 3 : L::ROW;
+    T c[9];
+#pragma unroll
+    for (int kj = 0; kj < 9; kj++) c[kj] = b2[kj * s];
+#pragma unroll
+    for (int kj = 0; kj < 9; kj++) b2[kj * s] = c[kj] + V[3 * kj + 2];
+  }
+  __syncwarp(amask);
+}
+
+// The tile's sums to scratch: the side buffer's columns added to their tile
+// entries, then one bulk copy of the tile.
+template <typename T, int NT>
+__device__ __forceinline__ void layer_dump(T *yt, T *side, const LayerThread &a, T *__restrict__ out)
+{
+  using L = LayerLayout<NT>;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned last = __ballot_sync(0xffffffffu, a.active && a.to_side);
+  if (last && lane < 27) {
+    const int kj = lane / 3, l = lane - 3 * kj;
+    yt[l * L::COMP + kj * L::ROW + 32 * (warp + 1)] += side[warp * 27 + lane];
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint32_t s = (uint32_t)__cvta_generic_to_shared(yt);
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out), "r"(s),
+                 "r"((uint32_t)(sizeof(T) * L::TILE))
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // before the tile's memory is given back
+  }
+}
+
+// One element (thread a), Gauss plane A: element_plane of the streaming
+// kernel on the layer tile's entries.
+template <typename T, int NT>
+__device__ __forceinline__ void layer_plane(int A, const T *ut, T *yt, T *side, const LayerThread &a, unsigned amask,
+                                            const T *__restrict__ Ke)
+{
+  using L = LayerLayout<NT>;
+  T G[3][3][9];  // [d][l][b*3+c]
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    T Q[9], R[9];
+    const T *ul = ut + l * L::COMP;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const T *p = ul + (i == 0 ? (int)threadIdx.x : (i == 1 ? a.od : a.en)) + j * L::ROW;
+        zeta_fwd_rt<T>(A, p[0], p[L::PLANE], p[2 * L::PLANE], Q[3 * j + i], R[3 * j + i]);
+      }
+    q2::plane_fwd(Q, R, G[0][l], G[1][l], G[2][l]);
+  }
+  // K of the next two points in flight while one computes, as in the streaming kernel
+  const T *kp = Ke + koff(9 * A, 0);
+  T Kn[9], Kn2[9];
+#pragma unroll
+  for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(0, r));
+#pragma unroll
+  for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(1, r));
+#pragma unroll
+  for (int p = 0; p < 9; p++) {
+    T Kq[9];
+#pragma unroll
+    for (int r = 0; r < 9; r++) Kq[r] = Kn[r];
+#pragma unroll
+    for (int r = 0; r < 9; r++) Kn[r] = Kn2[r];
+    if (p < 7) {
+#pragma unroll
+      for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(p + 2, r));
+    }
+    q2::qp_action_K(Kq, G, p);
+  }
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    T Qt[9], Rt[9];
+    q2::plane_bwd(G[0][l], G[1][l], G[2][l], Qt, Rt);
+    T C[27];
+#pragma unroll
+    for (int ji = 0; ji < 9; ji++) zeta_bwd_rt<T>(A, Qt[ji], Rt[ji], C[ji], C[9 + ji], C[18 + ji]);
+    layer_add<T, NT>(yt, side, a, amask, l, C);
+  }
+}
+
+// One tile; the whole CTA.  mbits: packed Dirichlet mask or null.
+template <typename T, int NT>
+__device__ __forceinline__ void layer_tile(const LayerGrid &g, int tile, const T *__restrict__ K,
+                                           const T *__restrict__ u, const uint32_t *__restrict__ mbits,
+                                           T *__restrict__ out)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *ut = reinterpret_cast<T *>(smem_raw);
+  T *yt = ut + L::TILE;
+  T *side = yt + L::TILE;
+  // the gather may be scheduled as soon as every tile has started; it waits
+  // for this grid's stores before it reads
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const LayerThread a = layer_thread<NT>(g, tile);
+  const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
+  prefetch_k(K, 0, e0, e1);
+  layer_fetch<T, NT>(ut, yt, g, tile, u, mbits);
+  __syncthreads();  // the stage is read: the y tile may be zeroed
+  layer_zero<T, NT>(yt);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const unsigned amask = __ballot_sync(0xffffffffu, a.active);
+  const T *Ke = K + kelem(a.e);
+#pragma unroll 1
+  for (int A = 0; A < 3; A++) {
+    if (A < 2) prefetch_k(K, A + 1, e0, e1);
+    if (a.active) layer_plane<T, NT>(A, ut, yt, side, a, amask, Ke);
+  }
+  layer_dump<T, NT>(yt, side, a, out + (int64_t)tile * L::TILE);
+}
+
+// FP64 256 threads per SM (252 registers, the streaming kernel's budget), FP32 512.
+template <typename T, int NT>
+constexpr int layer_min_blocks()
+{
+  return (sizeof(T) == 4 ? 512 : 256) / NT;
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(NT, layer_min_blocks<T, NT>()) a11_layer_kernel(LayerGrid g, int tile0,
+                                                                                  const T *__restrict__ K,
+                                                                                  const T *__restrict__ u,
+                                                                                  const uint32_t *__restrict__ mbits,
+                                                                                  T *__restrict__ out)
+{
+  layer_tile<T, NT>(g, tile0 + (int)blockIdx.x, K, u, mbits, out);
+}
+
+// diag(A11): the same tiles without an input, q2::diag_form_plane per plane
+// and component as in the streaming diagonal (kernels_diag.cuh).
+template <int NT>
+__global__ void __launch_bounds__(NT, 256 / NT) diag_layer_kernel(LayerGrid g, const double *__restrict__ K,
+                                                                  double *__restrict__ out)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *yt = reinterpret_cast<double *>(smem_raw);
+  double *side = yt + L::TILE;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
+  prefetch_k(K, 0, e0, e1);
+  layer_zero<double, NT>(yt);
+  __syncthreads();
+  const unsigned amask = __ballot_sync(0xffffffffu, a.active);
+  const double *Ke = K + kelem(a.e);
+#pragma unroll 1
+  for (int A = 0; A < 3; A++) {
+    if (A < 2) prefetch_k(K, A + 1, e0, e1);
+    if (!a.active) continue;
+    double z[3][3];
+#pragma unroll
+    for (int s = 0; s < 3; s++)
+#pragma unroll
+      for (int k = 0; k < 3; k++) z[s][k] = c_zdiag[A][s][k];
+    const double *kp = Ke + koff(9 * A, 0);
+    double S[27];
+#pragma unroll 1
+    for (int m = 0; m < 3; m++) {
+      const double *km = kp + koff(0, 3 * m);
+      double Q[27];
+      q2::diag_form_plane<double>([&](int p, int d) { return ldk(km + koff(p, d)); }, z, Q);
+#pragma unroll
+      for (int n = 0; n < 27; n++) S[n] = m == 0 ? Q[n] : S[n] + Q[n];
+      layer_add<double, NT>(yt, side, a, amask, m, Q);
+    }
+#pragma unroll 1
+    for (int l = 0; l < 3; l++) layer_add<double, NT>(yt, side, a, amask, l, S);
+  }
+  layer_dump<double, NT>(yt, side, a, out + (int64_t)tile * L::TILE);
+}
+
+// ---------------------------------------------------------------------------
+// The gather
+// ---------------------------------------------------------------------------
+enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2 };
+
+// Node t of the element box (i + NX (j + NY k)): the sum of its tile entries,
+// along x innermost, then rows, then layers, lower first.  BC_COPY: y_k = x_k
+// on Dirichlet dofs, BC_ONE: 1 there.
+template <typename T, int NT, int MODE>
+__device__ __forceinline__ void layer_gather_node(const LayerGrid &g, uint32_t t, const T *s,
+                                                  const T *__restrict__ x, const uint32_t *__restrict__ mbits,
+                                                  T *__restrict__ y)
+{
+  using L = LayerLayout<NT>;
+  const uint32_t jk = g.dNX.div(t);
+  const int i = (int)(t - jk * g.dNX.d);
+  const int k = (int)g.dNY.div(jk);
+  const int j = (int)(jk - (uint32_t)k * g.dNY.d);
+  const AxisNode ay = axis_node(j, g.my), az = axis_node(k, g.mz);
+  T acc[3] = {T(0), T(0), T(0)};
+#pragma unroll
+  for (int q = 0; q < 2; q++)
+#pragma unroll
+    for (int p = 0; p < 2; p++)
+      if (q < az.n && p < ay.n) {
+        int64_t at[2];
+        layer_slots<NT>(g, i, ay.e[p] + g.my * az.e[q], at);
+        const int o = az.l[q] * L::PLANE + ay.l[p] * L::ROW;
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+          if (at[b] >= 0) {
+            const T *e = s + at[b] + o;
+#pragma unroll
+            for (int l = 0; l < 3; l++) acc[l] += __ldcg(e + l * L::COMP);  // not before the wait
+          }
+      }
+  const int64_t k0 = 3 * (g.off + i + j * g.X + k * g.XY);
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    T v = acc[l];
+    if (MODE != LAYER_PLAIN && mbits && ((mbits[(k0 + l) >> 5] >> ((k0 + l) & 31)) & 1u))
+      v = MODE == LAYER_BC_COPY ? x[k0 + l] : T(1);
+    y[k0 + l] = v;
+  }
+}
+
+// Nodes [t0, t1) of the element box.
+template <typename T, int NT, int MODE>
+__global__ void __launch_bounds__(256) layer_gather_kernel(LayerGrid g, uint32_t t0, uint32_t t1,
+                                                           const T *s, const T *__restrict__ x,
+                                                           const uint32_t *__restrict__ mbits, T *__restrict__ y)
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const uint32_t t = t0 + blockIdx.x * 256u + threadIdx.x;
+  if (t < t1) layer_gather_node<T, NT, MODE>(g, t, s, x, mbits, y);
+}
+
+// Batched forms: one work item per tile (problem, tile) and one per
+// LAYER_GATHER_NODES nodes (problem, first node); a problem's sums lie at its
+// own offset of the batch's scratch.
+constexpr int LAYER_GATHER_NODES = 1024;
+
+template <typename T, int NT, bool MASKED>
+__global__ void __launch_bounds__(NT, layer_min_blocks<T, NT>()) a11_layer_batch_kernel(const BatchProb *__restrict__ probs,
+                                                                                        const int2 *__restrict__ items,
+                                                                                        const T *const *__restrict__ uptr,
+                                                                                        T *__restrict__ scratch)
+{
+  const int2 it = items[blockIdx.x];
+  const BatchProb &p = probs[it.x];
+  layer_tile<T, NT>(p.lg, it.y, reinterpret_cast<const T *>(p.K), uptr[it.x], MASKED ? p.mbits : nullptr,
+                    scratch + p.lay_off);
+}
+
+template <typename T, int NT, bool MASKED>
+__global__ void __launch_bounds__(256) layer_gather_batch_kernel(const BatchProb *__restrict__ probs,
+                                                                 const int2 *__restrict__ items,
+                                                                 const T *const *__restrict__ uptr, const T *scratch,
+                                                                 T *const *__restrict__ yptr)
+{
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int2 it = items[blockIdx.x];
+  const BatchProb &p = probs[it.x];
+  const LayerGrid g = p.lg;
+  const uint32_t nodes = g.nodes();
+  const T *s = scratch + p.lay_off, *u = uptr[it.x];
+  const uint32_t *mb = MASKED ? p.mbits : nullptr;
+  T *y = yptr[it.x];
+#pragma unroll 1
+  for (int k = 0; k < LAYER_GATHER_NODES; k += 256) {
+    const uint32_t t = (uint32_t)it.y + k + threadIdx.x;
+    if (t < nodes) layer_gather_node<T, NT, MASKED ? LAYER_BC_COPY : LAYER_PLAIN>(g, t, s, u, mb, y);
+  }
+}
+
+}  // namespace ptk

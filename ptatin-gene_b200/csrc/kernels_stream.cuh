@@ -46,6 +46,7 @@
 #include <cstdint>
 
 #include "kernels_colour.cuh"
+#include "layer_grid.cuh"
 #include "q2_core.cuh"
 #include "q2_plane.cuh"
 
@@ -58,21 +59,25 @@ struct StreamGrid {
   int px, py, pz;     // colour of this launch
   int nxc, nyc, nzcc; // tiles of this colour per axis
   int zc0;            // first z-chunk of this launch (parity pz; pz for a whole-box launch)
-  int64_t MXP;        // padded row length of the K array (elements)
 };
 
-// K index: ((row*27 + q)*9 + r)*MXP + ex,  row = ej + my*ek.
-__host__ __device__ __forceinline__ int64_t kidx(int64_t row, int q, int r, int64_t MXP, int ex)
-{
-  return ((row * 27 + q) * 9 + r) * MXP + ex;
-}
+// K is stored in blocks of 32 consecutive elements (element number
+// ex + mx*(ej + my*ek)), entry (q, r) of a block's elements side by side: a
+// warp of 32 consecutive elements reads whole lines whatever the row length,
+// nothing is padded but the last block, and the 243 offsets of an element are
+// compile-time constants.
+constexpr int KB = 32;
+constexpr int KBLOCK = 243 * KB;
+__host__ __device__ __forceinline__ int64_t kelem(int64_t e) { return e / KB * KBLOCK + e % KB; }
+__host__ __device__ constexpr int koff(int q, int r) { return (9 * q + r) * KB; }
+__host__ __device__ __forceinline__ int64_t ksize(int64_t nel) { return (nel + KB - 1) / KB * KBLOCK; }
 
 // ---------------------------------------------------------------------------
 // Set-up kernel: K for every element and Gauss point.  Returns through
 // *bad the number of points with c <= 0 or non-finite c.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(128) geom_kernel(Box bx, int64_t MXP, const double *__restrict__ coords,
+__global__ void __launch_bounds__(128) geom_kernel(Box bx, const double *__restrict__ coords,
                                                    const double *__restrict__ eta, T *__restrict__ K,
                                                    unsigned int *__restrict__ bad)
 {
@@ -96,21 +101,21 @@ __global__ void __launch_bounds__(128) geom_kernel(Box bx, int64_t MXP, const do
     T Kq[9];
     if (!q2::geom_K(J, q2::weight(q) * eta[27 * e + q], Kq)) nbad++;
 #pragma unroll
-    for (int r = 0; r < 9; r++) K[kidx(row, q, r, MXP, ei)] = Kq[r];
+    for (int r = 0; r < 9; r++) K[kelem(e) + koff(q, r)] = Kq[r];
   }
   if (nbad) atomicAdd(bad, nbad);
 }
 
-// Bulk L2 prefetch (TMA unit) of a contiguous K block, in pieces of at most
-// 32 KiB; addresses and sizes are multiples of 16 bytes (MXP is a multiple
-// of 32 elements).
-__device__ __forceinline__ void prefetch_k_plane(const void *p, uint32_t bytes)
+// Bulk L2 prefetch (TMA unit) of Gauss plane A of the K blocks that hold
+// elements [e0, e1), one thread per block (81 x 32 values, 16-byte aligned).
+template <typename T>
+__device__ __forceinline__ void prefetch_k(const T *K, int A, int64_t e0, int64_t e1)
 {
-  const char *c = reinterpret_cast<const char *>(p);
-  for (uint32_t off = 0; off < bytes; off += 32768u) {
-    const uint32_t n = min(32768u, bytes - off);
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(c + off), "r"(n) : "memory");
-  }
+  const int64_t b = e0 / KB + threadIdx.x;
+  if (b * KB < e1)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(K + b * KBLOCK + koff(9 * A, 0)),
+                 "r"((uint32_t)(sizeof(T) * 81 * KB))
+                 : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -373,15 +378,12 @@ __device__ __forceinline__ double ldk(const double *p)
 __device__ __forceinline__ float ldk(const float *p) { return *p; }
 
 // One element (thread t of the tile), quadrature plane A: forward from the u
-// tile, viscous action with K, transpose accumulated into the y tile.  KTX:
-// the K rows are one tile wide (MXP == TX), a compile-time stride whose
-// offsets fold into the loads (measured 2% faster in FP64 at 128^3, bitwise
-// the same result; no gain in FP32).
-template <typename T, int TX, bool KTX>
+// tile, viscous action with K (Ke: the element's entry (0, 0)), transpose
+// accumulated into the y tile.
+template <typename T, int TX>
 __device__ __forceinline__ void element_plane(int A, const T *ut, T *yt, T *side, const int sl[3], int t, int warp,
-                                              bool to_side, unsigned amask, const T *__restrict__ Ke, int64_t MXP_)
+                                              bool to_side, unsigned amask, const T *__restrict__ Ke)
 {
-  const int64_t MXP = KTX ? (int64_t)TX : MXP_;
   using L = TileLayout<TX>;
   T G[3][3][9];  // [d][l][b*3+c]
 #pragma unroll
@@ -401,13 +403,13 @@ __device__ __forceinline__ void element_plane(int A, const T *ut, T *yt, T *side
   // viscous action: K of the next two points is in flight while one computes
   // (measured at 128^3: FP64 2.18 -> 2.02 ms, FP32 1.20 -> 1.12 ms)
   constexpr bool DEEP = true;
-  const T *kp = Ke + (int64_t)(9 * A) * 9 * MXP;
+  const T *kp = Ke + koff(9 * A, 0);
   T Kn[9], Kn2[9];
 #pragma unroll
-  for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + (int64_t)r * MXP);
+  for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(0, r));
   if (DEEP) {
 #pragma unroll
-    for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + (int64_t)(9 + r) * MXP);
+    for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(1, r));
   }
 #pragma unroll
   for (int p = 0; p < 9; p++) {
@@ -419,11 +421,11 @@ __device__ __forceinline__ void element_plane(int A, const T *ut, T *yt, T *side
       for (int r = 0; r < 9; r++) Kn[r] = Kn2[r];
       if (p < 7) {
 #pragma unroll
-        for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + (int64_t)(9 * (p + 2) + r) * MXP);
+        for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(p + 2, r));
       }
     } else if (p < 8) {
 #pragma unroll
-      for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + (int64_t)(9 * (p + 1) + r) * MXP);
+      for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(p + 1, r));
     }
     q2::qp_action_K(Kq, G, p);
   }
@@ -445,13 +447,12 @@ __device__ __forceinline__ void element_plane(int A, const T *ut, T *yt, T *side
 // ---------------------------------------------------------------------------
 // One tile (x-tile tx, row ej, z-chunk zc) of one problem; the whole CTA.
 // MASKED (and mbits non-null): Dirichlet columns of u zeroed from the packed
-// mask mbits.  KTX: g.MXP == TX (one x-tile per row).
-template <typename T, int TX, bool MASKED, bool KTX = false, bool NULLABLE = false>
+// mask mbits.
+template <typename T, int TX, bool MASKED, bool NULLABLE = false>
 __device__ __forceinline__ void stream_tile(const StreamGrid &g, int tx, int ej, int zc, const T *__restrict__ K,
                                             const T *__restrict__ u, const uint32_t *__restrict__ mbits,
                                             T *__restrict__ y)
 {
-  const int64_t MXP = KTX ? (int64_t)TX : g.MXP;
   using L = TileLayout<TX>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *ut = reinterpret_cast<T *>(smem_raw);
@@ -501,11 +502,13 @@ __device__ __forceinline__ void stream_tile(const StreamGrid &g, int tx, int ej,
   // lane 31 of every warp but the last
   const bool to_side = (lane == 31) && (warp < L::NW - 1);
   const unsigned amask = __ballot_sync(0xffffffffu, active);
-  if (t == 0) prefetch_k_plane(K + kidx(ej + (int64_t)g.b.my * ek0, 0, 0, MXP, 0), (uint32_t)(sizeof(T) * 81 * MXP));
+  // first element of the tile's row in layer 0, and its elements
+  const int64_t e0 = ex0 + (int64_t)g.b.mx * ej, el = (int64_t)g.b.mx * g.b.my;
+  const int ne = min(TX, g.b.mx - ex0);
+  prefetch_k(K, 0, e0 + el * ek0, e0 + el * ek0 + ne);
 
 #pragma unroll 1
   for (int ek = ek0; ek < ek1; ek++) {
-    const int64_t row = ej + (int64_t)g.b.my * ek;
     const int s0 = (int)((2 * (int64_t)ek) % 3), s1 = (s0 + 1) % 3, s2 = (s0 + 2) % 3;
     const int sl[3] = {s0, s1, s2};
     const bool more = ek + 1 < ek1;
@@ -525,13 +528,13 @@ __device__ __forceinline__ void stream_tile(const StreamGrid &g, int tx, int ej,
 
     if (active) {
       // each quadrature plane's K is prefetched to L2 while the one before it computes
-      const int64_t krow = kidx(row, 0, 0, MXP, ex);
-      const uint32_t kb = (uint32_t)(sizeof(T) * 81 * MXP);
+      const int64_t e = e0 + el * ek;
+      const T *Ke = K + kelem(e + t);
 #pragma unroll 1
       for (int A = 0; A < 3; A++) {
-        if (t == 0 && (A < 2 || more))
-          prefetch_k_plane(A < 2 ? K + kidx(row, 9 * (A + 1), 0, MXP, 0) : K + kidx(row + g.b.my, 0, 0, MXP, 0), kb);
-        element_plane<T, TX, KTX>(A, ut, yt, side, sl, t, warp, to_side, amask, K + krow, MXP);
+        if (A < 2) prefetch_k(K, A + 1, e, e + ne);
+        else if (more) prefetch_k(K, 0, e + el, e + el + ne);
+        element_plane<T, TX>(A, ut, yt, side, sl, t, warp, to_side, amask, Ke);
       }
     }
     if (mk) fetch_wait();  // this thread's staged words
@@ -572,7 +575,7 @@ constexpr int stream_min_blocks()
   return (sizeof(T) == 4 && TX == 128) ? 4 : 256 / TX;
 }
 
-template <typename T, int TX, bool MASKED, bool KTX = false>
+template <typename T, int TX, bool MASKED>
 __global__ void __launch_bounds__(TX, stream_min_blocks<T, TX>()) a11_stream_kernel(StreamGrid g, const T *__restrict__ K,
                                                                   const T *__restrict__ u,
                                                                   const uint32_t *__restrict__ mbits,
@@ -581,7 +584,7 @@ __global__ void __launch_bounds__(TX, stream_min_blocks<T, TX>()) a11_stream_ker
   // tile of this CTA within the colour class
   const int bid = blockIdx.x;
   const int ixc = bid % g.nxc, iyc = (bid / g.nxc) % g.nyc, izc = bid / (g.nxc * g.nyc);
-  stream_tile<T, TX, MASKED, KTX>(g, g.px + 2 * ixc, g.py + 2 * iyc, g.zc0 + 2 * izc, K, u, mbits, y);
+  stream_tile<T, TX, MASKED>(g, g.px + 2 * ixc, g.py + 2 * iyc, g.zc0 + 2 * izc, K, u, mbits, y);
 }
 
 // ---------------------------------------------------------------------------
@@ -593,11 +596,13 @@ __global__ void __launch_bounds__(TX, stream_min_blocks<T, TX>()) a11_stream_ker
 struct BatchProb {
   Box b;
   int ntx, LZ, nzc;
-  int64_t MXP;
   const void *K;          // T* of the problem's Gauss-point factor
   const uint8_t *mask;    // Dirichlet mask (MatShell level) or null
   const uint32_t *mbits;  // the same mask packed one bit per dof
   int64_t nvel;           // length of the problem's vectors
+  bool layer;             // layer tiles (kernels_layer.cuh) instead of the coloured z-march
+  LayerGrid lg;           // their shape, and where the problem's sums start in the batch's scratch
+  int64_t lay_off;
 };
 
 template <typename T, int TX, bool MASKED>
@@ -610,11 +615,11 @@ __global__ void __launch_bounds__(TX, stream_min_blocks<T, TX>()) a11_stream_bat
   const BatchProb p = probs[it.x];
   StreamGrid g;
   g.b = p.b;
-  g.TX = TX; g.ntx = p.ntx; g.LZ = p.LZ; g.nzc = p.nzc; g.MXP = p.MXP;
+  g.TX = TX; g.ntx = p.ntx; g.LZ = p.LZ; g.nzc = p.nzc;
   g.px = px; g.py = py; g.pz = pz;
   g.nxc = g.nyc = g.nzcc = 0;
   g.zc0 = pz;
-  stream_tile<T, TX, MASKED, false, true>(g, it.y, it.z, it.w, reinterpret_cast<const T *>(p.K), uptr[it.x],
+  stream_tile<T, TX, MASKED, true>(g, it.y, it.z, it.w, reinterpret_cast<const T *>(p.K), uptr[it.x],
                              MASKED ? p.mbits : nullptr, yptr[it.x]);
 }
 

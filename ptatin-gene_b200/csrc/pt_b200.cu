@@ -6,6 +6,7 @@
 // Kernels live in kernels_*.cuh; this file does argument checking, memory,
 // streams and the BC fix-ups of the MatShell-level calls.
 #include <cuda_runtime.h>
+#include <pthread.h>
 
 #include <cmath>
 #include <cstdarg>
@@ -23,6 +24,7 @@
 #include "kernels_colour.cuh"
 #include "kernels_stream.cuh"
 #include "kernels_diag.cuh"
+#include "kernels_layer.cuh"
 #include "kernels_ebe.cuh"
 #include "kernels_markers.cuh"
 #include "kernels_bmat.cuh"
@@ -62,14 +64,20 @@ pt_status fail(pt_status s, const char *fmt, ...)
                   __LINE__);                                                                       \
   } while (0)
 
-enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3 };
+enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 
-// "b200" picks stored element matrices for one-rank boxes up to this many
-// elements (packed FP64 + FP32 matrices: 40 KB per element, 1.3 GB at 32^3)
-// and the streaming kernel above.  Measured FP64 / FP32 apply, stored
-// matrices vs streaming: 16^3 0.037 / 0.023 vs 0.26 / 0.22 ms, 32^3 0.24 /
-// 0.14 vs 0.35 / 0.30 ms, 40^3 0.45 / 0.27 vs 0.36 / 0.27 ms.
-constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 32768;
+// "b200" picks stored element matrices for one-rank boxes of up to
+// EBE_AUTO_MAX_ELEMENTS (FP64 / FP32 apply, matrices vs layer tiles: 10^3
+// 15.0 / 12.1 vs 21.0 / 20.9 us, 12^3 19.0 / 14.3 vs 20.9 / 20.4 us, 16^3
+// 36.5 / 19.8 vs 22.2 / 20.9 us); layer tiles above; and the streaming kernel
+// for boxes from STREAM_AUTO_MIN_ELEMENTS whose rows nearly fill its tiles
+// (layer tiles vs streaming: 56^3 162 / 115 vs 187 / 165 us, 64^3 216 / 153 vs
+// 205 / 181 us, 128x128x64 775 / 549 vs 731 / 493 us; rows that leave threads
+// idle: 80^3 417 / 301 vs 515 / 366 us, 97x70x81 440 / 313 vs 533 / 338 us).
+constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
+constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
+// layer tiles: node numbers stay below 2^31, scratch (460 B per element) below 4 GB
+constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
 constexpr int PIPE_LAYERS = 6;
@@ -93,7 +101,6 @@ struct pt_op {
   double *d_K;
   float *d_K32;
   unsigned int *d_bad;
-  int64_t MXP;
   int TX, ntx, LZ, nzc;
   bool geom_dirty, geom_ok, full_box, ebe_valid;
   bool be_valid;  // d_Be matches the coordinates
@@ -120,6 +127,11 @@ struct pt_op {
   // momentum residual: Gauss-point body force [27 nel][3] and its load vector
   double *d_fu, *d_F;
   bool has_fu, F_valid;
+  // layer tiles: shape, the tiles' sums between the two launches of an apply,
+  // and the lock that keeps those two launches of one host thread together
+  ptk::LayerGrid lg;
+  double *d_layer;
+  pthread_mutex_t layer_mu;
 };
 
 namespace {
@@ -282,7 +294,7 @@ pt_status stream_colours(pt_op *op, size_t smem, int zb, int ze, F &&launch)
   if (ze < 0) ze = op->nzc;
   ptk::StreamGrid g;
   g.b = op->box;
-  g.TX = TX; g.ntx = op->ntx; g.LZ = op->LZ; g.nzc = op->nzc; g.MXP = op->MXP;
+  g.TX = TX; g.ntx = op->ntx; g.LZ = op->LZ; g.nzc = op->nzc;
   cudaLaunchAttribute pdl[1] = {};
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
@@ -317,44 +329,32 @@ pt_status stream_colours(pt_op *op, size_t smem, int zb, int ze, F &&launch)
 // after an even one, or at the last chunk, so the node sums keep the order of
 // the whole-box launch (the even chunk of a boundary plane stores, the odd one
 // adds).
-// KTX: one x-tile per row (MXP == TX), the K stride a compile-time constant
-// (FP64 only: it measured no faster in FP32).
-template <typename T, int TX, bool MASKED, bool KTX>
-pt_status launch_stream_tx_k(pt_op *op, const T *K, const T *u, T *y, int zb, int ze)
+template <typename T, int TX, bool MASKED>
+pt_status launch_stream_tx(pt_op *op, const T *K, const T *u, T *y, int zb = 0, int ze = -1)
 {
   if (MASKED && !op->d_mbits) return fail(PT_ERR_STATE, "masked apply without the packed Dirichlet bits");
-  if (KTX && op->MXP != TX) return fail(PT_ERR_STATE, "K row stride differs from the tile width");
   constexpr size_t smem = ptk::stream_smem_bytes<T, TX>();
-  pt_status as = kernel_attrs((const void *)ptk::a11_stream_kernel<T, TX, MASKED, KTX>, smem);
+  pt_status as = kernel_attrs((const void *)ptk::a11_stream_kernel<T, TX, MASKED>, smem);
   if (as != PT_OK) return as;
   const uint32_t *mb = MASKED ? op->d_mbits : nullptr;
   return stream_colours<TX>(op, smem, zb, ze, [&](const cudaLaunchConfig_t &cfg, const ptk::StreamGrid &g) {
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, ptk::a11_stream_kernel<T, TX, MASKED, KTX>, g, K, u, mb, y);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, ptk::a11_stream_kernel<T, TX, MASKED>, g, K, u, mb, y);
     if (e != cudaSuccess) return fail(PT_ERR_CUDA, "streaming A11 launch: %s", cudaGetErrorString(e));
     return PT_OK;
   });
 }
 
-template <typename T, int TX, bool MASKED>
-pt_status launch_stream_tx(pt_op *op, const T *K, const T *u, T *y, int zb = 0, int ze = -1)
-{
-  if constexpr (sizeof(T) == 8) {
-    if (op->MXP == TX) return launch_stream_tx_k<T, TX, MASKED, true>(op, K, u, y, zb, ze);
-  }
-  return launch_stream_tx_k<T, TX, MASKED, false>(op, K, u, y, zb, ze);
-}
-
 // diag(A11) on the streaming tiles from the stored K (whole box, one launch
 // per colour class, programmatic like the apply).
-template <int TX, bool KTX>
+template <int TX>
 pt_status launch_diag_stream_tx(pt_op *op, double *d)
 {
   constexpr size_t smem = ptk::diag_smem_bytes<TX>();
-  pt_status as = kernel_attrs((const void *)ptk::diag_stream_kernel<TX, KTX>, smem);
+  pt_status as = kernel_attrs((const void *)ptk::diag_stream_kernel<TX>, smem);
   if (as != PT_OK) return as;
   const double *K = op->d_K;
   return stream_colours<TX>(op, smem, 0, -1, [&](const cudaLaunchConfig_t &cfg, const ptk::StreamGrid &g) {
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, ptk::diag_stream_kernel<TX, KTX>, g, K, d);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, ptk::diag_stream_kernel<TX>, g, K, d);
     if (e != cudaSuccess) return fail(PT_ERR_CUDA, "streaming diag launch: %s", cudaGetErrorString(e));
     return PT_OK;
   });
@@ -362,9 +362,99 @@ pt_status launch_diag_stream_tx(pt_op *op, double *d)
 
 pt_status launch_diag_stream(pt_op *op, double *d)
 {
-  if (op->TX == 32) return op->MXP == 32 ? launch_diag_stream_tx<32, true>(op, d) : launch_diag_stream_tx<32, false>(op, d);
-  if (op->TX == 64) return op->MXP == 64 ? launch_diag_stream_tx<64, true>(op, d) : launch_diag_stream_tx<64, false>(op, d);
-  return op->MXP == 128 ? launch_diag_stream_tx<128, true>(op, d) : launch_diag_stream_tx<128, false>(op, d);
+  if (op->TX == 32) return launch_diag_stream_tx<32>(op, d);
+  if (op->TX == 64) return launch_diag_stream_tx<64>(op, d);
+  return launch_diag_stream_tx<128>(op, d);
+}
+
+// ---- layer tiles ----------------------------------------------------------------
+
+constexpr int LNT = ptk::LAYER_NT;
+
+A11Kernel auto_kernel(const pt_op *op)
+{
+  if (op->full_box && op->nel <= EBE_AUTO_MAX_ELEMENTS) return A11_EBE;
+  const bool full_rows = 10 * (int64_t)op->mx >= 9 * (int64_t)op->ntx * op->TX;
+  const bool stream = op->nel > LAYER_MAX_ELEMENTS || (op->nel >= STREAM_AUTO_MIN_ELEMENTS && full_rows);
+  return stream ? A11_STREAM : A11_LAYER;
+}
+
+// The tiles' sums, once per op and sized for FP64 (an FP32 apply uses half).
+pt_status ensure_layer(pt_op *op)
+{
+  if (op->d_layer) return PT_OK;
+  PT_CUDA(op_alloc(op, (void **)&op->d_layer,
+                   sizeof(double) * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE));
+  return PT_OK;
+}
+
+// Holds the two launches of an apply together: they share the op's scratch, so
+// another host thread's apply of the same op must not be enqueued in between.
+struct LayerLock {
+  pt_op *op;
+  explicit LayerLock(pt_op *o) : op(o) { pthread_mutex_lock(&op->layer_mu); }
+  ~LayerLock() { pthread_mutex_unlock(&op->layer_mu); }
+};
+
+// The gather of nodes [t0, t1) as a programmatic launch behind the tiles'
+// kernel (it waits for that grid before it reads).
+template <typename T, int MODE>
+pt_status launch_layer_gather(pt_op *op, uint32_t t0, uint32_t t1, const T *x, T *y)
+{
+  cudaLaunchAttribute pdl[1] = {};
+  pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((t1 - t0 + 255) / 256);
+  cfg.blockDim = dim3(256);
+  cfg.stream = op->stream;
+  cfg.attrs = pdl;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, ptk::layer_gather_kernel<T, LNT, MODE>, op->lg, t0, t1,
+                                           reinterpret_cast<const T *>(op->d_layer), x,
+                                           (const uint32_t *)op->d_mbits, y);
+  if (e != cudaSuccess) return fail(PT_ERR_CUDA, "layer gather launch: %s", cudaGetErrorString(e));
+  PT_LAUNCHED(op);
+  return PT_OK;
+}
+
+// Tiles [tile0, tile1) and the gather of nodes [t0, t1).
+template <typename T>
+pt_status launch_layer_range(pt_op *op, const T *K, const T *u, T *y, bool masked, int tile0, int tile1, uint32_t t0,
+                             uint32_t t1)
+{
+  constexpr size_t smem = ptk::layer_smem_bytes<T, LNT>();
+  pt_status s = kernel_attrs((const void *)ptk::a11_layer_kernel<T, LNT>, smem);
+  if (s != PT_OK) return s;
+  ptk::a11_layer_kernel<T, LNT><<<(unsigned)(tile1 - tile0), LNT, smem, op->stream>>>(
+      op->lg, tile0, K, u, masked ? op->d_mbits : nullptr, reinterpret_cast<T *>(op->d_layer));
+  PT_LAUNCHED(op);
+  if (t1 == t0) return PT_OK;
+  return masked ? launch_layer_gather<T, ptk::LAYER_BC_COPY>(op, t0, t1, u, y)
+                : launch_layer_gather<T, ptk::LAYER_PLAIN>(op, t0, t1, u, y);
+}
+
+template <typename T>
+pt_status launch_layer(pt_op *op, const T *K, const T *u, T *y, bool masked)
+{
+  pt_status s = ensure_layer(op);
+  if (s != PT_OK) return s;
+  LayerLock lock(op);
+  return launch_layer_range<T>(op, K, u, y, masked, 0, (int)op->lg.tiles, 0, op->lg.nodes());
+}
+
+// diag(A11), Dirichlet entries 1 when `ones`
+pt_status launch_layer_diag(pt_op *op, double *d, bool ones)
+{
+  pt_status s = ensure_layer(op);
+  if (s != PT_OK) return s;
+  constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
+  if ((s = kernel_attrs((const void *)ptk::diag_layer_kernel<LNT>, smem)) != PT_OK) return s;
+  LayerLock lock(op);
+  ptk::diag_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, op->d_layer);
+  PT_LAUNCHED(op);
+  return ones ? launch_layer_gather<double, ptk::LAYER_BC_ONE>(op, 0, op->lg.nodes(), nullptr, d)
+              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, op->lg.nodes(), nullptr, d);
 }
 
 template <typename T, bool MASKED>
@@ -380,17 +470,21 @@ pt_status launch_stream(pt_op *op, const T *K, const T *u, T *y)
 pt_status ensure_geometry(pt_op *op)
 {
   if (!op->geom_dirty) return PT_OK;
-  const int64_t nk = (int64_t)op->my * op->mz * 243 * op->MXP;
+  const int64_t nk = ptk::ksize(op->nel);
   if (!op->d_K) {
     PT_CUDA(op_alloc(op, (void **)&op->d_K, sizeof(double) * nk));
     PT_CUDA(op_alloc(op, (void **)&op->d_K32, sizeof(float) * nk));
     PT_CUDA(op_alloc(op, (void **)&op->d_bad, sizeof(unsigned int)));
   }
+  if (op->a11_kernel == A11_LAYER) {
+    pt_status s = ensure_layer(op);
+    if (s != PT_OK) return s;
+  }
   PT_CUDA(cudaMemsetAsync(op->d_bad, 0, sizeof(unsigned int), op->stream));
-  ptk::geom_kernel<double><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->MXP, op->d_coords, op->d_eta,
+  ptk::geom_kernel<double><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
                                                                        op->d_K, op->d_bad);
   PT_LAUNCHED(op);
-  ptk::geom_kernel<float><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->MXP, op->d_coords, op->d_eta,
+  ptk::geom_kernel<float><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
                                                                       op->d_K32, op->d_bad);
   PT_LAUNCHED(op);
   unsigned int bad = 0;
@@ -463,11 +557,11 @@ pt_status launch_ebe(pt_op *op, const T *u, T *y, bool masked)
 
 // ---- A11 dispatch -----------------------------------------------------------
 
-// The streaming and stored-matrix applies set y_k = x_k on Dirichlet dofs
-// inside launch_a11, so MatMult needs no separate pass after them.
+// The streaming, layer and stored-matrix applies set y_k = x_k on Dirichlet
+// dofs inside launch_a11, so MatMult needs no separate pass after them.
 bool a11_sets_bc_rows(const pt_op *op)
 {
-  const bool stream = op->a11_kernel == A11_STREAM;
+  const bool stream = op->a11_kernel == A11_STREAM || op->a11_kernel == A11_LAYER;
   const bool ebe = op->a11_kernel == A11_EBE && op->full_box;
   return (stream || ebe) && op->geom_ok && !op->geom_dirty;
 }
@@ -487,11 +581,21 @@ pt_status launch_a11(pt_op *op, const T *coords, const T *eta, const T *u, T *y,
     if (s != PT_OK) return s;
     if (op->geom_ok) return launch_ebe<T>(op, u, y, masked);
   }
-  if (op->a11_kernel == A11_STREAM) {
+  if (op->a11_kernel == A11_STREAM || op->a11_kernel == A11_LAYER) {
     pt_status s = ensure_geometry(op);
     if (s != PT_OK) return s;
     if (op->geom_ok) {
       if (!op->full_box) PT_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * op->nvel, op->stream));
+      if (op->a11_kernel == A11_LAYER) {
+        if ((s = launch_layer<T>(op, op_K<T>(op), u, y, masked)) != PT_OK) return s;
+        // a ghosted box's Dirichlet dofs outside the element box
+        if (masked && !op->full_box) {
+          bc_bits_kernel<T><<<grid_stride_blocks((op->nvel + 31) / 32), 256, 0, op->stream>>>(op->d_mbits, u, y,
+                                                                                             op->nvel);
+          PT_LAUNCHED(op);
+        }
+        return PT_OK;
+      }
       if (masked) {
         // Dirichlet columns inside the kernel; rows y_k = x_k after its colour passes
         if ((s = launch_stream<T, true>(op, op_K<T>(op), u, y)) != PT_OK) return s;
@@ -516,9 +620,25 @@ pt_status launch_a11(pt_op *op, const T *coords, const T *eta, const T *u, T *y,
   return PT_OK;
 }
 
-pt_status diag_d(pt_op *op, double *d)
+pt_status bc_value(pt_op *op, double v, double *y);
+
+// diag(A11); `ones`: Dirichlet entries set to 1
+pt_status diag_d(pt_op *op, double *d, bool ones = false)
 {
   pt_status s;
+  ones = ones && op->has_mask;
+  if (op->a11_kernel == A11_LAYER) {
+    if ((s = ensure_geometry(op)) != PT_OK) return s;
+    if (op->geom_ok) {
+      if (!op->full_box) PT_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * op->nvel, op->stream));
+      if ((s = launch_layer_diag(op, d, ones && op->full_box)) != PT_OK) return s;
+      return ones && !op->full_box ? bc_value(op, 1.0, d) : PT_OK;
+    }
+  }
+  if (ones) {
+    if ((s = diag_d(op, d)) != PT_OK) return s;
+    return bc_value(op, 1.0, d);
+  }
   if (op->a11_kernel == A11_EBE && op->full_box) {
     // the stored element matrices carry the diagonal: one gather
     if ((s = ensure_geometry(op)) != PT_OK) return s;
@@ -664,14 +784,20 @@ bool is_pinned(const void *p)
 // launch_stream_tx), so the result is bitwise the one-shot apply's.  Used for
 // pinned host arrays on a one-rank box with the streaming kernel; returns
 // false when that does not apply.
+//
+// Layer tiles are cut by elements instead: a group's tiles run when the node
+// planes of their layers have arrived, and the planes below the first
+// incomplete layer are gathered and come down.
 template <bool MASKED>
 pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done)
 {
   *done = false;
-  if (!op->full_box || op->a11_kernel != A11_STREAM || !is_pinned(hu) || !is_pinned(hy)) return PT_OK;
+  const bool layer = op->a11_kernel == A11_LAYER;
+  if (!op->full_box || !(layer || op->a11_kernel == A11_STREAM) || !is_pinned(hu) || !is_pinned(hy)) return PT_OK;
   pt_status s = ensure_geometry(op);
   if (s != PT_OK) return s;
-  if (!op->geom_ok || op->nzc < 2) return PT_OK;
+  if (!op->geom_ok || (layer ? op->mz < 2 * PIPE_LAYERS : op->nzc < 2)) return PT_OK;
+  if (layer && (s = ensure_layer(op)) != PT_OK) return s;
   if (!op->pipe_ready) {
     PT_CUDA(cudaStreamCreateWithFlags(&op->h2d, cudaStreamNonBlocking));
     PT_CUDA(cudaStreamCreateWithFlags(&op->d2h, cudaStreamNonBlocking));
@@ -689,7 +815,12 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
   // compute); at 128^3 groups of 6 layers measured 10.3-10.6 ms against 11.0
   // for 8 groups, with pure copies in 8 pieces each way at 9.3 ms.
   std::vector<std::pair<int, int>> groups;
-  for (int per = std::max(1, (PIPE_LAYERS + op->LZ - 1) / op->LZ);; per++) {
+  if (layer) {  // element layers [first, second]
+    const int n = std::min(PIPE_GROUPS, op->mz / PIPE_LAYERS);
+    for (int g = 0; g < n; g++)
+      groups.push_back({(int)((int64_t)op->mz * g / n), (int)((int64_t)op->mz * (g + 1) / n) - 1});
+  }
+  for (int per = layer ? 0 : std::max(1, (PIPE_LAYERS + op->LZ - 1) / op->LZ); !layer; per++) {
     groups.clear();
     for (int c0 = 0; c0 < op->nzc;) {
       int c1 = std::min(op->nzc - 1, c0 + per - 1);
@@ -702,12 +833,14 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
   const int64_t plane = 3 * op->box.XY;  // doubles per node plane
   const int64_t nplanes = 2 * (int64_t)op->mz + 1;
   int64_t up = 0, down = 0;  // next plane to upload / download
+  int tile_g = 0;            // layer tiles: next tile to run
   PT_CUDA(cudaEventRecord(op->ev_done[0], op->stream));  // earlier work on the op's stream precedes the copies
   PT_CUDA(cudaStreamWaitEvent(op->h2d, op->ev_done[0], 0));
   for (size_t gi = 0; gi < groups.size(); gi++) {
     const int c0 = groups[gi].first, c1 = groups[gi].second;
     const bool last = gi + 1 == groups.size();
-    const int64_t top = 2 * (int64_t)std::min((c1 + 1) * op->LZ, op->mz);  // top node plane of the group
+    // top node plane of the group
+    const int64_t top = layer ? 2 * (int64_t)(c1 + 1) : 2 * (int64_t)std::min((c1 + 1) * op->LZ, op->mz);
     if (top + 1 > up) {
       PT_CUDA(cudaMemcpyAsync(op->d_u + up * plane, hu + up * plane, sizeof(double) * (top + 1 - up) * plane,
                               cudaMemcpyHostToDevice, op->h2d));
@@ -715,13 +848,25 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
     }
     PT_CUDA(cudaEventRecord(op->ev_in[gi], op->h2d));
     PT_CUDA(cudaStreamWaitEvent(op->stream, op->ev_in[gi], 0));
-    if (op->TX == 32) s = launch_stream_tx<double, 32, MASKED>(op, op->d_K, op->d_u, op->d_y, c0, c1 + 1);
+    int64_t fin = last ? nplanes : top;  // planes below `fin` are final
+    if (layer) {
+      // tiles whose elements all lie in the layers that have arrived
+      const int64_t layer_el = (int64_t)op->mx * op->my;
+      const int g1 = last ? op->lg.tiles : (int)((c1 + 1) * layer_el / op->lg.E);
+      if (!last) fin = 2 * ((int64_t)g1 * op->lg.E / layer_el);
+      const uint32_t pn = (uint32_t)(op->box.XY);
+      LayerLock lock(op);
+      if (g1 > tile_g)
+        s = launch_layer_range<double>(op, op->d_K, op->d_u, op->d_y, MASKED, tile_g, g1, (uint32_t)down * pn,
+                                       (uint32_t)fin * pn);
+      tile_g = g1;
+    }
+    else if (op->TX == 32) s = launch_stream_tx<double, 32, MASKED>(op, op->d_K, op->d_u, op->d_y, c0, c1 + 1);
     else if (op->TX == 64) s = launch_stream_tx<double, 64, MASKED>(op, op->d_K, op->d_u, op->d_y, c0, c1 + 1);
     else s = launch_stream_tx<double, 128, MASKED>(op, op->d_K, op->d_u, op->d_y, c0, c1 + 1);
     if (s != PT_OK) return s;
     PT_CUDA(cudaEventRecord(op->ev_done[gi], op->stream));
-    const int64_t fin = last ? nplanes : top;  // planes below `fin` are final
-    if (MASKED && fin > down) {  // their Dirichlet rows, y_k = x_k
+    if (MASKED && !layer && fin > down) {  // their Dirichlet rows, y_k = x_k
       const int64_t o = down * plane, m = (fin - down) * plane;
       bc_copy_kernel<double><<<grid_stride_blocks(m), 256, 0, op->stream>>>(op->d_mask + o, op->d_u + o, op->d_y + o, m);
       PT_LAUNCHED(op);
@@ -776,10 +921,12 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   op->npres = 4 * op->nel;
   op->full_box = (nx == 2 * (int64_t)desc->mx + 1) && (ny == 2 * (int64_t)desc->my + 1) &&
                  (nz == 2 * (int64_t)desc->mz + 1);
-  op->a11_kernel = (op->full_box && op->nel <= EBE_AUTO_MAX_ELEMENTS) ? A11_EBE : A11_STREAM;
+  pthread_mutex_init(&op->layer_mu, nullptr);
   op->TX = desc->mx <= 32 ? 32 : (desc->mx <= 64 ? 64 : 128);
   op->ntx = (desc->mx + op->TX - 1) / op->TX;
-  op->MXP = (int64_t)op->ntx * op->TX;
+  op->a11_kernel = auto_kernel(op);
+  if (op->nel <= LAYER_MAX_ELEMENTS)
+    op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
   pt_op_set_tiling(op, 0);
   op->geom_dirty = true;
   cudaError_t e = cudaGetDevice(&op->device);
@@ -816,7 +963,7 @@ pt_status pt_op_destroy(pt_op *op)
   if (op->stream && !op->pool) cudaStreamSynchronize(op->stream);
   void *bufs[] = {op->d_coords, op->d_eta, op->d_coords32, op->d_eta32, op->d_mask, op->d_u,
                   op->d_y, op->d_p, op->d_K, op->d_K32, op->d_bad, op->d_Ae, op->d_Ae32, op->d_ye,
-                  op->mk_scratch, op->d_Be, op->d_yp, op->d_mbits, op->d_fu, op->d_F};
+                  op->mk_scratch, op->d_Be, op->d_yp, op->d_mbits, op->d_fu, op->d_F, op->d_layer};
   for (void *b : bufs) op_free(op, b);
   for (int b = 0; b < 2; b++)
     if (op->h_stage[b]) {
@@ -835,6 +982,7 @@ pt_status pt_op_destroy(pt_op *op)
       cudaEventDestroy(op->ev_done[g]);
     }
   }
+  pthread_mutex_destroy(&op->layer_mu);
   free(op);
   return PT_OK;
 }
@@ -1100,9 +1248,10 @@ pt_status pt_matmult_a11_f32_d(pt_op *op, const float *x, float *y)
 
 pt_status pt_getdiag_a11_d(pt_op *op, double *d)
 {
-  pt_status s = pt_a11_diag_d(op, d);
+  pt_status s = check_ready(op, true);
   if (s != PT_OK) return s;
-  return bc_value(op, 1.0, d);
+  if (!d) return fail(PT_ERR_BAD_ARG, "NULL vector");
+  return diag_d(op, d, true);
 }
 
 pt_status pt_getdiag_a11_h(pt_op *op, double *d)
@@ -1405,9 +1554,14 @@ pt_status pt_project_markers_h(pt_op *op, int64_t n, const int32_t *wil, const d
 pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
 {
   if (!op || !name) return fail(PT_ERR_BAD_ARG, "NULL argument");
-  if (!strcmp(name, "b200")) op->a11_kernel = (op->full_box && op->nel <= EBE_AUTO_MAX_ELEMENTS) ? A11_EBE : A11_STREAM;
+  if (!strcmp(name, "b200")) op->a11_kernel = auto_kernel(op);
   else if (!strcmp(name, "b200_stream")) op->a11_kernel = A11_STREAM;
   else if (!strcmp(name, "b200_ebe")) op->a11_kernel = A11_EBE;
+  else if (!strcmp(name, "b200_layer")) {
+    if (op->nel > LAYER_MAX_ELEMENTS)
+      return fail(PT_ERR_UNSUPPORTED, "b200_layer takes boxes of at most %lld elements", (long long)LAYER_MAX_ELEMENTS);
+    op->a11_kernel = A11_LAYER;
+  }
   else if (!strcmp(name, "b200_colour")) op->a11_kernel = A11_COLOUR;
   else return fail(PT_ERR_BAD_ARG, "No -a11_op %s", name);
   return PT_OK;
@@ -1437,6 +1591,7 @@ const char *pt_op_get_a11_kernel(const pt_op *op)
   switch (op->a11_kernel) {
     case A11_STREAM: return "b200_stream";
     case A11_EBE: return "b200_ebe";
+    case A11_LAYER: return "b200_layer";
     default: return "b200_colour";
   }
 }
@@ -1562,13 +1717,13 @@ extern "C" pt_status pt_a11_apply_noalloc_d(const pt_mesh_desc *desc, const doub
   const int64_t nel = (int64_t)desc->mx * desc->my * desc->mz;
   // the counter keeps the previous call's value: clear it first
   PT_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st));
-  ptk::geom_kernel<double><<<nblocks(nel), TPB, 0, st>>>(bx, MXP, coords, eta, K, bad);
+  ptk::geom_kernel<double><<<nblocks(nel), TPB, 0, st>>>(bx, coords, eta, K, bad);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
 
   ptk::StreamGrid g;
   g.b = bx;
-  g.TX = TX; g.ntx = ntx; g.MXP = MXP;
+  g.TX = TX; g.ntx = ntx;
   {
     const int64_t txy = (int64_t)ntx * desc->my;
     int nzc = (int)((2048 + txy - 1) / txy);

@@ -453,15 +453,23 @@ namespace {
 
 size_t srv_bytes(const pt_mesh_desc &d, bool fp32)
 {
-  // op: coords (f64+f32), eta (f64+f32), mask, K (f64+f32, rows padded to 32);
+  // op: coords (f64+f32), eta (f64+f32), mask, K (f64+f32);
   // request: x r p q, z d az dinv, partials; set-up scratch (diagonal + Lanczos)
   const int64_t nx = 2 * (int64_t)d.mx + 1, ny = 2 * (int64_t)d.my + 1, nz = 2 * (int64_t)d.mz + 1;
   const int64_t nvel = 3 * nx * ny * nz, nel = (int64_t)d.mx * d.my * d.mz;
-  const int64_t tx = d.mx <= 32 ? 32 : (d.mx <= 64 ? 64 : 128);
-  const int64_t mxp = (d.mx + tx - 1) / tx * tx;
   const size_t ts = fp32 ? 4 : 8;
   const int64_t nch = (nvel + SRV_CH - 1) / SRV_CH;
-  const size_t op = nvel * 12 + 27 * nel * 12 + nvel + (size_t)d.my * d.mz * 243 * mxp * 12;
+  const size_t base = nvel * 12 + 27 * nel * 12 + nvel;
+  // K as the budget has always counted it, rows padded to the streaming tile
+  // width; the blocks that are stored and, for a box on layer tiles, its part
+  // of the batch's scratch where that is more (long rows: about 10% of a request)
+  const int64_t tx = d.mx <= 32 ? 32 : (d.mx <= 64 ? 64 : 128);
+  const size_t k_rows = (size_t)d.my * d.mz * 243 * ((d.mx + tx - 1) / tx * tx) * 12;
+  size_t k_blocks = (size_t)ptk::ksize(nel) * 12;
+  if (nel <= LAYER_MAX_ELEMENTS)
+    k_blocks += sizeof(double) * (size_t)ptk::LayerLayout<LNT>::TILE *
+                ptk::layer_grid<LNT>(d.mx, d.my, d.mz, 1, 1, 0).tiles;
+  const size_t op = base + std::max(k_rows, k_blocks);
   const size_t req = nvel * 32 + nvel * 4 * ts + 2 * 8 * nch;
   const size_t setup = nvel * 8 + sizeof(LzState) + 8 * nch;
   return op + req + setup;
@@ -523,15 +531,19 @@ pt_status srv_precond(pt_server *s, const int2 *items, int64_t nitems, cudaStrea
 // w*eta/detJ <= 0 goes to pinned memory, read when the set-up has completed.
 pt_status srv_geometry(pt_op *op, unsigned int *h_bad)
 {
-  const int64_t nk = (int64_t)op->my * op->mz * 243 * op->MXP;
+  const int64_t nk = ptk::ksize(op->nel);
   PT_CUDA(op_alloc(op, (void **)&op->d_K, sizeof(double) * nk));
   PT_CUDA(op_alloc(op, (void **)&op->d_K32, sizeof(float) * nk));
   PT_CUDA(op_alloc(op, (void **)&op->d_bad, sizeof(unsigned int)));
+  if (op->a11_kernel == A11_LAYER) {
+    pt_status s = ensure_layer(op);
+    if (s != PT_OK) return s;
+  }
   PT_CUDA(cudaMemsetAsync(op->d_bad, 0, sizeof(unsigned int), op->stream));
-  ptk::geom_kernel<double><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->MXP, op->d_coords, op->d_eta,
+  ptk::geom_kernel<double><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
                                                                        op->d_K, op->d_bad);
   PT_LAUNCHED(op);
-  ptk::geom_kernel<float><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->MXP, op->d_coords, op->d_eta,
+  ptk::geom_kernel<float><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
                                                                       op->d_K32, op->d_bad);
   PT_LAUNCHED(op);
   PT_CUDA(cudaMemcpyAsync(h_bad, op->d_bad, sizeof(unsigned int), cudaMemcpyDeviceToHost, op->stream));
@@ -551,7 +563,9 @@ pt_status srv_admit(pt_server *s, SrvReq *r, int slot)
   if (e != PT_OK) return e;
   pt_op *op = r->op;
   if (!op->full_box) return fail(PT_ERR_UNSUPPORTED, "request %lld: one-rank boxes only", (long long)r->id);
-  op->a11_kernel = A11_STREAM;  // the batch runs the streaming kernel; set-up applies use the same
+  // the batch runs layer or streaming tiles; set-up applies use the same
+  if (op->a11_kernel == A11_EBE) op->a11_kernel = A11_LAYER;
+  if (s->o.lz > 0) op->a11_kernel = A11_STREAM;
   if (s->o.lz > 0) {
     op->LZ = std::min(s->o.lz, op->mz);
     op->nzc = (op->mz + op->LZ - 1) / op->LZ;
@@ -658,7 +672,9 @@ pt_status srv_join(pt_server *s)
       s->done.push_back(r);
       continue;
     }
-    r->op->stream = s->main;  // its applies now run in the batch
+    r->op->stream = s->main;  // its applies now run in the batch, on the batch's scratch
+    op_free(r->op, r->op->d_layer);
+    r->op->d_layer = nullptr;
     r->joined = true;
     s->dirty = true;
   }
@@ -721,14 +737,14 @@ pt_status srv_iterate(pt_server *s)
   void **tab = (void **)s->d_ptrs;
   pt_status e = batch_apply<double, true>(s->batch, (const double *const *)tab, (double *const *)(tab + n), st);
   if (e != PT_OK) return e;
-  s->launches += s->batch->classes.size() + 1;
+  s->launches += pt_batch_launches_per_apply(s->batch) + (s->batch->coloured ? 1 : 0);
   srv_pq_kernel<<<ni, SRV_THREADS, 0, st>>>(s->d_items, s->d_slots, s->d_scal);
   srv_final_kernel<SRV_F_ALPHA><<<na, SRV_THREADS, 0, st>>>(s->d_act, s->d_slots, s->d_scal);
   srv_update_kernel<<<ni, SRV_THREADS, 0, st>>>(s->d_items, s->d_slots, s->d_scal);
   srv_final_kernel<SRV_F_RR><<<na, SRV_THREADS, 0, st>>>(s->d_act, s->d_slots, s->d_scal);
   s->launches += 4;
   e = srv_precond<T>(s, s->d_items, ni, st, [&]() {
-    s->launches += s->batch->classes.size() + 1;
+    s->launches += pt_batch_launches_per_apply(s->batch) + (s->batch->coloured ? 1 : 0);
     return batch_apply<T, true>(s->batch, (const T *const *)(tab + 2 * n), (T *const *)(tab + 3 * n), st);
   });
   if (e != PT_OK) return e;

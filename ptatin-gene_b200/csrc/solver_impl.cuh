@@ -388,7 +388,8 @@ pt_status mg_coarsen(const pt_op *f, const double *vf_f, double *vf_c, pt_op **o
   *out = c;  // the caller owns it from here on
   if ((st = pt_op_set_stream(c, (void *)f->stream)) != PT_OK) return st;
   // small levels keep their own element matrices (mg_level_setup)
-  c->a11_kernel = (f->a11_kernel == A11_EBE) ? A11_STREAM : f->a11_kernel;
+  if (f->a11_kernel == A11_COLOUR) c->a11_kernel = A11_COLOUR;
+  else if (c->a11_kernel == A11_EBE) c->a11_kernel = A11_LAYER;
   const MgBox fb = mgbox(f), cb = mgbox(c);
   inject_coords_kernel<<<vgrid(c->nnodes), 256, 0, c->stream>>>(fb, cb, f->d_coords, c->d_coords);
   PT_LAUNCHED(c);

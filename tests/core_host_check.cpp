@@ -5,7 +5,9 @@
 // CUDA kernels.
 #include <cstdint>
 #include <cstring>
+#include <vector>
 
+#include "layer_grid.cuh"
 #include "q2_core.cuh"
 #include "q2_plane.cuh"
 
@@ -206,3 +208,71 @@ extern "C" int core_diag_plane_f64(int mx, int my, int mz, const double *coords,
       }
   return bad;
 }
+
+// The layer tiles' index arithmetic on an mx x my x mz box: the segments of a
+// tile cover its threads; the entries that a thread writes lie inside its tile
+// and belong to no other node; and the gather of a node reads exactly the
+// entries that hold its elements' sums, each once, inside the scratch.  Returns 0, or the number of the check that failed.
+template <int NT>
+static int layer_walk(int mx, int my, int mz)
+{
+  using namespace ptk;
+  using L = LayerLayout<NT>;
+  const int64_t X = 2 * mx + 1, Y = 2 * my + 1, Z = 2 * mz + 1, rows = (int64_t)my * mz;
+  const LayerGrid g = layer_grid<NT>(mx, my, mz, X, X * Y, 0);
+  if (g.E < 1 || g.E > NT || g.nodes() != X * Y * Z || (int64_t)g.tiles * g.E < rows * mx) return 1;
+  const int64_t size = (int64_t)g.tiles * L::TILE;
+  std::vector<int64_t> node(size, -1);
+  std::vector<char> added(size, 0);
+  for (int tile = 0; tile < g.tiles; tile++) {
+    const int e0 = tile * g.E, n = g.nel - e0 < g.E ? g.nel - e0 : g.E;
+    const int row0 = (int)g.dmx.div(e0), segs = (int)g.dmx.div(e0 + n - 1) - row0 + 1;
+    if (row0 != e0 / mx || 2 * g.odd + segs > L::ROW || g.E > g.odd) return 2;
+    int covered = 0;
+    for (int sg = 0; sg < segs; sg++) {
+      int t0, len;
+      layer_segment(g, e0, row0, n, sg, t0, len);
+      if (t0 != covered || len < 1) return 3;
+      covered += len;
+      for (int t = t0; t < t0 + len; t++) {
+        const int e = e0 + t, row = row0 + sg, ex = e - row * mx, ej = row % my, ek = row / my;
+        if (ex < 0 || ex >= mx) return 4;
+        const bool last = e + 1 == (row + 1) * mx || t + 1 == g.E || t + 1 == n;
+        if (last != (t + 1 == t0 + len)) return 5;
+        for (int k = 0; k < 3; k++)
+          for (int j = 0; j < 3; j++)
+            for (int i = 0; i < 3; i++) {
+              const int col = i == 0 ? t : (i == 1 ? g.odd + t : (last ? 2 * g.odd + sg : t + 1));
+              if (col >= L::ROW || (i == 2 && !last && col >= g.odd)) return 6;
+              const int64_t at = (int64_t)tile * L::TILE + k * L::PLANE + j * L::ROW + col;
+              const int64_t nd = 2 * ex + i + X * (2 * ej + j + Y * (2 * (int64_t)ek + k));
+              if (node[at] >= 0 && node[at] != nd) return 7;
+              node[at] = nd;
+            }
+      }
+    }
+    if (covered != n) return 8;
+  }
+  for (uint32_t t = 0; t < g.nodes(); t++) {
+    const uint32_t jk = g.dNX.div(t);
+    const int i = (int)(t - jk * g.dNX.d), k = (int)g.dNY.div(jk), j = (int)(jk - (uint32_t)k * g.dNY.d);
+    if (jk != t / X || k != (int)(jk / Y)) return 9;
+    const AxisNode ay = axis_node(j, my), az = axis_node(k, mz);
+    for (int q = 0; q < az.n; q++)
+      for (int p = 0; p < ay.n; p++) {
+        int64_t at[2];
+        layer_slots<NT>(g, i, ay.e[p] + my * az.e[q], at);
+        for (int b = 0; b < 2; b++) {
+          if (at[b] < 0) continue;
+          const int64_t s = at[b] + az.l[q] * L::PLANE + ay.l[p] * L::ROW;
+          if (s + 2 * L::COMP >= size) return 10;
+          if (node[s] != (int64_t)t || added[s]++) return 11;
+        }
+      }
+  }
+  for (int64_t at = 0; at < size; at++)
+    if (node[at] >= 0 && !added[at]) return 12;
+  return 0;
+}
+
+extern "C" int core_layer_walk(int mx, int my, int mz) { return layer_walk<128>(mx, my, mz); }

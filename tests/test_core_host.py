@@ -76,3 +76,14 @@ def test_stream_diag_algorithm_matches_oracle(core, ora, workload):
     core.core_diag_plane_f64.argtypes = [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_double)] * 3
     assert core.core_diag_plane_f64(*m.dims, _p(m.coords), _p(eta), _p(d)) == 0
     assert relerr(d, ref) < 1e-13
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (1, 7, 3), (2, 3, 2), (7, 5, 3), (8, 8, 8), (31, 3, 4), (32, 4, 4), (33, 5, 2),
+                                  (41, 7, 5), (64, 3, 3), (97, 4, 3), (127, 2, 3), (128, 3, 2), (129, 2, 3), (130, 3, 1),
+                                  (257, 1, 2), (300, 2, 2), (2, 40, 9), (12, 9, 7), (13, 8, 8), (16, 16, 16), (17, 9, 5), (18, 7, 9),
+                                  (20, 11, 6), (21, 10, 9), (40, 12, 10), (56, 9, 8), (5, 30, 30)])
+def test_layer_tiles_cover_every_node_sum_once(core, dims):
+    """Index arithmetic of the layer tiles (csrc/layer_grid.cuh): one thread
+    per element, tile entries inside the tile, and a gather that reads every
+    element's contribution to a node once and nothing else."""
+    assert core.core_layer_walk(*dims) == 0
