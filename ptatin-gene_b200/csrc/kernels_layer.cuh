@@ -352,6 +352,162 @@ __global__ void __launch_bounds__(NT, 256 / NT) diag_layer_kernel(LayerGrid g, c
 }
 
 // ---------------------------------------------------------------------------
+// Set-up on the same tiles: the coordinates take the place of u
+// ---------------------------------------------------------------------------
+// G[d][l][p] = h^-1 d x_l / d xi_d at the 9 points of Gauss plane A.
+template <int NT>
+__device__ __forceinline__ void layer_jacobian(int A, const double *xt, const LayerThread &a, double G[3][3][9])
+{
+  using L = LayerLayout<NT>;
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double Q[9], R[9];
+    const double *xl = xt + l * L::COMP;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const double *p = xl + (i == 0 ? (int)threadIdx.x : (i == 1 ? a.od : a.en)) + j * L::ROW;
+        zeta_fwd_rt<double>(A, p[0], p[L::PLANE], p[2 * L::PLANE], Q[3 * j + i], R[3 * j + i]);
+      }
+    q2::plane_fwd(Q, R, G[0][l], G[1][l], G[2][l]);
+  }
+}
+
+// J at point p of a plane's scaled gradient
+__device__ __forceinline__ void layer_point(const double G[3][3][9], int p, double J[3][3])
+{
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+#pragma unroll
+    for (int l = 0; l < 3; l++) J[k][l] = q2::DH * G[k][l][p];
+}
+
+// The tile's coordinates in shared memory, for every thread.
+template <int NT>
+__device__ __forceinline__ void layer_fetch_coords(double *xt, void *stage, const LayerGrid &g, int tile,
+                                                   const double *__restrict__ coords)
+{
+  layer_fetch<double, NT>(xt, stage, g, tile, coords, nullptr);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+}
+
+constexpr int LAYER_STAGE_BYTES = 2048;  // segment table of a fetch without a mask (at most 68 entries)
+
+template <int NT>
+constexpr size_t layer_geom_smem_bytes()
+{
+  return sizeof(double) * (size_t)LayerLayout<NT>::TILE + LAYER_STAGE_BYTES;
+}
+
+// K at every Gauss point, in FP64 and (K32 not null) FP32 in one pass over the
+// coordinates; *bad counts the points with c = w eta / det <= 0 or not finite.
+// The live state is the coordinates at the element's 27 points, 81 values in
+// registers (arrays in local memory and a pass per precision took 4.1 ms at
+// 128^3), and the stores are whole lines of the K blocks.  J is formed by the
+// operations of element_jacobian in their order -- its entries are differences
+// of nearby coordinates, so another order moves K by 1e-14 -- which is why
+// this does not go plane by plane like the apply.
+template <int NT>
+__global__ void __launch_bounds__(NT, 256 / NT) geom_layer_kernel(LayerGrid g, const double *__restrict__ coords,
+                                                                  const double *__restrict__ eta,
+                                                                  double *__restrict__ K, float *__restrict__ K32,
+                                                                  unsigned int *__restrict__ bad)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *xt = reinterpret_cast<double *>(smem_raw);
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  layer_fetch_coords<NT>(xt, xt + L::TILE, g, tile, coords);
+  if (!a.active) return;
+  double I[3][27];
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double f[27];
+#pragma unroll
+    for (int n = 0; n < 27; n++)
+      f[n] = xt[l * L::COMP + n / 9 * L::PLANE + n / 3 % 3 * L::ROW +
+                (n % 3 == 0 ? (int)threadIdx.x : (n % 3 == 1 ? a.od : a.en))];
+    q2::interp(f, I[l]);
+  }
+  const double *ee = eta + 27 * (int64_t)a.e;
+  const int64_t k0 = kelem(a.e);
+  unsigned nbad = 0;
+#pragma unroll
+  for (int q = 0; q < 27; q++) {
+    const int qa = q / 9, qb = q / 3 % 3, qc = q % 3;
+    double J[3][3], Kq[9], e;
+    // one point at a time: square roots and divisions of several in flight spill
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(e) : "l"(ee + q) : "memory");
+#pragma unroll
+    for (int l = 0; l < 3; l++) {
+      const double *x = I[l];
+      J[0][l] = q2::lineD_at(x[9 * qa + 3 * qb], x[9 * qa + 3 * qb + 1], x[9 * qa + 3 * qb + 2], qc);
+      J[1][l] = q2::lineD_at(x[9 * qa + qc], x[9 * qa + 3 + qc], x[9 * qa + 6 + qc], qb);
+      J[2][l] = q2::lineD_at(x[3 * qb + qc], x[9 + 3 * qb + qc], x[18 + 3 * qb + qc], qa);
+    }
+    if (!q2::geom_K(J, q2::weight(q) * e, Kq)) nbad++;
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+      K[k0 + koff(q, r)] = Kq[r];
+      if (K32) K32[k0 + koff(q, r)] = (float)Kq[r];
+    }
+  }
+  if (nbad) atomicAdd(bad, nbad);
+}
+
+// Body-force load of the momentum residual (src/stokes_form_function.c:201-213):
+// F[n,l] = sum_q w_q det(J_q) N_n(q) Fu_l(q), fu = [27 nel][3], to scratch.
+template <int NT>
+__global__ void __launch_bounds__(NT, 256 / NT) body_force_layer_kernel(LayerGrid g, const double *__restrict__ coords,
+                                                                        const double *__restrict__ fu,
+                                                                        double *__restrict__ out)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *xt = reinterpret_cast<double *>(smem_raw);
+  double *yt = xt + L::TILE;
+  double *side = yt + L::TILE;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  layer_fetch_coords<NT>(xt, yt, g, tile, coords);
+  layer_zero<double, NT>(yt);
+  __syncthreads();
+  const unsigned amask = __ballot_sync(0xffffffffu, a.active);
+#pragma unroll 1
+  for (int A = 0; A < 3; A++) {
+    if (!a.active) continue;
+    double G[3][3][9], wd[9];
+    layer_jacobian<NT>(A, xt, a, G);
+#pragma unroll
+    for (int p = 0; p < 9; p++) {
+      double J[3][3], adj[3][3];
+      layer_point(G, p, J);
+      wd[p] = q2::weight(p) * (A == 1 ? q2::W1 / q2::W0 : 1.0) * q2::adjugate(J, adj);
+    }
+    const double *f = fu + 3 * (27 * (int64_t)a.e + 9 * A);
+#pragma unroll 1
+    for (int l = 0; l < 3; l++) {
+      double r[9], Sx[9], Qt[9], V[27];
+#pragma unroll
+      for (int p = 0; p < 9; p++) r[p] = wd[p] * f[3 * p + l];
+#pragma unroll
+      for (int c = 0; c < 3; c++) q2::lineBt(r[c], r[3 + c], r[6 + c], Sx[c], Sx[3 + c], Sx[6 + c]);
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+        q2::lineBt(Sx[3 * j], Sx[3 * j + 1], Sx[3 * j + 2], Qt[3 * j], Qt[3 * j + 1], Qt[3 * j + 2]);
+#pragma unroll
+      for (int ji = 0; ji < 9; ji++) zeta_bwd_rt<double>(A, Qt[ji], 0.0, V[ji], V[9 + ji], V[18 + ji]);
+      layer_add<double, NT>(yt, side, a, amask, l, V);
+    }
+  }
+  layer_dump<double, NT>(yt, side, a, out + (int64_t)tile * L::TILE);
+}
+
+// ---------------------------------------------------------------------------
 // The gather
 // ---------------------------------------------------------------------------
 enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2 };

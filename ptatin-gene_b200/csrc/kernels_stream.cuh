@@ -72,40 +72,6 @@ __host__ __device__ __forceinline__ int64_t kelem(int64_t e) { return e / KB * K
 __host__ __device__ constexpr int koff(int q, int r) { return (9 * q + r) * KB; }
 __host__ __device__ __forceinline__ int64_t ksize(int64_t nel) { return (nel + KB - 1) / KB * KBLOCK; }
 
-// ---------------------------------------------------------------------------
-// Set-up kernel: K for every element and Gauss point.  Returns through
-// *bad the number of points with c <= 0 or non-finite c.
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(128) geom_kernel(Box bx, const double *__restrict__ coords,
-                                                   const double *__restrict__ eta, T *__restrict__ K,
-                                                   unsigned int *__restrict__ bad)
-{
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (int64_t)bx.mx * bx.my * bx.mz) return;
-  const int ei = (int)(e % bx.mx);
-  const int64_t row = e / bx.mx;
-  const int ej = (int)(row % bx.my), ek = (int)(row / bx.my);
-  int64_t nid[27];
-  element_nodes(bx, ei, ej, ek, nid);
-  double Jg[3][3][27], Xq[3][27];
-  element_jacobian(coords, nid, Jg, Xq);
-  unsigned nbad = 0;
-#pragma unroll 1
-  for (int q = 0; q < 27; q++) {
-    double J[3][3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-      for (int l = 0; l < 3; l++) J[k][l] = Jg[k][l][q];
-    T Kq[9];
-    if (!q2::geom_K(J, q2::weight(q) * eta[27 * e + q], Kq)) nbad++;
-#pragma unroll
-    for (int r = 0; r < 9; r++) K[kelem(e) + koff(q, r)] = Kq[r];
-  }
-  if (nbad) atomicAdd(bad, nbad);
-}
-
 // Bulk L2 prefetch (TMA unit) of Gauss plane A of the K blocks that hold
 // elements [e0, e1), one thread per block (81 x 32 values, 16-byte aligned).
 template <typename T>

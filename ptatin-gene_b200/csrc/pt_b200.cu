@@ -78,6 +78,9 @@ constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
 constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
 // layer tiles: node numbers stay below 2^31, scratch (460 B per element) below 4 GB
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
+// the set-up kernels use the same tiles for every box (node numbers below
+// 2^31; K of a larger box is more than any device holds)
+constexpr int64_t TILE_MAX_ELEMENTS = (int64_t)1 << 27;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
 constexpr int PIPE_LAYERS = 6;
@@ -465,11 +468,25 @@ pt_status launch_stream(pt_op *op, const T *K, const T *u, T *y)
   return launch_stream_tx<T, 128, MASKED>(op, K, u, y);
 }
 
+// K in FP64 and FP32 and the count of points with c <= 0, on the op's stream.
+pt_status launch_geometry(pt_op *op)
+{
+  constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
+  pt_status s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT>, smem);
+  if (s != PT_OK) return s;
+  PT_CUDA(cudaMemsetAsync(op->d_bad, 0, sizeof(unsigned int), op->stream));
+  ptk::geom_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_eta,
+                                                                                op->d_K, op->d_K32, op->d_bad);
+  PT_LAUNCHED(op);
+  return PT_OK;
+}
+
 // Recompute K when coordinates or viscosity changed.  Sets geom_ok = false
 // (and the op falls back to the colour kernel) if any c = w eta / det <= 0.
 pt_status ensure_geometry(pt_op *op)
 {
   if (!op->geom_dirty) return PT_OK;
+  if (op->nel > TILE_MAX_ELEMENTS) return fail(PT_ERR_OOM, "%lld elements: more geometry than a device holds", (long long)op->nel);
   const int64_t nk = ptk::ksize(op->nel);
   if (!op->d_K) {
     PT_CUDA(op_alloc(op, (void **)&op->d_K, sizeof(double) * nk));
@@ -480,13 +497,8 @@ pt_status ensure_geometry(pt_op *op)
     pt_status s = ensure_layer(op);
     if (s != PT_OK) return s;
   }
-  PT_CUDA(cudaMemsetAsync(op->d_bad, 0, sizeof(unsigned int), op->stream));
-  ptk::geom_kernel<double><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
-                                                                       op->d_K, op->d_bad);
-  PT_LAUNCHED(op);
-  ptk::geom_kernel<float><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
-                                                                      op->d_K32, op->d_bad);
-  PT_LAUNCHED(op);
+  pt_status gs = launch_geometry(op);
+  if (gs != PT_OK) return gs;
   unsigned int bad = 0;
   PT_CUDA(cudaMemcpyAsync(&bad, op->d_bad, sizeof bad, cudaMemcpyDeviceToHost, op->stream));
   PT_CUDA(cudaStreamSynchronize(op->stream));
@@ -607,6 +619,12 @@ pt_status launch_a11(pt_op *op, const T *coords, const T *eta, const T *u, T *y,
     }
   }
   PT_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * op->nvel, op->stream));
+  if (sizeof(T) == 4) {  // only this kernel reads the FP32 coordinates and viscosity
+    to_f32_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_coords, op->d_coords32, op->nvel);
+    PT_LAUNCHED(op);
+    to_f32_kernel<<<grid_stride_blocks(27 * op->nel), 256, 0, op->stream>>>(op->d_eta, op->d_eta32, 27 * op->nel);
+    PT_LAUNCHED(op);
+  }
   for (int c = 0; c < 8; c++) {
     ptk::ColourGrid g = ptk::colour_grid(op->box, c);
     const int64_t n = (int64_t)g.ncx * g.ncy * g.ncz;
@@ -925,7 +943,7 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   op->TX = desc->mx <= 32 ? 32 : (desc->mx <= 64 ? 64 : 128);
   op->ntx = (desc->mx + op->TX - 1) / op->TX;
   op->a11_kernel = auto_kernel(op);
-  if (op->nel <= LAYER_MAX_ELEMENTS)
+  if (op->nel <= TILE_MAX_ELEMENTS)
     op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
   pt_op_set_tiling(op, 0);
   op->geom_dirty = true;
@@ -1008,8 +1026,6 @@ pt_status pt_op_get_sizes(const pt_op *op, int64_t *nvel, int64_t *npres, int64_
 
 static pt_status finish_coords(pt_op *op)
 {
-  to_f32_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_coords, op->d_coords32, op->nvel);
-  PT_LAUNCHED(op);
   op->has_coords = true;
   op->geom_dirty = true;
   op->be_valid = false;
@@ -1020,8 +1036,6 @@ static pt_status finish_coords(pt_op *op)
 
 static pt_status finish_eta(pt_op *op)
 {
-  to_f32_kernel<<<grid_stride_blocks(27 * op->nel), 256, 0, op->stream>>>(op->d_eta, op->d_eta32, 27 * op->nel);
-  PT_LAUNCHED(op);
   op->has_eta = true;
   op->geom_dirty = true;
   op->state++;
@@ -1397,14 +1411,16 @@ static pt_status ensure_body_force(pt_op *op)
 {
   if (op->F_valid) return PT_OK;
   if (!op->d_F) PT_CUDA(op_alloc(op, (void **)&op->d_F, sizeof(double) * op->nvel));
-  PT_CUDA(cudaMemsetAsync(op->d_F, 0, sizeof(double) * op->nvel, op->stream));
-  for (int c = 0; c < 8; c++) {
-    ptk::ColourGrid g = ptk::colour_grid(op->box, c);
-    const int64_t n = (int64_t)g.ncx * g.ncy * g.ncz;
-    if (n == 0) continue;
-    ptk::body_force_colour_kernel<<<nblocks(n), TPB, 0, op->stream>>>(g, op->d_coords, op->d_fu, op->d_F);
-    PT_LAUNCHED(op);
-  }
+  if (!op->full_box) PT_CUDA(cudaMemsetAsync(op->d_F, 0, sizeof(double) * op->nvel, op->stream));
+  pt_status s = ensure_layer(op);
+  if (s != PT_OK) return s;
+  constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
+  if ((s = kernel_attrs((const void *)ptk::body_force_layer_kernel<LNT>, smem)) != PT_OK) return s;
+  LayerLock lock(op);
+  ptk::body_force_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_fu,
+                                                                                      op->d_layer);
+  PT_LAUNCHED(op);
+  if ((s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, op->lg.nodes(), nullptr, op->d_F)) != PT_OK) return s;
   op->F_valid = true;
   return PT_OK;
 }
@@ -1717,7 +1733,10 @@ extern "C" pt_status pt_a11_apply_noalloc_d(const pt_mesh_desc *desc, const doub
   const int64_t nel = (int64_t)desc->mx * desc->my * desc->mz;
   // the counter keeps the previous call's value: clear it first
   PT_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st));
-  ptk::geom_kernel<double><<<nblocks(nel), TPB, 0, st>>>(bx, coords, eta, K, bad);
+  constexpr size_t gsmem = ptk::layer_geom_smem_bytes<LNT>();
+  if ((s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT>, gsmem)) != PT_OK) return s;
+  const ptk::LayerGrid lg = ptk::layer_grid<LNT>(bx.mx, bx.my, bx.mz, bx.X, bx.XY, bx.off);
+  ptk::geom_layer_kernel<LNT><<<(unsigned)lg.tiles, LNT, gsmem, st>>>(lg, coords, eta, K, nullptr, bad);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
 

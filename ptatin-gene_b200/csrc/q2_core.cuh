@@ -81,6 +81,17 @@ PT_HD void lineD(T x0, T x1, T x2, T &y0, T &y1, T &y2)
   y2 = y1 + T(2) * h * t;           //  h x0 - 4h x1 + 3h x2
 }
 
+// one entry of y = Dc x (the same operations as lineD)
+template <typename T>
+PT_HD T lineD_at(T x0, T x1, T x2, int q)
+{
+  const T h = T(DH);
+  const T y1 = h * (x2 - x0);
+  if (q == 1) return y1;
+  const T t = (x0 + x2) - T(2) * x1;
+  return q == 0 ? y1 - T(2) * h * t : y1 + T(2) * h * t;
+}
+
 // y (+)= Dc^T x
 template <typename T, bool ACC>
 PT_HD void lineDt(T x0, T x1, T x2, T &y0, T &y1, T &y2)

@@ -539,13 +539,8 @@ pt_status srv_geometry(pt_op *op, unsigned int *h_bad)
     pt_status s = ensure_layer(op);
     if (s != PT_OK) return s;
   }
-  PT_CUDA(cudaMemsetAsync(op->d_bad, 0, sizeof(unsigned int), op->stream));
-  ptk::geom_kernel<double><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
-                                                                       op->d_K, op->d_bad);
-  PT_LAUNCHED(op);
-  ptk::geom_kernel<float><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
-                                                                      op->d_K32, op->d_bad);
-  PT_LAUNCHED(op);
+  pt_status s = launch_geometry(op);
+  if (s != PT_OK) return s;
   PT_CUDA(cudaMemcpyAsync(h_bad, op->d_bad, sizeof(unsigned int), cudaMemcpyDeviceToHost, op->stream));
   op->geom_dirty = false;
   op->geom_ok = true;  // provisional: the request fails at join if h_bad > 0
