@@ -354,24 +354,30 @@ __global__ void __launch_bounds__(NT, 256 / NT) diag_layer_kernel(LayerGrid g, c
 // ---------------------------------------------------------------------------
 // Set-up on the same tiles: the coordinates take the place of u
 // ---------------------------------------------------------------------------
+// Gradient of component l of a tile's field at Gauss plane A (h^-1 d/dxi).
+template <int NT>
+__device__ __forceinline__ void layer_gradient(int A, const double *t, const LayerThread &a, int l, double G0[9],
+                                               double G1[9], double G2[9])
+{
+  using L = LayerLayout<NT>;
+  double Q[9], R[9];
+  const double *tl = t + l * L::COMP;
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double *p = tl + (i == 0 ? (int)threadIdx.x : (i == 1 ? a.od : a.en)) + j * L::ROW;
+      zeta_fwd_rt<double>(A, p[0], p[L::PLANE], p[2 * L::PLANE], Q[3 * j + i], R[3 * j + i]);
+    }
+  q2::plane_fwd(Q, R, G0, G1, G2);
+}
+
 // G[d][l][p] = h^-1 d x_l / d xi_d at the 9 points of Gauss plane A.
 template <int NT>
 __device__ __forceinline__ void layer_jacobian(int A, const double *xt, const LayerThread &a, double G[3][3][9])
 {
-  using L = LayerLayout<NT>;
 #pragma unroll
-  for (int l = 0; l < 3; l++) {
-    double Q[9], R[9];
-    const double *xl = xt + l * L::COMP;
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        const double *p = xl + (i == 0 ? (int)threadIdx.x : (i == 1 ? a.od : a.en)) + j * L::ROW;
-        zeta_fwd_rt<double>(A, p[0], p[L::PLANE], p[2 * L::PLANE], Q[3 * j + i], R[3 * j + i]);
-      }
-    q2::plane_fwd(Q, R, G[0][l], G[1][l], G[2][l]);
-  }
+  for (int l = 0; l < 3; l++) layer_gradient<NT>(A, xt, a, l, G[0][l], G[1][l], G[2][l]);
 }
 
 // J at point p of a plane's scaled gradient
@@ -393,12 +399,49 @@ __device__ __forceinline__ void layer_fetch_coords(double *xt, void *stage, cons
   __syncthreads();
 }
 
-constexpr int LAYER_STAGE_BYTES = 2048;  // segment table of a fetch without a mask (at most 68 entries)
+// Segment table and mask words of a fetch that has no tile to stage them in:
+// most for rows of one element (40 segments of 9 lines, 2 words each).
+constexpr int LAYER_STAGE_BYTES = 4096;
 
 template <int NT>
 constexpr size_t layer_geom_smem_bytes()
 {
   return sizeof(double) * (size_t)LayerLayout<NT>::TILE + LAYER_STAGE_BYTES;
+}
+
+// Node n of component l of the thread's element in a tile.
+template <int NT>
+__device__ __forceinline__ double layer_node(const double *t, const LayerThread &a, int l, int n)
+{
+  using L = LayerLayout<NT>;
+  return t[l * L::COMP + n / 9 * L::PLANE + n / 3 % 3 * L::ROW +
+           (n % 3 == 0 ? (int)threadIdx.x : (n % 3 == 1 ? a.od : a.en))];
+}
+
+// I[l][q] = coordinate l at the element's 27 Gauss points.
+template <int NT>
+__device__ __forceinline__ void layer_points(const double *xt, const LayerThread &a, double I[3][27])
+{
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double f[27];
+#pragma unroll
+    for (int n = 0; n < 27; n++) f[n] = layer_node<NT>(xt, a, l, n);
+    q2::interp(f, I[l]);
+  }
+}
+
+// J at point q from the coordinates at the points
+__device__ __forceinline__ void layer_point_jacobian(const double I[3][27], int q, double J[3][3])
+{
+  const int qa = q / 9, qb = q / 3 % 3, qc = q % 3;
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    const double *x = I[l];
+    J[0][l] = q2::lineD_at(x[9 * qa + 3 * qb], x[9 * qa + 3 * qb + 1], x[9 * qa + 3 * qb + 2], qc);
+    J[1][l] = q2::lineD_at(x[9 * qa + qc], x[9 * qa + 3 + qc], x[9 * qa + 6 + qc], qb);
+    J[2][l] = q2::lineD_at(x[3 * qb + qc], x[9 + 3 * qb + qc], x[18 + 3 * qb + qc], qa);
+  }
 }
 
 // K at every Gauss point, in FP64 and (K32 not null) FP32 in one pass over the
@@ -423,31 +466,16 @@ __global__ void __launch_bounds__(NT, 256 / NT) geom_layer_kernel(LayerGrid g, c
   layer_fetch_coords<NT>(xt, xt + L::TILE, g, tile, coords);
   if (!a.active) return;
   double I[3][27];
-#pragma unroll
-  for (int l = 0; l < 3; l++) {
-    double f[27];
-#pragma unroll
-    for (int n = 0; n < 27; n++)
-      f[n] = xt[l * L::COMP + n / 9 * L::PLANE + n / 3 % 3 * L::ROW +
-                (n % 3 == 0 ? (int)threadIdx.x : (n % 3 == 1 ? a.od : a.en))];
-    q2::interp(f, I[l]);
-  }
+  layer_points<NT>(xt, a, I);
   const double *ee = eta + 27 * (int64_t)a.e;
   const int64_t k0 = kelem(a.e);
   unsigned nbad = 0;
 #pragma unroll
   for (int q = 0; q < 27; q++) {
-    const int qa = q / 9, qb = q / 3 % 3, qc = q % 3;
     double J[3][3], Kq[9], e;
     // one point at a time: square roots and divisions of several in flight spill
     asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(e) : "l"(ee + q) : "memory");
-#pragma unroll
-    for (int l = 0; l < 3; l++) {
-      const double *x = I[l];
-      J[0][l] = q2::lineD_at(x[9 * qa + 3 * qb], x[9 * qa + 3 * qb + 1], x[9 * qa + 3 * qb + 2], qc);
-      J[1][l] = q2::lineD_at(x[9 * qa + qc], x[9 * qa + 3 + qc], x[9 * qa + 6 + qc], qb);
-      J[2][l] = q2::lineD_at(x[3 * qb + qc], x[9 + 3 * qb + qc], x[18 + 3 * qb + qc], qa);
-    }
+    layer_point_jacobian(I, q, J);
     if (!q2::geom_K(J, q2::weight(q) * e, Kq)) nbad++;
 #pragma unroll
     for (int r = 0; r < 9; r++) {
@@ -508,13 +536,183 @@ __global__ void __launch_bounds__(NT, 256 / NT) body_force_layer_kernel(LayerGri
 }
 
 // ---------------------------------------------------------------------------
+// Divergence and gradient
+// ---------------------------------------------------------------------------
+// D: the factors of B and B^T, 12 per Gauss point, blocked like K: entries
+// 3k + d (k, d = 0..2) are -h w adj(J)[k][d] and 9 + d the P1GRel basis
+// function x^_d of P3D_ConstructNi_P1GRel_3D (src/element_utils_q2.c:183-224).
+// With G' = h^-1 grad_xi u, w det div u = -sum_kd D[3k+d] G'[d][k], so
+//   (B u)_i = sum_q Np_i sum_kd D[3k+d] G'[d][k],    Np = {1, x^_0, x^_1, x^_2}
+//   dv'[d][l] = (sum_i p_i Np_i) D[3l+d]              (the transpose's input)
+// (MatMultMF_Stokes_MixedFEM3d_A21 / _A12, src/stokes_q2p1_mf_operators_def.c:
+// 423-538).  324 values per element like the 4 x 81 blocks of B itself, but
+// formed in one pass over the coordinates (the blocks took 12 transposed
+// contractions per element and scattered stores: 64x48x40 1,031 us) and
+// read in whole lines by one thread per element.  Coordinates only: a
+// viscosity update keeps them.
+constexpr int DN = 12;
+constexpr int DBLOCK = 27 * DN * KB;
+__host__ __device__ __forceinline__ int64_t delem(int64_t e) { return e / KB * DBLOCK + e % KB; }
+__host__ __device__ constexpr int doff(int q, int r) { return (DN * q + r) * KB; }
+__host__ __device__ __forceinline__ int64_t dsize(int64_t nel) { return (nel + KB - 1) / KB * DBLOCK; }
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 256 / NT) div_layer_kernel(LayerGrid g, const double *__restrict__ coords,
+                                                                 double *__restrict__ D)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *xt = reinterpret_cast<double *>(smem_raw);
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  layer_fetch_coords<NT>(xt, xt + L::TILE, g, tile, coords);
+  if (!a.active) return;
+  double mean[3], invL[3];
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double s = 0.0;
+#pragma unroll
+    for (int n = 0; n < 27; n++) s += layer_node<NT>(xt, a, l, n);
+    mean[l] = (1.0 / 27.0) * s;
+  }
+  invL[0] = 1.0 / (layer_node<NT>(xt, a, 0, 14) - layer_node<NT>(xt, a, 0, 12));
+  invL[1] = 1.0 / (layer_node<NT>(xt, a, 1, 16) - layer_node<NT>(xt, a, 1, 10));
+  invL[2] = 1.0 / (layer_node<NT>(xt, a, 2, 22) - layer_node<NT>(xt, a, 2, 4));
+  double I[3][27];
+  layer_points<NT>(xt, a, I);
+  double *De = D + delem(a.e);
+#pragma unroll
+  for (int q = 0; q < 27; q++) {
+    double J[3][3], adj[3][3];
+    layer_point_jacobian(I, q, J);
+    (void)q2::adjugate(J, adj);
+    const double s = -q2::DH * q2::weight(q);
+#pragma unroll
+    for (int r = 0; r < 9; r++) De[doff(q, r)] = s * adj[r / 3][r % 3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) De[doff(q, 9 + d)] = (I[d][q] - mean[d]) * invL[d];
+    asm volatile("" ::: "memory");  // one point at a time
+  }
+}
+
+// B and B^T go component by component, so their live state is one component's
+// gradient (27 values) and three tiles fit an SM instead of the apply's two.
+constexpr int DIV_TILES_PER_SM = 3;
+
+// yp = B u (Dirichlet entries of u as zeros where mbits is given): gradient and
+// divergence per point, four sums per element, nothing to scatter.
+template <int NT>
+__global__ void __launch_bounds__(NT, DIV_TILES_PER_SM) a21_layer_kernel(LayerGrid g, const double *__restrict__ D,
+                                                                         const double *__restrict__ u,
+                                                                         const uint32_t *__restrict__ mbits,
+                                                                         double *__restrict__ yp)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *ut = reinterpret_cast<double *>(smem_raw);
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
+  prefetch_k<double, DN>(D, 0, e0, e1);
+  layer_fetch<double, NT>(ut, ut + L::TILE, g, tile, u, mbits);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const double *De = D + delem(a.e);
+  double Y[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int A = 0; A < 3; A++) {
+    if (A < 2) prefetch_k<double, DN>(D, A + 1, e0, e1);
+    if (!a.active) continue;
+    const double *dp = De + doff(9 * A, 0);
+    double f[9];
+#pragma unroll
+    for (int p = 0; p < 9; p++) f[p] = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) {
+      double m[27], G[3][9];
+#pragma unroll
+      for (int p = 0; p < 9; p++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) m[3 * p + d] = ldk(dp + doff(p, 0) + (3 * k + d) * KB);
+      layer_gradient<NT>(A, ut, a, k, G[0], G[1], G[2]);
+#pragma unroll
+      for (int p = 0; p < 9; p++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) f[p] = fma(m[3 * p + d], G[d][p], f[p]);
+    }
+#pragma unroll
+    for (int p = 0; p < 9; p++) {
+      Y[0] += f[p];
+#pragma unroll
+      for (int d = 0; d < 3; d++) Y[1 + d] = fma(f[p], ldk(dp + doff(p, 9 + d)), Y[1 + d]);
+    }
+  }
+  if (!a.active) return;
+  double *y = yp + 4 * (int64_t)a.e;
+  if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
+    reinterpret_cast<double2 *>(y)[0] = make_double2(Y[0], Y[1]);
+    reinterpret_cast<double2 *>(y)[1] = make_double2(Y[2], Y[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i++) y[i] = Y[i];
+  }
+}
+
+// B^T p to scratch.
+template <int NT>
+__global__ void __launch_bounds__(NT, DIV_TILES_PER_SM) a12_layer_kernel(LayerGrid g, const double *__restrict__ D,
+                                                                         const double *__restrict__ p,
+                                                                         double *__restrict__ out)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *yt = reinterpret_cast<double *>(smem_raw);
+  double *side = yt + L::TILE;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
+  prefetch_k<double, DN>(D, 0, e0, e1);
+  layer_zero<double, NT>(yt);
+  double pe[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) pe[i] = a.active ? p[4 * (int64_t)a.e + i] : 0.0;
+  __syncthreads();
+  const unsigned amask = __ballot_sync(0xffffffffu, a.active);
+  const double *De = D + delem(a.e);
+#pragma unroll 1
+  for (int A = 0; A < 3; A++) {
+    if (A < 2) prefetch_k<double, DN>(D, A + 1, e0, e1);
+    if (!a.active) continue;
+    const double *dp = De + doff(9 * A, 0);
+    double pq[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++)
+      pq[q] = pe[0] + (pe[1] * ldk(dp + doff(q, 9)) + (pe[2] * ldk(dp + doff(q, 10)) + pe[3] * ldk(dp + doff(q, 11))));
+#pragma unroll 1
+    for (int l = 0; l < 3; l++) {
+      double G[3][9], Qt[9], Rt[9], V[27];
+#pragma unroll
+      for (int q = 0; q < 9; q++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) G[d][q] = pq[q] * ldk(dp + doff(q, 0) + (3 * l + d) * KB);
+      q2::plane_bwd(G[0], G[1], G[2], Qt, Rt);
+#pragma unroll
+      for (int ji = 0; ji < 9; ji++) zeta_bwd_rt<double>(A, Qt[ji], Rt[ji], V[ji], V[9 + ji], V[18 + ji]);
+      layer_add<double, NT>(yt, side, a, amask, l, V);
+    }
+  }
+  layer_dump<double, NT>(yt, side, a, out + (int64_t)tile * L::TILE);
+}
+
+// ---------------------------------------------------------------------------
 // The gather
 // ---------------------------------------------------------------------------
-enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2 };
+enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2, LAYER_BC_ZERO = 3, LAYER_ADD = 4 };
 
 // Node t of the element box (i + NX (j + NY k)): the sum of its tile entries,
 // along x innermost, then rows, then layers, lower first.  BC_COPY: y_k = x_k
-// on Dirichlet dofs, BC_ONE: 1 there.
+// on Dirichlet dofs, BC_ONE / BC_ZERO: 1 / 0 there, ADD: added to y.
 template <typename T, int NT, int MODE>
 __device__ __forceinline__ void layer_gather_node(const LayerGrid &g, uint32_t t, const T *s,
                                                   const T *__restrict__ x, const uint32_t *__restrict__ mbits,
@@ -547,8 +745,9 @@ __device__ __forceinline__ void layer_gather_node(const LayerGrid &g, uint32_t t
 #pragma unroll
   for (int l = 0; l < 3; l++) {
     T v = acc[l];
-    if (MODE != LAYER_PLAIN && mbits && ((mbits[(k0 + l) >> 5] >> ((k0 + l) & 31)) & 1u))
-      v = MODE == LAYER_BC_COPY ? x[k0 + l] : T(1);
+    if (MODE == LAYER_ADD) v += y[k0 + l];
+    else if (MODE != LAYER_PLAIN && mbits && ((mbits[(k0 + l) >> 5] >> ((k0 + l) & 31)) & 1u))
+      v = MODE == LAYER_BC_COPY ? x[k0 + l] : T(MODE == LAYER_BC_ONE ? 1 : 0);
     y[k0 + l] = v;
   }
 }

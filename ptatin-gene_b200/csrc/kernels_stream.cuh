@@ -73,14 +73,15 @@ __host__ __device__ constexpr int koff(int q, int r) { return (9 * q + r) * KB; 
 __host__ __device__ __forceinline__ int64_t ksize(int64_t nel) { return (nel + KB - 1) / KB * KBLOCK; }
 
 // Bulk L2 prefetch (TMA unit) of Gauss plane A of the K blocks that hold
-// elements [e0, e1), one thread per block (81 x 32 values, 16-byte aligned).
-template <typename T>
+// elements [e0, e1), one thread per block (16-byte aligned pieces).
+// R: values per Gauss point (9 for K).
+template <typename T, int R = 9>
 __device__ __forceinline__ void prefetch_k(const T *K, int A, int64_t e0, int64_t e1)
 {
   const int64_t b = e0 / KB + threadIdx.x;
   if (b * KB < e1)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(K + b * KBLOCK + koff(9 * A, 0)),
-                 "r"((uint32_t)(sizeof(T) * 81 * KB))
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(K + (b * 27 + 9 * A) * R * KB),
+                 "r"((uint32_t)(sizeof(T) * 9 * R * KB))
                  : "memory");
 }
 

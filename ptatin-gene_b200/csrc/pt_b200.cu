@@ -27,7 +27,6 @@
 #include "kernels_layer.cuh"
 #include "kernels_ebe.cuh"
 #include "kernels_markers.cuh"
-#include "kernels_bmat.cuh"
 #include "kernels_galerkin.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
@@ -78,9 +77,8 @@ constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
 constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
 // layer tiles: node numbers stay below 2^31, scratch (460 B per element) below 4 GB
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
-// the set-up kernels use the same tiles for every box (node numbers below
-// 2^31; K of a larger box is more than any device holds)
-constexpr int64_t TILE_MAX_ELEMENTS = (int64_t)1 << 27;
+// every box: element-node numbers stay below 2^31
+constexpr int64_t MAX_ELEMENTS = (int64_t)1 << 28;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
 constexpr int PIPE_LAYERS = 6;
@@ -106,8 +104,8 @@ struct pt_op {
   unsigned int *d_bad;
   int TX, ntx, LZ, nzc;
   bool geom_dirty, geom_ok, full_box, ebe_valid;
-  bool be_valid;  // d_Be matches the coordinates
-  double *d_Be;   // divergence blocks [nel][4][81] (one-rank boxes, built on first B / B^T use)
+  bool d_valid;   // d_D matches the coordinates
+  double *d_D;    // factors of B and B^T at the Gauss points (built on first use)
   int a11_kernel;
   int64_t launches;
   uint64_t state;  // bumped whenever coordinates, viscosity or the mask change
@@ -486,7 +484,6 @@ pt_status launch_geometry(pt_op *op)
 pt_status ensure_geometry(pt_op *op)
 {
   if (!op->geom_dirty) return PT_OK;
-  if (op->nel > TILE_MAX_ELEMENTS) return fail(PT_ERR_OOM, "%lld elements: more geometry than a device holds", (long long)op->nel);
   const int64_t nk = ptk::ksize(op->nel);
   if (!op->d_K) {
     PT_CUDA(op_alloc(op, (void **)&op->d_K, sizeof(double) * nk));
@@ -688,60 +685,48 @@ pt_status diag_d(pt_op *op, double *d, bool ones = false)
   return PT_OK;
 }
 
-// Divergence blocks of the current coordinates (one-rank boxes), built on first use.
-pt_status ensure_be(pt_op *op)
+// Factors of B and B^T for the current coordinates, built on first use.
+pt_status ensure_div(pt_op *op)
 {
-  if (op->be_valid) return PT_OK;
-  if (!op->d_Be) PT_CUDA(op_alloc(op, (void **)&op->d_Be, sizeof(double) * ptk::BMAT_LD * op->nel));
-  ptk::bmat_kernel<<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, op->d_Be);
+  if (op->d_valid) return PT_OK;
+  if (!op->d_D) PT_CUDA(op_alloc(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel)));
+  pt_status s = ensure_layer(op);
+  if (s != PT_OK) return s;
+  constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
+  if ((s = kernel_attrs((const void *)ptk::div_layer_kernel<LNT>, smem)) != PT_OK) return s;
+  ptk::div_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_D);
   PT_LAUNCHED(op);
-  op->be_valid = true;
+  op->d_valid = true;
   return PT_OK;
 }
 
 pt_status a21_d(pt_op *op, const double *u, double *yp, bool masked)
 {
-  if (op->full_box) {
-    pt_status s = ensure_be(op);
-    if (s != PT_OK) return s;
-    if (masked)
-      ptk::bmat_a21_kernel<true><<<nblocks(32 * op->nel), TPB, 0, op->stream>>>(op->box, op->d_Be, u, op->d_mask, yp);
-    else
-      ptk::bmat_a21_kernel<false><<<nblocks(32 * op->nel), TPB, 0, op->stream>>>(op->box, op->d_Be, u, nullptr, yp);
-    PT_LAUNCHED(op);
-    return PT_OK;
-  }
-  if (masked)
-    ptk::a21_kernel<true><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, u, op->d_mask, yp);
-  else
-    ptk::a21_kernel<false><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, u, nullptr, yp);
+  pt_status s = ensure_div(op);
+  if (s != PT_OK) return s;
+  constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
+  if ((s = kernel_attrs((const void *)ptk::a21_layer_kernel<LNT>, smem)) != PT_OK) return s;
+  ptk::a21_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, u,
+                                                                               masked ? op->d_mbits : nullptr, yp);
   PT_LAUNCHED(op);
   return PT_OK;
 }
 
-// yu = B^T p, or yu += B^T p (accumulate)
-pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false)
+// yu = B^T p (`zero`: Dirichlet rows 0), or yu += B^T p (accumulate)
+pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false, bool zero = false)
 {
-  if (op->full_box) {
-    // one-rank box: node by node from the stored blocks
-    pt_status s = ensure_be(op);
-    if (s != PT_OK) return s;
-    if (accumulate)
-      ptk::bmat_a12_gather_kernel<true><<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->box, op->d_Be, p, yu);
-    else
-      ptk::bmat_a12_gather_kernel<false><<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->box, op->d_Be, p, yu);
-    PT_LAUNCHED(op);
-    return PT_OK;
-  }
-  if (!accumulate) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
-  for (int c = 0; c < 8; c++) {
-    ptk::ColourGrid g = ptk::colour_grid(op->box, c);
-    const int64_t n = (int64_t)g.ncx * g.ncy * g.ncz;
-    if (n == 0) continue;
-    ptk::a12_colour_kernel<<<nblocks(n), TPB, 0, op->stream>>>(g, op->d_coords, p, yu);
-    PT_LAUNCHED(op);
-  }
-  return PT_OK;
+  pt_status s = ensure_div(op);
+  if (s != PT_OK) return s;
+  constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
+  if ((s = kernel_attrs((const void *)ptk::a12_layer_kernel<LNT>, smem)) != PT_OK) return s;
+  if (!accumulate && !op->full_box) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
+  LayerLock lock(op);
+  ptk::a12_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, p, op->d_layer);
+  PT_LAUNCHED(op);
+  const uint32_t n = op->lg.nodes();
+  if (accumulate) return launch_layer_gather<double, ptk::LAYER_ADD>(op, 0, n, nullptr, yu);
+  return zero && op->has_mask ? launch_layer_gather<double, ptk::LAYER_BC_ZERO>(op, 0, n, nullptr, yu)
+                              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, n, nullptr, yu);
 }
 
 pt_status bc_copy(pt_op *op, const double *x, double *y)
@@ -927,6 +912,11 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
                 desc->ox, desc->oy, desc->oz, desc->mx, desc->my, desc->mz, (long long)nx, (long long)ny, (long long)nz);
   const int64_t nnodes = nx * ny * nz;
   if (nnodes > ((int64_t)1 << 40)) return fail(PT_ERR_BAD_ARG, "mesh too large");
+  // element and element-node numbers are 32-bit in the tile kernels: past what
+  // any device holds (coordinates and viscosity alone 600 bytes per element)
+  if ((int64_t)desc->mx * desc->my * desc->mz > MAX_ELEMENTS ||
+      (2 * (int64_t)desc->mx + 1) * (2 * (int64_t)desc->my + 1) * (2 * (int64_t)desc->mz + 1) > INT32_MAX)
+    return fail(PT_ERR_OOM, "%d x %d x %d elements do not fit a device", desc->mx, desc->my, desc->mz);
   pt_op *op = (pt_op *)calloc(1, sizeof(pt_op));
   if (!op) return fail(PT_ERR_OOM, "host allocation failed");
   op->mx = desc->mx; op->my = desc->my; op->mz = desc->mz;
@@ -943,8 +933,7 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   op->TX = desc->mx <= 32 ? 32 : (desc->mx <= 64 ? 64 : 128);
   op->ntx = (desc->mx + op->TX - 1) / op->TX;
   op->a11_kernel = auto_kernel(op);
-  if (op->nel <= TILE_MAX_ELEMENTS)
-    op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
+  op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
   pt_op_set_tiling(op, 0);
   op->geom_dirty = true;
   cudaError_t e = cudaGetDevice(&op->device);
@@ -981,7 +970,7 @@ pt_status pt_op_destroy(pt_op *op)
   if (op->stream && !op->pool) cudaStreamSynchronize(op->stream);
   void *bufs[] = {op->d_coords, op->d_eta, op->d_coords32, op->d_eta32, op->d_mask, op->d_u,
                   op->d_y, op->d_p, op->d_K, op->d_K32, op->d_bad, op->d_Ae, op->d_Ae32, op->d_ye,
-                  op->mk_scratch, op->d_Be, op->d_yp, op->d_mbits, op->d_fu, op->d_F, op->d_layer};
+                  op->mk_scratch, op->d_D, op->d_yp, op->d_mbits, op->d_fu, op->d_F, op->d_layer};
   for (void *b : bufs) op_free(op, b);
   for (int b = 0; b < 2; b++)
     if (op->h_stage[b]) {
@@ -1028,7 +1017,7 @@ static pt_status finish_coords(pt_op *op)
 {
   op->has_coords = true;
   op->geom_dirty = true;
-  op->be_valid = false;
+  op->d_valid = false;
   op->F_valid = false;
   op->state++;
   return PT_OK;
@@ -1278,9 +1267,10 @@ pt_status pt_getdiag_a11_h(pt_op *op, double *d)
 
 pt_status pt_matmult_a12_d(pt_op *op, const double *p, double *yu)
 {
-  pt_status s = pt_a12_apply_d(op, p, yu);
+  pt_status s = check_ready(op, false);
   if (s != PT_OK) return s;
-  return bc_value(op, 0.0, yu);
+  if (!p || !yu) return fail(PT_ERR_BAD_ARG, "NULL vector");
+  return a12_d(op, p, yu, false, true);
 }
 
 pt_status pt_matmult_a12_h(pt_op *op, const double *p, double *yu)

@@ -105,3 +105,23 @@ def test_pinned_host_apply_of_layer_tiles_is_bitwise_the_device_apply(workload):
         assert np.array_equal(yp.numpy(), op.MatMult_MFStokes_A11(x.cuda()).cpu().numpy())
         op.MFStokesWrapper_A11(xp.numpy(), yp.numpy())
         assert np.array_equal(yp.numpy(), op.MFStokesWrapper_A11(x.cuda()).cpu().numpy())
+
+
+@pytest.mark.parametrize("workload", SHAPES)
+def test_divergence_and_gradient_match_oracle(ora, workload):
+    """B u and B^T p from the Gauss-point factors, MatShell and SpMVOp level,
+    before any viscosity is set, into a pressure vector of odd alignment too."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, _, mask = M.problem(workload, seed=17)
+    u, p = M.uniform_vec(m.nvel, 18), M.uniform_vec(m.npres, 19)
+    with MatStokesMF(*m.dims) as op:
+        op.set_coords(m.coords)
+        op.set_bc_mask(mask)
+        ud, buf = torch.from_numpy(u).cuda(), torch.empty(m.npres + 1, dtype=torch.float64, device="cuda")
+        for yp in (buf[:-1], buf[1:]):
+            assert relerr(op.MatMult_MFStokes_A21(ud, yp).cpu().numpy(), ora.matmult_a21(m.dims, m.coords, mask, u)) < TOL64
+        assert relerr(op.MFStokesWrapper_A21(u), ora.a21(m.dims, m.coords, u)) < TOL64
+        assert relerr(op.MatMult_MFStokes_A12(p), ora.matmult_a12(m.dims, m.coords, mask, p)) < TOL64
+        assert relerr(op.MFStokesWrapper_A12(p), ora.a12(m.dims, m.coords, p)) < TOL64
