@@ -306,6 +306,143 @@ __global__ void __launch_bounds__(NT, layer_min_blocks<T, NT>()) a11_layer_kerne
   layer_tile<T, NT>(g, tile0 + (int)blockIdx.x, K, u, mbits, out);
 }
 
+// P: four factors per point beyond K, in blocks like K (geom_layer_kernel).
+constexpr int PN = 4;
+constexpr int PBLOCK = 27 * PN * KB;
+__host__ __device__ __forceinline__ int64_t pelem(int64_t e) { return e / KB * PBLOCK + e % KB; }
+__host__ __device__ constexpr int poff(int q, int r) { return (PN * q + r) * KB; }
+__host__ __device__ __forceinline__ int64_t psize(int64_t nel) { return (nel + KB - 1) / KB * PBLOCK; }
+
+// Gradient of component l of a tile's field at Gauss plane A (h^-1 d/dxi).
+template <int NT>
+__device__ __forceinline__ void layer_gradient(int A, const double *t, const LayerThread &a, int l, double G0[9],
+                                               double G1[9], double G2[9])
+{
+  using L = LayerLayout<NT>;
+  double Q[9], R[9];
+  const double *tl = t + l * L::COMP;
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double *p = tl + (i == 0 ? (int)threadIdx.x : (i == 1 ? a.od : a.en)) + j * L::ROW;
+      zeta_fwd_rt<double>(A, p[0], p[L::PLANE], p[2 * L::PLANE], Q[3 * j + i], R[3 * j + i]);
+    }
+  q2::plane_fwd(Q, R, G0, G1, G2);
+}
+
+// G[d][l][p] = h^-1 d x_l / d xi_d at the 9 points of Gauss plane A.
+template <int NT>
+__device__ __forceinline__ void layer_jacobian(int A, const double *xt, const LayerThread &a, double G[3][3][9])
+{
+#pragma unroll
+  for (int l = 0; l < 3; l++) layer_gradient<NT>(A, xt, a, l, G[0][l], G[1][l], G[2][l]);
+}
+
+// Element e's four pressure sums.
+__device__ __forceinline__ void store_p(double *__restrict__ yp, int e, const double Y[4])
+{
+  double *y = yp + 4 * (int64_t)e;
+  if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
+    reinterpret_cast<double2 *>(y)[0] = make_double2(Y[0], Y[1]);
+    reinterpret_cast<double2 *>(y)[1] = make_double2(Y[2], Y[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i++) y[i] = Y[i];
+  }
+}
+
+// The whole Stokes operator on the A11 tiles: with P (four more factors per
+// point, see the set-up) the pressure is one number added to the symmetric
+// stress before it meets K again, and the divergence is the trace that the
+// viscous action has formed, so A12 and A21 cost neither a forward nor a
+// transposed contraction nor a scatter of their own.  DIV: yp = B u.
+template <int NT, bool DIV>
+__device__ __forceinline__ void stokes_plane(int A, const double *ut, double *yt, double *side, const LayerThread &a,
+                                             unsigned amask, const double *__restrict__ Ke,
+                                             const double *__restrict__ Pe, const double pe[4], double Y[4])
+{
+  double G[3][3][9];
+  layer_jacobian<NT>(A, ut, a, G);
+  // the next point's factors are in flight while one computes
+  const double *kp = Ke + koff(9 * A, 0), *pp = Pe + poff(9 * A, 0);
+  double Kn[9], Pn[4];
+#pragma unroll
+  for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(0, r));
+#pragma unroll
+  for (int r = 0; r < 4; r++) Pn[r] = ldk(pp + poff(0, r));
+#pragma unroll
+  for (int p = 0; p < 9; p++) {
+    double Kq[9], Pq[4];
+#pragma unroll
+    for (int r = 0; r < 9; r++) Kq[r] = Kn[r];
+#pragma unroll
+    for (int r = 0; r < 4; r++) Pq[r] = Pn[r];
+    if (p < 8) {
+#pragma unroll
+      for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(p + 1, r));
+#pragma unroll
+      for (int r = 0; r < 4; r++) Pn[r] = ldk(pp + poff(p + 1, r));
+    }
+    const double pq = pe[0] + (pe[1] * Pq[1] + (pe[2] * Pq[2] + pe[3] * Pq[3]));
+    const double f = Pq[0] * q2::qp_action_Ks<double, true>(Kq, G, p, Pq[0] * pq);
+    if (DIV) {
+      Y[0] += f;
+#pragma unroll
+      for (int d = 0; d < 3; d++) Y[1 + d] = fma(f, Pq[1 + d], Y[1 + d]);
+    }
+  }
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double Qt[9], Rt[9], C[27];
+    q2::plane_bwd(G[0][l], G[1][l], G[2][l], Qt, Rt);
+#pragma unroll
+    for (int ji = 0; ji < 9; ji++) zeta_bwd_rt<double>(A, Qt[ji], Rt[ji], C[ji], C[9 + ji], C[18 + ji]);
+    layer_add<double, NT>(yt, side, a, amask, l, C);
+  }
+}
+
+template <int NT, bool DIV>
+__global__ void __launch_bounds__(NT, 256 / NT) stokes_layer_kernel(LayerGrid g, const double *__restrict__ K,
+                                                                    const double *__restrict__ P,
+                                                                    const double *__restrict__ u,
+                                                                    const double *__restrict__ pr,
+                                                                    const uint32_t *__restrict__ mbits,
+                                                                    double *__restrict__ out, double *__restrict__ yp)
+{
+  using L = LayerLayout<NT>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *ut = reinterpret_cast<double *>(smem_raw);
+  double *yt = ut + L::TILE;
+  double *side = yt + L::TILE;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tile = blockIdx.x;
+  const LayerThread a = layer_thread<NT>(g, tile);
+  const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
+  prefetch_k(K, 0, e0, e1);
+  prefetch_k<double, PN>(P, 0, e0, e1);
+  layer_fetch<double, NT>(ut, yt, g, tile, u, mbits);
+  __syncthreads();  // the stage is read: the y tile may be zeroed
+  layer_zero<double, NT>(yt);
+  double pe[4], Y[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < 4; i++) pe[i] = a.active ? pr[4 * (int64_t)a.e + i] : 0.0;
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const unsigned amask = __ballot_sync(0xffffffffu, a.active);
+  const double *Ke = K + kelem(a.e), *Pe = P + pelem(a.e);
+#pragma unroll 1
+  for (int A = 0; A < 3; A++) {
+    if (A < 2) {
+      prefetch_k(K, A + 1, e0, e1);
+      prefetch_k<double, PN>(P, A + 1, e0, e1);
+    }
+    if (a.active) stokes_plane<NT, DIV>(A, ut, yt, side, a, amask, Ke, Pe, pe, Y);
+  }
+  if (DIV && a.active) store_p(yp, a.e, Y);
+  layer_dump<double, NT>(yt, side, a, out + (int64_t)tile * L::TILE);
+}
+
 // diag(A11): the same tiles without an input, q2::diag_form_plane per plane
 // and component as in the streaming diagonal (kernels_diag.cuh).
 template <int NT>
@@ -354,32 +491,6 @@ __global__ void __launch_bounds__(NT, 256 / NT) diag_layer_kernel(LayerGrid g, c
 // ---------------------------------------------------------------------------
 // Set-up on the same tiles: the coordinates take the place of u
 // ---------------------------------------------------------------------------
-// Gradient of component l of a tile's field at Gauss plane A (h^-1 d/dxi).
-template <int NT>
-__device__ __forceinline__ void layer_gradient(int A, const double *t, const LayerThread &a, int l, double G0[9],
-                                               double G1[9], double G2[9])
-{
-  using L = LayerLayout<NT>;
-  double Q[9], R[9];
-  const double *tl = t + l * L::COMP;
-#pragma unroll
-  for (int j = 0; j < 3; j++)
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      const double *p = tl + (i == 0 ? (int)threadIdx.x : (i == 1 ? a.od : a.en)) + j * L::ROW;
-      zeta_fwd_rt<double>(A, p[0], p[L::PLANE], p[2 * L::PLANE], Q[3 * j + i], R[3 * j + i]);
-    }
-  q2::plane_fwd(Q, R, G0, G1, G2);
-}
-
-// G[d][l][p] = h^-1 d x_l / d xi_d at the 9 points of Gauss plane A.
-template <int NT>
-__device__ __forceinline__ void layer_jacobian(int A, const double *xt, const LayerThread &a, double G[3][3][9])
-{
-#pragma unroll
-  for (int l = 0; l < 3; l++) layer_gradient<NT>(A, xt, a, l, G[0][l], G[1][l], G[2][l]);
-}
-
 // J at point p of a plane's scaled gradient
 __device__ __forceinline__ void layer_point(const double G[3][3][9], int p, double J[3][3])
 {
@@ -431,6 +542,22 @@ __device__ __forceinline__ void layer_points(const double *xt, const LayerThread
   }
 }
 
+// The P1GRel frame: mean of the element's nodes and inverse extents.
+template <int NT>
+__device__ __forceinline__ void layer_frame(const double *xt, const LayerThread &a, double mean[3], double invL[3])
+{
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double s = 0.0;
+#pragma unroll
+    for (int n = 0; n < 27; n++) s += layer_node<NT>(xt, a, l, n);
+    mean[l] = (1.0 / 27.0) * s;
+  }
+  invL[0] = 1.0 / (layer_node<NT>(xt, a, 0, 14) - layer_node<NT>(xt, a, 0, 12));
+  invL[1] = 1.0 / (layer_node<NT>(xt, a, 1, 16) - layer_node<NT>(xt, a, 1, 10));
+  invL[2] = 1.0 / (layer_node<NT>(xt, a, 2, 22) - layer_node<NT>(xt, a, 2, 4));
+}
+
 // J at point q from the coordinates at the points
 __device__ __forceinline__ void layer_point_jacobian(const double I[3][27], int q, double J[3][3])
 {
@@ -452,10 +579,15 @@ __device__ __forceinline__ void layer_point_jacobian(const double I[3][27], int 
 // operations of element_jacobian in their order -- its entries are differences
 // of nearby coordinates, so another order moves K by 1e-14 -- which is why
 // this does not go plane by plane like the apply.
-template <int NT>
+//
+// PRESSURE: also P, the factors of the whole Stokes operator beyond K, four per
+// point and blocked like K: S = -w / sqrt(c), and the P1GRel basis functions
+// x^_d of P3D_ConstructNi_P1GRel_3D (src/element_utils_q2.c:183-224).
+template <int NT, bool PRESSURE>
 __global__ void __launch_bounds__(NT, 256 / NT) geom_layer_kernel(LayerGrid g, const double *__restrict__ coords,
                                                                   const double *__restrict__ eta,
                                                                   double *__restrict__ K, float *__restrict__ K32,
+                                                                  double *__restrict__ P,
                                                                   unsigned int *__restrict__ bad)
 {
   using L = LayerLayout<NT>;
@@ -465,6 +597,8 @@ __global__ void __launch_bounds__(NT, 256 / NT) geom_layer_kernel(LayerGrid g, c
   const LayerThread a = layer_thread<NT>(g, tile);
   layer_fetch_coords<NT>(xt, xt + L::TILE, g, tile, coords);
   if (!a.active) return;
+  double mean[3], invL[3];
+  if (PRESSURE) layer_frame<NT>(xt, a, mean, invL);
   double I[3][27];
   layer_points<NT>(xt, a, I);
   const double *ee = eta + 27 * (int64_t)a.e;
@@ -476,11 +610,18 @@ __global__ void __launch_bounds__(NT, 256 / NT) geom_layer_kernel(LayerGrid g, c
     // one point at a time: square roots and divisions of several in flight spill
     asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(e) : "l"(ee + q) : "memory");
     layer_point_jacobian(I, q, J);
-    if (!q2::geom_K(J, q2::weight(q) * e, Kq)) nbad++;
+    double root;
+    if (!q2::geom_K(J, q2::weight(q) * e, Kq, &root)) nbad++;
 #pragma unroll
     for (int r = 0; r < 9; r++) {
       K[k0 + koff(q, r)] = Kq[r];
       if (K32) K32[k0 + koff(q, r)] = (float)Kq[r];
+    }
+    if (PRESSURE) {
+      double *Pe = P + pelem(a.e) + poff(q, 0);
+      Pe[0] = -q2::weight(q) / root;
+#pragma unroll
+      for (int d = 0; d < 3; d++) Pe[(1 + d) * KB] = (I[d][q] - mean[d]) * invL[d];
     }
   }
   if (nbad) atomicAdd(bad, nbad);
@@ -568,16 +709,7 @@ __global__ void __launch_bounds__(NT, 256 / NT) div_layer_kernel(LayerGrid g, co
   layer_fetch_coords<NT>(xt, xt + L::TILE, g, tile, coords);
   if (!a.active) return;
   double mean[3], invL[3];
-#pragma unroll
-  for (int l = 0; l < 3; l++) {
-    double s = 0.0;
-#pragma unroll
-    for (int n = 0; n < 27; n++) s += layer_node<NT>(xt, a, l, n);
-    mean[l] = (1.0 / 27.0) * s;
-  }
-  invL[0] = 1.0 / (layer_node<NT>(xt, a, 0, 14) - layer_node<NT>(xt, a, 0, 12));
-  invL[1] = 1.0 / (layer_node<NT>(xt, a, 1, 16) - layer_node<NT>(xt, a, 1, 10));
-  invL[2] = 1.0 / (layer_node<NT>(xt, a, 2, 22) - layer_node<NT>(xt, a, 2, 4));
+  layer_frame<NT>(xt, a, mean, invL);
   double I[3][27];
   layer_points<NT>(xt, a, I);
   double *De = D + delem(a.e);
@@ -647,15 +779,7 @@ __global__ void __launch_bounds__(NT, DIV_TILES_PER_SM) a21_layer_kernel(LayerGr
       for (int d = 0; d < 3; d++) Y[1 + d] = fma(f[p], ldk(dp + doff(p, 9 + d)), Y[1 + d]);
     }
   }
-  if (!a.active) return;
-  double *y = yp + 4 * (int64_t)a.e;
-  if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
-    reinterpret_cast<double2 *>(y)[0] = make_double2(Y[0], Y[1]);
-    reinterpret_cast<double2 *>(y)[1] = make_double2(Y[2], Y[3]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; i++) y[i] = Y[i];
-  }
+  if (a.active) store_p(yp, a.e, Y);
 }
 
 // B^T p to scratch.
@@ -708,11 +832,12 @@ __global__ void __launch_bounds__(NT, DIV_TILES_PER_SM) a12_layer_kernel(LayerGr
 // ---------------------------------------------------------------------------
 // The gather
 // ---------------------------------------------------------------------------
-enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2, LAYER_BC_ZERO = 3, LAYER_ADD = 4 };
+enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2, LAYER_BC_ZERO = 3, LAYER_ADD = 4, LAYER_SUB = 5 };
 
 // Node t of the element box (i + NX (j + NY k)): the sum of its tile entries,
 // along x innermost, then rows, then layers, lower first.  BC_COPY: y_k = x_k
-// on Dirichlet dofs, BC_ONE / BC_ZERO: 1 / 0 there, ADD: added to y.
+// on Dirichlet dofs, BC_ONE / BC_ZERO: 1 / 0 there, ADD: added to y,
+// SUB: x subtracted.
 template <typename T, int NT, int MODE>
 __device__ __forceinline__ void layer_gather_node(const LayerGrid &g, uint32_t t, const T *s,
                                                   const T *__restrict__ x, const uint32_t *__restrict__ mbits,
@@ -746,6 +871,7 @@ __device__ __forceinline__ void layer_gather_node(const LayerGrid &g, uint32_t t
   for (int l = 0; l < 3; l++) {
     T v = acc[l];
     if (MODE == LAYER_ADD) v += y[k0 + l];
+    else if (MODE == LAYER_SUB) v -= x[k0 + l];
     else if (MODE != LAYER_PLAIN && mbits && ((mbits[(k0 + l) >> 5] >> ((k0 + l) & 31)) & 1u))
       v = MODE == LAYER_BC_COPY ? x[k0 + l] : T(MODE == LAYER_BC_ONE ? 1 : 0);
     y[k0 + l] = v;

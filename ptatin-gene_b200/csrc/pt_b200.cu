@@ -106,6 +106,7 @@ struct pt_op {
   bool geom_dirty, geom_ok, full_box, ebe_valid;
   bool d_valid;   // d_D matches the coordinates
   double *d_D;    // factors of B and B^T at the Gauss points (built on first use)
+  double *d_P;    // factors of the whole Stokes operator beyond K (from its first use, with K)
   int a11_kernel;
   int64_t launches;
   uint64_t state;  // bumped whenever coordinates, viscosity or the mask change
@@ -466,15 +467,18 @@ pt_status launch_stream(pt_op *op, const T *K, const T *u, T *y)
   return launch_stream_tx<T, 128, MASKED>(op, K, u, y);
 }
 
-// K in FP64 and FP32 and the count of points with c <= 0, on the op's stream.
+// K in FP64 and FP32, P once the whole operator has been used, and the count of
+// points with c <= 0, on the op's stream.
 pt_status launch_geometry(pt_op *op)
 {
   constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
-  pt_status s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT>, smem);
+  pt_status s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT, false>, smem);
+  if (s == PT_OK) s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT, true>, smem);
   if (s != PT_OK) return s;
   PT_CUDA(cudaMemsetAsync(op->d_bad, 0, sizeof(unsigned int), op->stream));
-  ptk::geom_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_eta,
-                                                                                op->d_K, op->d_K32, op->d_bad);
+  auto kernel = op->d_P ? ptk::geom_layer_kernel<LNT, true> : ptk::geom_layer_kernel<LNT, false>;
+  kernel<<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_eta, op->d_K, op->d_K32,
+                                                            op->d_P, op->d_bad);
   PT_LAUNCHED(op);
   return PT_OK;
 }
@@ -729,6 +733,49 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
                               : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, n, nullptr, yu);
 }
 
+// Yu = A11 u + B^T p (- x when mode is LAYER_SUB) and, unless yp is null,
+// Yp = B u, in one pass over the tiles; *done = false where the geometry does
+// not allow K (the caller then runs the blocks one by one).  masked: Dirichlet
+// columns of u as zeros, rows copied from u.
+pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double *x, double *yu, double *yp, int mode,
+                       bool *done)
+{
+  *done = false;
+  if (op->a11_kernel == A11_COLOUR) return PT_OK;
+  pt_status s = ensure_geometry(op);
+  if (s != PT_OK) return s;
+  if (!op->geom_ok) return PT_OK;
+  if (!op->d_P) {
+    PT_CUDA(op_alloc(op, (void **)&op->d_P, sizeof(double) * ptk::psize(op->nel)));
+    if ((s = launch_geometry(op)) != PT_OK) return s;  // K again with the same values, and P
+  }
+  if ((s = ensure_layer(op)) != PT_OK) return s;
+  constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
+  if ((s = kernel_attrs((const void *)ptk::stokes_layer_kernel<LNT, true>, smem)) != PT_OK) return s;
+  if ((s = kernel_attrs((const void *)ptk::stokes_layer_kernel<LNT, false>, smem)) != PT_OK) return s;
+  if (!op->full_box) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
+  const bool masked = mode == ptk::LAYER_BC_COPY;
+  {
+    LayerLock lock(op);
+    auto kernel = yp ? ptk::stokes_layer_kernel<LNT, true> : ptk::stokes_layer_kernel<LNT, false>;
+    kernel<<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, op->d_P, u, p,
+                                                              masked ? op->d_mbits : nullptr, op->d_layer, yp);
+    PT_LAUNCHED(op);
+    const uint32_t n = op->lg.nodes();
+    if (masked) s = launch_layer_gather<double, ptk::LAYER_BC_COPY>(op, 0, n, x, yu);
+    else if (mode == ptk::LAYER_SUB) s = launch_layer_gather<double, ptk::LAYER_SUB>(op, 0, n, x, yu);
+    else s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, n, nullptr, yu);
+    if (s != PT_OK) return s;
+  }
+  if (!op->full_box && masked) {  // Dirichlet dofs outside the element box
+    bc_bits_kernel<double><<<grid_stride_blocks((op->nvel + 31) / 32), 256, 0, op->stream>>>(op->d_mbits, x, yu,
+                                                                                            op->nvel);
+    PT_LAUNCHED(op);
+  }
+  *done = true;
+  return PT_OK;
+}
+
 pt_status bc_copy(pt_op *op, const double *x, double *y)
 {
   if (!op->has_mask) return PT_OK;
@@ -970,7 +1017,7 @@ pt_status pt_op_destroy(pt_op *op)
   if (op->stream && !op->pool) cudaStreamSynchronize(op->stream);
   void *bufs[] = {op->d_coords, op->d_eta, op->d_coords32, op->d_eta32, op->d_mask, op->d_u,
                   op->d_y, op->d_p, op->d_K, op->d_K32, op->d_bad, op->d_Ae, op->d_Ae32, op->d_ye,
-                  op->mk_scratch, op->d_D, op->d_yp, op->d_mbits, op->d_fu, op->d_F, op->d_layer};
+                  op->mk_scratch, op->d_D, op->d_P, op->d_yp, op->d_mbits, op->d_fu, op->d_F, op->d_layer};
   for (void *b : bufs) op_free(op, b);
   for (int b = 0; b < 2; b++)
     if (op->h_stage[b]) {
@@ -1305,6 +1352,8 @@ pt_status pt_stokes_a_apply_d(pt_op *op, const double *u, const double *p, doubl
   if (s != PT_OK) return s;
   if (!u || !p || !yu || !yp) return fail(PT_ERR_BAD_ARG, "NULL vector");
   if (u == yu) return fail(PT_ERR_BAD_ARG, "u and yu must not alias");
+  bool done;
+  if ((s = stokes_fused(op, u, p, nullptr, yu, yp, ptk::LAYER_PLAIN, &done)) != PT_OK || done) return s;
   if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, u, yu, false)) != PT_OK) return s;
   if ((s = a12_d(op, p, yu, true)) != PT_OK) return s;
   return a21_d(op, u, yp, false);
@@ -1316,6 +1365,9 @@ pt_status pt_matmult_a_d(pt_op *op, const double *xu, const double *xp, double *
   if (s != PT_OK) return s;
   if (!xu || !xp || !yu || !yp) return fail(PT_ERR_BAD_ARG, "NULL vector");
   if (xu == yu) return fail(PT_ERR_BAD_ARG, "xu and yu must not alias");
+  bool done;
+  s = stokes_fused(op, xu, xp, xu, yu, yp, op->has_mask ? ptk::LAYER_BC_COPY : ptk::LAYER_PLAIN, &done);
+  if (s != PT_OK || done) return s;
   // Dirichlet columns zeroed inside the masked kernels; rows set back to x after B^T p
   if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, xu, yu, op->has_mask)) != PT_OK) return s;
   if ((s = a12_d(op, xp, yu, true)) != PT_OK) return s;
@@ -1423,9 +1475,11 @@ pt_status pt_residual_u_d(pt_op *op, const double *u, const double *p, double *r
   if (!u || !p || !ru) return fail(PT_ERR_BAD_ARG, "NULL vector");
   if (u == ru) return fail(PT_ERR_BAD_ARG, "u and ru must not alias");
   // u as given (the caller inserted the Dirichlet values): no column rule
+  bool done;
+  if ((s = ensure_body_force(op)) != PT_OK) return s;
+  if ((s = stokes_fused(op, u, p, op->d_F, ru, nullptr, ptk::LAYER_SUB, &done)) != PT_OK || done) return s;
   if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, u, ru, false)) != PT_OK) return s;
   if ((s = a12_d(op, p, ru, true)) != PT_OK) return s;
-  if ((s = ensure_body_force(op)) != PT_OK) return s;
   sub_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_F, ru, op->nvel);
   PT_LAUNCHED(op);
   return PT_OK;
@@ -1724,9 +1778,9 @@ extern "C" pt_status pt_a11_apply_noalloc_d(const pt_mesh_desc *desc, const doub
   // the counter keeps the previous call's value: clear it first
   PT_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st));
   constexpr size_t gsmem = ptk::layer_geom_smem_bytes<LNT>();
-  if ((s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT>, gsmem)) != PT_OK) return s;
+  if ((s = kernel_attrs((const void *)ptk::geom_layer_kernel<LNT, false>, gsmem)) != PT_OK) return s;
   const ptk::LayerGrid lg = ptk::layer_grid<LNT>(bx.mx, bx.my, bx.mz, bx.X, bx.XY, bx.off);
-  ptk::geom_layer_kernel<LNT><<<(unsigned)lg.tiles, LNT, gsmem, st>>>(lg, coords, eta, K, nullptr, bad);
+  ptk::geom_layer_kernel<LNT, false><<<(unsigned)lg.tiles, LNT, gsmem, st>>>(lg, coords, eta, K, nullptr, nullptr, bad);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
 

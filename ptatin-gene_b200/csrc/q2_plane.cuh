@@ -120,9 +120,12 @@ PT_HD void plane_bwd(const T G0[9], const T G1[9], const T G2[9], T Qt[9], T Rt[
   }
 }
 
-// Viscous action at point p of a plane: G[d][l][p] <- dv'[d][l] = ((K G)+(K G)^T) K
-template <typename T>
-PT_HD void qp_action_K(const T Kq[9], T G[3][3][9], int p)
+// Viscous action at point p of a plane: G[d][l][p] <- dv'[d][l] =
+// ((K G)+(K G)^T + s I) K; returns the trace of K G.  s = 0 is the viscous
+// block alone; the pressure enters as s = S p(q), and S tr(K G) is the
+// divergence's integrand (S = -sqrt(w det J / eta), kernels_layer.cuh).
+template <typename T, bool PRESSURE>
+PT_HD T qp_action_Ks(const T Kq[9], T G[3][3][9], int p, T s)
 {
   T A[3][3];
 #pragma unroll
@@ -136,10 +139,22 @@ PT_HD void qp_action_K(const T Kq[9], T G[3][3][9], int p)
   S[0][1] = S[1][0] = A[0][1] + A[1][0];
   S[0][2] = S[2][0] = A[0][2] + A[2][0];
   S[1][2] = S[2][1] = A[1][2] + A[2][1];
+  if (PRESSURE) {
+    S[0][0] += s;
+    S[1][1] += s;
+    S[2][2] += s;
+  }
 #pragma unroll
   for (int k = 0; k < 3; k++)
 #pragma unroll
     for (int l = 0; l < 3; l++) G[k][l][p] = S[0][l] * Kq[k] + (S[1][l] * Kq[3 + k] + S[2][l] * Kq[6 + k]);
+  return (A[0][0] + A[1][1]) + A[2][2];
+}
+
+template <typename T>
+PT_HD void qp_action_K(const T Kq[9], T G[3][3][9], int p)
+{
+  (void)qp_action_Ks<T, false>(Kq, G, p, T(0));
 }
 
 // ---------------------------------------------------------------------------
@@ -251,15 +266,17 @@ PT_HD void diag_form_plane(KR kr, const T z[3][3], T Q[27])
 }
 
 // K at one Gauss point from J (d x_l / d xi_d) and the weight*eta product.
-// Returns false when c = w eta / det is not positive and finite.
+// Returns false when c = w eta / det is not positive and finite; *root = sqrt(c).
 template <typename T>
-PT_HD bool geom_K(const double J[3][3], double w_eta, T Kq[9])
+PT_HD bool geom_K(const double J[3][3], double w_eta, T Kq[9], double *root = nullptr)
 {
   double adj[3][3];
   const double det = adjugate(J, adj);
   const double c = w_eta / det;
   const bool ok = (c > 0.0) && (c < 1.0e308);
-  const double f = DH * (ok ? sqrt(c) : 0.0);
+  const double r = ok ? sqrt(c) : 0.0;
+  const double f = DH * r;
+  if (root) *root = r;
 #pragma unroll
   for (int k = 0; k < 3; k++)
 #pragma unroll

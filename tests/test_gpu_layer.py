@@ -125,3 +125,57 @@ def test_divergence_and_gradient_match_oracle(ora, workload):
         assert relerr(op.MFStokesWrapper_A21(u), ora.a21(m.dims, m.coords, u)) < TOL64
         assert relerr(op.MatMult_MFStokes_A12(p), ora.matmult_a12(m.dims, m.coords, mask, p)) < TOL64
         assert relerr(op.MFStokesWrapper_A12(p), ora.a12(m.dims, m.coords, p)) < TOL64
+
+
+@pytest.mark.parametrize("workload", SHAPES)
+def test_whole_operator_matches_oracle_and_follows_its_coefficients(ora, workload):
+    """A11 and the pressure blocks in one pass, MatShell and SpMVOp level and
+    the residual; new viscosity and new coordinates reach its factors."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, eta, mask = M.problem(workload, seed=27)
+    m2 = M.make_mesh(*m.dims, perturb=0.05, seed=28)
+    eta2 = 1.0 + eta[::-1].copy()
+    u, p, fu = M.uniform_vec(m.nvel, 29), M.uniform_vec(m.npres, 30), M.uniform_vec(81 * m.nel, 31)
+    ud, pd = torch.from_numpy(u).cuda(), torch.from_numpy(p).cuda()
+    with MatStokesMF(*m.dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        op.set_body_force(fu)
+        for c, e in ((m.coords, eta), (m.coords, eta2), (m2.coords, eta2)):
+            op.set_coords(c)
+            op.set_eta(e)
+            yu, yp = op.MatMult_MFStokes_A(ud, pd)
+            ru, rp = ora.matmult_a(m.dims, c, e, mask, u, p)
+            assert relerr(yu.cpu().numpy(), ru) < TOL64 and relerr(yp.cpu().numpy(), rp) < TOL64
+            yu, yp = op.MFStokesWrapper_A(ud, pd)
+            a = ora.a11(m.dims, c, e, u) + ora.a12(m.dims, c, p)
+            assert relerr(yu.cpu().numpy(), a) < TOL64 and relerr(yp.cpu().numpy(), ora.a21(m.dims, c, u)) < TOL64
+            assert relerr(op.FormFunctionLocal_U(ud, pd).cpu().numpy(), ora.residual_u(m.dims, c, e, fu, u, p)) < TOL64
+
+
+def test_whole_operator_on_a_ghosted_box_is_the_sum_of_its_blocks():
+    import torch
+
+    from pt_b200 import MatStokesMF
+    sub, off, nb = (37, 4, 3), (2, 0, 1), (37 * 2 + 1 + 4, 4 * 2 + 1 + 2, 3 * 2 + 1 + 3)
+    rng = np.random.default_rng(7)
+    m, eta, _ = M.problem("box:%d,%d,%d" % sub, seed=8)
+    sl = tuple(slice(o, o + 2 * n + 1) for o, n in zip(off[::-1], sub[::-1]))
+    cg = rng.uniform(size=(nb[2], nb[1], nb[0], 3))
+    cg[sl] = m.coords.reshape(cg[sl].shape)
+    mask = (rng.uniform(size=cg.size) < 0.1).astype(np.uint8)
+    u = torch.from_numpy(rng.uniform(-1, 1, size=cg.size)).cuda()
+    p = torch.from_numpy(rng.uniform(-1, 1, size=4 * m.nel)).cuda()
+    with MatStokesMF(*sub, node_box=(*nb, *off)) as op:
+        op.SetUp(np.ascontiguousarray(cg.reshape(-1)), eta, mask)
+        yu, yp = op.MFStokesWrapper_A(u, p)
+        ref = op.MFStokesWrapper_A11(u) + op.MFStokesWrapper_A12(p)
+        assert float((yu - ref).abs().max()) < 1e-13 * float(ref.abs().max())
+        rp = op.MFStokesWrapper_A21(u)
+        assert float((yp - rp).abs().max()) < 1e-13 * float(rp.abs().max())
+        yu, yp = op.MatMult_MFStokes_A(u, p)
+        bc = torch.from_numpy(mask != 0).cuda()
+        ref = torch.where(bc, u, op.MatMult_MFStokes_A11(u) + op.MFStokesWrapper_A12(p))
+        assert float((yu - ref).abs().max()) < 1e-13 * float(ref.abs().max())
+        assert torch.equal(yu[bc], u[bc])
