@@ -66,25 +66,57 @@ struct LayerSeg {
   int t0, len;
 };
 
-// Fetches the tile's node values of u (Dirichlet entries as zeros where mbits
-// is given) with asynchronous copies, every copy of the tile in flight at
-// once, a warp to a line (one of a segment's 9 node rows).  The mask words of
-// all lines are staged first (`stage`: shared memory that nothing else uses
-// yet, the size of a tile), so the copies wait for one round trip and not for
-// one each.  Ends with the copies committed; `stage` is free after the next
-// barrier.
+// Segment table and lines of a tile (a line is one of a segment's 9 node rows).
+struct LayerLines {
+  const LayerSeg *seg;
+  int lines;
+  int words;  // mask words that cover a line, wherever it starts
+};
+
+// Line `line`: its first dof, its first entry in the tile, its nodes' elements
+// and its end entry from the first one.
+template <int NT>
+__device__ __forceinline__ int64_t layer_line(const LayerGrid &g, const LayerLines &ll, int line, int &first, int &len,
+                                              int &end)
+{
+  using L = LayerLayout<NT>;
+  const int sg = line / 9, kj = line - 9 * sg, k = kj / 3, j = kj - 3 * k;
+  const LayerSeg s = ll.seg[sg];
+  first = k * L::PLANE + j * L::ROW + s.t0;
+  len = s.len;
+  end = 2 * g.odd + sg - s.t0;
+  return s.k0 + 3 * (j * g.X + k * g.XY);
+}
+
+// Entry of value d (node d/3, component d%3) of a line, from the line's first.
+template <int NT>
+__device__ __forceinline__ int layer_entry(const LayerGrid &g, int d, int len, int end)
+{
+  const int m = (d * 43691) >> 17, c = d - 3 * m;  // d / 3 for d < 2^16
+  const int h = m >> 1;
+  return c * LayerLayout<NT>::COMP + ((m & 1) ? g.odd + h : (h == len ? end : h));
+}
+
+// Fetches the tile's node values of u with asynchronous copies, every copy of
+// the tile in flight at once, a warp to a line: a lane works out one of its
+// warp's lines and the warp then takes them from lane to lane (worked out by
+// the whole warp one after the other, the lines of a tile of short rows took
+// 8 us of a 27 us apply).  `stage`: shared memory for the segment table.  Ends
+// with the copies committed.
 template <typename T, int NT>
-__device__ __forceinline__ void layer_fetch(T *ut, void *stage, const LayerGrid &g, int tile, const T *__restrict__ u,
-                                            const uint32_t *__restrict__ mbits)
+__device__ __forceinline__ LayerLines layer_fetch(T *ut, void *stage, const LayerGrid &g, int tile,
+                                                  const T *__restrict__ u)
 {
   using L = LayerLayout<NT>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e0 = tile * g.E, n = min(g.E, g.nel - e0);
   const int row0 = (int)g.dmx.div((uint32_t)e0);
-  const int segs = (int)g.dmx.div((uint32_t)(e0 + n - 1)) - row0 + 1, lines = 9 * segs;
+  const int segs = (int)g.dmx.div((uint32_t)(e0 + n - 1)) - row0 + 1;
   LayerSeg *seg = reinterpret_cast<LayerSeg *>(stage);
-  uint32_t *words = reinterpret_cast<uint32_t *>(seg + segs);
-  const int mw = (3 * (2 * min(g.mx, n) + 1) + 31) / 32 + 1;  // words that cover a line, wherever it starts
+  LayerLines ll;
+  ll.seg = seg;
+  ll.lines = 9 * segs;
+  ll.words = (3 * (2 * min(g.mx, n) + 1) + 31) / 32 + 1;
   if ((int)threadIdx.x < segs) {
     LayerSeg s;
     const int row = row0 + threadIdx.x;
@@ -94,45 +126,85 @@ __device__ __forceinline__ void layer_fetch(T *ut, void *stage, const LayerGrid 
     seg[threadIdx.x] = s;
   }
   __syncthreads();
-  if (mbits) {
-    for (int line = warp; line < lines; line += L::NW) {
-      const int sg = line / 9, kj = line - 9 * sg, k = kj / 3, j = kj - 3 * k;
-      const LayerSeg s = seg[sg];
-      const int64_t k0 = s.k0 + 3 * (j * g.X + k * g.XY);
-      const int64_t w0 = k0 >> 5;
-      const int nw = (int)(((k0 + 3 * (2 * s.len + 1) - 1) >> 5) - w0 + 1);
-      if (lane < nw) words[line * mw + lane] = mbits[w0 + lane];
+  const int nl = (ll.lines - warp + L::NW - 1) / L::NW;  // lines of this warp
+  for (int b = 0; b < nl; b += 32) {
+    int64_t k0 = 0;
+    uint32_t pack = 0;  // first (12 bits), len (8), end (10)
+    if (b + lane < nl) {
+      int first, len, end;
+      k0 = layer_line<NT>(g, ll, warp + L::NW * (b + lane), first, len, end);
+      pack = (uint32_t)first | (uint32_t)len << 12 | (uint32_t)end << 20;
     }
-    __syncthreads();
-  }
-  for (int line = warp; line < lines; line += L::NW) {
-    const int sg = line / 9, kj = line - 9 * sg, k = kj / 3, j = kj - 3 * k;
-    const LayerSeg s = seg[sg];
-    const int64_t k0 = s.k0 + 3 * (j * g.X + k * g.XY);
-    const int nd = 3 * (2 * s.len + 1);
-    const T *src = u + k0;
-    T *row = ut + k * L::PLANE + j * L::ROW + s.t0;
-    const int end = 2 * g.odd + sg - s.t0;  // the end entry, from `row`
-    const uint32_t *w = words + line * mw;
-    const int b0 = (int)(k0 & 31);
+    const int cnt = min(32, nl - b);
+    for (int i = 0; i < cnt; i++) {
+      const uint32_t pk = __shfl_sync(0xffffffffu, pack, i);
+      const T *src = u + __shfl_sync(0xffffffffu, k0, i);
+      const int len = (pk >> 12) & 255, end = pk >> 20, nd = 3 * (2 * len + 1);
+      T *row = ut + (pk & 4095);
 #pragma unroll 4
-    for (int d = lane; d < nd; d += 32) {
-      const int m = (d * 43691) >> 17, c = d - 3 * m;  // d / 3 for d < 2^16
-      const int h = m >> 1;
-      T *dst = row + c * L::COMP + ((m & 1) ? g.odd + h : (h == s.len ? end : h));
-      uint32_t bytes = sizeof(T);
-      if (mbits) {
-        const int pos = b0 + d;
-        if ((w[pos >> 5] >> (pos & 31)) & 1u) bytes = 0;  // zero-filled
+      for (int d = lane; d < nd; d += 32) {
+        const uint32_t sd = (uint32_t)__cvta_generic_to_shared(row + layer_entry<NT>(g, d, len, end));
+        if (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sd), "l"(src + d) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sd), "l"(src + d) : "memory");
       }
-      const uint32_t sd = (uint32_t)__cvta_generic_to_shared(dst);
-      if (sizeof(T) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sd), "l"(src + d), "r"(bytes) : "memory");
-      else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sd), "l"(src + d), "r"(bytes) : "memory");
     }
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
+  return ll;
+}
+
+// Waits for the tile's copies and zeroes its Dirichlet entries (mbits not
+// null): a thread per mask word of a line, read while the copies fly.  The
+// tile is complete for every thread on return, the stage free.
+template <typename T, int NT>
+__device__ __forceinline__ void layer_land(T *ut, const LayerGrid &g, const LayerLines &ll,
+                                           const uint32_t *__restrict__ mbits)
+{
+  constexpr int AHEAD = 4;  // words per thread in flight (a tile of 128 elements has about 250 to 400)
+  if (!mbits) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    return;
+  }
+  const int total = ll.lines * ll.words;
+  for (int i0 = threadIdx.x; i0 - (int)threadIdx.x < total; i0 += AHEAD * NT) {
+    uint32_t w[AHEAD];
+    int d0[AHEAD], line[AHEAD];  // value of the word's first bit
+#pragma unroll
+    for (int a = 0; a < AHEAD; a++) {
+      const int i = i0 + a * NT;
+      w[a] = 0;
+      if (i < total) {
+        line[a] = i / ll.words;
+        int first, len, end;
+        const int64_t k0 = layer_line<NT>(g, ll, line[a], first, len, end);
+        const int64_t wi = (k0 >> 5) + (i - line[a] * ll.words);
+        const int nd = 3 * (2 * len + 1);
+        d0[a] = (int)(32 * wi - k0);
+        if (d0[a] < nd) {
+          w[a] = mbits[wi];
+          if (d0[a] < 0) w[a] &= ~0u << -d0[a];           // the line starts within the word
+          if (nd - d0[a] < 32) w[a] &= (1u << (nd - d0[a])) - 1;  // or ends in it
+        }
+      }
+    }
+    if (i0 == (int)threadIdx.x) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+    }
+#pragma unroll
+    for (int a = 0; a < AHEAD; a++)
+      if (w[a]) {
+        int first, len, end;
+        (void)layer_line<NT>(g, ll, line[a], first, len, end);
+        while (w[a]) {
+          const int d = d0[a] + __ffs(w[a]) - 1;
+          w[a] &= w[a] - 1;
+          ut[first + layer_entry<NT>(g, d, len, end)] = T(0);
+        }
+      }
+  }
+  __syncthreads();
 }
 
 template <typename T, int NT>
@@ -274,10 +346,9 @@ __device__ __forceinline__ void layer_tile(const LayerGrid &g, int tile, const T
   const LayerThread a = layer_thread<NT>(g, tile);
   const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
   prefetch_k(K, 0, e0, e1);
-  layer_fetch<T, NT>(ut, yt, g, tile, u, mbits);
-  __syncthreads();  // the stage is read: the y tile may be zeroed
-  layer_zero<T, NT>(yt);
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  const LayerLines ll = layer_fetch<T, NT>(ut, yt, g, tile, u);
+  layer_land<T, NT>(ut, g, ll, mbits);
+  layer_zero<T, NT>(yt);  // the stage was there
   __syncthreads();
   const unsigned amask = __ballot_sync(0xffffffffu, a.active);
   const T *Ke = K + kelem(a.e);
@@ -421,13 +492,12 @@ __global__ void __launch_bounds__(NT, 256 / NT) stokes_layer_kernel(LayerGrid g,
   const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
   prefetch_k(K, 0, e0, e1);
   prefetch_k<double, PN>(P, 0, e0, e1);
-  layer_fetch<double, NT>(ut, yt, g, tile, u, mbits);
-  __syncthreads();  // the stage is read: the y tile may be zeroed
-  layer_zero<double, NT>(yt);
+  const LayerLines ll = layer_fetch<double, NT>(ut, yt, g, tile, u);
   double pe[4], Y[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int i = 0; i < 4; i++) pe[i] = a.active ? pr[4 * (int64_t)a.e + i] : 0.0;
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  layer_land<double, NT>(ut, g, ll, mbits);
+  layer_zero<double, NT>(yt);  // the stage was there
   __syncthreads();
   const unsigned amask = __ballot_sync(0xffffffffu, a.active);
   const double *Ke = K + kelem(a.e), *Pe = P + pelem(a.e);
@@ -505,14 +575,11 @@ template <int NT>
 __device__ __forceinline__ void layer_fetch_coords(double *xt, void *stage, const LayerGrid &g, int tile,
                                                    const double *__restrict__ coords)
 {
-  layer_fetch<double, NT>(xt, stage, g, tile, coords, nullptr);
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
+  const LayerLines ll = layer_fetch<double, NT>(xt, stage, g, tile, coords);
+  layer_land<double, NT>(xt, g, ll, nullptr);
 }
 
-// Segment table and mask words of a fetch that has no tile to stage them in:
-// most for rows of one element (40 segments of 9 lines, 2 words each).
-constexpr int LAYER_STAGE_BYTES = 4096;
+constexpr int LAYER_STAGE_BYTES = 1024;  // segment table of a fetch that has no second tile (at most 40 entries)
 
 template <int NT>
 constexpr size_t layer_geom_smem_bytes()
@@ -746,9 +813,8 @@ __global__ void __launch_bounds__(NT, DIV_TILES_PER_SM) a21_layer_kernel(LayerGr
   const LayerThread a = layer_thread<NT>(g, tile);
   const int64_t e0 = (int64_t)tile * g.E, e1 = min(e0 + g.E, (int64_t)g.nel);
   prefetch_k<double, DN>(D, 0, e0, e1);
-  layer_fetch<double, NT>(ut, ut + L::TILE, g, tile, u, mbits);
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
+  const LayerLines ll = layer_fetch<double, NT>(ut, ut + L::TILE, g, tile, u);
+  layer_land<double, NT>(ut, g, ll, mbits);
   const double *De = D + delem(a.e);
   double Y[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1

@@ -10,10 +10,10 @@
 //   element's 27 node values.
 //
 // Deterministic without atomics: markers are sorted by element (stable radix
-// sort, so each element keeps its markers in input order), one warp sums an
-// element's markers into per-element node partials (lane = node), and a
-// per-node gather adds the (<= 8) element partials in a fixed order.  Node
-// arrays are indexed compactly over the element box's own nodes.
+// sort, so each element keeps its markers in input order), eight lanes sum an
+// element's markers (lane = vertex), and a per-node gather adds the (<= 8)
+// element sums in a fixed order.  Node arrays are indexed compactly over the
+// element box's own nodes.
 #pragma once
 
 #include <cstdint>
@@ -29,9 +29,6 @@ __device__ __forceinline__ double mk_q1(int v, double x, double y, double z)
   const double c = (v & 4) ? 1.0 + z : 1.0 - z;
   return 0.125 * a * b * c;
 }
-
-// Q2 node of vertex v
-__device__ __forceinline__ int mk_vertex_node(int v) { return 2 * (v & 1) + 6 * ((v >> 1) & 1) + 18 * (v >> 2); }
 
 // Sort keys and payload: key = element index, with every index outside
 // [0, nel) mapped to nel so that a radix sort over the bits of nel suffices;
@@ -60,56 +57,63 @@ __global__ void mk_starts_kernel(const int32_t *__restrict__ keys, int64_t n, in
   }
 }
 
-// One warp per element, lane i < 27 = node i: part[(e*27 + i)*3 + {0,1,2}] =
-// sums over the element's markers of (N_i eta, N_i rho, N_i).  The warp reads
-// up to 32 markers at a time (one per lane) and broadcasts them, so the sum
-// over markers runs in marker order without a chain of dependent loads.
+// Sums over an element's markers, 27 values: (N eta, N rho, N) for its 8
+// vertices and, once for the other 19 nodes whose weight is 1, (eta, rho, 1).
+// Eight lanes per element, lane v = vertex v, four elements per warp; every
+// lane walks the element's markers in order (the eight read the same address),
+// MK_AHEAD of them loaded before they are used.  A warp per element with one
+// lane per node kept 81 sums per element, 19 times the same ones, and moved
+// every marker through ten shuffles: 64^3 with 2.1 M markers 186 us.
+constexpr int MK_SUMS = 27;
+constexpr int MK_AHEAD = 4;
+
 __global__ void __launch_bounds__(128) mk_element_kernel(int64_t nel, const int64_t *__restrict__ start,
                                                          const int32_t *__restrict__ order,
                                                          const double *__restrict__ xi, const double *__restrict__ eta,
                                                          const double *__restrict__ rho, double *__restrict__ part)
 {
-  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (e >= nel) return;  // whole warp
-  // lane's vertex (or -1): nodes 0,2,6,8,18,20,24,26 are vertices 0..7
-  const int c = lane % 3, b = (lane / 3) % 3, a = lane / 9;
-  const int v = (lane < 27 && c != 1 && b != 1 && a != 1) ? (c >> 1) + 2 * (b >> 1) + 4 * (a >> 1) : -1;
-  double s1 = 0.0, s2 = 0.0, sb = 0.0;
+  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int v = threadIdx.x & 7;
+  if (e >= nel) return;
+  double s1 = 0.0, s2 = 0.0, sb = 0.0, c1 = 0.0, c2 = 0.0;
   const int64_t m0 = start[e], m1 = start[e + 1];
-  for (int64_t c0 = m0; c0 < m1; c0 += 32) {
-    const int cnt = (int)min((int64_t)32, m1 - c0);
-    double x0 = 0.0, x1 = 0.0, x2 = 0.0, ee = 0.0, rr = 0.0;
-    if (lane < cnt) {
-      const int64_t p = order[c0 + lane];
-      x0 = xi[3 * p];
-      x1 = xi[3 * p + 1];
-      x2 = xi[3 * p + 2];
-      ee = eta[p];
-      rr = rho[p];
-    }
-    for (int k = 0; k < cnt; k++) {
-      const double y0 = __shfl_sync(0xffffffffu, x0, k), y1 = __shfl_sync(0xffffffffu, x1, k);
-      const double y2 = __shfl_sync(0xffffffffu, x2, k), ek = __shfl_sync(0xffffffffu, ee, k);
-      const double rk = __shfl_sync(0xffffffffu, rr, k);
-      const double N = v >= 0 ? mk_q1(v, y0, y1, y2) : 1.0;
-      s1 += N * ek;
-      s2 += N * rk;
-      sb += N;
-    }
+  for (int64_t c0 = m0; c0 < m1; c0 += MK_AHEAD) {
+    double x[MK_AHEAD], y[MK_AHEAD], z[MK_AHEAD], ee[MK_AHEAD], rr[MK_AHEAD];
+#pragma unroll
+    for (int k = 0; k < MK_AHEAD; k++)
+      if (c0 + k < m1) {
+        const int64_t p = order[c0 + k];
+        x[k] = xi[3 * p];
+        y[k] = xi[3 * p + 1];
+        z[k] = xi[3 * p + 2];
+        ee[k] = eta[p];
+        rr[k] = rho[p];
+      }
+#pragma unroll
+    for (int k = 0; k < MK_AHEAD; k++)
+      if (c0 + k < m1) {
+        const double N = mk_q1(v, x[k], y[k], z[k]);
+        s1 += N * ee[k];
+        s2 += N * rr[k];
+        sb += N;
+        c1 += ee[k];
+        c2 += rr[k];
+      }
   }
-  if (lane < 27) {
-    double *o = part + (e * 27 + lane) * 3;
-    o[0] = s1;
-    o[1] = s2;
-    o[2] = sb;
+  double *o = part + e * MK_SUMS;
+  o[3 * v] = s1;
+  o[3 * v + 1] = s2;
+  o[3 * v + 2] = sb;
+  if (v == 0) {
+    o[24] = c1;
+    o[25] = c2;
+    o[26] = (double)(m1 - m0);
   }
 }
 
 // Per node of the element box (compact index i + j X + k X Y, X = 2mx+1):
-// add the element partials in a fixed order, divide.
-__global__ void mk_node_kernel(int mx, int my, int mz, const double *__restrict__ part, double *__restrict__ v1,
-                               double *__restrict__ v2)
+// the element sums in a fixed order, divided; (viscosity, density) side by side.
+__global__ void mk_node_kernel(int mx, int my, int mz, const double *__restrict__ part, double2 *__restrict__ v12)
 {
   // node count < 2^31 (checked by the caller): 32-bit index arithmetic
   const unsigned X = 2 * mx + 1, Y = 2 * my + 1;
@@ -117,84 +121,101 @@ __global__ void mk_node_kernel(int mx, int my, int mz, const double *__restrict_
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < nn; t += gridDim.x * blockDim.x) {
     const unsigned txy = t / X;
     const int i = (int)(t - txy * X), j = (int)(txy % Y), k = (int)(txy / Y);
-    int ex[2], lx[2], nx = 0, ey[2], ly[2], ny = 0, ez[2], lz[2], nz = 0;
-    if (i & 1) { ex[0] = i >> 1; lx[0] = 1; nx = 1; }
-    else {
-      if (i > 0) { ex[nx] = (i >> 1) - 1; lx[nx++] = 2; }
-      if ((i >> 1) < mx) { ex[nx] = i >> 1; lx[nx++] = 0; }
-    }
-    if (j & 1) { ey[0] = j >> 1; ly[0] = 1; ny = 1; }
-    else {
-      if (j > 0) { ey[ny] = (j >> 1) - 1; ly[ny++] = 2; }
-      if ((j >> 1) < my) { ey[ny] = j >> 1; ly[ny++] = 0; }
-    }
-    if (k & 1) { ez[0] = k >> 1; lz[0] = 1; nz = 1; }
-    else {
-      if (k > 0) { ez[nz] = (k >> 1) - 1; lz[nz++] = 2; }
-      if ((k >> 1) < mz) { ez[nz] = k >> 1; lz[nz++] = 0; }
-    }
+    const bool vertex = !((i | j | k) & 1);
     double a1 = 0.0, a2 = 0.0, b = 0.0;
-    for (int cz = 0; cz < nz; cz++)
-      for (int cy = 0; cy < ny; cy++)
-        for (int cx = 0; cx < nx; cx++) {
-          const int64_t e = ex[cx] + (int64_t)mx * (ey[cy] + (int64_t)my * ez[cz]);
-          const double *o = part + (e * 27 + lx[cx] + 3 * ly[cy] + 9 * lz[cz]) * 3;
+#pragma unroll
+    for (int cz = 0; cz < 2; cz++)
+#pragma unroll
+      for (int cy = 0; cy < 2; cy++)
+#pragma unroll
+        for (int cx = 0; cx < 2; cx++) {
+          // elements i/2 - 1 and i/2 of an even node, i/2 of an odd one
+          const int ex = (i >> 1) - 1 + cx, ey = (j >> 1) - 1 + cy, ez = (k >> 1) - 1 + cz;
+          if ((cx == 0 && (i & 1)) || (cy == 0 && (j & 1)) || (cz == 0 && (k & 1))) continue;
+          if (ex < 0 || ey < 0 || ez < 0 || ex >= mx || ey >= my || ez >= mz) continue;
+          const int64_t e = ex + (int64_t)mx * (ey + (int64_t)my * ez);
+          // this node within the element: its high vertex where the element is the lower one
+          const int w = vertex ? (1 - cx) + 2 * (1 - cy) + 4 * (1 - cz) : 8;
+          const double *o = part + e * MK_SUMS + 3 * w;
           a1 += o[0];
           a2 += o[1];
           b += o[2];
         }
-    v1[t] = a1 / b;
-    v2[t] = a2 / b;
+    v12[t] = make_double2(a1 / b, a2 / b);
   }
 }
 
 // Gauss point q of element e: Q1 interpolant of the vertex values, clamped to
-// the element's 27 node values.  One warp per element: lane n < 27 reads node
-// n once, the range is a warp reduction, the vertex values are broadcast, and
-// lane q writes Gauss point q.  Abscissae of QuadratureCreateGauss_3pnt_3D
-// (src/quadrature.c:136-167).
-__global__ void __launch_bounds__(128) mk_qp_kernel(int mx, int my, int mz, const double *__restrict__ v1,
-                                                    const double *__restrict__ v2, double *__restrict__ eta_qp,
-                                                    double *__restrict__ rho_qp)
+// the element's 27 node values, abscissae of QuadratureCreateGauss_3pnt_3D
+// (src/quadrature.c:136-167).  One thread per element: the interpolant is
+// formed axis by axis (a warp per element paid 72 shuffles for the range and
+// the vertices: 64^3 122 us), and a block's points, which lie side by side in
+// the result, leave through shared memory in whole lines.  eta2: a second copy
+// of the viscosity, or null.
+constexpr int MK_QP_THREADS = 128;
+
+__global__ void __launch_bounds__(MK_QP_THREADS) mk_qp_kernel(int mx, int my, int mz, const double2 *__restrict__ v12,
+                                                              double *__restrict__ eta_qp, double *__restrict__ eta2,
+                                                              double *__restrict__ rho_qp)
 {
+  __shared__ double sh[27 * MK_QP_THREADS];
   // element count < 2^31 (checked by the caller): 32-bit index arithmetic
   const unsigned nel = (unsigned)mx * my * mz;
-  const unsigned e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (e >= nel) return;  // whole warp
-  const int X = 2 * mx + 1, Y = 2 * my + 1;
-  const unsigned exy = e / mx;
-  const int ei = (int)(e - exy * mx), ej = (int)(exy % my), ek = (int)(exy / my);
-  const int64_t base = 2 * (int64_t)ei + 2 * (int64_t)ej * X + 2 * (int64_t)ek * X * Y;
-  // lanes 27..31 read node 0 again, so the range reduction needs no sentinel
-  const int n = lane < 27 ? lane : 0;
-  const int64_t nd = base + (n % 3) + ((n / 3) % 3) * (int64_t)X + (n / 9) * (int64_t)X * Y;
-  const double a = v1[nd], b = v2[nd];
-  double lo1 = a, hi1 = a, lo2 = b, hi2 = b;
+  const unsigned e0 = blockIdx.x * MK_QP_THREADS, e = e0 + threadIdx.x;
+  const unsigned n = min((unsigned)MK_QP_THREADS, nel - e0);
+  double lo[2], hi[2], vx[2][8];
+  if (e < nel) {
+    const int X = 2 * mx + 1, Y = 2 * my + 1;
+    const unsigned exy = e / mx;
+    const int ei = (int)(e - exy * mx), ej = (int)(exy % my), ek = (int)(exy / my);
+    const double2 *base = v12 + 2 * (int64_t)ei + 2 * (int64_t)ej * X + 2 * (int64_t)ek * X * Y;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    lo1 = fmin(lo1, __shfl_xor_sync(0xffffffffu, lo1, o));
-    hi1 = fmax(hi1, __shfl_xor_sync(0xffffffffu, hi1, o));
-    lo2 = fmin(lo2, __shfl_xor_sync(0xffffffffu, lo2, o));
-    hi2 = fmax(hi2, __shfl_xor_sync(0xffffffffu, hi2, o));
+    for (int m = 0; m < 27; m++) {
+      const double2 a = base[(m % 3) + ((m / 3) % 3) * (int64_t)X + (m / 9) * (int64_t)X * Y];
+      lo[0] = m == 0 ? a.x : fmin(lo[0], a.x);
+      hi[0] = m == 0 ? a.x : fmax(hi[0], a.x);
+      lo[1] = m == 0 ? a.y : fmin(lo[1], a.y);
+      hi[1] = m == 0 ? a.y : fmax(hi[1], a.y);
+      if (m % 3 != 1 && m / 3 % 3 != 1 && m / 9 != 1) {
+        const int v = (m % 3) / 2 + (m / 3 % 3) + 2 * (m / 9);
+        vx[0][v] = a.x;
+        vx[1][v] = a.y;
+      }
+    }
   }
-  const double g[3] = {-0.774596669241483, 0.0, 0.774596669241483};
-  const double x = g[n % 3], y = g[(n / 3) % 3], z = g[n / 9];
-  double s1 = 0.0, s2 = 0.0;
+  const double g = 0.774596669241483;
+  const double w0[3] = {0.5 * (1.0 + g), 0.5, 0.5 * (1.0 - g)};  // weight of the lower node; the upper one's mirrored
 #pragma unroll
-  for (int v = 0; v < 8; v++) {
-    const int vn = mk_vertex_node(v);
-    const double N = mk_q1(v, x, y, z);
-    s1 += N * __shfl_sync(0xffffffffu, a, vn);
-    s2 += N * __shfl_sync(0xffffffffu, b, vn);
+  for (int f = 0; f < 2; f++) {
+    double *const out = f == 0 ? eta_qp : rho_qp;
+    if (f == 1 && !out) break;
+    if (e < nel) {
+      double a[3][4];  // along x
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int yz = 0; yz < 4; yz++) a[c][yz] = w0[c] * vx[f][2 * yz] + w0[2 - c] * vx[f][2 * yz + 1];
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double b0 = w0[b] * a[c][0] + w0[2 - b] * a[c][1], b1 = w0[b] * a[c][2] + w0[2 - b] * a[c][3];
+#pragma unroll
+          for (int d = 0; d < 3; d++) {
+            double s = w0[d] * b0 + w0[2 - d] * b1;
+            if (s < lo[f]) s = lo[f];
+            if (s > hi[f]) s = hi[f];
+            sh[27 * threadIdx.x + 9 * d + 3 * b + c] = s;
+          }
+        }
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < 27 * n; i += MK_QP_THREADS) {
+      if (out) out[27 * (int64_t)e0 + i] = sh[i];
+      if (f == 0 && eta2) eta2[27 * (int64_t)e0 + i] = sh[i];
+    }
+    __syncthreads();
   }
-  if (lane >= 27) return;
-  if (s1 < lo1) s1 = lo1;
-  if (s1 > hi1) s1 = hi1;
-  if (s2 < lo2) s2 = lo2;
-  if (s2 > hi2) s2 = hi2;
-  if (eta_qp) eta_qp[27 * (int64_t)e + lane] = s1;
-  if (rho_qp) rho_qp[27 * (int64_t)e + lane] = s2;
 }
 
 }  // namespace ptk

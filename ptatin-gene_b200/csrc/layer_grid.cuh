@@ -83,8 +83,8 @@ inline int layer_segments(int E, int mx)
 
 // Elements per tile: NT where their segments fit the 8 end entries beside NT
 // even and odd ones (rows of 21 elements and more, and of 16), else 7/8 of NT
-// (40 end entries with NT = 128), fewer only for rows of one or two elements;
-// then whole warps fewer while there are not enough tiles for every SM.
+// (40 end entries with NT = 128), fewer only for rows of one or two elements.
+// The shape depends on the box alone, so its sums are the same in any batch.
 template <int NT>
 inline LayerGrid layer_grid(int mx, int my, int mz, int64_t X, int64_t XY, int64_t off)
 {
@@ -96,11 +96,6 @@ inline LayerGrid layer_grid(int mx, int my, int mz, int64_t X, int64_t XY, int64
   const int ends = LayerLayout<NT>::ROW - 2 * g.odd;
   g.E = g.odd;
   while (layer_segments(g.E, mx) > ends) g.E--;
-  while (g.E > 32 && (g.nel + g.E - 1) / g.E < 148) {
-    const int E = (g.E - 1) / 32 * 32;
-    if (layer_segments(E, mx) > ends) break;
-    g.E = E;
-  }
   g.tiles = (g.nel + g.E - 1) / g.E;
   g.dNX = fast_div(2 * mx + 1);
   g.dNY = fast_div(2 * my + 1);

@@ -1515,8 +1515,7 @@ pt_status pt_project_markers_d(pt_op *op, int64_t n, const int32_t *wil, const d
   int bits = 1;
   while (bits < 31 && (int64_t(1) << bits) <= nel) bits++;
   // scratch (op-owned, grown on demand and reused): keys in and sorted, marker
-  // indices in and sorted, starts, element partials, node values, qp outputs
-  // when the caller passes none, sort workspace
+  // indices in and sorted, starts, element sums, node values, sort workspace
   const int64_t nm = n > 0 ? n : 1;
   size_t tmp_bytes = 0;
   cudaError_t e = cudaSuccess;
@@ -1525,9 +1524,10 @@ pt_status pt_project_markers_d(pt_op *op, int64_t n, const int32_t *wil, const d
                                         (const int32_t *)nullptr, (int32_t *)nullptr, (int)n, 0, bits, st);
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "marker projection: %s", cudaGetErrorString(e));
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t sz[9] = {up(4 * nm),         up(4 * nm),     up(4 * nm),
-                        up(8 * (nel + 1)),   up(8 * 81 * nel), up(8 * 2 * nn),
-                        eta_qp ? 0 : up(8 * 27 * nel), up(tmp_bytes), up(4 * nm)};
+  const size_t sz[8] = {up(4 * nm),        up(4 * nm),
+                        up(4 * nm),        up(8 * (nel + 1)),
+                        up(8 * ptk::MK_SUMS * nel), up(16 * nn),
+                        up(tmp_bytes),     up(4 * nm)};
   size_t total = 0;
   for (size_t b : sz) total += b;
   if (total > op->mk_bytes) {
@@ -1538,17 +1538,17 @@ pt_status pt_project_markers_d(pt_op *op, int64_t n, const int32_t *wil, const d
     op->mk_bytes = total;
   }
   char *cur = (char *)op->mk_scratch;
-  void *ptrs[9];
-  for (int i = 0; i < 9; i++) {
+  void *ptrs[8];
+  for (int i = 0; i < 8; i++) {
     ptrs[i] = sz[i] ? cur : nullptr;
     cur += sz[i];
   }
   int32_t *keys = (int32_t *)ptrs[0], *iota = (int32_t *)ptrs[1], *order = (int32_t *)ptrs[2];
   int64_t *start = (int64_t *)ptrs[3];
-  double *part = (double *)ptrs[4], *v1 = (double *)ptrs[5];
-  double *eq = eta_qp ? eta_qp : (double *)ptrs[6], *rq = rho_qp;
-  void *tmp = ptrs[7];
-  int32_t *kin = (int32_t *)ptrs[8];
+  double *part = (double *)ptrs[4];
+  double2 *v12 = (double2 *)ptrs[5];
+  void *tmp = ptrs[6];
+  int32_t *kin = (int32_t *)ptrs[7];
   pt_status s = PT_OK;
   if (e == cudaSuccess) {
     if (n > 0) {
@@ -1557,9 +1557,11 @@ pt_status pt_project_markers_d(pt_op *op, int64_t n, const int32_t *wil, const d
     }
     if (e == cudaSuccess) {
       ptk::mk_starts_kernel<<<grid_stride_blocks(nel + 1), 256, 0, st>>>(keys, n, nel, start);
-      ptk::mk_element_kernel<<<nblocks(32 * nel), TPB, 0, st>>>(nel, start, order, xi, eta, rho, part);
-      ptk::mk_node_kernel<<<grid_stride_blocks(nn), 256, 0, st>>>(op->mx, op->my, op->mz, part, v1, v1 + nn);
-      ptk::mk_qp_kernel<<<nblocks(32 * nel), TPB, 0, st>>>(op->mx, op->my, op->mz, v1, v1 + nn, eq, rq);
+      ptk::mk_element_kernel<<<nblocks(8 * nel), TPB, 0, st>>>(nel, start, order, xi, eta, rho, part);
+      ptk::mk_node_kernel<<<grid_stride_blocks(nn), 256, 0, st>>>(op->mx, op->my, op->mz, part, v12);
+      // installed: written to the op's viscosity in the same pass
+      ptk::mk_qp_kernel<<<nblocks(nel, ptk::MK_QP_THREADS), ptk::MK_QP_THREADS, 0, st>>>(
+          op->mx, op->my, op->mz, v12, eta_qp, install ? op->d_eta : nullptr, rho_qp);
       e = cudaGetLastError();
       op->launches += 4 + (n > 0 ? 2 : 0);
     }
@@ -1567,7 +1569,7 @@ pt_status pt_project_markers_d(pt_op *op, int64_t n, const int32_t *wil, const d
     // projected: report them
     int64_t inside = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&inside, start + nel, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess && install) s = pt_op_set_eta_d(op, eq);
+    if (e == cudaSuccess && install) s = finish_eta(op);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess && s == PT_OK && inside != n)
       s = fail(PT_ERR_BAD_ARG, "%lld markers have an element index outside [0, %lld)", (long long)(n - inside),

@@ -179,3 +179,32 @@ def test_whole_operator_on_a_ghosted_box_is_the_sum_of_its_blocks():
         ref = torch.where(bc, u, op.MatMult_MFStokes_A11(u) + op.MFStokesWrapper_A12(p))
         assert float((yu - ref).abs().max()) < 1e-13 * float(ref.abs().max())
         assert torch.equal(yu[bc], u[bc])
+
+
+@pytest.mark.parametrize("dims,counts", [((1, 1, 1), (3, 3)), ((2, 1, 3), (1, 1)), ((33, 5, 2), (1, 9)), ((129, 1, 2), (2, 5))])
+def test_marker_projection_with_uneven_counts_matches_oracle(ora, dims, counts):
+    """Elements of different marker counts (around the loop's load-ahead), a last
+    block that is not full, viscosity only or density too, installed or not."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, eta, _ = M.problem("box:%d,%d,%d" % dims, seed=3)
+    rng = np.random.default_rng(4)
+    wil = np.repeat(np.arange(m.nel, dtype=np.int32), rng.integers(counts[0], counts[1] + 1, size=m.nel))
+    wil = rng.permutation(wil).astype(np.int32)
+    xi = rng.uniform(-1, 1, size=(len(wil), 3))
+    e, r = 10.0 ** rng.uniform(-3, 3, size=len(wil)), rng.uniform(1, 2, size=len(wil))
+    ref_e, ref_r = ora.marker_project(m.dims, wil, xi, e, r)
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    u = M.uniform_vec(m.nvel, 5)
+    with MatStokesMF(*m.dims) as op:
+        op.SetUp(m.coords, eta)
+        before = op.MFStokesWrapper_A11(u)
+        for install in (False, True):
+            eq, rq = op.ProjectMarkers(t(wil), t(xi), t(e), t(r), install=install)
+            assert relerr(eq.cpu().numpy(), ref_e) < TOL64 and relerr(rq.cpu().numpy(), ref_r) < TOL64
+            y = op.MFStokesWrapper_A11(u)
+            if not install:
+                assert np.array_equal(y, before)
+            else:
+                assert relerr(y, ora.a11(m.dims, m.coords, ref_e, u)) < TOL64
