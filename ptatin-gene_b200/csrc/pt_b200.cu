@@ -67,14 +67,17 @@ enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 
 // "b200" picks stored element matrices for one-rank boxes of up to
 // EBE_AUTO_MAX_ELEMENTS (FP64 / FP32 apply, matrices vs layer tiles: 10^3
-// 15.0 / 12.1 vs 21.0 / 20.9 us, 12^3 19.0 / 14.3 vs 20.9 / 20.4 us, 16^3
-// 36.5 / 19.8 vs 22.2 / 20.9 us); layer tiles above; and the streaming kernel
-// for boxes from STREAM_AUTO_MIN_ELEMENTS whose rows nearly fill its tiles
-// (layer tiles vs streaming: 56^3 162 / 115 vs 187 / 165 us, 64^3 216 / 153 vs
-// 205 / 181 us, 128x128x64 775 / 549 vs 731 / 493 us; rows that leave threads
-// idle: 80^3 417 / 301 vs 515 / 366 us, 97x70x81 440 / 313 vs 533 / 338 us).
+// 15.0 / 12.1 vs 25 / 23 us, 13^3 21.0 / 15.3 vs 23.6 / 23.0 us, 16^3 36.5 /
+// 19.8 vs 25.0 / 24.9 us); layer tiles above; and, in FP64, the streaming
+// kernel for boxes from STREAM_AUTO_MIN_ELEMENTS whose rows nearly fill its
+// tiles (layer tiles vs streaming: 56^3 162 vs 187 us, 80^3 398 vs 515 us,
+// 96^3 619 vs 738 us; 64^3 198 vs 205 us, 128^3 1365 vs 1427 us applied again
+// and again to one box but 1560 vs 1511 us taking turns among three).  Such a
+// box's FP32 applies use layer tiles below LAYER_F32_MAX_ELEMENTS (64^3 142 vs
+// 175 us, 128x32x64 140 vs 172 us; 128^3 1025 vs 1014 us).
 constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
 constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
+constexpr int64_t LAYER_F32_MAX_ELEMENTS = 1000000;
 // layer tiles: node numbers stay below 2^31, scratch (460 B per element) below 4 GB
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
 // every box: element-node numbers stay below 2^31
@@ -108,6 +111,7 @@ struct pt_op {
   double *d_D;    // factors of B and B^T at the Gauss points (built on first use)
   double *d_P;    // factors of the whole Stokes operator beyond K (from its first use, with K)
   int a11_kernel;
+  bool a11_auto;  // chosen by auto_kernel ("b200"), not by name
   int64_t launches;
   uint64_t state;  // bumped whenever coordinates, viscosity or the mask change
   int device;
@@ -494,7 +498,7 @@ pt_status ensure_geometry(pt_op *op)
     PT_CUDA(op_alloc(op, (void **)&op->d_K32, sizeof(float) * nk));
     PT_CUDA(op_alloc(op, (void **)&op->d_bad, sizeof(unsigned int)));
   }
-  if (op->a11_kernel == A11_LAYER) {
+  if (op->a11_kernel == A11_LAYER || (op->a11_kernel == A11_STREAM && op->a11_auto && op->nel < LAYER_F32_MAX_ELEMENTS)) {
     pt_status s = ensure_layer(op);
     if (s != PT_OK) return s;
   }
@@ -599,7 +603,7 @@ pt_status launch_a11(pt_op *op, const T *coords, const T *eta, const T *u, T *y,
     if (s != PT_OK) return s;
     if (op->geom_ok) {
       if (!op->full_box) PT_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * op->nvel, op->stream));
-      if (op->a11_kernel == A11_LAYER) {
+      if (op->a11_kernel == A11_LAYER || (sizeof(T) == 4 && op->a11_auto && op->nel < LAYER_F32_MAX_ELEMENTS)) {
         if ((s = launch_layer<T>(op, op_K<T>(op), u, y, masked)) != PT_OK) return s;
         // a ghosted box's Dirichlet dofs outside the element box
         if (masked && !op->full_box) {
@@ -980,6 +984,7 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   op->TX = desc->mx <= 32 ? 32 : (desc->mx <= 64 ? 64 : 128);
   op->ntx = (desc->mx + op->TX - 1) / op->TX;
   op->a11_kernel = auto_kernel(op);
+  op->a11_auto = true;
   op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
   pt_op_set_tiling(op, 0);
   op->geom_dirty = true;
@@ -1616,7 +1621,8 @@ pt_status pt_project_markers_h(pt_op *op, int64_t n, const int32_t *wil, const d
 pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
 {
   if (!op || !name) return fail(PT_ERR_BAD_ARG, "NULL argument");
-  if (!strcmp(name, "b200")) op->a11_kernel = auto_kernel(op);
+  const bool by_name = strcmp(name, "b200") != 0;
+  if (!by_name) op->a11_kernel = auto_kernel(op);
   else if (!strcmp(name, "b200_stream")) op->a11_kernel = A11_STREAM;
   else if (!strcmp(name, "b200_ebe")) op->a11_kernel = A11_EBE;
   else if (!strcmp(name, "b200_layer")) {
@@ -1626,6 +1632,7 @@ pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
   }
   else if (!strcmp(name, "b200_colour")) op->a11_kernel = A11_COLOUR;
   else return fail(PT_ERR_BAD_ARG, "No -a11_op %s", name);
+  op->a11_auto = !by_name;
   return PT_OK;
 }
 

@@ -228,6 +228,7 @@ struct pt_solver {
   pt_mg *mg;
   bool setup_done;
   uint64_t op_state;  // op->state the set-up was made for
+  cudaMemPool_t pool; // the hierarchy's memory
 };
 
 namespace {
@@ -362,15 +363,54 @@ pt_status sv_estimate_lambda(pt_solver *s) { return sv_lanczos(s, s->op, s->n, s
 
 // ---- multigrid set-up -------------------------------------------------------
 
-void mg_free(pt_mg *mg)
+// The hierarchy lives in a pool of the solver's: a Picard step rebuilds it for
+// every new viscosity, and 66 cudaMalloc and 78 cudaFree per rebuild (each a
+// device-wide wait) were 15 to 60 ms of a 65 ms solve at 40^3.  What is freed
+// stays in the pool for the next rebuild up to MG_POOL_KEEP bytes (a 64^3
+// hierarchy's FP64 Galerkin matrices are 7 GB: not kept), and all of it goes
+// back with the solver.
+constexpr uint64_t MG_POOL_KEEP = (uint64_t)1 << 30;
+
+pt_status mg_pool(pt_solver *s)
 {
+  if (s->pool) return PT_OK;
+  cudaMemPoolProps pp{};
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = s->op->device;
+  PT_CUDA(cudaMemPoolCreate(&s->pool, &pp));
+  uint64_t keep = MG_POOL_KEEP;
+  PT_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  return PT_OK;
+}
+
+template <typename T>
+cudaError_t mg_alloc(pt_solver *s, T **p, size_t bytes)
+{
+  return cudaMallocFromPoolAsync((void **)p, bytes, s->pool, s->op->stream);
+}
+
+void mg_release(pt_solver *s, void *p)
+{
+  if (p) cudaFreeAsync(p, s->op->stream);
+}
+
+// Gives the hierarchy back to the pool behind the work queued on `st`.
+void mg_free(pt_solver *s, cudaStream_t st)
+{
+  pt_mg *mg = s->mg;
+  s->mg = nullptr;
   if (!mg) return;
   if (mg->gexec) cudaGraphExecDestroy(mg->gexec);
   for (pt_mg_level &L : mg->lv) {
     void *p[] = {L.dinv64, L.dinv32, L.x, L.b, L.r, L.d, L.az, L.dl, L.t1, L.Ae, L.ye, L.Ainv, L.Ah, L.Ascale};
-    for (void *q : p) cudaFree(q);
-    if (L.Ae64 && (void *)L.Ae64 != L.Ae) cudaFree(L.Ae64);
-    if (L.own && L.op) pt_op_destroy(L.op);
+    for (void *q : p)
+      if (q) cudaFreeAsync(q, st);
+    if (L.Ae64 && (void *)L.Ae64 != L.Ae) cudaFreeAsync(L.Ae64, st);
+    if (L.own && L.op) {
+      L.op->stream = st;
+      pt_op_destroy(L.op);
+    }
   }
   delete mg;
 }
@@ -378,15 +418,14 @@ void mg_free(pt_mg *mg)
 // Coarse level of level f: half the elements per axis, coordinates and
 // Dirichlet mask injected; vf_c (the coarse vertex viscosity) restricted from
 // vf_f and interpolated to the coarse Gauss points.
-pt_status mg_coarsen(const pt_op *f, const double *vf_f, double *vf_c, pt_op **out)
+pt_status mg_coarsen(pt_solver *s, const pt_op *f, const double *vf_f, double *vf_c, pt_op **out)
 {
   pt_mesh_desc d{};
   d.mx = f->mx / 2; d.my = f->my / 2; d.mz = f->mz / 2;
   pt_op *c = nullptr;
-  pt_status st = pt_op_create(&d, &c);
+  pt_status st = op_create_impl(&d, s->pool, f->stream, &c);
   if (st != PT_OK) return st;
   *out = c;  // the caller owns it from here on
-  if ((st = pt_op_set_stream(c, (void *)f->stream)) != PT_OK) return st;
   // small levels keep their own element matrices (mg_level_setup)
   if (f->a11_kernel == A11_COLOUR) c->a11_kernel = A11_COLOUR;
   else if (c->a11_kernel == A11_EBE) c->a11_kernel = A11_LAYER;
@@ -412,13 +451,13 @@ constexpr int64_t MG_DENSE_MAX_DOFS = 1200;     // coarsest level solved by a de
 // Dense inverse of the coarsest level's masked operator (Dirichlet rows and
 // columns replaced by the identity), from its FP64 element matrices:
 // assembled on the host, Cholesky-factored, inverted, uploaded as T.
-pt_status mg_dense_inverse(pt_mg_level &L, bool fp32)
+pt_status mg_dense_inverse(pt_solver *s, pt_mg_level &L, bool fp32)
 {
   const pt_op *op = L.op;
   const int64_t n = L.n, nel = op->nel;
   double *dAe = L.Ae64;  // Galerkin level: its own matrices; else re-discretised ones
   if (!dAe) {
-    PT_CUDA(cudaMalloc(&dAe, sizeof(double) * ptk::EBE_LD * nel));
+    PT_CUDA(mg_alloc(s, &dAe, sizeof(double) * ptk::EBE_LD * nel));
     ptk::element_matrix_kernel<double><<<(unsigned)nel, 96, 0, op->stream>>>(op->box, op->d_coords, op->d_eta, dAe);
   }
   std::vector<double> Ae(ptk::EBE_LD * nel), A(n * n, 0.0);
@@ -427,7 +466,7 @@ pt_status mg_dense_inverse(pt_mg_level &L, bool fp32)
   if (e == cudaSuccess) e = cudaMemcpyAsync(Ae.data(), dAe, sizeof(double) * Ae.size(), cudaMemcpyDeviceToHost, op->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(mask.data(), op->d_mask, n, cudaMemcpyDeviceToHost, op->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(op->stream);
-  if (dAe != L.Ae64) cudaFree(dAe);
+  if (dAe != L.Ae64) mg_release(s, dAe);
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "coarse element matrices: %s", cudaGetErrorString(e));
   const int64_t X = op->box.X, XY = op->box.XY;
   for (int64_t el = 0; el < nel; el++) {
@@ -476,12 +515,14 @@ pt_status mg_dense_inverse(pt_mg_level &L, bool fp32)
       inv[i * n + j] = inv[j * n + i] = v;
     }
   const size_t ts = fp32 ? sizeof(float) : sizeof(double);
-  PT_CUDA(cudaMalloc(&L.Ainv, ts * n * n));
+  PT_CUDA(mg_alloc(s, &L.Ainv, ts * n * n));
   if (fp32) {
     std::vector<float> f(inv.begin(), inv.end());
-    PT_CUDA(cudaMemcpy(L.Ainv, f.data(), ts * n * n, cudaMemcpyHostToDevice));
+    PT_CUDA(cudaMemcpyAsync(L.Ainv, f.data(), ts * n * n, cudaMemcpyHostToDevice, op->stream));
+    PT_CUDA(cudaStreamSynchronize(op->stream));
   } else {
-    PT_CUDA(cudaMemcpy(L.Ainv, inv.data(), ts * n * n, cudaMemcpyHostToDevice));
+    PT_CUDA(cudaMemcpyAsync(L.Ainv, inv.data(), ts * n * n, cudaMemcpyHostToDevice, op->stream));
+    PT_CUDA(cudaStreamSynchronize(op->stream));
   }
   return PT_OK;
 }
@@ -493,19 +534,19 @@ pt_status mg_level_setup(pt_solver *s, pt_mg &mg, pt_mg_level &L, const pt_op *n
   const size_t ts = mg.fp32 ? sizeof(float) : sizeof(double);
   L.n = L.op->nvel;
   L.nel = L.op->nel;
-  PT_CUDA(cudaMalloc(&L.dinv64, sizeof(double) * L.n));
-  PT_CUDA(cudaMalloc(&L.dinv32, sizeof(float) * L.n));
+  PT_CUDA(mg_alloc(s, &L.dinv64, sizeof(double) * L.n));
+  PT_CUDA(mg_alloc(s, &L.dinv32, sizeof(float) * L.n));
   void **vecs[] = {&L.x, &L.b, &L.r, &L.d, &L.az, &L.dl};
-  for (void **v : vecs) PT_CUDA(cudaMalloc(v, ts * L.n));
+  for (void **v : vecs) PT_CUDA(mg_alloc(s, v, ts * L.n));
   if (next) {  // transfer temporaries: 3 (2mcx+1)(2my+1)(2mz+1) values each
     const int64_t nt = 3LL * (2 * next->mx + 1) * (2 * L.op->my + 1) * (2 * L.op->mz + 1);
-    PT_CUDA(cudaMalloc(&L.t1, 2 * ts * nt));
+    PT_CUDA(mg_alloc(s, &L.t1, 2 * ts * nt));
     L.t2 = (char *)L.t1 + ts * nt;
   }
   pt_status st = PT_OK;
   if (L.Ae64) {
     // Galerkin level: diagonal, lambda_max and applies from its element matrices
-    PT_CUDA(cudaMalloc(&L.ye, sizeof(double) * 81 * L.nel));
+    PT_CUDA(mg_alloc(s, &L.ye, sizeof(double) * 81 * L.nel));
     ptk::ebe_diag_kernel<<<vgrid(L.n), 256, 0, L.op->stream>>>(L.op->box, L.Ae64, s->t1);
     PT_LAUNCHED(L.op);
     if ((st = bc_value(L.op, 1.0, s->t1)) != PT_OK) return st;
@@ -525,14 +566,14 @@ pt_status mg_level_setup(pt_solver *s, pt_mg &mg, pt_mg_level &L, const pt_op *n
       return PT_OK;
     });
     if (st != PT_OK) return st;
-    if (!next && L.n <= MG_DENSE_MAX_DOFS) return mg_dense_inverse(L, mg.fp32);
+    if (!next && L.n <= MG_DENSE_MAX_DOFS) return mg_dense_inverse(s, L, mg.fp32);
     if (mg.fp32 && mg.coarse_half) {
-      PT_CUDA(cudaMalloc(&L.Ah, sizeof(__half) * ptk::EBE_LD * L.nel));
-      PT_CUDA(cudaMalloc(&L.Ascale, sizeof(float) * L.nel));
+      PT_CUDA(mg_alloc(s, &L.Ah, sizeof(__half) * ptk::EBE_LD * L.nel));
+      PT_CUDA(mg_alloc(s, &L.Ascale, sizeof(float) * L.nel));
       ptk::ebe_to_half_kernel<<<(unsigned)L.nel, 128, 0, L.op->stream>>>(L.Ae64, L.Ah, L.Ascale);
       PT_LAUNCHED(L.op);
     } else if (mg.fp32) {
-      PT_CUDA(cudaMalloc(&L.Ae, sizeof(float) * ptk::EBE_LD * L.nel));
+      PT_CUDA(mg_alloc(s, &L.Ae, sizeof(float) * ptk::EBE_LD * L.nel));
       ptk::convert_kernel<float><<<vgrid(ptk::EBE_LD * L.nel), 256, 0, L.op->stream>>>(L.Ae64, (float *)L.Ae,
                                                                                      ptk::EBE_LD * L.nel);
       PT_LAUNCHED(L.op);
@@ -543,10 +584,10 @@ pt_status mg_level_setup(pt_solver *s, pt_mg &mg, pt_mg_level &L, const pt_op *n
   }
   if ((st = sv_lanczos(s, L.op, L.n, L.dinv64, &L.lmax)) != PT_OK) return st;
   if (!mg.assembled) return PT_OK;
-  if (!next && L.n <= MG_DENSE_MAX_DOFS && (st = mg_dense_inverse(L, mg.fp32)) != PT_OK) return st;
+  if (!next && L.n <= MG_DENSE_MAX_DOFS && (st = mg_dense_inverse(s, L, mg.fp32)) != PT_OK) return st;
   if (L.nel <= MG_EBE_MAX_ELEMENTS && !L.Ainv) {
-    PT_CUDA(cudaMalloc(&L.Ae, ts * ptk::EBE_LD * L.nel));
-    PT_CUDA(cudaMalloc(&L.ye, ts * 81 * L.nel));
+    PT_CUDA(mg_alloc(s, &L.Ae, ts * ptk::EBE_LD * L.nel));
+    PT_CUDA(mg_alloc(s, &L.ye, ts * 81 * L.nel));
     if (mg.fp32)
       ptk::element_matrix_kernel<float><<<(unsigned)L.nel, 96, 0, L.op->stream>>>(L.op->box, L.op->d_coords, L.op->d_eta,
                                                                              (float *)L.Ae);
@@ -565,7 +606,7 @@ constexpr int64_t MG_GALERKIN_MAX_ELEMENTS = 262144;  // Galerkin levels up to 6
 // P^T A P from the level above -- from that level's quadrature when it runs
 // matrix-free (the reference's OP_TYPE_MFGALERKIN), from its Galerkin
 // matrices below that (OP_TYPE_GALERKIN).  Levels above stay re-discretised.
-pt_status mg_galerkin(pt_mg &mg)
+pt_status mg_galerkin(pt_solver *s, pt_mg &mg)
 {
   constexpr size_t smem = ptk::galerkin_smem_bytes();
   pt_status as = kernel_attrs((const void *)ptk::galerkin_kernel<true>, smem, false);
@@ -574,7 +615,7 @@ pt_status mg_galerkin(pt_mg &mg)
   for (size_t l = 1; l < mg.lv.size(); l++) {
     pt_mg_level &F = mg.lv[l - 1], &C = mg.lv[l];
     if (!F.Ae64 && C.op->nel > MG_GALERKIN_MAX_ELEMENTS) continue;
-    PT_CUDA(cudaMalloc(&C.Ae64, sizeof(double) * ptk::EBE_LD * C.op->nel));
+    PT_CUDA(mg_alloc(s, &C.Ae64, sizeof(double) * ptk::EBE_LD * C.op->nel));
     ptk::GalerkinArgs a;
     a.fb = F.op->box;
     a.cmx = C.op->mx; a.cmy = C.op->my; a.cmz = C.op->mz;
@@ -593,6 +634,8 @@ pt_status mg_galerkin(pt_mg &mg)
 pt_status mg_build(pt_solver *s)
 {
   if (!s->op->full_box) return fail(PT_ERR_UNSUPPORTED, "multigrid needs a one-rank box (node box = element box)");
+  pt_status ps = mg_pool(s);
+  if (ps != PT_OK) return ps;
   pt_mg *mg = new (std::nothrow) pt_mg();
   if (!mg) return fail(PT_ERR_OOM, "host allocation failed");
   s->mg = mg;  // freed by pt_solver_destroy, also after a failure here
@@ -615,7 +658,7 @@ pt_status mg_build(pt_solver *s)
   const pt_op *op = s->op;
   const int64_t nv0 = (int64_t)(op->mx + 1) * (op->my + 1) * (op->mz + 1);
   double *vf[2] = {nullptr, nullptr};
-  PT_CUDA(cudaMalloc(&vf[0], sizeof(double) * 2 * nv0));
+  PT_CUDA(mg_alloc(s, &vf[0], sizeof(double) * 2 * nv0));
   vf[1] = vf[0] + nv0;
   vertex_field_kernel<<<vgrid(nv0), 256, 0, op->stream>>>(mgbox(op), op->d_eta, vf[0]);
   st = cudaGetLastError() == cudaSuccess ? PT_OK : fail(PT_ERR_CUDA, "vertex field kernel launch failed");
@@ -626,12 +669,12 @@ pt_status mg_build(pt_solver *s)
     L.own = true;
     mg->lv.push_back(L);
     const int cur = ((int)mg->lv.size() - 2) & 1;
-    st = mg_coarsen(f, vf[cur], vf[cur ^ 1], &mg->lv.back().op);
+    st = mg_coarsen(s, f, vf[cur], vf[cur ^ 1], &mg->lv.back().op);
   }
   if (st == PT_OK && cudaStreamSynchronize(op->stream) != cudaSuccess) st = fail(PT_ERR_CUDA, "multigrid set-up failed");
-  cudaFree(vf[0]);
+  mg_release(s, vf[0]);
   if (st != PT_OK) return st;
-  if (s->o.mg_assembled == 2 && (st = mg_galerkin(*mg)) != PT_OK) return st;
+  if (s->o.mg_assembled == 2 && (st = mg_galerkin(s, *mg)) != PT_OK) return st;
   for (size_t l = 0; l < mg->lv.size(); l++) {
     const pt_op *next = l + 1 < mg->lv.size() ? mg->lv[l + 1].op : nullptr;
     if ((st = mg_level_setup(s, *mg, mg->lv[l], next)) != PT_OK) return st;
@@ -640,7 +683,7 @@ pt_status mg_build(pt_solver *s)
   if (mg->fp32)
     for (pt_mg_level &L : mg->lv)
       if (L.Ae64 && (void *)L.Ae64 != L.Ae) {
-        cudaFree(L.Ae64);
+        mg_release(s, L.Ae64);
         L.Ae64 = nullptr;
       }
   s->lambda_max = mg->lv[0].lmax;
@@ -689,6 +732,7 @@ template <typename T>
 pt_status mg_run(pt_solver *s)
 {
   pt_mg &mg = *s->mg;
+  for (pt_mg_level &L : mg.lv) L.op->stream = s->op->stream;  // the op may have been given another one
   if (!mg.use_graph) return mg_vcycle<T>(mg, 0);
   if (!mg.gexec) {
     pt_status st = mg_capture<T>(s);
@@ -707,15 +751,13 @@ pt_status sv_setup(pt_solver *s)
   if (s->setup_done && s->op_state == s->op->state) return PT_OK;
   s->have_diag = false;
   s->lambda_max = 0.0;
-  mg_free(s->mg);
-  s->mg = nullptr;
+  mg_free(s, s->op->stream);
   s->setup_done = false;
   pt_status st = PT_OK;
   if (s->o.pc != PT_PC_NONE && (st = sv_setup_diag(s)) != PT_OK) return st;
   if (s->o.pc == PT_PC_CHEBY_JACOBI && (st = sv_estimate_lambda(s)) != PT_OK) return st;
   if (s->o.pc == PT_PC_MG && (st = mg_build(s)) != PT_OK) {
-    mg_free(s->mg);
-    s->mg = nullptr;
+    mg_free(s, s->op->stream);
     return st;
   }
   s->setup_done = true;
@@ -1019,7 +1061,8 @@ pt_status pt_solver_destroy(pt_solver *s)
                   s->az32, s->partial, s->dres, s->hbuf, (void *)s->dptr};
   for (void *p : ptrs) cudaFree(p);
   if (s->hhost) cudaFreeHost(s->hhost);
-  mg_free(s->mg);
+  mg_free(s, nullptr);  // the solver's work is done: any stream will do
+  if (s->pool) cudaMemPoolDestroy(s->pool);
   delete s;
   return PT_OK;
 }
