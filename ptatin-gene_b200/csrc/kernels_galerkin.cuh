@@ -45,11 +45,21 @@ struct GalerkinArgs {
 
 constexpr int GAL_THREADS = 256;
 
-// smem (doubles): child matrix, work matrix, g table [q][n][3], c[q], child coords
+// smem (doubles): child matrix, work matrix, g table [q][n][3], basis gradients
+// [q][n][3], J then adj(J) [q][9], c[q], child coords
 constexpr size_t galerkin_smem_bytes()
 {
-  return sizeof(double) * (2 * 6561 + 27 * 27 * 3 + 27 + 81) + 96;
+  return sizeof(double) * (2 * 6561 + 2 * 27 * 27 * 3 + 243 + 27 + 81) + 96;
 }
+
+// The child matrix from quadrature: a thread takes three nodes n against one
+// node m, the node triples' upper triangle only (135 of 243), and all 27
+// points, so a point's 13 values feed three pairs of 9 multiply-adds (a thread
+// per pair read seven for one pair), the symmetric half is not computed twice
+// and there is nothing to reduce.  (Tiles of 3 x 3 nodes with the points dealt
+// to five thread groups read less but spent longer adding the groups up: 13.4
+// ms for the 20^3 level of a 40^3 box, a thread per pair 8.7 ms.)
+constexpr int GAL_UNITS = 135;
 
 // 1-D Q2 interpolation from a coarse element's nodes M to child h's nodes m:
 // fine node m of child h sits at coarse xi = -1 + h + m/2.
@@ -123,7 +133,9 @@ __global__ void __launch_bounds__(GAL_THREADS) galerkin_kernel(GalerkinArgs a)
   double *A = reinterpret_cast<double *>(smem_raw);  // child matrix, then P^T (.) P
   double *B = A + 6561;                              // A P
   double *G = B + 6561;                              // g[q][n][3]
-  double *cq = G + 27 * 27 * 3;
+  double *dN = G + 27 * 27 * 3;                      // d N_n / d xi_k at q: [q][n][k]
+  double *Jq = dN + 27 * 27 * 3;                     // J[k][l], then adj(J)
+  double *cq = Jq + 243;
   double *xe = cq + 27;
   uint8_t *mk = reinterpret_cast<uint8_t *>(xe + 81);
   const int t = threadIdx.x;
@@ -132,6 +144,20 @@ __global__ void __launch_bounds__(GAL_THREADS) galerkin_kernel(GalerkinArgs a)
   double acc[26];
 #pragma unroll
   for (int k = 0; k < 26; k++) acc[k] = 0.0;
+  if (MF)
+    for (int i = t; i < 27 * 27 * 3; i += GAL_THREADS) {
+      const int k = i % 3, n = i / 3 % 27, q = i / 81;
+      const int qi = q % 3, qj = q / 3 % 3, qk = q / 9, ni = n % 3, nj = n / 3 % 3, nk = n / 9;
+      dN[i] = (k == 0 ? gal_d1(qi, ni) : gal_n1(qi, ni)) * (k == 1 ? gal_d1(qj, nj) : gal_n1(qj, nj)) *
+              (k == 2 ? gal_d1(qk, nk) : gal_n1(qk, nk));
+    }
+  // this thread's node triple 3*nt.. and node m >= 3*nt
+  int nt = 0, m = t;
+  while (nt < 8 && m >= 27 - 3 * nt) {
+    m -= 27 - 3 * nt;
+    nt++;
+  }
+  m += 3 * nt;
 
 #pragma unroll 1
   for (int ch = 0; ch < 8; ch++) {
@@ -147,56 +173,66 @@ __global__ void __launch_bounds__(GAL_THREADS) galerkin_kernel(GalerkinArgs a)
     }
     __syncthreads();
     if (MF) {
-      // per Gauss point: c = w eta / det and g_n = adj(J) grad_xi N_n
-      if (t < 27) {
-        const int q = t, pc = q % 3, pb = (q / 3) % 3, pa = q / 9;
-        double Jm[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        for (int n = 0; n < 27; n++) {
-          const int ni = n % 3, nj = (n / 3) % 3, nk = n / 9;
-          const double d0 = gal_d1(pc, ni) * gal_n1(pb, nj) * gal_n1(pa, nk);
-          const double d1 = gal_n1(pc, ni) * gal_d1(pb, nj) * gal_n1(pa, nk);
-          const double d2 = gal_n1(pc, ni) * gal_n1(pb, nj) * gal_d1(pa, nk);
-          for (int l = 0; l < 3; l++) {
-            const double x = xe[3 * n + l];
-            Jm[0][l] = fma(d0, x, Jm[0][l]);
-            Jm[1][l] = fma(d1, x, Jm[1][l]);
-            Jm[2][l] = fma(d2, x, Jm[2][l]);
-          }
-        }
-        double adj[3][3];
-        const double det = q2::adjugate(Jm, adj);
-        cq[q] = q2::weight(q) * a.eta[27 * e + q] / det;
-        for (int n = 0; n < 27; n++) {
-          const int ni = n % 3, nj = (n / 3) % 3, nk = n / 9;
-          const double d[3] = {gal_d1(pc, ni) * gal_n1(pb, nj) * gal_n1(pa, nk),
-                               gal_n1(pc, ni) * gal_d1(pb, nj) * gal_n1(pa, nk),
-                               gal_n1(pc, ni) * gal_n1(pb, nj) * gal_d1(pa, nk)};
-          for (int l = 0; l < 3; l++) G[(q * 27 + n) * 3 + l] = adj[l][0] * d[0] + adj[l][1] * d[1] + adj[l][2] * d[2];
-        }
+      // J at the 27 points, one entry per thread
+      if (t < 243) {
+        const int q = t / 9, k = t / 3 % 3, l = t % 3;
+        double v = 0.0;
+#pragma unroll 9
+        for (int n = 0; n < 27; n++) v = fma(dN[(q * 27 + n) * 3 + k], xe[3 * n + l], v);
+        Jq[t] = v;
       }
       __syncthreads();
-      for (int p = t; p < 729; p += GAL_THREADS) {
-        const int n = p / 27, m = p % 27;
-        double S = 0.0, T[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+      // c = w eta / det, J <- adj(J)
+      if (t < 27) {
+        double Jm[3][3], adj[3][3];
+#pragma unroll
+        for (int i = 0; i < 9; i++) Jm[i / 3][i % 3] = Jq[9 * t + i];
+        const double det = q2::adjugate(Jm, adj);
+        cq[t] = q2::weight(t) * a.eta[27 * e + t] / det;
+#pragma unroll
+        for (int i = 0; i < 9; i++) Jq[9 * t + i] = adj[i / 3][i % 3];
+      }
+      __syncthreads();
+      // g_n = adj(J) grad_xi N_n
+      for (int i = t; i < 27 * 27 * 3; i += GAL_THREADS) {
+        const int l = i % 3, qn = i / 3, q = qn / 27;
+        const double *d = dN + 3 * qn, *ad = Jq + 9 * q + 3 * l;
+        G[i] = ad[0] * d[0] + ad[1] * d[1] + ad[2] * d[2];
+      }
+      __syncthreads();
+      // row dof (n, ra), column dof (m, cb): delta S + g_n[cb] g_m[ra]  (T[3 cb + ra]), S = g_n . g_m
+      if (t < GAL_UNITS) {
+        double T[3][9];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+          for (int r = 0; r < 9; r++) T[i][r] = 0.0;
+#pragma unroll 3
         for (int q = 0; q < 27; q++) {
-          const double *gn = G + (q * 27 + n) * 3, *gm = G + (q * 27 + m) * 3;
+          const double *gn = G + (q * 27 + 3 * nt) * 3, *gm = G + (q * 27 + m) * 3;
           const double c = cq[q];
-          const double gn0 = c * gn[0], gn1 = c * gn[1], gn2 = c * gn[2];
-          const double gm0 = gm[0], gm1 = gm[1], gm2 = gm[2];
-          S = fma(gn0, gm0, fma(gn1, gm1, fma(gn2, gm2, S)));
-          T[0][0] = fma(gn0, gm0, T[0][0]); T[0][1] = fma(gn1, gm0, T[0][1]); T[0][2] = fma(gn2, gm0, T[0][2]);
-          T[1][0] = fma(gn0, gm1, T[1][0]); T[1][1] = fma(gn1, gm1, T[1][1]); T[1][2] = fma(gn2, gm1, T[1][2]);
-          T[2][0] = fma(gn0, gm2, T[2][0]); T[2][1] = fma(gn1, gm2, T[2][1]); T[2][2] = fma(gn2, gm2, T[2][2]);
+          double vm[3];
+#pragma unroll
+          for (int i = 0; i < 3; i++) vm[i] = c * gm[i];
+#pragma unroll
+          for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int r = 0; r < 9; r++) T[i][r] = fma(gn[3 * i + r / 3], vm[r % 3], T[i][r]);
         }
-        // row dof (n, ra), column dof (m, cb): delta S + g_n[cb] g_m[ra]  (T[ra][cb])
 #pragma unroll
-        for (int ra = 0; ra < 3; ra++)
+        for (int i = 0; i < 3; i++) {
+          const int n = 3 * nt + i;
+          const double S = (T[i][0] + T[i][4]) + T[i][8];
 #pragma unroll
-          for (int cb = 0; cb < 3; cb++) {
-            const int i = 3 * n + ra, j = 3 * m + cb;
-            const double v = (ra == cb ? S : 0.0) + T[ra][cb];
-            A[j * 81 + i] = (mk[i] || mk[j]) ? 0.0 : v;
-          }
+          for (int ra = 0; ra < 3; ra++)
+#pragma unroll
+            for (int cb = 0; cb < 3; cb++) {
+              const int r = 3 * n + ra, k = 3 * m + cb;
+              const double v = (mk[r] || mk[k]) ? 0.0 : (ra == cb ? S : 0.0) + T[i][3 * cb + ra];
+              A[k * 81 + r] = v;
+              if (m >= 3 * nt + 3) A[r * 81 + k] = v;  // the mirrored triple is nobody's
+            }
+        }
       }
     } else {
       const double *src = a.Af + e * EBE_LD;
