@@ -24,6 +24,18 @@
 
 namespace ptk {
 
+// Start of a kernel that may be launched programmatically behind another one:
+// the next launch may be scheduled from here on, and nothing that the previous
+// grid writes is read or written before it is complete and flushed.  Pointers
+// that such kernels read after it are not __restrict__, so no load is moved up
+// as read-only.  Both instructions do nothing for an ordinary launch.  A chain
+// of small kernels saves about a microsecond per launch.
+__device__ __forceinline__ void chain_wait()
+{
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr int EBE_LD = 3328;  // packed upper triangle (3321) padded to a multiple of 16 bytes
 
 // Packed position of entry (i, j) of a symmetric element matrix.
@@ -164,8 +176,8 @@ __device__ __forceinline__ T ebe_row(uint32_t sbase, int t, const T *ue)
 // entries of u taken as 0).  The element's packed block is copied to shared
 // memory with 16-byte cp.async while u is gathered.
 template <typename T, bool MASKED>
-__global__ void __launch_bounds__(96) ebe_apply_kernel(Box b, const T *__restrict__ Ae, const T *__restrict__ u,
-                                                       const uint8_t *__restrict__ mask, T *__restrict__ ye)
+__global__ void __launch_bounds__(96) ebe_apply_kernel(Box b, const T *__restrict__ Ae, const T *u,
+                                                       const uint8_t *__restrict__ mask, T *ye)
 {
   __shared__ __align__(16) T S[EBE_LD];
   __shared__ __align__(16) T ue[84];
@@ -180,6 +192,7 @@ __global__ void __launch_bounds__(96) ebe_apply_kernel(Box b, const T *__restric
                    : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  chain_wait();  // u and ye; the matrices are complete before any apply is launched programmatically
   const int ei = (int)(e % b.mx), ej = (int)((e / b.mx) % b.my), ek = (int)(e / ((int64_t)b.mx * b.my));
   if (t < 84) {
     T v = T(0);
@@ -224,8 +237,8 @@ __global__ void __launch_bounds__(128) ebe_to_half_kernel(const double *__restri
 // element instead of 13.3 KB.
 template <bool MASKED>
 __global__ void __launch_bounds__(96) ebe_apply_h_kernel(Box b, const __half *__restrict__ Ah,
-                                                         const float *__restrict__ scale, const float *__restrict__ u,
-                                                         const uint8_t *__restrict__ mask, float *__restrict__ ye)
+                                                         const float *__restrict__ scale, const float *u,
+                                                         const uint8_t *__restrict__ mask, float *ye)
 {
   __shared__ __align__(16) __half S[EBE_LD];
   __shared__ __align__(16) float ue[84];
@@ -240,6 +253,7 @@ __global__ void __launch_bounds__(96) ebe_apply_h_kernel(Box b, const __half *__
                    : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  chain_wait();
   const int ei = (int)(e % b.mx), ej = (int)((e / b.mx) % b.my), ek = (int)(e / ((int64_t)b.mx * b.my));
   if (t < 84) {
     float v = 0.0f;
@@ -257,46 +271,64 @@ __global__ void __launch_bounds__(96) ebe_apply_h_kernel(Box b, const __half *__
 }
 
 // y_k = sum over the (<= 8) elements of node k of their ye entry, in a fixed
-// order (MASKED: y_k = x_k on Dirichlet dofs; ACC: added to y).  One-rank
-// boxes (node box = element box).
-template <typename T, bool MASKED, bool ACC = false>
-__global__ void ebe_gather_kernel(Box b, const T *__restrict__ ye, const T *__restrict__ x,
-                                  const uint8_t *__restrict__ mask, T *__restrict__ y)
+// order (MASKED: y_k = x_k on Dirichlet dofs).  One-rank boxes (node box =
+// element box).
+template <typename T>
+__device__ __forceinline__ T ebe_node_sum(const Box &b, int64_t t, const T *ye)
 {
+  const int l = (int)(t % 3);
+  const int64_t node = t / 3;
+  const int i = (int)(node % b.X), j = (int)((node / b.X) % (2 * b.my + 1)), k = (int)(node / b.XY);
+  // per axis: (element, local index) pairs, lower element first
+  int ex[2], lx[2], nx = 0, ey[2], ly[2], ny = 0, ez[2], lz[2], nz = 0;
+  if (i & 1) { ex[0] = i >> 1; lx[0] = 1; nx = 1; }
+  else {
+    if (i > 0) { ex[nx] = (i >> 1) - 1; lx[nx++] = 2; }
+    if ((i >> 1) < b.mx) { ex[nx] = i >> 1; lx[nx++] = 0; }
+  }
+  if (j & 1) { ey[0] = j >> 1; ly[0] = 1; ny = 1; }
+  else {
+    if (j > 0) { ey[ny] = (j >> 1) - 1; ly[ny++] = 2; }
+    if ((j >> 1) < b.my) { ey[ny] = j >> 1; ly[ny++] = 0; }
+  }
+  if (k & 1) { ez[0] = k >> 1; lz[0] = 1; nz = 1; }
+  else {
+    if (k > 0) { ez[nz] = (k >> 1) - 1; lz[nz++] = 2; }
+    if ((k >> 1) < b.mz) { ez[nz] = k >> 1; lz[nz++] = 0; }
+  }
+  T acc = T(0);
+  for (int c = 0; c < nz; c++)
+    for (int bb = 0; bb < ny; bb++)
+      for (int a = 0; a < nx; a++) {
+        const int64_t e = ex[a] + (int64_t)b.mx * (ey[bb] + (int64_t)b.my * ez[c]);
+        acc += ye[e * 81 + 3 * (lx[a] + 3 * ly[bb] + 9 * lz[c]) + l];
+      }
+  return acc;
+}
+
+template <typename T, bool MASKED>
+__global__ void ebe_gather_kernel(Box b, const T *ye, const T *x, const uint8_t *__restrict__ mask, T *y)
+{
+  chain_wait();
+  const int64_t n = 3 * b.XY * (2 * (int64_t)b.mz + 1);
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
+    y[t] = MASKED && mask[t] ? x[t] : ebe_node_sum<T>(b, t, ye);
+}
+
+// The masked gather and a Chebyshev step in one pass: with az = A z (z_k on
+// Dirichlet dofs), d = alpha d + beta dinv (r - az), z += d.
+template <typename T>
+__global__ void ebe_gather_cheb_kernel(Box b, const T *ye, const uint8_t *__restrict__ mask, T alpha, T beta,
+                                       const T *__restrict__ dinv, const T *r, T *d, T *z)
+{
+  chain_wait();
   const int64_t n = 3 * b.XY * (2 * (int64_t)b.mz + 1);
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
-    if (MASKED && mask[t]) {
-      y[t] = x[t];
-      continue;
-    }
-    const int l = (int)(t % 3);
-    const int64_t node = t / 3;
-    const int i = (int)(node % b.X), j = (int)((node / b.X) % (2 * b.my + 1)), k = (int)(node / b.XY);
-    // per axis: (element, local index) pairs, lower element first
-    int ex[2], lx[2], nx = 0, ey[2], ly[2], ny = 0, ez[2], lz[2], nz = 0;
-    if (i & 1) { ex[0] = i >> 1; lx[0] = 1; nx = 1; }
-    else {
-      if (i > 0) { ex[nx] = (i >> 1) - 1; lx[nx++] = 2; }
-      if ((i >> 1) < b.mx) { ex[nx] = i >> 1; lx[nx++] = 0; }
-    }
-    if (j & 1) { ey[0] = j >> 1; ly[0] = 1; ny = 1; }
-    else {
-      if (j > 0) { ey[ny] = (j >> 1) - 1; ly[ny++] = 2; }
-      if ((j >> 1) < b.my) { ey[ny] = j >> 1; ly[ny++] = 0; }
-    }
-    if (k & 1) { ez[0] = k >> 1; lz[0] = 1; nz = 1; }
-    else {
-      if (k > 0) { ez[nz] = (k >> 1) - 1; lz[nz++] = 2; }
-      if ((k >> 1) < b.mz) { ez[nz] = k >> 1; lz[nz++] = 0; }
-    }
-    T acc = T(0);
-    for (int c = 0; c < nz; c++)
-      for (int bb = 0; bb < ny; bb++)
-        for (int a = 0; a < nx; a++) {
-          const int64_t e = ex[a] + (int64_t)b.mx * (ey[bb] + (int64_t)b.my * ez[c]);
-          acc += ye[e * 81 + 3 * (lx[a] + 3 * ly[bb] + 9 * lz[c]) + l];
-        }
-    y[t] = ACC ? y[t] + acc : acc;
+    const T zt = z[t];
+    const T az = mask[t] ? zt : ebe_node_sum<T>(b, t, ye);
+    const T v = alpha * d[t] + beta * dinv[t] * (r[t] - az);
+    d[t] = v;
+    z[t] = zt + v;
   }
 }
 

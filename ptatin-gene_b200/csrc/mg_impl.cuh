@@ -179,9 +179,10 @@ struct Dims3 {
 };
 
 template <typename T, int AXIS, bool PROLONG, int FINAL>
-__global__ void transfer_axis_kernel(Dims3 din, Dims3 dout, const T *__restrict__ in, T *__restrict__ out,
+__global__ void transfer_axis_kernel(Dims3 din, Dims3 dout, const T *in, T *out,
                                      const uint8_t *__restrict__ mask)
 {
+  ptk::chain_wait();
   // FINAL: 0 = write, 1 = out = mask ? 0 : out + v (prolongation into x), 2 = out = mask ? 0 : v
   const int64_t nout = 3 * (int64_t)dout.n[0] * dout.n[1] * dout.n[2];
   const int64_t s_in = AXIS == 0 ? 3 : (AXIS == 1 ? 3 * (int64_t)din.n[0] : 3 * (int64_t)din.n[0] * din.n[1]);
@@ -231,8 +232,9 @@ __global__ void transfer_axis_kernel(Dims3 din, Dims3 dout, const T *__restrict_
 
 // x = Ainv b on the coarsest level (dense symmetric inverse, one warp per row).
 template <typename T>
-__global__ void dense_apply_kernel(int n, const T *__restrict__ Ainv, const T *__restrict__ b, T *__restrict__ x)
+__global__ void dense_apply_kernel(int n, const T *Ainv, const T *b, T *x)
 {
+  ptk::chain_wait();
   const int lane = threadIdx.x & 31;
   const int row = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   if (row >= n) return;
@@ -245,15 +247,17 @@ __global__ void dense_apply_kernel(int n, const T *__restrict__ Ainv, const T *_
 }
 
 template <typename T>
-__global__ void sub_kernel(const T *__restrict__ b, const T *__restrict__ ax, T *__restrict__ r, int64_t n)
+__global__ void sub_kernel(const T *b, const T *ax, T *r, int64_t n)
 {
+  ptk::chain_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     r[i] = b[i] - ax[i];
 }
 
 template <typename T>
-__global__ void add_kernel(const T *__restrict__ a, T *__restrict__ x, int64_t n)
+__global__ void add_kernel(const T *a, T *x, int64_t n)
 {
+  ptk::chain_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] += a[i];
 }
@@ -304,33 +308,58 @@ struct pt_mg {
 
 namespace {
 
-template <typename T>
-pt_status mg_matmult(pt_mg &mg, pt_mg_level &L, const T *x, T *y)
+// Launch programmatically behind the kernel before it on the stream; the kernel
+// starts with chain_wait().
+template <typename... P, typename... A>
+void chain(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st, A... args)
 {
-  if (L.op == mg.lv[0].op) mg.fine_applies++;
-  else mg.coarse_work += (double)L.op->nel / (double)mg.lv[0].op->nel;
+  cudaLaunchAttribute pdl[1] = {};
+  pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cfg.attrs = pdl;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // PT_LAUNCHED reports its error
+}
+
+// Per-element outputs A_e x into L.ye where the level has element matrices;
+// false where it does not.
+template <typename T>
+bool mg_element_apply(pt_mg &mg, pt_mg_level &L, const T *x)
+{
+  const cudaStream_t st = L.op->stream;
   if constexpr (std::is_same<T, float>::value) {
     if (L.Ah) {
       ebe_h_carveout<true>();
-      ptk::ebe_apply_h_kernel<true><<<(unsigned)L.nel, 96, 0, L.op->stream>>>(L.op->box, L.Ah, L.Ascale, x,
-                                                                               L.op->d_mask, (float *)L.ye);
-      PT_LAUNCHED(L.op);
-      ptk::ebe_gather_kernel<float, true><<<vgrid(L.n), 256, 0, L.op->stream>>>(L.op->box, (const float *)L.ye, x,
-                                                                                L.op->d_mask, y);
-      PT_LAUNCHED(L.op);
-      return PT_OK;
+      mg.coarse_work += (double)L.op->nel / (double)mg.lv[0].op->nel;
+      chain(ptk::ebe_apply_h_kernel<true>, (unsigned)L.nel, 96, st, L.op->box, L.Ah, L.Ascale, x, L.op->d_mask,
+            (float *)L.ye);
+      L.op->launches++;
+      return true;
     }
   }
-  if (L.Ae) {
-    ebe_carveout<T, true>();
-    ptk::ebe_apply_kernel<T, true><<<(unsigned)L.nel, 96, 0, L.op->stream>>>(L.op->box, (const T *)L.Ae, x,
-                                                                              L.op->d_mask, (T *)L.ye);
-    PT_LAUNCHED(L.op);
-    ptk::ebe_gather_kernel<T, true><<<vgrid(L.n), 256, 0, L.op->stream>>>(L.op->box, (const T *)L.ye, x,
-                                                                          L.op->d_mask, y);
+  if (!L.Ae) return false;
+  ebe_carveout<T, true>();
+  if (L.op == mg.lv[0].op) mg.fine_applies++;
+  else mg.coarse_work += (double)L.op->nel / (double)mg.lv[0].op->nel;
+  chain(ptk::ebe_apply_kernel<T, true>, (unsigned)L.nel, 96, st, L.op->box, (const T *)L.Ae, x, L.op->d_mask, (T *)L.ye);
+  L.op->launches++;
+  return true;
+}
+
+template <typename T>
+pt_status mg_matmult(pt_mg &mg, pt_mg_level &L, const T *x, T *y)
+{
+  if (mg_element_apply<T>(mg, L, x)) {
+    chain(ptk::ebe_gather_kernel<T, true>, vgrid(L.n), 256, L.op->stream, L.op->box, (const T *)L.ye, x, L.op->d_mask, y);
     PT_LAUNCHED(L.op);
     return PT_OK;
   }
+  if (L.op == mg.lv[0].op) mg.fine_applies++;
+  else mg.coarse_work += (double)L.op->nel / (double)mg.lv[0].op->nel;
   if (std::is_same<T, double>::value) return pt_matmult_a11_d(L.op, (const double *)x, (double *)y);
   return pt_matmult_a11_f32_d(L.op, (const float *)x, (float *)y);
 }
@@ -356,25 +385,31 @@ pt_status mg_cheby(pt_mg &mg, pt_mg_level &L, const T *b, T *x, bool x_zero, int
   const T *rr = b;
   if (!x_zero) {
     if ((s = mg_matmult<T>(mg, L, x, az)) != PT_OK) return s;
-    sub_kernel<T><<<vgrid(n), 256, 0, st>>>(b, az, r, n);
+    chain(sub_kernel<T>, vgrid(n), 256, st, b, (const T *)az, r, n);
     PT_LAUNCHED(L.op);
     rr = r;
   }
   // correction dl (= z of the recurrence) from residual rr
-  cheb_first_kernel<T><<<vgrid(n), 256, 0, st>>>((T)(1.0 / theta), mg_dinv<T>(L), rr, d, dl, n);
+  chain(cheb_first_kernel<T>, vgrid(n), 256, st, (T)(1.0 / theta), mg_dinv<T>(L), rr, d, dl, n);
   PT_LAUNCHED(L.op);
   for (int i = 1; i < k; i++) {
-    if ((s = mg_matmult<T>(mg, L, dl, az)) != PT_OK) return s;
     const double rho_new = 1.0 / (2.0 * sigma - rho);
-    cheb_step_kernel<T><<<vgrid(n), 256, 0, st>>>((T)(rho_new * rho), (T)(2.0 * rho_new / delta), mg_dinv<T>(L), rr,
-                                                   az, d, dl, n);
-    PT_LAUNCHED(L.op);
+    const T alpha = (T)(rho_new * rho), beta = (T)(2.0 * rho_new / delta);
+    if (mg_element_apply<T>(mg, L, dl)) {
+      chain(ptk::ebe_gather_cheb_kernel<T>, vgrid(n), 256, st, L.op->box, (const T *)L.ye, L.op->d_mask, alpha, beta,
+            mg_dinv<T>(L), rr, d, dl);
+      PT_LAUNCHED(L.op);
+    } else {
+      if ((s = mg_matmult<T>(mg, L, dl, az)) != PT_OK) return s;
+      chain(cheb_step_kernel<T>, vgrid(n), 256, st, alpha, beta, mg_dinv<T>(L), rr, az, d, dl, n);
+      PT_LAUNCHED(L.op);
+    }
     rho = rho_new;
   }
   if (x_zero) {
     PT_CUDA(cudaMemcpyAsync(x, dl, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
   } else {
-    add_kernel<T><<<vgrid(n), 256, 0, st>>>(dl, x, n);
+    chain(add_kernel<T>, vgrid(n), 256, st, dl, x, n);
     PT_LAUNCHED(L.op);
   }
   return PT_OK;
@@ -388,8 +423,8 @@ pt_status mg_vcycle(pt_mg &mg, int l)
   pt_status s;
   if (l + 1 == (int)mg.lv.size()) {
     if (L.Ainv) {
-      dense_apply_kernel<T><<<(unsigned)((L.n * 32 + 255) / 256), 256, 0, L.op->stream>>>((int)L.n, (const T *)L.Ainv,
-                                                                                          b, x);
+      chain(dense_apply_kernel<T>, (unsigned)((L.n * 32 + 255) / 256), 256, L.op->stream, (int)L.n, (const T *)L.Ainv,
+            b, x);
       PT_LAUNCHED(L.op);
       return PT_OK;
     }
@@ -400,7 +435,7 @@ pt_status mg_vcycle(pt_mg &mg, int l)
   // residual -> coarse rhs
   pt_mg_level &C = mg.lv[l + 1];
   if ((s = mg_matmult<T>(mg, L, x, (T *)L.az)) != PT_OK) return s;
-  sub_kernel<T><<<vgrid(L.n), 256, 0, L.op->stream>>>(b, (T *)L.az, (T *)L.r, L.n);
+  chain(sub_kernel<T>, vgrid(L.n), 256, L.op->stream, b, (T *)L.az, (T *)L.r, L.n);
   PT_LAUNCHED(L.op);
   const cudaStream_t st = L.op->stream;
   const int fx = 2 * L.op->mx + 1, fy = 2 * L.op->my + 1, fz = 2 * L.op->mz + 1;
@@ -408,19 +443,19 @@ pt_status mg_vcycle(pt_mg &mg, int l)
   const Dims3 dF{{fx, fy, fz}}, dXf{{cx, fy, fz}}, dXYf{{cx, cy, fz}}, dC{{cx, cy, cz}};
   T *t1 = (T *)L.t1, *t2 = (T *)L.t2;
   // b_c = R r_f: x, then y, then z (masked)
-  transfer_axis_kernel<T, 0, false, 0><<<vgrid(3LL * cx * fy * fz), 256, 0, st>>>(dF, dXf, (T *)L.r, t1, nullptr);
+  chain(transfer_axis_kernel<T, 0, false, 0>, vgrid(3LL * cx * fy * fz), 256, st, dF, dXf, (T *)L.r, t1, nullptr);
   PT_LAUNCHED(L.op);
-  transfer_axis_kernel<T, 1, false, 0><<<vgrid(3LL * cx * cy * fz), 256, 0, st>>>(dXf, dXYf, t1, t2, nullptr);
+  chain(transfer_axis_kernel<T, 1, false, 0>, vgrid(3LL * cx * cy * fz), 256, st, dXf, dXYf, t1, t2, nullptr);
   PT_LAUNCHED(L.op);
-  transfer_axis_kernel<T, 2, false, 2><<<vgrid(C.n), 256, 0, st>>>(dXYf, dC, t2, (T *)C.b, C.op->d_mask);
+  chain(transfer_axis_kernel<T, 2, false, 2>, vgrid(C.n), 256, st, dXYf, dC, t2, (T *)C.b, C.op->d_mask);
   PT_LAUNCHED(L.op);
   if ((s = mg_vcycle<T>(mg, l + 1)) != PT_OK) return s;
   // x_f += P x_c: z, then y, then x (masked add)
-  transfer_axis_kernel<T, 2, true, 0><<<vgrid(3LL * cx * cy * fz), 256, 0, st>>>(dC, dXYf, (T *)C.x, t2, nullptr);
+  chain(transfer_axis_kernel<T, 2, true, 0>, vgrid(3LL * cx * cy * fz), 256, st, dC, dXYf, (T *)C.x, t2, nullptr);
   PT_LAUNCHED(L.op);
-  transfer_axis_kernel<T, 1, true, 0><<<vgrid(3LL * cx * fy * fz), 256, 0, st>>>(dXYf, dXf, t2, t1, nullptr);
+  chain(transfer_axis_kernel<T, 1, true, 0>, vgrid(3LL * cx * fy * fz), 256, st, dXYf, dXf, t2, t1, nullptr);
   PT_LAUNCHED(L.op);
-  transfer_axis_kernel<T, 0, true, 1><<<vgrid(L.n), 256, 0, st>>>(dXf, dF, t1, x, L.op->d_mask);
+  chain(transfer_axis_kernel<T, 0, true, 1>, vgrid(L.n), 256, st, dXf, dF, t1, x, L.op->d_mask);
   PT_LAUNCHED(L.op);
   return mg_cheby<T>(mg, L, b, x, false, degree);
 }

@@ -115,8 +115,9 @@ __global__ void resid_kernel(const double *__restrict__ b, double *__restrict__ 
 }
 
 template <typename TO, typename TI>
-__global__ void convert_kernel(const TI *__restrict__ a, TO *__restrict__ b, int64_t n)
+__global__ void convert_kernel(const TI *a, TO *b, int64_t n)
 {
+  ptk::chain_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     b[i] = (TO)a[i];
 }
@@ -133,9 +134,10 @@ __global__ void reciprocal_kernel(const double *__restrict__ d, double *__restri
 
 // z = s * dinv .* r ; d = z
 template <typename T>
-__global__ void cheb_first_kernel(T s, const T *__restrict__ dinv, const T *__restrict__ r, T *__restrict__ d,
-                                  T *__restrict__ z, int64_t n)
+__global__ void cheb_first_kernel(T s, const T *__restrict__ dinv, const T *r, T *d,
+                                  T *z, int64_t n)
 {
+  ptk::chain_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T v = s * dinv[i] * r[i];
     d[i] = v;
@@ -145,9 +147,10 @@ __global__ void cheb_first_kernel(T s, const T *__restrict__ dinv, const T *__re
 
 // az holds A z on entry: d = alpha d + beta dinv .* (r - A z); z += d
 template <typename T>
-__global__ void cheb_step_kernel(T alpha, T beta, const T *__restrict__ dinv, const T *__restrict__ r,
-                                 const T *__restrict__ az, T *__restrict__ d, T *__restrict__ z, int64_t n)
+__global__ void cheb_step_kernel(T alpha, T beta, const T *__restrict__ dinv, const T *r,
+                                 const T *az, T *d, T *z, int64_t n)
 {
+  ptk::chain_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T v = alpha * d[i] + beta * dinv[i] * (r[i] - az[i]);
     d[i] = v;
