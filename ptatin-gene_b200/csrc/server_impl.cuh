@@ -75,6 +75,20 @@ __device__ __forceinline__ double srv_block_sum(double v, double *sh)
   return r;
 }
 
+// A thread's SRV_PER values of a chunk, all loaded before any is stored: the
+// loops of the chunk kernels were chains of dependent round trips (5 to 10 us
+// per kernel for a handful of requests).
+constexpr int SRV_PER = SRV_CH / SRV_THREADS;
+template <typename F>
+__device__ __forceinline__ void srv_each(int64_t i0, int64_t i1, F f)
+{
+#pragma unroll
+  for (int k = 0; k < SRV_PER; k++) {
+    const int64_t i = i0 + threadIdx.x + k * SRV_THREADS;
+    if (i < i1) f(k, i);
+  }
+}
+
 // chunk c of slot s: [c*CH, min(n, (c+1)*CH))
 __device__ __forceinline__ void srv_chunk(const SrvSlot &S, int c, int64_t &i0, int64_t &i1)
 {
@@ -83,9 +97,10 @@ __device__ __forceinline__ void srv_chunk(const SrvSlot &S, int c, int64_t &i0, 
 }
 
 // partial[c][0] = p.q over the chunk
-__global__ void __launch_bounds__(SRV_THREADS) srv_pq_kernel(const int2 *__restrict__ items, const SrvSlot *slots,
+__global__ void __launch_bounds__(SRV_THREADS) srv_pq_kernel(const int2 *items, const SrvSlot *slots,
                                                              const SrvScal *scal)
 {
+  ptk::chain_wait();
   __shared__ double sh[SRV_THREADS];
   const int2 it = items[blockIdx.x];
   const SrvSlot S = slots[it.x];
@@ -93,15 +108,21 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_pq_kernel(const int2 *__restr
   int64_t i0, i1;
   srv_chunk(S, it.y, i0, i1);
   double a = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SRV_THREADS) a = fma(S.p[i], S.q[i], a);
+  double p[SRV_PER] = {}, q[SRV_PER] = {};
+  srv_each(i0, i1, [&](int k, int64_t i) {
+    p[k] = S.p[i];
+    q[k] = S.q[i];
+  });
+  srv_each(i0, i1, [&](int k, int64_t) { a = fma(p[k], q[k], a); });
   a = srv_block_sum<double>(a, sh);
   if (threadIdx.x == 0) S.part[2 * it.y] = a;
 }
 
 // x += alpha p; r -= alpha q; partial[c][0] = r.r
-__global__ void __launch_bounds__(SRV_THREADS) srv_update_kernel(const int2 *__restrict__ items, const SrvSlot *slots,
+__global__ void __launch_bounds__(SRV_THREADS) srv_update_kernel(const int2 *items, const SrvSlot *slots,
                                                                  const SrvScal *scal)
 {
+  ptk::chain_wait();
   __shared__ double sh[SRV_THREADS];
   const int2 it = items[blockIdx.x];
   const SrvSlot S = slots[it.x];
@@ -110,21 +131,29 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_update_kernel(const int2 *__r
   int64_t i0, i1;
   srv_chunk(S, it.y, i0, i1);
   double a = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SRV_THREADS) {
-    S.x[i] = fma(alpha, S.p[i], S.x[i]);
-    const double r = fma(-alpha, S.q[i], S.r[i]);
-    S.r[i] = r;
-    a = fma(r, r, a);
-  }
+  double x[SRV_PER], p[SRV_PER], q[SRV_PER], r[SRV_PER];
+  srv_each(i0, i1, [&](int k, int64_t i) {
+    x[k] = S.x[i];
+    p[k] = S.p[i];
+    q[k] = S.q[i];
+    r[k] = S.r[i];
+  });
+  srv_each(i0, i1, [&](int k, int64_t i) {
+    S.x[i] = fma(alpha, p[k], x[k]);
+    r[k] = fma(-alpha, q[k], r[k]);
+    S.r[i] = r[k];
+    a = fma(r[k], r[k], a);
+  });
   a = srv_block_sum<double>(a, sh);
   if (threadIdx.x == 0) S.part[2 * it.y] = a;
 }
 
 // z = d = theta^-1 D^-1 r  (smoother precision)
 template <typename T>
-__global__ void __launch_bounds__(SRV_THREADS) srv_cheb_first_kernel(const int2 *__restrict__ items,
+__global__ void __launch_bounds__(SRV_THREADS) srv_cheb_first_kernel(const int2 *items,
                                                                      const SrvSlot *slots, const SrvScal *scal)
 {
+  ptk::chain_wait();
   const int2 it = items[blockIdx.x];
   const SrvSlot S = slots[it.x];
   if (scal[it.x].status != SRV_ACTIVE) return;
@@ -133,18 +162,20 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_cheb_first_kernel(const int2 
   T *z = (T *)S.z, *d = (T *)S.d;
   int64_t i0, i1;
   srv_chunk(S, it.y, i0, i1);
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SRV_THREADS) {
-    const T v = s * dinv[i] * (T)S.r[i];
-    d[i] = v;
-    z[i] = v;
-  }
+  T v[SRV_PER];
+  srv_each(i0, i1, [&](int k, int64_t i) { v[k] = s * dinv[i] * (T)S.r[i]; });
+  srv_each(i0, i1, [&](int k, int64_t i) {
+    d[i] = v[k];
+    z[i] = v[k];
+  });
 }
 
 // step k: d = ca[k] d + cb[k] D^-1 (r - A z); z += d
 template <typename T>
-__global__ void __launch_bounds__(SRV_THREADS) srv_cheb_step_kernel(const int2 *__restrict__ items,
+__global__ void __launch_bounds__(SRV_THREADS) srv_cheb_step_kernel(const int2 *items,
                                                                     const SrvSlot *slots, const SrvScal *scal, int k)
 {
+  ptk::chain_wait();
   const int2 it = items[blockIdx.x];
   const SrvSlot S = slots[it.x];
   const SrvScal &P = scal[it.x];
@@ -154,18 +185,23 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_cheb_step_kernel(const int2 *
   T *z = (T *)S.z, *d = (T *)S.d;
   int64_t i0, i1;
   srv_chunk(S, it.y, i0, i1);
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SRV_THREADS) {
-    const T v = ca * d[i] + cb * dinv[i] * ((T)S.r[i] - az[i]);
-    d[i] = v;
-    z[i] += v;
-  }
+  T v[SRV_PER], zz[SRV_PER];
+  srv_each(i0, i1, [&](int m, int64_t i) {
+    v[m] = ca * d[i] + cb * dinv[i] * ((T)S.r[i] - az[i]);
+    zz[m] = z[i];
+  });
+  srv_each(i0, i1, [&](int m, int64_t i) {
+    d[i] = v[m];
+    z[i] = zz[m] + v[m];
+  });
 }
 
 // partial[c] = (z.r, z.q)
 template <typename T>
-__global__ void __launch_bounds__(SRV_THREADS) srv_zdots_kernel(const int2 *__restrict__ items, const SrvSlot *slots,
+__global__ void __launch_bounds__(SRV_THREADS) srv_zdots_kernel(const int2 *items, const SrvSlot *slots,
                                                                 const SrvScal *scal)
 {
+  ptk::chain_wait();
   __shared__ double sh[SRV_THREADS];
   const int2 it = items[blockIdx.x];
   const SrvSlot S = slots[it.x];
@@ -174,11 +210,16 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_zdots_kernel(const int2 *__re
   int64_t i0, i1;
   srv_chunk(S, it.y, i0, i1);
   double a = 0.0, b = 0.0;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SRV_THREADS) {
-    const double zi = (double)z[i];
-    a = fma(zi, S.r[i], a);
-    b = fma(zi, S.q[i], b);
-  }
+  double zi[SRV_PER], r[SRV_PER], q[SRV_PER];
+  srv_each(i0, i1, [&](int k, int64_t i) {
+    zi[k] = (double)z[i];
+    r[k] = S.r[i];
+    q[k] = S.q[i];
+  });
+  srv_each(i0, i1, [&](int k, int64_t) {
+    a = fma(zi[k], r[k], a);
+    b = fma(zi[k], q[k], b);
+  });
   a = srv_block_sum<double>(a, sh);
   b = srv_block_sum<double>(b, sh);
   if (threadIdx.x == 0) {
@@ -189,9 +230,10 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_zdots_kernel(const int2 *__re
 
 // p = z + beta p
 template <typename T>
-__global__ void __launch_bounds__(SRV_THREADS) srv_p_kernel(const int2 *__restrict__ items, const SrvSlot *slots,
+__global__ void __launch_bounds__(SRV_THREADS) srv_p_kernel(const int2 *items, const SrvSlot *slots,
                                                             const SrvScal *scal)
 {
+  ptk::chain_wait();
   const int2 it = items[blockIdx.x];
   const SrvSlot S = slots[it.x];
   if (scal[it.x].status != SRV_ACTIVE) return;
@@ -199,7 +241,9 @@ __global__ void __launch_bounds__(SRV_THREADS) srv_p_kernel(const int2 *__restri
   const T *z = (const T *)S.z;
   int64_t i0, i1;
   srv_chunk(S, it.y, i0, i1);
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += SRV_THREADS) S.p[i] = fma(beta, S.p[i], (double)z[i]);
+  double v[SRV_PER];
+  srv_each(i0, i1, [&](int k, int64_t i) { v[k] = fma(beta, S.p[i], (double)z[i]); });
+  srv_each(i0, i1, [&](int k, int64_t i) { S.p[i] = v[k]; });
 }
 
 enum { SRV_F_ALPHA = 0, SRV_F_RR = 1, SRV_F_BETA = 2, SRV_F_INIT_RR = 3, SRV_F_INIT_RZ = 4 };
@@ -207,9 +251,10 @@ enum { SRV_F_ALPHA = 0, SRV_F_RR = 1, SRV_F_BETA = 2, SRV_F_INIT_RR = 3, SRV_F_I
 // Per slot (block): reduce the slot's chunk partials in a fixed order, then
 // the scalar recurrences.
 template <int PHASE>
-__global__ void __launch_bounds__(SRV_THREADS) srv_final_kernel(const int *__restrict__ act, const SrvSlot *slots,
+__global__ void __launch_bounds__(SRV_THREADS) srv_final_kernel(const int *act, const SrvSlot *slots,
                                                                 SrvScal *scal)
 {
+  ptk::chain_wait();
   __shared__ double sh[SRV_THREADS];
   const int s = act[blockIdx.x];
   const SrvSlot S = slots[s];
@@ -369,22 +414,49 @@ __global__ void __launch_bounds__(SRV_THREADS) lz_sum_kernel(int64_t nch, const 
 
 // lambda_max from the Lanczos tridiagonal, then the Chebyshev coefficients
 // (Saad, Alg. 12.1) of degree deg on [emin, emax] * lambda_max.
-__global__ void lz_finish_kernel(const LzState *L, double emin, double emax, int deg, SrvScal *P)
+// One warp: lane i counts the eigenvalues below the i-th of 32 points of the
+// bracket, so a round narrows it 33 times and 16 rounds do what one thread's
+// 200 bisections did in 300 us.
+__global__ void __launch_bounds__(32) lz_finish_kernel(const LzState *L, double emin, double emax, int deg, SrvScal *P)
 {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int m = L->m;
-  double a[SRV_MAX_LZ], b[SRV_MAX_LZ];
-  for (int k = 0; k < m; k++) {
+  __shared__ double a[SRV_MAX_LZ], b[SRV_MAX_LZ];
+  const int m = L->m, lane = threadIdx.x;
+  for (int k = lane; k < m; k += 32) {
     a[k] = 1.0 / L->alpha[k] + (k > 0 ? L->beta[k - 1] / L->alpha[k - 1] : 0.0);
-    if (k + 1 < m) b[k] = sqrt(L->beta[k]) / L->alpha[k];
+    b[k] = k + 1 < m ? sqrt(L->beta[k]) / L->alpha[k] : 0.0;
   }
-  const double lmax = tridiag_lmax(a, b, m);
+  __syncwarp();
+  double lo = 0.0, hi = 0.0;
+  for (int i = 0; i < m; i++) {  // Gershgorin
+    const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i + 1 < m ? fabs(b[i]) : 0.0);
+    lo = i == 0 ? a[0] - r : fmin(lo, a[i] - r);
+    hi = i == 0 ? a[0] + r : fmax(hi, a[i] + r);
+  }
+  for (int it = 0; it < 16 && m > 0; it++) {
+    const double x = lo + (hi - lo) * ((lane + 1) * (1.0 / 33.0));
+    double q = a[0] - x;
+    int c = q < 0.0;
+    for (int i = 1; i < m; i++) {
+      const double qq = (q == 0.0) ? 1e-300 : q;
+      q = a[i] - x - b[i - 1] * b[i - 1] / qq;
+      c += q < 0.0;
+    }
+    // the points above every eigenvalue: the lowest of them is the new upper end
+    const unsigned above = __ballot_sync(0xffffffffu, c >= m);
+    const int first = above ? __ffs(above) - 1 : 32;
+    const double up = __shfl_sync(0xffffffffu, x, first & 31), dn = __shfl_sync(0xffffffffu, x, (first - 1) & 31);
+    if (first < 32) hi = up;
+    if (first > 0) lo = dn;
+  }
+  const double lmax = m > 0 ? hi : 0.0;
+  if (lane != 0) return;
   P->lmax = lmax;
   if (!(lmax > 0.0)) {
     P->status = SRV_BREAKDOWN;
     return;
   }
-  const double hi = emax * lmax, lo = emin * lmax;
+  hi = emax * lmax;
+  lo = emin * lmax;
   const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), sigma = theta / delta;
   P->theta_inv = 1.0 / theta;
   double rho = 1.0 / sigma;
@@ -514,12 +586,12 @@ pt_status srv_apply_single<double>(pt_op *op, const double *u, double *y) { retu
 template <typename T, typename F>
 pt_status srv_precond(pt_server *s, const int2 *items, int64_t nitems, cudaStream_t st, F apply)
 {
-  srv_cheb_first_kernel<T><<<(unsigned)nitems, SRV_THREADS, 0, st>>>(items, s->d_slots, s->d_scal);
+  chain(srv_cheb_first_kernel<T>, (unsigned)nitems, SRV_THREADS, st, items, s->d_slots, s->d_scal);
   s->launches++;
   for (int k = 1; k < s->o.cheby_degree; k++) {
     pt_status e = apply();
     if (e != PT_OK) return e;
-    srv_cheb_step_kernel<T><<<(unsigned)nitems, SRV_THREADS, 0, st>>>(items, s->d_slots, s->d_scal, k);
+    chain(srv_cheb_step_kernel<T>, (unsigned)nitems, SRV_THREADS, st, items, s->d_slots, s->d_scal, k);
     s->launches++;
   }
   cudaError_t e = cudaGetLastError();
@@ -615,7 +687,7 @@ pt_status srv_admit(pt_server *s, SrvReq *r, int slot)
     lz_sum_kernel<2><<<1, SRV_THREADS, 0, st>>>(r->nch, lpart, L, k);
     lz_p_kernel<<<nb, SRV_THREADS, 0, st>>>(n, L, k, rr, p);
   }
-  lz_finish_kernel<<<1, 1, 0, st>>>(L, s->o.cheby_emin, s->o.cheby_emax, s->o.cheby_degree, s->d_scal + slot);
+  lz_finish_kernel<<<1, 32, 0, st>>>(L, s->o.cheby_emin, s->o.cheby_emax, s->o.cheby_degree, s->d_scal + slot);
   s->launches += 3 + 5 * its;
   // Krylov start: x = 0, p = 0, q = 0, r = f
   PT_CUDA(cudaMemsetAsync(r->vec, 0, sizeof(double) * (4 * n + 2 * r->nch), st));
@@ -734,19 +806,19 @@ pt_status srv_iterate(pt_server *s)
   pt_status e = batch_apply<double, true>(s->batch, (const double *const *)tab, (double *const *)(tab + n), st);
   if (e != PT_OK) return e;
   s->launches += pt_batch_launches_per_apply(s->batch) + (s->batch->coloured ? 1 : 0);
-  srv_pq_kernel<<<ni, SRV_THREADS, 0, st>>>(s->d_items, s->d_slots, s->d_scal);
-  srv_final_kernel<SRV_F_ALPHA><<<na, SRV_THREADS, 0, st>>>(s->d_act, s->d_slots, s->d_scal);
-  srv_update_kernel<<<ni, SRV_THREADS, 0, st>>>(s->d_items, s->d_slots, s->d_scal);
-  srv_final_kernel<SRV_F_RR><<<na, SRV_THREADS, 0, st>>>(s->d_act, s->d_slots, s->d_scal);
+  chain(srv_pq_kernel, ni, SRV_THREADS, st, s->d_items, s->d_slots, s->d_scal);
+  chain(srv_final_kernel<SRV_F_ALPHA>, na, SRV_THREADS, st, s->d_act, s->d_slots, s->d_scal);
+  chain(srv_update_kernel, ni, SRV_THREADS, st, s->d_items, s->d_slots, s->d_scal);
+  chain(srv_final_kernel<SRV_F_RR>, na, SRV_THREADS, st, s->d_act, s->d_slots, s->d_scal);
   s->launches += 4;
   e = srv_precond<T>(s, s->d_items, ni, st, [&]() {
     s->launches += pt_batch_launches_per_apply(s->batch) + (s->batch->coloured ? 1 : 0);
     return batch_apply<T, true>(s->batch, (const T *const *)(tab + 2 * n), (T *const *)(tab + 3 * n), st);
   });
   if (e != PT_OK) return e;
-  srv_zdots_kernel<T><<<ni, SRV_THREADS, 0, st>>>(s->d_items, s->d_slots, s->d_scal);
-  srv_final_kernel<SRV_F_BETA><<<na, SRV_THREADS, 0, st>>>(s->d_act, s->d_slots, s->d_scal);
-  srv_p_kernel<T><<<ni, SRV_THREADS, 0, st>>>(s->d_items, s->d_slots, s->d_scal);
+  chain(srv_zdots_kernel<T>, ni, SRV_THREADS, st, s->d_items, s->d_slots, s->d_scal);
+  chain(srv_final_kernel<SRV_F_BETA>, na, SRV_THREADS, st, s->d_act, s->d_slots, s->d_scal);
+  chain(srv_p_kernel<T>, ni, SRV_THREADS, st, s->d_items, s->d_slots, s->d_scal);
   s->launches += 3;
   cudaError_t ce = cudaGetLastError();
   if (ce != cudaSuccess) return fail(PT_ERR_CUDA, "server iteration launch: %s", cudaGetErrorString(ce));

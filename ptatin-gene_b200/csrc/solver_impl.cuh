@@ -177,8 +177,8 @@ unsigned vgrid(int64_t n)
 }
 
 // Largest eigenvalue of a symmetric tridiagonal matrix (diagonal a[0..n),
-// off-diagonal b[0..n-1)) by bisection on Sturm counts.  Host and device.
-__host__ __device__ inline double tridiag_lmax(const double *a, const double *b, int n)
+// off-diagonal b[0..n-1)) by bisection on Sturm counts.
+inline double tridiag_lmax(const double *a, const double *b, int n)
 {
   if (n == 0) return 0.0;
   double lo = a[0], hi = a[0];
