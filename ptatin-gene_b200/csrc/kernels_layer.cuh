@@ -904,61 +904,81 @@ enum { LAYER_PLAIN = 0, LAYER_BC_COPY = 1, LAYER_BC_ONE = 2, LAYER_BC_ZERO = 3, 
 // along x innermost, then rows, then layers, lower first.  BC_COPY: y_k = x_k
 // on Dirichlet dofs, BC_ONE / BC_ZERO: 1 / 0 there, ADD: added to y,
 // SUB: x subtracted.
-template <typename T, int NT, int MODE>
-__device__ __forceinline__ void layer_gather_node(const LayerGrid &g, uint32_t t, const T *s,
-                                                  const T *__restrict__ x, const uint32_t *__restrict__ mbits,
-                                                  T *__restrict__ y)
+struct LayerNode {
+  int64_t at[2][2][2];  // scratch offsets of the node's sums, -1 where there is none
+  int64_t k0;           // its first dof
+};
+template <int NT>
+__device__ __forceinline__ LayerNode layer_node_slots(const LayerGrid &g, uint32_t t)
 {
   using L = LayerLayout<NT>;
+  LayerNode n;
   const uint32_t jk = g.dNX.div(t);
   const int i = (int)(t - jk * g.dNX.d);
   const int k = (int)g.dNY.div(jk);
   const int j = (int)(jk - (uint32_t)k * g.dNY.d);
   const AxisNode ay = axis_node(j, g.my), az = axis_node(k, g.mz);
-  T acc[3] = {T(0), T(0), T(0)};
 #pragma unroll
   for (int q = 0; q < 2; q++)
 #pragma unroll
-    for (int p = 0; p < 2; p++)
+    for (int p = 0; p < 2; p++) {
+      n.at[q][p][0] = n.at[q][p][1] = -1;
       if (q < az.n && p < ay.n) {
-        int64_t at[2];
-        layer_slots<NT>(g, i, ay.e[p] + g.my * az.e[q], at);
+        layer_slots<NT>(g, i, ay.e[p] + g.my * az.e[q], n.at[q][p]);
         const int o = az.l[q] * L::PLANE + ay.l[p] * L::ROW;
 #pragma unroll
         for (int b = 0; b < 2; b++)
-          if (at[b] >= 0) {
-            const T *e = s + at[b] + o;
-#pragma unroll
-            for (int l = 0; l < 3; l++) acc[l] += __ldcg(e + l * L::COMP);  // not before the wait
-          }
+          if (n.at[q][p][b] >= 0) n.at[q][p][b] += o;
       }
-  const int64_t k0 = 3 * (g.off + i + j * g.X + k * g.XY);
+    }
+  n.k0 = 3 * (g.off + i + j * g.X + k * g.XY);
+  return n;
+}
+
+template <typename T, int NT, int MODE>
+__device__ __forceinline__ void layer_gather_node(const LayerNode &n, const T *s, const T *__restrict__ x,
+                                                  const uint32_t *__restrict__ mbits, T *__restrict__ y)
+{
+  using L = LayerLayout<NT>;
+  T acc[3] = {T(0), T(0), T(0)};
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int64_t at = n.at[i >> 2][i >> 1 & 1][i & 1];
+    if (at >= 0) {
+#pragma unroll
+      for (int l = 0; l < 3; l++) acc[l] += __ldcg(s + at + l * L::COMP);  // not before the wait
+    }
+  }
 #pragma unroll
   for (int l = 0; l < 3; l++) {
+    const int64_t k = n.k0 + l;
     T v = acc[l];
-    if (MODE == LAYER_ADD) v += y[k0 + l];
-    else if (MODE == LAYER_SUB) v -= x[k0 + l];
-    else if (MODE != LAYER_PLAIN && mbits && ((mbits[(k0 + l) >> 5] >> ((k0 + l) & 31)) & 1u))
-      v = MODE == LAYER_BC_COPY ? x[k0 + l] : T(MODE == LAYER_BC_ONE ? 1 : 0);
-    y[k0 + l] = v;
+    if (MODE == LAYER_ADD) v += y[k];
+    else if (MODE == LAYER_SUB) v -= x[k];
+    else if (MODE != LAYER_PLAIN && mbits && ((mbits[k >> 5] >> (k & 31)) & 1u))
+      v = MODE == LAYER_BC_COPY ? x[k] : T(MODE == LAYER_BC_ONE ? 1 : 0);
+    y[k] = v;
   }
 }
 
-// Nodes [t0, t1) of the element box.
+// Nodes [t0, t1) of the element box.  The offsets are worked out while the
+// tiles' kernel runs.
 template <typename T, int NT, int MODE>
 __global__ void __launch_bounds__(256) layer_gather_kernel(LayerGrid g, uint32_t t0, uint32_t t1,
                                                            const T *s, const T *__restrict__ x,
                                                            const uint32_t *__restrict__ mbits, T *__restrict__ y)
 {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t t = t0 + blockIdx.x * 256u + threadIdx.x;
-  if (t < t1) layer_gather_node<T, NT, MODE>(g, t, s, x, mbits, y);
+  if (t >= t1) return;
+  const LayerNode n = layer_node_slots<NT>(g, t);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  layer_gather_node<T, NT, MODE>(n, s, x, mbits, y);
 }
 
 // Batched forms: one work item per tile (problem, tile) and one per
 // LAYER_GATHER_NODES nodes (problem, first node); a problem's sums lie at its
 // own offset of the batch's scratch.
-constexpr int LAYER_GATHER_NODES = 1024;
+constexpr int LAYER_GATHER_NODES = 512;
 
 template <typename T, int NT, bool MASKED>
 __global__ void __launch_bounds__(NT, layer_min_blocks<T, NT>()) a11_layer_batch_kernel(const BatchProb *__restrict__ probs,
@@ -978,7 +998,6 @@ __global__ void __launch_bounds__(256) layer_gather_batch_kernel(const BatchProb
                                                                  const T *const *__restrict__ uptr, const T *scratch,
                                                                  T *const *__restrict__ yptr)
 {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int2 it = items[blockIdx.x];
   const BatchProb &p = probs[it.x];
   const LayerGrid g = p.lg;
@@ -986,10 +1005,16 @@ __global__ void __launch_bounds__(256) layer_gather_batch_kernel(const BatchProb
   const T *s = scratch + p.lay_off, *u = uptr[it.x];
   const uint32_t *mb = MASKED ? p.mbits : nullptr;
   T *y = yptr[it.x];
-#pragma unroll 1
-  for (int k = 0; k < LAYER_GATHER_NODES; k += 256) {
-    const uint32_t t = (uint32_t)it.y + k + threadIdx.x;
-    if (t < nodes) layer_gather_node<T, NT, MASKED ? LAYER_BC_COPY : LAYER_PLAIN>(g, t, s, u, mb, y);
+  uint32_t t = (uint32_t)it.y + threadIdx.x;
+  if (t >= nodes) return;
+  const uint32_t t1 = min(nodes, (uint32_t)it.y + LAYER_GATHER_NODES);
+  LayerNode n = layer_node_slots<NT>(g, t);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (;;) {
+    layer_gather_node<T, NT, MASKED ? LAYER_BC_COPY : LAYER_PLAIN>(n, s, u, mb, y);
+    t += 256;
+    if (t >= t1) break;
+    n = layer_node_slots<NT>(g, t);
   }
 }
 
