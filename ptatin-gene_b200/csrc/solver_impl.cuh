@@ -308,42 +308,151 @@ pt_status sv_setup_diag(pt_solver *s)
   return PT_OK;
 }
 
-// lambda_max(D^-1 A) of operator `op` (n dofs, inverse diagonal dinv) from
+// ---- Lanczos estimate on the device ------------------------------------------
+// The Jacobi-PCG recurrence without a host read per dot product: alpha_k and
+// beta_k are formed by the last block of the reduction that they need (a count
+// of finished blocks; nobody waits) and stay on the device, so a step is the
+// apply and three launches.  (Two host round trips and nine enqueues a step
+// were a third of a 40^3 hierarchy's set-up.)
+struct LanczosState {
+  double rz;
+  int m, stop;
+  unsigned done;  // finished blocks of the reduction under way
+};
+
+// Adds up `a` over the grid in a fixed order; true in every thread of the block
+// that finished last, with the sum in *sum.
+__device__ __forceinline__ bool lanczos_sum(double a, double *partial, LanczosState *L, double *sh, double *sum)
+{
+  __shared__ bool last;
+  a = block_sum<double>(a, sh);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = a;
+    __threadfence();
+    last = atomicAdd(&L->done, 1u) + 1 == gridDim.x;
+    if (last) L->done = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return false;
+  double t = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += RED_THREADS) t += __ldcg(partial + b);
+  *sum = block_sum<double>(t, sh);
+  return true;
+}
+
+// r = hash, z = p = D^-1 r, rz = r.z
+__global__ void __launch_bounds__(RED_THREADS) lanczos_start_kernel(int64_t n, const double *__restrict__ dinv, double *r,
+                                                                   double *p, double *partial, LanczosState *L)
+{
+  __shared__ double sh[RED_THREADS];
+  double a = 0.0, t;
+  for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)RED_BLOCKS * RED_THREADS) {
+    const double z = dinv[i] * r[i];
+    p[i] = z;
+    a = fma(r[i], z, a);
+  }
+  if (lanczos_sum(a, partial, L, sh, &t) && threadIdx.x == 0) {
+    L->rz = t;
+    L->m = 0;
+    L->stop = !(t > 0.0);
+  }
+}
+
+// alpha_k = rz / p.q
+__global__ void __launch_bounds__(RED_THREADS) lanczos_alpha_kernel(int64_t n, const double *p, const double *q, int k,
+                                                                   double *alpha, double *partial, LanczosState *L)
+{
+  __shared__ double sh[RED_THREADS];
+  if (L->stop) return;
+  double a = 0.0, t;
+  for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)RED_BLOCKS * RED_THREADS)
+    a = fma(p[i], q[i], a);
+  if (lanczos_sum(a, partial, L, sh, &t) && threadIdx.x == 0) {
+    if (t > 0.0) alpha[k] = L->rz / t;
+    else L->stop = 1;
+  }
+}
+
+// r -= alpha_k q; z = D^-1 r; beta_k = r.z / rz
+__global__ void __launch_bounds__(RED_THREADS) lanczos_beta_kernel(int64_t n, const double *__restrict__ dinv,
+                                                                  const double *q, double *r, double *z, int k,
+                                                                  const double *alpha, double *beta, double *partial,
+                                                                  LanczosState *L)
+{
+  __shared__ double sh[RED_THREADS];
+  if (L->stop) return;
+  const double al = alpha[k];
+  double a = 0.0, t;
+  for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)RED_BLOCKS * RED_THREADS) {
+    const double rv = fma(-al, q[i], r[i]), zv = dinv[i] * rv;
+    r[i] = rv;
+    z[i] = zv;
+    a = fma(rv, zv, a);
+  }
+  if (lanczos_sum(a, partial, L, sh, &t) && threadIdx.x == 0) {
+    beta[k] = t / L->rz;
+    L->rz = t;
+    L->m = k + 1;
+    if (!(t > 0.0)) L->stop = 1;
+  }
+}
+
+// p = z + beta_k p
+__global__ void lanczos_p_kernel(int64_t n, const double *z, double *p, int k, const double *beta, const LanczosState *L)
+{
+  if (L->stop) return;
+  const double b = beta[k];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    p[i] = fma(b, p[i], z[i]);
+}
+
+pt_status mg_pool(pt_solver *s);
+template <typename T>
+cudaError_t mg_alloc(pt_solver *s, T **p, size_t bytes);
+void mg_release(pt_solver *s, void *p);
+
+// lambda_max(D^-1 A) of an operator (n dofs, inverse diagonal dinv) from
 // eig_its steps of Jacobi-PCG on a pseudo-random rhs (Lanczos tridiagonal).
 // Uses the solver's FP64 work vectors (fine-level size >= n).
 template <typename ApplyFn>
 pt_status sv_lanczos_fn(pt_solver *s, int64_t n, const double *dinv, double *lmax, ApplyFn apply)
 {
-  double *b = s->t2, *p = s->t3, *q = s->w, *r = s->r, *z = s->t1;
+  double *p = s->t3, *q = s->w, *r = s->r, *z = s->t1;
   cudaStream_t st = s->op->stream;
-  hash_vec_kernel<<<vgrid(n), 256, 0, st>>>(b, n, 12345u);
-  PT_LAUNCHED(s->op);
-  PT_CUDA(cudaMemcpyAsync(r, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  cheb_first_kernel<double><<<vgrid(n), 256, 0, st>>>(1.0, dinv, r, z, p, n);  // z = p = D^-1 r
-  PT_LAUNCHED(s->op);
-  double rz;
-  pt_status stt = sv_dot(s, r, z, &rz, n);
+  const int its = std::max(0, s->o.eig_its);
+  pt_status stt = mg_pool(s);
   if (stt != PT_OK) return stt;
-  std::vector<double> alphas, betas, diag, off;
-  for (int k = 0; k < s->o.eig_its && rz > 0.0; k++) {
-    if ((stt = apply(p, q)) != PT_OK) return stt;
-    double pq;
-    if ((stt = sv_dot(s, p, q, &pq, n)) != PT_OK) return stt;
-    if (!(pq > 0.0)) break;
-    const double alpha = rz / pq;
-    if ((stt = sv_axpby<double>(s, -alpha, q, 1.0, r, n)) != PT_OK) return stt;
-    cheb_first_kernel<double><<<vgrid(n), 256, 0, st>>>(1.0, dinv, r, z, z, n);
-    PT_LAUNCHED(s->op);
-    double rz_new;
-    if ((stt = sv_dot(s, r, z, &rz_new, n)) != PT_OK) return stt;
-    const double beta = rz_new / rz;
-    if ((stt = sv_axpby<double>(s, 1.0, z, beta, p, n)) != PT_OK) return stt;
-    alphas.push_back(alpha);
-    betas.push_back(beta);
-    rz = rz_new;
+  // state, then alpha and beta
+  char *buf = nullptr;
+  const size_t head = 32, bytes = head + sizeof(double) * 2 * (size_t)std::max(1, its);
+  static_assert(sizeof(LanczosState) <= head, "state block");
+  PT_CUDA(mg_alloc(s, &buf, bytes));
+  LanczosState *L = reinterpret_cast<LanczosState *>(buf);
+  double *alpha = reinterpret_cast<double *>(buf + head), *beta = alpha + std::max(1, its);
+  cudaError_t e = cudaMemsetAsync(buf, 0, bytes, st);
+  hash_vec_kernel<<<vgrid(n), 256, 0, st>>>(r, n, 12345u);
+  lanczos_start_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, dinv, r, p, s->partial, L);
+  s->op->launches += 2;
+  for (int k = 0; k < its && e == cudaSuccess && stt == PT_OK; k++) {
+    if ((stt = apply(p, q)) != PT_OK) break;
+    lanczos_alpha_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, p, q, k, alpha, s->partial, L);
+    lanczos_beta_kernel<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, dinv, q, r, z, k, alpha, beta, s->partial, L);
+    lanczos_p_kernel<<<vgrid(n), 256, 0, st>>>(n, z, p, k, beta, L);
+    s->op->launches += 3;
+    e = cudaGetLastError();
   }
-  const int m = (int)alphas.size();
+  std::vector<char> host(bytes);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(host.data(), buf, bytes, cudaMemcpyDeviceToHost, st);
+  mg_release(s, buf);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (stt != PT_OK) return stt;
+  if (e != cudaSuccess) return fail(PT_ERR_CUDA, "eigenvalue estimate: %s", cudaGetErrorString(e));
+  const LanczosState *h = reinterpret_cast<const LanczosState *>(host.data());
+  const double *alphas = reinterpret_cast<const double *>(host.data() + head), *betas = alphas + std::max(1, its);
+  const int m = h->m;
   if (m == 0) return fail(PT_ERR_STATE, "eigenvalue estimate failed (A11 not positive definite?)");
+  std::vector<double> diag, off;
   for (int k = 0; k < m; k++) {
     double t = 1.0 / alphas[k];
     if (k > 0) t += betas[k - 1] / alphas[k - 1];
