@@ -28,6 +28,7 @@
 #include "kernels_ebe.cuh"
 #include "kernels_markers.cuh"
 #include "kernels_galerkin.cuh"
+#include "kernels_dense.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 

@@ -561,81 +561,42 @@ constexpr int64_t MG_EBE_MAX_ELEMENTS = 32768;  // levels up to 32^3 elements st
 constexpr int64_t MG_DENSE_MAX_DOFS = 1200;     // coarsest level solved by a dense inverse up to this size
 
 // Dense inverse of the coarsest level's masked operator (Dirichlet rows and
-// columns replaced by the identity), from its FP64 element matrices:
-// assembled on the host, Cholesky-factored, inverted, uploaded as T.
+// columns replaced by the identity), from its FP64 element matrices.
 pt_status mg_dense_inverse(pt_solver *s, pt_mg_level &L, bool fp32)
 {
   const pt_op *op = L.op;
-  const int64_t n = L.n, nel = op->nel;
-  double *dAe = L.Ae64;  // Galerkin level: its own matrices; else re-discretised ones
-  if (!dAe) {
-    PT_CUDA(mg_alloc(s, &dAe, sizeof(double) * ptk::EBE_LD * nel));
-    ptk::element_matrix_kernel<double><<<(unsigned)nel, 96, 0, op->stream>>>(op->box, op->d_coords, op->d_eta, dAe);
+  const cudaStream_t st = op->stream;
+  const int n = (int)L.n, nb = (n + ptk::DN_B - 1) / ptk::DN_B, np = nb * ptk::DN_B;
+  double *Ae = L.Ae64;  // Galerkin level: its own matrices; else re-discretised ones
+  if (!Ae) {
+    PT_CUDA(mg_alloc(s, &Ae, sizeof(double) * ptk::EBE_LD * op->nel));
+    ptk::element_matrix_kernel<double><<<(unsigned)op->nel, 96, 0, st>>>(op->box, op->d_coords, op->d_eta, Ae);
   }
-  std::vector<double> Ae(ptk::EBE_LD * nel), A(n * n, 0.0);
-  std::vector<uint8_t> mask(n);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(Ae.data(), dAe, sizeof(double) * Ae.size(), cudaMemcpyDeviceToHost, op->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(mask.data(), op->d_mask, n, cudaMemcpyDeviceToHost, op->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(op->stream);
-  if (dAe != L.Ae64) mg_release(s, dAe);
-  if (e != cudaSuccess) return fail(PT_ERR_CUDA, "coarse element matrices: %s", cudaGetErrorString(e));
-  const int64_t X = op->box.X, XY = op->box.XY;
-  for (int64_t el = 0; el < nel; el++) {
-    const int64_t ei = el % op->mx, ej = (el / op->mx) % op->my, ek = el / ((int64_t)op->mx * op->my);
-    int64_t g[81];
-    for (int nn = 0; nn < 27; nn++) {
-      const int64_t node = (2 * ei + nn % 3) + (2 * ej + (nn / 3) % 3) * X + (2 * ek + nn / 9) * XY;
-      for (int l = 0; l < 3; l++) g[3 * nn + l] = 3 * node + l;
-    }
-    const double *m = &Ae[el * ptk::EBE_LD];
-    for (int jj = 0; jj < 81; jj++) {
-      if (mask[g[jj]]) continue;
-      for (int ii = 0; ii < 81; ii++)
-        if (!mask[g[ii]]) A[g[ii] * n + g[jj]] += m[ptk::ebe_sym(ii, jj)];
-    }
+  // the matrix, the panels, the pivot block's inverse, the check
+  double *A = nullptr;
+  const size_t values = (size_t)np * np + 2 * (size_t)np * ptk::DN_B + ptk::DN_B * ptk::DN_B;
+  PT_CUDA(mg_alloc(s, &A, sizeof(double) * values + sizeof(int)));
+  double *R = A + (size_t)np * np, *C = R + (size_t)np * ptk::DN_B, *D = C + (size_t)np * ptk::DN_B;
+  int *bad = reinterpret_cast<int *>(A + values);
+  PT_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
+  ptk::dense_assemble_kernel<<<(unsigned)np, 96, 0, st>>>(op->box, Ae, op->d_mask, n, np, A);
+  for (int k = 0; k < nb; k++) {
+    ptk::dense_pivot_kernel<<<1, ptk::DN_B * ptk::DN_B, 0, st>>>(A, np, k, D, bad);
+    ptk::dense_panel_kernel<<<(unsigned)nb, 256, 0, st>>>(A, np, k, D, R, C);
+    ptk::dense_update_kernel<<<dim3((unsigned)nb, (unsigned)nb), 256, 0, st>>>(A, np, k, R, C);
   }
-  for (int64_t i = 0; i < n; i++)
-    if (mask[i]) A[i * n + i] = 1.0;
-  // A = L L^T (lower triangle in place), W = L^-1, A^-1 = W^T W
-  for (int64_t j = 0; j < n; j++) {
-    double d = A[j * n + j];
-    for (int64_t k = 0; k < j; k++) d -= A[j * n + k] * A[j * n + k];
-    if (!(d > 0.0)) return fail(PT_ERR_STATE, "coarse operator is not positive definite");
-    d = std::sqrt(d);
-    A[j * n + j] = d;
-    for (int64_t i = j + 1; i < n; i++) {
-      double v = A[i * n + j];
-      for (int64_t k = 0; k < j; k++) v -= A[i * n + k] * A[j * n + k];
-      A[i * n + j] = v / d;
-    }
-  }
-  std::vector<double> W(n * n, 0.0);
-  for (int64_t c = 0; c < n; c++) {  // column c of L^-1 by forward substitution
-    W[c * n + c] = 1.0 / A[c * n + c];
-    for (int64_t i = c + 1; i < n; i++) {
-      double v = 0.0;
-      for (int64_t k = c; k < i; k++) v -= A[i * n + k] * W[k * n + c];
-      W[i * n + c] = v / A[i * n + i];
-    }
-  }
-  std::vector<double> inv(n * n, 0.0);
-  for (int64_t i = 0; i < n; i++)
-    for (int64_t j = 0; j <= i; j++) {
-      double v = 0.0;
-      for (int64_t k = i; k < n; k++) v += W[k * n + i] * W[k * n + j];
-      inv[i * n + j] = inv[j * n + i] = v;
-    }
-  const size_t ts = fp32 ? sizeof(float) : sizeof(double);
-  PT_CUDA(mg_alloc(s, &L.Ainv, ts * n * n));
-  if (fp32) {
-    std::vector<float> f(inv.begin(), inv.end());
-    PT_CUDA(cudaMemcpyAsync(L.Ainv, f.data(), ts * n * n, cudaMemcpyHostToDevice, op->stream));
-    PT_CUDA(cudaStreamSynchronize(op->stream));
-  } else {
-    PT_CUDA(cudaMemcpyAsync(L.Ainv, inv.data(), ts * n * n, cudaMemcpyHostToDevice, op->stream));
-    PT_CUDA(cudaStreamSynchronize(op->stream));
-  }
+  L.op->launches += 1 + 3 * nb;
+  PT_CUDA(mg_alloc(s, &L.Ainv, (fp32 ? sizeof(float) : sizeof(double)) * (size_t)n * n));
+  if (fp32) ptk::dense_copy_kernel<float><<<vgrid((int64_t)n * n), 256, 0, st>>>(A, np, n, (float *)L.Ainv);
+  else ptk::dense_copy_kernel<double><<<vgrid((int64_t)n * n), 256, 0, st>>>(A, np, n, (double *)L.Ainv);
+  PT_LAUNCHED(L.op);
+  int h_bad = 0;
+  cudaError_t e = cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  mg_release(s, A);
+  if (Ae != L.Ae64) mg_release(s, Ae);
+  if (e != cudaSuccess) return fail(PT_ERR_CUDA, "coarse inverse: %s", cudaGetErrorString(e));
+  if (h_bad) return fail(PT_ERR_STATE, "coarse operator is not positive definite");
   return PT_OK;
 }
 
