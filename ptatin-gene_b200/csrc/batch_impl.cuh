@@ -263,6 +263,10 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
         uint64_t keep = UINT64_MAX;  // kept from apply to apply, given back with the batch
         e = cudaMemPoolSetAttribute(b->lay_pool, cudaMemPoolAttrReleaseThreshold, &keep);
       }
+      // one FP64 apply's scratch is there before the first apply
+      void *first = nullptr;
+      if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&first, sizeof(double) * (size_t)b->lay_values, b->lay_pool, stream);
+      if (e == cudaSuccess) e = cudaFreeAsync(first, stream);
     }
   }
   if (e != cudaSuccess) {

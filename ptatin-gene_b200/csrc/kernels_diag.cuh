@@ -116,9 +116,8 @@ __device__ __forceinline__ void diag_tile(const StreamGrid &g, int tx, int ej, i
     }
     __syncthreads();
     if (ek == ek0) asm volatile("griddepcontrol.wait;" ::: "memory");
-    flush_plane<double, TX>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek, s0, ek == ek0 && zlo_shared, y);
-    flush_plane<double, TX>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek + 1, s1, false, y);
-    if (!more) flush_plane<double, TX>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek + 2, s2, zhi_shared, y);
+    flush_planes<double, TX, 2>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek, s0, ek == ek0 && zlo_shared, y);
+    if (!more) flush_planes<double, TX, 1>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek + 2, s2, zhi_shared, y);
     // the flushed slots (zeroed as read) take the next layer's sums
     if (more) __syncthreads();
   }

@@ -153,37 +153,47 @@ __device__ __forceinline__ void stage_mask(uint32_t *mw, const StreamGrid &g, in
   }
 }
 
-// Fetches node plane P (rows 0..2) of u into slot s with asynchronous 4- or
-// 8-byte copies straight into the component-planar tile (cp.async: no
-// registers, the copies run while the thread flushes y).  MASKED: the
-// Dirichlet entries, whose bits the slot's staged mask words hold (visible to
-// every thread), are written as zeros instead -- the MatShell apply's column
-// rule.  The caller commits and waits.
-template <typename T, int TX, bool MASKED>
-__device__ __forceinline__ void fetch_plane(T *ut, const uint32_t *mw, const StreamGrid &g, int ex0, int ej, int64_t P,
-                                            int s, const T *__restrict__ u, bool mk)
+// Fetches node planes P0 .. P0+NP-1 (rows 0..2) of u into slots s0, s0+1, ..
+// (modulo 3) with asynchronous 4- or 8-byte copies straight into the
+// component-planar tile (cp.async: no registers, the copies run while the
+// thread flushes y).  A thread's values d = t, t + TX, .. of a row lie at the
+// same entries in every row and plane, so the entry is worked out once per d
+// and the 3 NP rows' copies are issued side by side.  MASKED: the Dirichlet
+// entries, whose bits the slots' staged mask words hold (visible to every
+// thread), are zero-filled instead -- the MatShell apply's column rule.  The
+// caller commits and waits.
+template <typename T, int TX, bool MASKED, int NP>
+__device__ __forceinline__ void fetch_planes(T *ut, const uint32_t *mw, const StreamGrid &g, int ex0, int ej,
+                                             int64_t P0, int s0, const T *__restrict__ u, bool mk)
 {
   using L = TileLayout<TX>;
   const int nd = 3 * min(L::NXN, 2 * (g.b.mx - ex0) + 1);
+  const int64_t k00 = 3 * row_node0(g, ex0, ej, 0, P0);
 #pragma unroll 1
-  for (int r = 0; r < 3; r++) {
-    const int64_t k0 = 3 * row_node0(g, ex0, ej, r, P);
-    const T *src = u + k0;
-    const uint32_t *w = mw + (s * 3 + r) * mask_row_words<TX>();
-    const int b0 = (int)(k0 & 31);
-    for (int d = threadIdx.x; d < nd; d += TX) {
-      const int n = d / 3, c = d - 3 * n;
-      T *dst = &ut[L::at(c, s, r, n)];
-      if (MASKED && mk) {
-        const int pos = b0 + d;
-        if ((w[pos >> 5] >> (pos & 31)) & 1u) {
-          *dst = T(0);
-          continue;
+  for (int d = threadIdx.x; d < nd; d += TX) {
+    const int n = d / 3, c = d - 3 * n;
+    T *dst = ut + L::at(c, 0, 0, n);
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      const int s = s0 + k < 3 ? s0 + k : s0 + k - 3;
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        const int64_t k0 = k00 + 3 * (k * g.b.XY + r * g.b.X);
+        uint32_t bytes = sizeof(T);
+        if (MASKED && mk) {
+          const int pos = (int)(k0 & 31) + d;
+          if ((mw[(s * 3 + r) * mask_row_words<TX>() + (pos >> 5)] >> (pos & 31)) & 1u) bytes = 0;
         }
+        const uint32_t sd = (uint32_t)__cvta_generic_to_shared(dst + s * L::PLANE + r * L::ROW);
+        if (!MASKED && sizeof(T) == 8)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sd), "l"(u + k0 + d) : "memory");
+        else if (!MASKED)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sd), "l"(u + k0 + d) : "memory");
+        else if (sizeof(T) == 8)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(sd), "l"(u + k0 + d), "r"(bytes) : "memory");
+        else
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sd), "l"(u + k0 + d), "r"(bytes) : "memory");
       }
-      const uint32_t sd = (uint32_t)__cvta_generic_to_shared(dst);
-      if (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sd), "l"(src + d) : "memory");
-      else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sd), "l"(src + d) : "memory");
     }
   }
 }
@@ -221,43 +231,63 @@ __device__ __forceinline__ void zero_slot(T *yt, T *side, int s)
   }
 }
 
-// Flush node plane P (in slot s) to global y, zeroing each y-tile (and side
-// buffer) entry as it is read, so the slot is ready for its next plane with
-// no further pass or barrier.  zshared: the plane is the chunk's first/last
-// plane and shared with a neighbouring chunk.  A node on a
+// Flush node planes P0 .. P0+NP-1 (in slots s0, s0+1, .. modulo 3) to global y,
+// zeroing each y-tile (and side buffer) entry as it is read, so the slots are
+// ready for their next planes with no further pass or barrier.  zshared: P0 is
+// shared with a neighbouring chunk.  A node on a
 // tile boundary is stored by the first colour that touches it and added to
 // by the later ones; the colours are separate launches in a fixed order and
 // a launch touches each node from one CTA only, so the adds (red.global.add,
 // no read-back) happen in a fixed order: the sums are deterministic and equal
 // to a read-modify-write.  Dirichlet rows are set after the colour passes.
-template <typename T, int TX>
-__device__ __forceinline__ void flush_plane(T *yt, T *side, const StreamGrid &g, int tx, int ex0, int ej, int64_t P,
-                                            int s, bool zshared, T *__restrict__ y)
+// As in the fetch an entry is worked out once for its 3 NP rows, whose reads
+// are issued side by side.
+template <typename T, int TX, int NP>
+__device__ __forceinline__ void flush_planes(T *yt, T *side, const StreamGrid &g, int tx, int ex0, int ej, int64_t P0,
+                                             int s0, bool zshared, T *__restrict__ y)
 {
   using L = TileLayout<TX>;
-  const int nvalid = min(L::NXN, 2 * (g.b.mx - ex0) + 1);
+  const int nd = 3 * min(L::NXN, 2 * (g.b.mx - ex0) + 1);
   const bool xlo = tx > 0, xhi = ex0 + TX < g.b.mx;
-  const bool ylo = ej > 0, yhi = ej < g.b.my - 1;
-  const int nd = 3 * nvalid;
+  const int64_t k00 = 3 * row_node0(g, ex0, ej, 0, P0);
+  // rows (bit 3k + r) that an earlier colour has stored, wherever along x
+  unsigned later = 0;
+  if (g.py) later |= (ej > 0 ? 1u : 0u) * 0x49u | (ej < g.b.my - 1 ? 1u : 0u) * 0x124u;
+  if (zshared && g.pz) later |= 7u;
 #pragma unroll 1
-  for (int r = 0; r < 3; r++) {
-    const int64_t node0 = row_node0(g, ex0, ej, r, P);
-    const bool yb = (r == 0 && ylo) || (r == 2 && yhi);
-    for (int d = threadIdx.x; d < nd; d += TX) {
-      const int n = d / 3, c = d - 3 * n;
-      T v = yt[L::at(c, s, r, n)];
-      yt[L::at(c, s, r, n)] = T(0);
-      if (L::NW > 1 && (n & 63) == 0 && n > 0 && n < 2 * TX) {
-        T *sb = &side[((n >> 6) - 1) * 27 + s * 9 + r * 3 + c];
-        v += *sb;
-        *sb = T(0);
-      }
-      const int64_t k = 3 * node0 + d;
-      const bool xb = (n == 0 && xlo) || (n == 2 * TX && xhi);
-      const bool first = !((xb && g.px) || (yb && g.py) || (zshared && g.pz));
-      if (first) y[k] = v;
-      else atomicAdd(&y[k], v);
+  for (int d = threadIdx.x; d < nd; d += TX) {
+    const int n = d / 3, c = d - 3 * n;
+    T *src = yt + L::at(c, 0, 0, n);
+    const bool seam = L::NW > 1 && (n & 63) == 0 && n > 0 && n < 2 * TX;
+    T v[3 * NP];
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      const int s = s0 + k < 3 ? s0 + k : s0 + k - 3;
+#pragma unroll
+      for (int r = 0; r < 3; r++) v[3 * k + r] = src[s * L::PLANE + r * L::ROW];
     }
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      const int s = s0 + k < 3 ? s0 + k : s0 + k - 3;
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        src[s * L::PLANE + r * L::ROW] = T(0);
+        if (seam) {
+          T *sb = &side[((n >> 6) - 1) * 27 + s * 9 + r * 3 + c];
+          v[3 * k + r] += *sb;
+          *sb = T(0);
+        }
+      }
+    }
+    const bool xb = g.px && ((n == 0 && xlo) || (n == 2 * TX && xhi));
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        T *p = y + k00 + 3 * (k * g.b.XY + r * g.b.X) + d;
+        if (xb || ((later >> (3 * k + r)) & 1u)) atomicAdd(p, v[3 * k + r]);
+        else *p = v[3 * k + r];
+      }
   }
 }
 
@@ -457,10 +487,7 @@ __device__ __forceinline__ void stream_tile(const StreamGrid &g, int tx, int ej,
   }
   for (int k = 0; k < 3; k++) zero_slot<T, TX>(yt, side, (int)((2 * (int64_t)ek0 + k) % 3));
   __syncthreads();
-  for (int k = 0; k < 3; k++) {
-    const int64_t P = 2 * (int64_t)ek0 + k;
-    fetch_plane<T, TX, MASKED>(ut, mw, g, ex0, ej, P, (int)(P % 3), u, mk);
-  }
+  fetch_planes<T, TX, MASKED, 3>(ut, mw, g, ex0, ej, 2 * (int64_t)ek0, (int)(2 * (int64_t)ek0 % 3), u, mk);
   fetch_commit();
   fetch_wait();
   __syncthreads();
@@ -511,8 +538,7 @@ __device__ __forceinline__ void stream_tile(const StreamGrid &g, int tx, int ej,
     // planes 2ek and 2ek+1 (complete for this CTA) are flushed and their y
     // slots zeroed for the next layer
     if (more) {
-      fetch_plane<T, TX, MASKED>(ut, mw, g, ex0, ej, 2 * (int64_t)ek + 3, s0, u, mk);
-      fetch_plane<T, TX, MASKED>(ut, mw, g, ex0, ej, 2 * (int64_t)ek + 4, s1, u, mk);
+      fetch_planes<T, TX, MASKED, 2>(ut, mw, g, ex0, ej, 2 * (int64_t)ek + 3, s0, u, mk);
       fetch_commit();
     }
     // y is written from here on: the previous grid in the stream (an earlier
@@ -521,9 +547,8 @@ __device__ __forceinline__ void stream_tile(const StreamGrid &g, int tx, int ej,
     // point, so a programmatic launch is only made where the previous grid
     // does not write them (the colours after the first of one apply).
     if (ek == ek0) asm volatile("griddepcontrol.wait;" ::: "memory");
-    flush_plane<T, TX>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek, s0, ek == ek0 && zlo_shared, y);
-    flush_plane<T, TX>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek + 1, s1, false, y);
-    if (!more) flush_plane<T, TX>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek + 2, s2, zhi_shared, y);
+    flush_planes<T, TX, 2>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek, s0, ek == ek0 && zlo_shared, y);
+    if (!more) flush_planes<T, TX, 1>(yt, side, g, tx, ex0, ej, 2 * (int64_t)ek + 2, s2, zhi_shared, y);
     if (more) {
       fetch_wait();
       __syncthreads();

@@ -472,6 +472,27 @@ pt_status launch_stream(pt_op *op, const T *K, const T *u, T *y)
   return launch_stream_tx<T, 128, MASKED>(op, K, u, y);
 }
 
+// FP32 copies of coordinates and viscosity for the 8-colour FP32 kernel,
+// allocated as soon as an op turns to that kernel.
+pt_status ensure_f32(pt_op *op)
+{
+  if (op->d_eta32) return PT_OK;
+  if (!op->d_coords32) PT_CUDA(op_alloc(op, (void **)&op->d_coords32, sizeof(float) * op->nvel));
+  PT_CUDA(op_alloc(op, (void **)&op->d_eta32, sizeof(float) * 27 * op->nel));
+  return PT_OK;
+}
+
+// K in FP64, in FP32 and the check counter, one allocation.
+pt_status alloc_geometry(pt_op *op)
+{
+  if (op->d_K) return PT_OK;
+  const size_t nk = (size_t)ptk::ksize(op->nel);
+  PT_CUDA(op_alloc(op, (void **)&op->d_K, (sizeof(double) + sizeof(float)) * nk + sizeof(unsigned int)));
+  op->d_K32 = reinterpret_cast<float *>(op->d_K + nk);
+  op->d_bad = reinterpret_cast<unsigned int *>(op->d_K32 + nk);
+  return PT_OK;
+}
+
 // K in FP64 and FP32, P once the whole operator has been used, and the count of
 // points with c <= 0, on the op's stream.
 pt_status launch_geometry(pt_op *op)
@@ -493,12 +514,8 @@ pt_status launch_geometry(pt_op *op)
 pt_status ensure_geometry(pt_op *op)
 {
   if (!op->geom_dirty) return PT_OK;
-  const int64_t nk = ptk::ksize(op->nel);
-  if (!op->d_K) {
-    PT_CUDA(op_alloc(op, (void **)&op->d_K, sizeof(double) * nk));
-    PT_CUDA(op_alloc(op, (void **)&op->d_K32, sizeof(float) * nk));
-    PT_CUDA(op_alloc(op, (void **)&op->d_bad, sizeof(unsigned int)));
-  }
+  pt_status ks = alloc_geometry(op);
+  if (ks != PT_OK) return ks;
   if (op->a11_kernel == A11_LAYER || (op->a11_kernel == A11_STREAM && op->a11_auto && op->nel < LAYER_F32_MAX_ELEMENTS)) {
     pt_status s = ensure_layer(op);
     if (s != PT_OK) return s;
@@ -509,6 +526,10 @@ pt_status ensure_geometry(pt_op *op)
   PT_CUDA(cudaMemcpyAsync(&bad, op->d_bad, sizeof bad, cudaMemcpyDeviceToHost, op->stream));
   PT_CUDA(cudaStreamSynchronize(op->stream));
   op->geom_ok = (bad == 0);
+  if (!op->geom_ok) {
+    pt_status fs = ensure_f32(op);
+    if (fs != PT_OK) return fs;
+  }
   op->geom_dirty = false;
   op->ebe_valid = false;
   return PT_OK;
@@ -605,7 +626,7 @@ template <>
 const float *op_K<float>(const pt_op *op) { return op->d_K32; }
 
 template <typename T>
-pt_status launch_a11(pt_op *op, const T *coords, const T *eta, const T *u, T *y, bool masked)
+pt_status launch_a11(pt_op *op, const T *u, T *y, bool masked)
 {
   if (op->a11_kernel == A11_EBE && op->full_box) {
     pt_status s = ensure_geometry(op);
@@ -638,7 +659,15 @@ pt_status launch_a11(pt_op *op, const T *coords, const T *eta, const T *u, T *y,
     }
   }
   PT_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * op->nvel, op->stream));
-  if (sizeof(T) == 4) {  // only this kernel reads the FP32 coordinates and viscosity
+  const T *coords = nullptr, *eta = nullptr;
+  if constexpr (sizeof(T) == 8) {
+    coords = op->d_coords;
+    eta = op->d_eta;
+  } else {  // only this kernel reads the FP32 coordinates and viscosity
+    pt_status s = ensure_f32(op);
+    if (s != PT_OK) return s;
+    coords = op->d_coords32;
+    eta = op->d_eta32;
     to_f32_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_coords, op->d_coords32, op->nvel);
     PT_LAUNCHED(op);
     to_f32_kernel<<<grid_stride_blocks(27 * op->nel), 256, 0, op->stream>>>(op->d_eta, op->d_eta32, 27 * op->nel);
@@ -1012,8 +1041,6 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   }
   if (e == cudaSuccess) e = op_alloc(op, (void **)&op->d_coords, sizeof(double) * op->nvel);
   if (e == cudaSuccess) e = op_alloc(op, (void **)&op->d_eta, sizeof(double) * 27 * op->nel);
-  if (e == cudaSuccess) e = op_alloc(op, (void **)&op->d_coords32, sizeof(float) * op->nvel);
-  if (e == cudaSuccess) e = op_alloc(op, (void **)&op->d_eta32, sizeof(float) * 27 * op->nel);
   if (e == cudaSuccess) e = op_alloc(op, (void **)&op->d_mask, op->nvel);
   if (e == cudaSuccess) e = cudaMemsetAsync(op->d_mask, 0, op->nvel, op->stream);
   if (e == cudaSuccess && !pool) e = cudaStreamSynchronize(op->stream);
@@ -1035,7 +1062,7 @@ pt_status pt_op_destroy(pt_op *op)
   // pooled ops free in stream order (after the op's queued work); others wait
   if (op->stream && !op->pool) cudaStreamSynchronize(op->stream);
   void *bufs[] = {op->d_coords, op->d_eta, op->d_coords32, op->d_eta32, op->d_mask, op->d_u,
-                  op->d_y, op->d_p, op->d_K, op->d_K32, op->d_bad, op->d_Ae, op->d_Ae32, op->d_ye,
+                  op->d_y, op->d_p, op->d_K, op->d_Ae, op->d_Ae32, op->d_ye,
                   op->mk_scratch, op->d_D, op->d_P, op->d_yp, op->d_mbits, op->d_fu, op->d_F, op->d_layer};
   for (void *b : bufs) op_free(op, b);
   for (int b = 0; b < 2; b++)
@@ -1208,7 +1235,7 @@ pt_status pt_a11_apply_d(pt_op *op, const double *u, double *y)
   pt_status s = check_ready(op, true);
   if (s != PT_OK) return s;
   if (!u || !y) return fail(PT_ERR_BAD_ARG, "NULL vector");
-  return launch_a11<double>(op, op->d_coords, op->d_eta, u, y, false);
+  return launch_a11<double>(op, u, y, false);
 }
 
 pt_status pt_a11_apply_h(pt_op *op, const double *u, double *y)
@@ -1220,7 +1247,7 @@ pt_status pt_a11_apply_h(pt_op *op, const double *u, double *y)
   if (u && y && (s = a11_host_pipelined<false>(op, u, y, &done)) != PT_OK) return s;
   if (done) return PT_OK;
   return host_call(op, u, op->nvel, op->d_u, y, op->nvel, op->d_y,
-                   [&]() { return launch_a11<double>(op, op->d_coords, op->d_eta, op->d_u, op->d_y, false); });
+                   [&]() { return launch_a11<double>(op, op->d_u, op->d_y, false); });
 }
 
 pt_status pt_a11_apply_f32_d(pt_op *op, const float *u, float *y)
@@ -1228,7 +1255,7 @@ pt_status pt_a11_apply_f32_d(pt_op *op, const float *u, float *y)
   pt_status s = check_ready(op, true);
   if (s != PT_OK) return s;
   if (!u || !y) return fail(PT_ERR_BAD_ARG, "NULL vector");
-  return launch_a11<float>(op, op->d_coords32, op->d_eta32, u, y, false);
+  return launch_a11<float>(op, u, y, false);
 }
 
 pt_status pt_a11_diag_d(pt_op *op, double *d)
@@ -1287,7 +1314,7 @@ pt_status pt_matmult_a11_d(pt_op *op, const double *x, double *y)
   if (s != PT_OK) return s;
   if (!x || !y) return fail(PT_ERR_BAD_ARG, "NULL vector");
   if (x == y) return fail(PT_ERR_BAD_ARG, "x and y must not alias");
-  if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, x, y, op->has_mask)) != PT_OK) return s;
+  if ((s = launch_a11<double>(op, x, y, op->has_mask)) != PT_OK) return s;
   if (a11_sets_bc_rows(op)) return PT_OK;
   return bc_copy(op, x, y);
 }
@@ -1310,7 +1337,7 @@ pt_status pt_matmult_a11_f32_d(pt_op *op, const float *x, float *y)
   if (s != PT_OK) return s;
   if (!x || !y) return fail(PT_ERR_BAD_ARG, "NULL vector");
   if (x == y) return fail(PT_ERR_BAD_ARG, "x and y must not alias");
-  if ((s = launch_a11<float>(op, op->d_coords32, op->d_eta32, x, y, op->has_mask)) != PT_OK) return s;
+  if ((s = launch_a11<float>(op, x, y, op->has_mask)) != PT_OK) return s;
   if (a11_sets_bc_rows(op)) return PT_OK;
   return bc_copy32(op, x, y);
 }
@@ -1373,7 +1400,7 @@ pt_status pt_stokes_a_apply_d(pt_op *op, const double *u, const double *p, doubl
   if (u == yu) return fail(PT_ERR_BAD_ARG, "u and yu must not alias");
   bool done;
   if ((s = stokes_fused(op, u, p, nullptr, yu, yp, ptk::LAYER_PLAIN, &done)) != PT_OK || done) return s;
-  if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, u, yu, false)) != PT_OK) return s;
+  if ((s = launch_a11<double>(op, u, yu, false)) != PT_OK) return s;
   if ((s = a12_d(op, p, yu, true)) != PT_OK) return s;
   return a21_d(op, u, yp, false);
 }
@@ -1388,7 +1415,7 @@ pt_status pt_matmult_a_d(pt_op *op, const double *xu, const double *xp, double *
   s = stokes_fused(op, xu, xp, xu, yu, yp, op->has_mask ? ptk::LAYER_BC_COPY : ptk::LAYER_PLAIN, &done);
   if (s != PT_OK || done) return s;
   // Dirichlet columns zeroed inside the masked kernels; rows set back to x after B^T p
-  if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, xu, yu, op->has_mask)) != PT_OK) return s;
+  if ((s = launch_a11<double>(op, xu, yu, op->has_mask)) != PT_OK) return s;
   if ((s = a12_d(op, xp, yu, true)) != PT_OK) return s;
   if ((s = bc_copy(op, xu, yu)) != PT_OK) return s;
   return a21_d(op, xu, yp, op->has_mask);
@@ -1497,7 +1524,7 @@ pt_status pt_residual_u_d(pt_op *op, const double *u, const double *p, double *r
   bool done;
   if ((s = ensure_body_force(op)) != PT_OK) return s;
   if ((s = stokes_fused(op, u, p, op->d_F, ru, nullptr, ptk::LAYER_SUB, &done)) != PT_OK || done) return s;
-  if ((s = launch_a11<double>(op, op->d_coords, op->d_eta, u, ru, false)) != PT_OK) return s;
+  if ((s = launch_a11<double>(op, u, ru, false)) != PT_OK) return s;
   if ((s = a12_d(op, p, ru, true)) != PT_OK) return s;
   sub_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_F, ru, op->nvel);
   PT_LAUNCHED(op);
@@ -1644,7 +1671,11 @@ pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
       return fail(PT_ERR_UNSUPPORTED, "b200_layer takes boxes of at most %lld elements", (long long)LAYER_MAX_ELEMENTS);
     op->a11_kernel = A11_LAYER;
   }
-  else if (!strcmp(name, "b200_colour")) op->a11_kernel = A11_COLOUR;
+  else if (!strcmp(name, "b200_colour")) {
+    pt_status s = ensure_f32(op);
+    if (s != PT_OK) return s;
+    op->a11_kernel = A11_COLOUR;
+  }
   else return fail(PT_ERR_BAD_ARG, "No -a11_op %s", name);
   op->a11_auto = !by_name;
   return PT_OK;

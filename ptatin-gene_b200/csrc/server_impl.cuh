@@ -603,10 +603,8 @@ pt_status srv_precond(pt_server *s, const int2 *items, int64_t nitems, cudaStrea
 // w*eta/detJ <= 0 goes to pinned memory, read when the set-up has completed.
 pt_status srv_geometry(pt_op *op, unsigned int *h_bad)
 {
-  const int64_t nk = ptk::ksize(op->nel);
-  PT_CUDA(op_alloc(op, (void **)&op->d_K, sizeof(double) * nk));
-  PT_CUDA(op_alloc(op, (void **)&op->d_K32, sizeof(float) * nk));
-  PT_CUDA(op_alloc(op, (void **)&op->d_bad, sizeof(unsigned int)));
+  pt_status ks = alloc_geometry(op);
+  if (ks != PT_OK) return ks;
   if (op->a11_kernel == A11_LAYER) {
     pt_status s = ensure_layer(op);
     if (s != PT_OK) return s;
