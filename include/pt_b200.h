@@ -388,7 +388,8 @@ pt_status pt_residual_u_h(pt_op *op, const double *u, const double *p, double *r
 pt_status pt_op_set_a11_kernel(pt_op *op, const char *name);
 const char *pt_op_get_a11_kernel(const pt_op *op);
 /* Tile schedule of the streaming kernel: element layers per z-chunk of a CTA
- * (0 = the default, about 2048 tiles); the other kernels have none.  Changes the summation order, so
+ * (0 = the default: about 2048 tiles for a small box, else the depth that fills
+ * the resident tiles best); the other kernels have none.  Changes the summation order, so
  * results differ in the last bits between schedules (each is deterministic).
  * No counterpart in the reference; set by the autotuner. */
 pt_status pt_op_set_tiling(pt_op *op, int32_t lz);

@@ -1681,17 +1681,69 @@ pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
   return PT_OK;
 }
 
+// Layers that one colour class of n chunks (the last one `tail` layers long when
+// has_tail) by `lines` tiles takes on `slots` resident tiles, one wave after the
+// other, the short tiles last.
+static double class_layers(int64_t n, int64_t lines, int lz, int tail, bool has_tail, int64_t slots)
+{
+  const int64_t full = (n - (has_tail ? 1 : 0)) * lines;
+  int64_t shorts = has_tail ? lines : 0;
+  const int64_t q = full / slots, rem = full % slots;
+  double t = (double)(q + (rem ? 1 : 0)) * lz;
+  if (rem && tail > 0) shorts -= std::min(shorts, (slots - rem) * (lz / tail));  // beside the last full wave
+  return t + (double)((shorts + slots - 1) / slots) * tail;
+}
+
+// Layers that all colour classes take, one after the other, with chunks of lz
+// layers on `slots` resident tiles, a start-up of half a layer per wave included.
+static double tiling_layers(const pt_op *op, int lz, int64_t slots)
+{
+  const int n = (op->mz + lz - 1) / lz, tail = op->mz - (n - 1) * lz;
+  double c = 0.0;
+  for (int pz = 0; pz < 2; pz++)
+    for (int py = 0; py < 2; py++)
+      for (int px = 0; px < 2; px++) {
+        const int64_t nz = (n - pz + 1) / 2, lines = (int64_t)((op->my - py + 1) / 2) * ((op->ntx - px + 1) / 2);
+        if (nz * lines == 0) continue;
+        const bool has_tail = tail < lz && ((n - 1) & 1) == pz;
+        c += class_layers(nz, lines, lz, tail, has_tail, slots) + 0.5 * (double)(nz * lines) / (double)slots;
+      }
+  return c;
+}
+
+// Element layers per z-chunk.  Small boxes: about 2048 tiles, at least 2 layers.
+// From 2048 tiles on, the depth whose colour classes take the fewest layers in
+// FP64 (256 threads per SM) and FP32 (512 with 128-wide tiles; its layers take
+// about 0.6 of the time).  128^3: classes of 1.7 waves with 8 layers (64 layers
+// in all), of 1.95 with 7 (60) -- measured 1415 and 1282 us, FP32 892 and 838;
+// 128x128x64 4 / 7 / 8 / 16 layers 718 / 842 / 720 / 1219 us, FP32 432 / 595 /
+// 624 / 1008; 64^3 2 / 3 / 4 layers 187 / 231 / 270 us.
+static int default_lz(const pt_op *op)
+{
+  const int64_t txy = (int64_t)op->ntx * op->my;
+  int nzc = (int)((2048 + txy - 1) / txy);
+  nzc = nzc < 1 ? 1 : (nzc > (op->mz + 1) / 2 ? (op->mz + 1) / 2 : nzc);
+  if (nzc < 1) nzc = 1;
+  const int lz0 = (op->mz + nzc - 1) / nzc;
+  if (txy * ((op->mz + 1) / 2) < 2048) return lz0;
+  const int64_t slots = 148 * (256 / op->TX), slots32 = op->TX == 128 ? 2 * slots : slots;
+  int best = lz0;
+  double cost = -1.0;
+  for (int lz = std::min(16, op->mz); lz >= 2; lz--) {
+    const double c = tiling_layers(op, lz, slots) + 0.6 * (double)(slots32 / slots) * tiling_layers(op, lz, slots32);
+    if (cost < 0.0 || c < cost - 1e-9) {
+      cost = c;
+      best = lz;
+    }
+  }
+  return best;
+}
+
 pt_status pt_op_set_tiling(pt_op *op, int32_t lz)
 {
   if (!op) return fail(PT_ERR_BAD_ARG, "op is NULL");
   if (lz < 0) return fail(PT_ERR_BAD_ARG, "lz must be >= 0");
-  if (lz == 0) {  // the default: about 2048 CTAs, at least 2 layers per z-chunk where possible
-    const int64_t txy = (int64_t)op->ntx * op->my;
-    int nzc = (int)((2048 + txy - 1) / txy);
-    nzc = nzc < 1 ? 1 : (nzc > (op->mz + 1) / 2 ? (op->mz + 1) / 2 : nzc);
-    if (nzc < 1) nzc = 1;
-    lz = (op->mz + nzc - 1) / nzc;
-  }
+  if (lz == 0) lz = default_lz(op);
   op->LZ = lz < op->mz ? lz : op->mz;
   op->nzc = (op->mz + op->LZ - 1) / op->LZ;
   return PT_OK;
