@@ -7,6 +7,8 @@
  * stream of its own; device-pointer (_d) calls are asynchronous on the op's
  * stream, so a caller whose producers/consumers run on another stream hands
  * that stream over with pt_op_set_stream (NULL = the legacy default stream).
+ * Calls on one op share its scratch: graphs captured from one op are replayed
+ * one after another.
  * Every entry point returns pt_status and never exits the process (the
  * reference CUDA back-end calls cudaDeviceReset()+exit on errors,
  * src/stokes_operators_cuda.cu:46-57).
