@@ -19,6 +19,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200, sm_100a)")
 
 
+def pytest_runtest_setup(item):
+    """Tests against the reference's own operators are skipped, not errors, where
+    neither its compiled library nor its sources are at hand."""
+    import oracle
+    for fixture, lib in (("ref", "libptref.so"), ("shim", "libshimtest.so")):
+        if fixture in getattr(item, "fixturenames", ()) and not oracle.reference_tree() \
+                and not os.path.exists(os.path.join(REPO, "oracle", "_ref", lib)):
+            pytest.skip(f"oracle/_ref/{lib} is not built and the reference's sources are absent")
+
+
 def golden_names():
     """Operator fixtures (inputs and the reference's A11/diag/B/B^T/A outputs)."""
     return sorted(os.path.basename(p)[:-4] for p in glob.glob(os.path.join(GOLDEN_DIR, "*.npz"))
