@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <optional>
 #include <new>
 #include <string>
 #include <type_traits>
@@ -386,22 +387,24 @@ A11Kernel auto_kernel(const pt_op *op)
   return stream ? A11_STREAM : A11_LAYER;
 }
 
-// The tiles' sums, once per op and sized for FP64 (an FP32 apply uses half).
-pt_status ensure_layer(pt_op *op)
-{
-  if (op->d_layer) return PT_OK;
-  PT_CUDA(op_alloc(op, (void **)&op->d_layer,
-                   sizeof(double) * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE));
-  return PT_OK;
-}
-
-// Holds the two launches of an apply together: they share the op's scratch, so
-// another host thread's apply of the same op must not be enqueued in between.
+// Holds the launches of an apply together, from the first tile that writes the
+// op's scratch to the last gather that reads it: another host thread's apply of
+// the same op must not be enqueued in between.
 struct LayerLock {
   pt_op *op;
   explicit LayerLock(pt_op *o) : op(o) { pthread_mutex_lock(&op->layer_mu); }
   ~LayerLock() { pthread_mutex_unlock(&op->layer_mu); }
 };
+
+// The tiles' sums, once per op and sized for FP64 (an FP32 apply uses half).
+pt_status ensure_layer(pt_op *op)
+{
+  LayerLock lock(op);
+  if (op->d_layer) return PT_OK;
+  PT_CUDA(op_alloc(op, (void **)&op->d_layer,
+                   sizeof(double) * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE));
+  return PT_OK;
+}
 
 // The gather of nodes [t0, t1) as a programmatic launch behind the tiles'
 // kernel (it waits for that grid before it reads).
@@ -931,6 +934,9 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
   const int64_t nplanes = 2 * (int64_t)op->mz + 1;
   int64_t up = 0, down = 0;  // next plane to upload / download
   int tile_g = 0;            // layer tiles: next tile to run
+  // a group's gather reads sums that the groups before it left in the scratch
+  std::optional<LayerLock> lock;
+  if (layer) lock.emplace(op);
   PT_CUDA(cudaEventRecord(op->ev_done[0], op->stream));  // earlier work on the op's stream precedes the copies
   PT_CUDA(cudaStreamWaitEvent(op->h2d, op->ev_done[0], 0));
   for (size_t gi = 0; gi < groups.size(); gi++) {
@@ -952,7 +958,6 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
       const int g1 = last ? op->lg.tiles : (int)((c1 + 1) * layer_el / op->lg.E);
       if (!last) fin = 2 * ((int64_t)g1 * op->lg.E / layer_el);
       const uint32_t pn = (uint32_t)(op->box.XY);
-      LayerLock lock(op);
       if (g1 > tile_g)
         s = launch_layer_range<double>(op, op->d_K, op->d_u, op->d_y, MASKED, tile_g, g1, (uint32_t)down * pn,
                                        (uint32_t)fin * pn);
@@ -976,6 +981,7 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
       down = fin;
     }
   }
+  lock.reset();  // everything is enqueued
   PT_CUDA(cudaStreamSynchronize(op->d2h));
   *done = true;
   return PT_OK;
