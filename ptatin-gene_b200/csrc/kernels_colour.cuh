@@ -190,4 +190,123 @@ __global__ void __launch_bounds__(128) diag_colour_kernel(ColourGrid g, const do
     for (int d = 0; d < 3; d++) y[3 * nid[n] + d] += acc[n][d];
 }
 
+// ---------------------------------------------------------------------------
+// P1 "global relative" pressure basis (src/element_utils_q2.c:183-224):
+// Np = {1, (x_q - mean)/Lx, (y_q - mean)/Ly, (z_q - mean)/Lz}.
+// Returns the per-element offsets/scales; x_q comes from Xq.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void p1grel_frame(const double *__restrict__ coords, const int64_t nid[27],
+                                             double mean[3], double invL[3])
+{
+#pragma unroll
+  for (int l = 0; l < 3; l++) {
+    double s = 0.0;
+#pragma unroll
+    for (int n = 0; n < 27; n++) s += coords[3 * nid[n] + l];
+    mean[l] = (1.0 / 27.0) * s;
+  }
+  invL[0] = 1.0 / (coords[3 * nid[14]] - coords[3 * nid[12]]);
+  invL[1] = 1.0 / (coords[3 * nid[16] + 1] - coords[3 * nid[10] + 1]);
+  invL[2] = 1.0 / (coords[3 * nid[22] + 2] - coords[3 * nid[4] + 2]);
+}
+
+// ---------------------------------------------------------------------------
+// A21 (B u):  Yp[e,i] = -sum_q w det div(u)_q Np_i(q)
+//             = -sum_q w Np_i(q) trace(adj Gu)      (det cancels)
+// No scatter conflicts: one thread writes its own 4 pressure dofs.
+// ---------------------------------------------------------------------------
+template <bool MASKED>
+__global__ void __launch_bounds__(128) a21_kernel(Box bx, const double *__restrict__ coords,
+                                                  const double *__restrict__ u, const uint8_t *__restrict__ mask,
+                                                  double *__restrict__ yp)
+{
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (int64_t)bx.mx * bx.my * bx.mz) return;
+  const int ei = (int)(e % bx.mx), ej = (int)((e / bx.mx) % bx.my), ek = (int)(e / ((int64_t)bx.mx * bx.my));
+  int64_t nid[27];
+  element_nodes(bx, ei, ej, ek, nid);
+  double Jg[3][3][27], Xq[3][27];
+  element_jacobian(coords, nid, Jg, Xq);
+  double mean[3], invL[3];
+  p1grel_frame(coords, nid, mean, invL);
+
+  double Ug[3][3][27];
+#pragma unroll 1
+  for (int l = 0; l < 3; l++) {
+    double f[27], I[27];
+#pragma unroll
+    for (int n = 0; n < 27; n++) {
+      const int64_t k = 3 * nid[n] + l;
+      double v = u[k];
+      if (MASKED && mask[k]) v = 0.0;
+      f[n] = v;
+    }
+    q2::interp(f, I);
+    q2::grad_colloc(I, Ug[0][l], Ug[1][l], Ug[2][l]);
+  }
+  double Y[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int q = 0; q < 27; q++) {
+    double J[3][3], adj[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+      for (int l = 0; l < 3; l++) J[k][l] = Jg[k][l][q];
+    (void)q2::adjugate(J, adj);
+    double tr = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) tr += adj[k][0] * Ug[0][k][q] + adj[k][1] * Ug[1][k][q] + adj[k][2] * Ug[2][k][q];
+    const double f = -q2::weight(q) * tr;
+    Y[0] += f;
+    Y[1] += f * ((Xq[0][q] - mean[0]) * invL[0]);
+    Y[2] += f * ((Xq[1][q] - mean[1]) * invL[1]);
+    Y[3] += f * ((Xq[2][q] - mean[2]) * invL[2]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) yp[4 * e + i] = Y[i];
+}
+
+// ---------------------------------------------------------------------------
+// A12 (B^T p):  Yu[n,l] = -sum_q w det p_q dN_n/dx_l,
+//   dv[k][l] = -w p_q adj[l][k],  Yu_l = (B x B x B)^T sum_k Dc_k^T dv[k][l]
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) a12_colour_kernel(ColourGrid g, const double *__restrict__ coords,
+                                                         const double *__restrict__ p, double *__restrict__ yu)
+{
+  int ei, ej, ek;
+  if (!colour_element(g, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, ei, ej, ek)) return;
+  const int64_t e = ei + (int64_t)g.b.mx * (ej + (int64_t)g.b.my * ek);
+  int64_t nid[27];
+  element_nodes(g.b, ei, ej, ek, nid);
+  double Jg[3][3][27], Xq[3][27];
+  element_jacobian(coords, nid, Jg, Xq);
+  double mean[3], invL[3];
+  p1grel_frame(coords, nid, mean, invL);
+  const double p0 = p[4 * e], p1 = p[4 * e + 1], p2 = p[4 * e + 2], p3 = p[4 * e + 3];
+#pragma unroll 1
+  for (int q = 0; q < 27; q++) {
+    double J[3][3], adj[3][3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+      for (int l = 0; l < 3; l++) J[k][l] = Jg[k][l][q];
+    (void)q2::adjugate(J, adj);
+    const double pq = p0 + p1 * ((Xq[0][q] - mean[0]) * invL[0]) + p2 * ((Xq[1][q] - mean[1]) * invL[1]) +
+                      p3 * ((Xq[2][q] - mean[2]) * invL[2]);
+    const double s = -q2::weight(q) * pq;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+      for (int l = 0; l < 3; l++) Jg[k][l][q] = s * adj[l][k];
+  }
+#pragma unroll 1
+  for (int l = 0; l < 3; l++) {
+    double r[27], f[27];
+    q2::grad_colloc_t(Jg[0][l], Jg[1][l], Jg[2][l], r);
+    q2::interp_t(r, f);
+#pragma unroll
+    for (int n = 0; n < 27; n++) yu[3 * nid[n] + l] += f[n];
+  }
+}
+
 }  // namespace ptk

@@ -159,6 +159,17 @@ void op_free(pt_op *op, void *p)
   else cudaFree(p);
 }
 
+// The op's stream is being captured: nothing may be allocated.
+bool capturing(const pt_op *op)
+{
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(op->stream, &st) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream beside a capture of another one
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 constexpr int TPB = 128;
 
 inline unsigned nblocks(int64_t n, int tpb = TPB) { return (unsigned)((n + tpb - 1) / tpb); }
@@ -739,25 +750,45 @@ pt_status diag_d(pt_op *op, double *d, bool ones = false)
   return PT_OK;
 }
 
-// Factors of B and B^T for the current coordinates, built on first use.
-pt_status ensure_div(pt_op *op)
+// Factors of B and B^T for the current coordinates.
+pt_status launch_div(pt_op *op)
 {
-  if (op->d_valid) return PT_OK;
-  if (!op->d_D) PT_CUDA(op_alloc(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel)));
-  pt_status s = ensure_layer(op);
-  if (s != PT_OK) return s;
   constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
-  if ((s = kernel_attrs((const void *)ptk::div_layer_kernel<LNT>, smem)) != PT_OK) return s;
+  pt_status s = kernel_attrs((const void *)ptk::div_layer_kernel<LNT>, smem);
+  if (s != PT_OK) return s;
   ptk::div_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_D);
   PT_LAUNCHED(op);
   op->d_valid = true;
   return PT_OK;
 }
 
+// The factors, built on first use; *have = false in a capture that comes before
+// it (the colour kernels, which need nothing but the coordinates, run there).
+// Ghosted boxes keep them up to date from then on (finish_coords), so a graph of
+// B u or B^T p sees coordinates that are set after it was captured.
+pt_status ensure_div(pt_op *op, bool *have)
+{
+  *have = op->d_D || !capturing(op);
+  if (!*have || op->d_valid) return PT_OK;
+  pt_status s = ensure_layer(op);
+  if (s != PT_OK) return s;
+  if (!op->d_D) PT_CUDA(op_alloc(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel)));
+  return launch_div(op);
+}
+
 pt_status a21_d(pt_op *op, const double *u, double *yp, bool masked)
 {
-  pt_status s = ensure_div(op);
+  bool have;
+  pt_status s = ensure_div(op, &have);
   if (s != PT_OK) return s;
+  if (!have) {
+    if (masked)
+      ptk::a21_kernel<true><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, u, op->d_mask, yp);
+    else
+      ptk::a21_kernel<false><<<nblocks(op->nel), TPB, 0, op->stream>>>(op->box, op->d_coords, u, nullptr, yp);
+    PT_LAUNCHED(op);
+    return PT_OK;
+  }
   constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
   if ((s = kernel_attrs((const void *)ptk::a21_layer_kernel<LNT>, smem)) != PT_OK) return s;
   ptk::a21_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, u,
@@ -769,11 +800,22 @@ pt_status a21_d(pt_op *op, const double *u, double *yp, bool masked)
 // yu = B^T p (`zero`: Dirichlet rows 0), or yu += B^T p (accumulate)
 pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false, bool zero = false)
 {
-  pt_status s = ensure_div(op);
+  bool have;
+  pt_status s = ensure_div(op, &have);
   if (s != PT_OK) return s;
+  if (!accumulate && (!op->full_box || !have)) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
+  if (!have) {
+    for (int c = 0; c < 8; c++) {
+      ptk::ColourGrid g = ptk::colour_grid(op->box, c);
+      const int64_t n = (int64_t)g.ncx * g.ncy * g.ncz;
+      if (n == 0) continue;
+      ptk::a12_colour_kernel<<<nblocks(n), TPB, 0, op->stream>>>(g, op->d_coords, p, yu);
+      PT_LAUNCHED(op);
+    }
+    return zero ? bc_value(op, 0.0, yu) : PT_OK;
+  }
   constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
   if ((s = kernel_attrs((const void *)ptk::a12_layer_kernel<LNT>, smem)) != PT_OK) return s;
-  if (!accumulate && !op->full_box) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
   LayerLock lock(op);
   ptk::a12_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, p, op->d_layer);
   PT_LAUNCHED(op);
@@ -785,8 +827,9 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
 
 // Yu = A11 u + B^T p (- x when mode is LAYER_SUB) and, unless yp is null,
 // Yp = B u, in one pass over the tiles; *done = false where the geometry does
-// not allow K (the caller then runs the blocks one by one).  masked: Dirichlet
-// columns of u as zeros, rows copied from u.
+// not allow K, and in a capture that comes before the first use (the caller
+// then runs the blocks one by one).  masked: Dirichlet columns of u as zeros,
+// rows copied from u.
 pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double *x, double *yu, double *yp, int mode,
                        bool *done)
 {
@@ -795,6 +838,7 @@ pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double
   pt_status s = ensure_geometry(op);
   if (s != PT_OK) return s;
   if (!op->geom_ok) return PT_OK;
+  if ((!op->d_P || !op->d_layer) && capturing(op)) return PT_OK;
   if (!op->d_P) {
     PT_CUDA(op_alloc(op, (void **)&op->d_P, sizeof(double) * ptk::psize(op->nel)));
     if ((s = launch_geometry(op)) != PT_OK) return s;  // K again with the same values, and P
@@ -1119,7 +1163,7 @@ static pt_status finish_coords(pt_op *op)
   op->d_valid = false;
   op->F_valid = false;
   op->state++;
-  return PT_OK;
+  return op->d_D && !op->full_box ? launch_div(op) : PT_OK;  // ensure_div
 }
 
 static pt_status finish_eta(pt_op *op)

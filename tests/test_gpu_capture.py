@@ -1,0 +1,89 @@
+"""Applies recorded in CUDA graphs: first uses inside a capture, inputs that change
+between replays, several graphs of one op."""
+import numpy as np
+import pytest
+
+from conftest import relerr
+from pt_b200 import mesh as M
+
+pytestmark = pytest.mark.gpu
+
+TOL64 = 1e-12  # the project's parity bar for FP64 operators
+SUB, OFF, NB = (37, 4, 3), (2, 0, 1), (37 * 2 + 1 + 4, 4 * 2 + 1 + 2, 3 * 2 + 1 + 3)
+
+
+def _ghosted(seed):
+    """Coordinates of a ghosted box (a rank's node box around SUB elements)."""
+    rng = np.random.default_rng(seed)
+    m, eta, _ = M.problem("box:%d,%d,%d" % SUB, seed=seed)
+    c = rng.uniform(size=(NB[2], NB[1], NB[0], 3))
+    sl = tuple(slice(o, o + 2 * n + 1) for o, n in zip(OFF[::-1], SUB[::-1]))
+    c[sl] = m.coords.reshape(c[sl].shape)
+    return np.ascontiguousarray(c.reshape(-1)), eta, rng.uniform(-1, 1, size=c.size)
+
+
+def _record(op, call):
+    import torch
+    st = torch.cuda.Stream()
+    op.set_stream(st)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        call()
+    return g, st
+
+
+def test_ghosted_b_and_bt_recorded_before_their_first_use(ora):
+    """No warm-up is needed, and replays follow the coordinates."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    c, eta, u = _ghosted(3)
+    p = np.random.default_rng(4).uniform(-1, 1, size=4 * eta.size // 27)
+    ud, pd = torch.from_numpy(u).cuda(), torch.from_numpy(p).cuda()
+    yp, yu = torch.empty_like(pd), torch.empty_like(ud)
+
+    def calls(op):
+        op.MFStokesWrapper_A21(ud, yp)
+        op.MFStokesWrapper_A12(pd, yu)
+
+    for warm in (False, True):
+        with MatStokesMF(*SUB, node_box=(*NB, *OFF)) as op, MatStokesMF(*SUB, node_box=(*NB, *OFF)) as own:
+            op.set_coords(c)
+            if warm:
+                calls(op)
+            g, st = _record(op, lambda: calls(op))
+            for seed in (3, 8):
+                cs = _ghosted(seed)[0]
+                op.set_coords(cs)
+                own.set_coords(cs)
+                yp.fill_(np.nan)
+                yu.fill_(np.nan)
+                torch.cuda.synchronize()
+                g.replay()
+                torch.cuda.synchronize()
+                assert relerr(yp.cpu(), own.MFStokesWrapper_A21(u)) < TOL64, (warm, seed)
+                assert relerr(yu.cpu(), own.MFStokesWrapper_A12(p)) < TOL64, (warm, seed)
+
+
+@pytest.mark.parametrize("workload", ["box:8,8,8", "box:21,13,17"])
+def test_whole_operator_recorded_after_its_blocks(ora, workload):
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, eta, mask = M.problem(workload, seed=7)
+    u, p = M.uniform_vec(m.nvel, 8), M.uniform_vec(m.npres, 9)
+    ud, pd = torch.from_numpy(u).cuda(), torch.from_numpy(p).cuda()
+    yu, yp = torch.empty_like(ud), torch.empty_like(pd)
+    with MatStokesMF(*m.dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        op.MatMult_MFStokes_A11(ud, yu)
+        op.MatMult_MFStokes_A12(pd, yu)
+        op.MatMult_MFStokes_A21(ud, yp)
+        g, st = _record(op, lambda: op.MatMult_MFStokes_A(ud, pd, yu, yp))
+        yu.fill_(np.nan)
+        yp.fill_(np.nan)
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        wu, wp = op.MatMult_MFStokes_A(u, p)
+        assert relerr(yu.cpu(), wu) < TOL64 and relerr(yp.cpu(), wp) < TOL64
