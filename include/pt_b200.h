@@ -7,8 +7,11 @@
  * stream of its own; device-pointer (_d) calls are asynchronous on the op's
  * stream, so a caller whose producers/consumers run on another stream hands
  * that stream over with pt_op_set_stream (NULL = the legacy default stream).
- * Calls on one op share its scratch: graphs captured from one op are replayed
- * one after another.
+ * Graphs captured from one op may be replayed at the same time, each on its own
+ * vectors: on layer and streaming tiles a recorded apply brings its own scratch
+ * (memory nodes of the graph, so such a graph has one executable instance and
+ * is nobody's child graph).  Applies from stored element matrices share the
+ * op's: their graphs are replayed one after another.
  * Every entry point returns pt_status and never exits the process (the
  * reference CUDA back-end calls cudaDeviceReset()+exit on errors,
  * src/stokes_operators_cuda.cu:46-57).

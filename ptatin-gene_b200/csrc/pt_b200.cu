@@ -140,6 +140,7 @@ struct pt_op {
   ptk::LayerGrid lg;
   double *d_layer;
   pthread_mutex_t layer_mu;
+  bool graph_own;  // the capture under way is a solver's (LayerScratch)
 };
 
 namespace {
@@ -417,10 +418,39 @@ pt_status ensure_layer(pt_op *op)
   return PT_OK;
 }
 
+// The scratch of an apply: the op's own or, in a capture, memory of the graph
+// (an allocation and a free recorded with the apply), so that graphs captured
+// from one op may run at the same time on several streams.  A solver's graph
+// runs on the op's stream only and uses the op's scratch (graph_own).
+struct LayerScratch {
+  pt_op *op;
+  double *p = nullptr;
+  bool of_graph = false;
+  std::optional<LayerLock> lock;
+  explicit LayerScratch(pt_op *o) : op(o) {}
+  pt_status get(size_t value_bytes)
+  {
+    if (!op->graph_own && capturing(op)) {
+      PT_CUDA(cudaMallocAsync((void **)&p, value_bytes * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE, op->stream));
+      of_graph = true;
+      return PT_OK;
+    }
+    pt_status s = ensure_layer(op);
+    if (s != PT_OK) return s;
+    lock.emplace(op);
+    p = op->d_layer;
+    return PT_OK;
+  }
+  ~LayerScratch()
+  {
+    if (of_graph) cudaFreeAsync(p, op->stream);
+  }
+};
+
 // The gather of nodes [t0, t1) as a programmatic launch behind the tiles'
 // kernel (it waits for that grid before it reads).
 template <typename T, int MODE>
-pt_status launch_layer_gather(pt_op *op, uint32_t t0, uint32_t t1, const T *x, T *y)
+pt_status launch_layer_gather(pt_op *op, const void *scratch, uint32_t t0, uint32_t t1, const T *x, T *y)
 {
   cudaLaunchAttribute pdl[1] = {};
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -432,7 +462,7 @@ pt_status launch_layer_gather(pt_op *op, uint32_t t0, uint32_t t1, const T *x, T
   cfg.attrs = pdl;
   cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, ptk::layer_gather_kernel<T, LNT, MODE>, op->lg, t0, t1,
-                                           reinterpret_cast<const T *>(op->d_layer), x,
+                                           static_cast<const T *>(scratch), x,
                                            (const uint32_t *)op->d_mbits, y);
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "layer gather launch: %s", cudaGetErrorString(e));
   PT_LAUNCHED(op);
@@ -441,41 +471,41 @@ pt_status launch_layer_gather(pt_op *op, uint32_t t0, uint32_t t1, const T *x, T
 
 // Tiles [tile0, tile1) and the gather of nodes [t0, t1).
 template <typename T>
-pt_status launch_layer_range(pt_op *op, const T *K, const T *u, T *y, bool masked, int tile0, int tile1, uint32_t t0,
-                             uint32_t t1)
+pt_status launch_layer_range(pt_op *op, void *scratch, const T *K, const T *u, T *y, bool masked, int tile0, int tile1,
+                             uint32_t t0, uint32_t t1)
 {
   constexpr size_t smem = ptk::layer_smem_bytes<T, LNT>();
   pt_status s = kernel_attrs((const void *)ptk::a11_layer_kernel<T, LNT>, smem);
   if (s != PT_OK) return s;
   ptk::a11_layer_kernel<T, LNT><<<(unsigned)(tile1 - tile0), LNT, smem, op->stream>>>(
-      op->lg, tile0, K, u, masked ? op->d_mbits : nullptr, reinterpret_cast<T *>(op->d_layer));
+      op->lg, tile0, K, u, masked ? op->d_mbits : nullptr, static_cast<T *>(scratch));
   PT_LAUNCHED(op);
   if (t1 == t0) return PT_OK;
-  return masked ? launch_layer_gather<T, ptk::LAYER_BC_COPY>(op, t0, t1, u, y)
-                : launch_layer_gather<T, ptk::LAYER_PLAIN>(op, t0, t1, u, y);
+  return masked ? launch_layer_gather<T, ptk::LAYER_BC_COPY>(op, scratch, t0, t1, u, y)
+                : launch_layer_gather<T, ptk::LAYER_PLAIN>(op, scratch, t0, t1, u, y);
 }
 
 template <typename T>
 pt_status launch_layer(pt_op *op, const T *K, const T *u, T *y, bool masked)
 {
-  pt_status s = ensure_layer(op);
+  LayerScratch sc(op);
+  pt_status s = sc.get(sizeof(T));
   if (s != PT_OK) return s;
-  LayerLock lock(op);
-  return launch_layer_range<T>(op, K, u, y, masked, 0, (int)op->lg.tiles, 0, op->lg.nodes());
+  return launch_layer_range<T>(op, sc.p, K, u, y, masked, 0, (int)op->lg.tiles, 0, op->lg.nodes());
 }
 
 // diag(A11), Dirichlet entries 1 when `ones`
 pt_status launch_layer_diag(pt_op *op, double *d, bool ones)
 {
-  pt_status s = ensure_layer(op);
-  if (s != PT_OK) return s;
   constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
-  if ((s = kernel_attrs((const void *)ptk::diag_layer_kernel<LNT>, smem)) != PT_OK) return s;
-  LayerLock lock(op);
-  ptk::diag_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, op->d_layer);
+  pt_status s = kernel_attrs((const void *)ptk::diag_layer_kernel<LNT>, smem);
+  if (s != PT_OK) return s;
+  LayerScratch sc(op);
+  if ((s = sc.get(sizeof(double))) != PT_OK) return s;
+  ptk::diag_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, sc.p);
   PT_LAUNCHED(op);
-  return ones ? launch_layer_gather<double, ptk::LAYER_BC_ONE>(op, 0, op->lg.nodes(), nullptr, d)
-              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, op->lg.nodes(), nullptr, d);
+  return ones ? launch_layer_gather<double, ptk::LAYER_BC_ONE>(op, sc.p, 0, op->lg.nodes(), nullptr, d)
+              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, op->lg.nodes(), nullptr, d);
 }
 
 template <typename T, bool MASKED>
@@ -770,8 +800,6 @@ pt_status ensure_div(pt_op *op, bool *have)
 {
   *have = op->d_D || !capturing(op);
   if (!*have || op->d_valid) return PT_OK;
-  pt_status s = ensure_layer(op);
-  if (s != PT_OK) return s;
   if (!op->d_D) PT_CUDA(op_alloc(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel)));
   return launch_div(op);
 }
@@ -816,13 +844,14 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
   }
   constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
   if ((s = kernel_attrs((const void *)ptk::a12_layer_kernel<LNT>, smem)) != PT_OK) return s;
-  LayerLock lock(op);
-  ptk::a12_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, p, op->d_layer);
+  LayerScratch sc(op);
+  if ((s = sc.get(sizeof(double))) != PT_OK) return s;
+  ptk::a12_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, p, sc.p);
   PT_LAUNCHED(op);
   const uint32_t n = op->lg.nodes();
-  if (accumulate) return launch_layer_gather<double, ptk::LAYER_ADD>(op, 0, n, nullptr, yu);
-  return zero && op->has_mask ? launch_layer_gather<double, ptk::LAYER_BC_ZERO>(op, 0, n, nullptr, yu)
-                              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, n, nullptr, yu);
+  if (accumulate) return launch_layer_gather<double, ptk::LAYER_ADD>(op, sc.p, 0, n, nullptr, yu);
+  return zero && op->has_mask ? launch_layer_gather<double, ptk::LAYER_BC_ZERO>(op, sc.p, 0, n, nullptr, yu)
+                              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, n, nullptr, yu);
 }
 
 // Yu = A11 u + B^T p (- x when mode is LAYER_SUB) and, unless yp is null,
@@ -838,27 +867,27 @@ pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double
   pt_status s = ensure_geometry(op);
   if (s != PT_OK) return s;
   if (!op->geom_ok) return PT_OK;
-  if ((!op->d_P || !op->d_layer) && capturing(op)) return PT_OK;
+  if (!op->d_P && capturing(op)) return PT_OK;
   if (!op->d_P) {
     PT_CUDA(op_alloc(op, (void **)&op->d_P, sizeof(double) * ptk::psize(op->nel)));
     if ((s = launch_geometry(op)) != PT_OK) return s;  // K again with the same values, and P
   }
-  if ((s = ensure_layer(op)) != PT_OK) return s;
   constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
   if ((s = kernel_attrs((const void *)ptk::stokes_layer_kernel<LNT, true>, smem)) != PT_OK) return s;
   if ((s = kernel_attrs((const void *)ptk::stokes_layer_kernel<LNT, false>, smem)) != PT_OK) return s;
   if (!op->full_box) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
   const bool masked = mode == ptk::LAYER_BC_COPY;
   {
-    LayerLock lock(op);
+    LayerScratch sc(op);
+    if ((s = sc.get(sizeof(double))) != PT_OK) return s;
     auto kernel = yp ? ptk::stokes_layer_kernel<LNT, true> : ptk::stokes_layer_kernel<LNT, false>;
     kernel<<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, op->d_P, u, p,
-                                                              masked ? op->d_mbits : nullptr, op->d_layer, yp);
+                                                              masked ? op->d_mbits : nullptr, sc.p, yp);
     PT_LAUNCHED(op);
     const uint32_t n = op->lg.nodes();
-    if (masked) s = launch_layer_gather<double, ptk::LAYER_BC_COPY>(op, 0, n, x, yu);
-    else if (mode == ptk::LAYER_SUB) s = launch_layer_gather<double, ptk::LAYER_SUB>(op, 0, n, x, yu);
-    else s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, n, nullptr, yu);
+    if (masked) s = launch_layer_gather<double, ptk::LAYER_BC_COPY>(op, sc.p, 0, n, x, yu);
+    else if (mode == ptk::LAYER_SUB) s = launch_layer_gather<double, ptk::LAYER_SUB>(op, sc.p, 0, n, x, yu);
+    else s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, n, nullptr, yu);
     if (s != PT_OK) return s;
   }
   if (!op->full_box && masked) {  // Dirichlet dofs outside the element box
@@ -941,7 +970,6 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
   pt_status s = ensure_geometry(op);
   if (s != PT_OK) return s;
   if (!op->geom_ok || (layer ? op->mz < 2 * PIPE_LAYERS : op->nzc < 2)) return PT_OK;
-  if (layer && (s = ensure_layer(op)) != PT_OK) return s;
   if (!op->pipe_ready) {
     PT_CUDA(cudaStreamCreateWithFlags(&op->h2d, cudaStreamNonBlocking));
     PT_CUDA(cudaStreamCreateWithFlags(&op->d2h, cudaStreamNonBlocking));
@@ -979,8 +1007,8 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
   int64_t up = 0, down = 0;  // next plane to upload / download
   int tile_g = 0;            // layer tiles: next tile to run
   // a group's gather reads sums that the groups before it left in the scratch
-  std::optional<LayerLock> lock;
-  if (layer) lock.emplace(op);
+  LayerScratch sc(op);
+  if (layer && (s = sc.get(sizeof(double))) != PT_OK) return s;
   PT_CUDA(cudaEventRecord(op->ev_done[0], op->stream));  // earlier work on the op's stream precedes the copies
   PT_CUDA(cudaStreamWaitEvent(op->h2d, op->ev_done[0], 0));
   for (size_t gi = 0; gi < groups.size(); gi++) {
@@ -1003,7 +1031,7 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
       if (!last) fin = 2 * ((int64_t)g1 * op->lg.E / layer_el);
       const uint32_t pn = (uint32_t)(op->box.XY);
       if (g1 > tile_g)
-        s = launch_layer_range<double>(op, op->d_K, op->d_u, op->d_y, MASKED, tile_g, g1, (uint32_t)down * pn,
+        s = launch_layer_range<double>(op, sc.p, op->d_K, op->d_u, op->d_y, MASKED, tile_g, g1, (uint32_t)down * pn,
                                        (uint32_t)fin * pn);
       tile_g = g1;
     }
@@ -1025,7 +1053,7 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
       down = fin;
     }
   }
-  lock.reset();  // everything is enqueued
+  sc.lock.reset();  // everything is enqueued
   PT_CUDA(cudaStreamSynchronize(op->d2h));
   *done = true;
   return PT_OK;
@@ -1550,15 +1578,16 @@ static pt_status ensure_body_force(pt_op *op)
   if (op->F_valid) return PT_OK;
   if (!op->d_F) PT_CUDA(op_alloc(op, (void **)&op->d_F, sizeof(double) * op->nvel));
   if (!op->full_box) PT_CUDA(cudaMemsetAsync(op->d_F, 0, sizeof(double) * op->nvel, op->stream));
-  pt_status s = ensure_layer(op);
-  if (s != PT_OK) return s;
   constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
-  if ((s = kernel_attrs((const void *)ptk::body_force_layer_kernel<LNT>, smem)) != PT_OK) return s;
-  LayerLock lock(op);
+  pt_status s = kernel_attrs((const void *)ptk::body_force_layer_kernel<LNT>, smem);
+  if (s != PT_OK) return s;
+  LayerScratch sc(op);
+  if ((s = sc.get(sizeof(double))) != PT_OK) return s;
   ptk::body_force_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_fu,
-                                                                                      op->d_layer);
+                                                                                      sc.p);
   PT_LAUNCHED(op);
-  if ((s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, 0, op->lg.nodes(), nullptr, op->d_F)) != PT_OK) return s;
+  if ((s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, op->lg.nodes(), nullptr, op->d_F)) != PT_OK)
+    return s;
   op->F_valid = true;
   return PT_OK;
 }

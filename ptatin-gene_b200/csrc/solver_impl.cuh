@@ -779,6 +779,7 @@ pt_status mg_capture(pt_solver *s)
   for (pt_mg_level &L : mg.lv) {
     saved.push_back(L.op->stream);
     L.op->stream = cap;
+    L.op->graph_own = true;
   }
   const int64_t f0 = mg.fine_applies;
   const double c0 = mg.coarse_work;
@@ -788,7 +789,10 @@ pt_status mg_capture(pt_solver *s)
     st = mg_vcycle<T>(mg, 0);
     e = cudaStreamEndCapture(cap, &g);
   }
-  for (size_t i = 0; i < mg.lv.size(); i++) mg.lv[i].op->stream = saved[i];
+  for (size_t i = 0; i < mg.lv.size(); i++) {
+    mg.lv[i].op->stream = saved[i];
+    mg.lv[i].op->graph_own = false;
+  }
   mg.graph_fine = mg.fine_applies - f0;
   mg.graph_coarse = mg.coarse_work - c0;
   mg.fine_applies = f0;

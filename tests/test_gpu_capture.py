@@ -87,3 +87,40 @@ def test_whole_operator_recorded_after_its_blocks(ora, workload):
         torch.cuda.synchronize()
         wu, wp = op.MatMult_MFStokes_A(u, p)
         assert relerr(yu.cpu(), wu) < TOL64 and relerr(yp.cpu(), wp) < TOL64
+
+
+def test_graphs_of_one_op_on_two_streams():
+    """Replayed at the same time, each gives what its call gives alone."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, eta, mask = M.problem("box:33,30,28", seed=5)
+    xs = [torch.from_numpy(M.uniform_vec(m.nvel, 6 + i)).cuda() for i in range(3)]
+    pd = torch.from_numpy(M.uniform_vec(m.npres, 9)).cuda()
+    with MatStokesMF(*m.dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        assert op.a11_op == "b200_layer"
+        calls = [lambda y: op.MatMult_MFStokes_A11(xs[0], y), lambda y: op.MFStokesWrapper_A11(xs[1], y),
+                 lambda y: op.MatMult_MFStokes_A(xs[2], pd, y, yp), lambda y: op.MatMult_MFStokes_A12(pd, y),
+                 lambda y: op.MatGetDiagonal_MFStokes_A11(y)]
+        yp = torch.empty_like(pd)
+        want = []
+        for c in calls:
+            y = torch.empty_like(xs[0])
+            c(y)
+            torch.cuda.synchronize()
+            want.append(y)
+        got = [torch.empty_like(xs[0]) for _ in calls]
+        graphs = [_record(op, lambda: c(y))[0] for c, y in zip(calls, got)]
+        streams = [torch.cuda.Stream() for _ in calls]
+        for _ in range(20):
+            for y in got:
+                y.fill_(np.nan)
+            torch.cuda.synchronize()
+            for g, st in zip(graphs, streams):
+                with torch.cuda.stream(st):
+                    for _ in range(3):
+                        g.replay()
+            torch.cuda.synchronize()
+            for k, (y, w) in enumerate(zip(got, want)):
+                assert torch.equal(y, w), k
