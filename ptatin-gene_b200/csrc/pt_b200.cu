@@ -141,6 +141,7 @@ struct pt_op {
   double *d_layer;
   pthread_mutex_t layer_mu;
   bool graph_own;  // the capture under way is a solver's (LayerScratch)
+  bool lean;       // the device had no room for what alloc_if_room wanted
 };
 
 namespace {
@@ -158,6 +159,21 @@ void op_free(pt_op *op, void *p)
   if (!p) return;
   if (op->pool) cudaFreeAsync(p, op->stream);
   else cudaFree(p);
+}
+
+// Memory that a faster route wants beside K.  Where the device has no room *p
+// stays null, the caller takes the route that does without, and nothing more of
+// this kind is tried until the coordinates change.
+pt_status alloc_if_room(pt_op *op, void **p, size_t bytes)
+{
+  if (op->lean) return PT_OK;
+  const cudaError_t e = op_alloc(op, p, bytes);
+  if (e == cudaSuccess) return PT_OK;
+  *p = nullptr;
+  cudaGetLastError();
+  if (e != cudaErrorMemoryAllocation) return fail(PT_ERR_CUDA, "device memory: %s", cudaGetErrorString(e));
+  op->lean = true;
+  return PT_OK;
 }
 
 // The op's stream is being captured: nothing may be allocated.
@@ -408,17 +424,18 @@ struct LayerLock {
   ~LayerLock() { pthread_mutex_unlock(&op->layer_mu); }
 };
 
-// The tiles' sums, once per op and sized for FP64 (an FP32 apply uses half).
+// The tiles' sums, once per op and sized for FP64 (an FP32 apply uses half);
+// null where there is no room.
 pt_status ensure_layer(pt_op *op)
 {
   LayerLock lock(op);
   if (op->d_layer) return PT_OK;
-  PT_CUDA(op_alloc(op, (void **)&op->d_layer,
-                   sizeof(double) * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE));
-  return PT_OK;
+  return alloc_if_room(op, (void **)&op->d_layer,
+                       sizeof(double) * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE);
 }
 
-// The scratch of an apply: the op's own or, in a capture, memory of the graph
+// The scratch of an apply (p null where there is no room): the op's own or, in a
+// capture, memory of the graph
 // (an allocation and a free recorded with the apply), so that graphs captured
 // from one op may run at the same time on several streams.  A solver's graph
 // runs on the op's stream only and uses the op's scratch (graph_own).
@@ -485,23 +502,27 @@ pt_status launch_layer_range(pt_op *op, void *scratch, const T *K, const T *u, T
                 : launch_layer_gather<T, ptk::LAYER_PLAIN>(op, scratch, t0, t1, u, y);
 }
 
+// *done = false where there is no room for the scratch.
 template <typename T>
-pt_status launch_layer(pt_op *op, const T *K, const T *u, T *y, bool masked)
+pt_status launch_layer(pt_op *op, const T *K, const T *u, T *y, bool masked, bool *done)
 {
   LayerScratch sc(op);
   pt_status s = sc.get(sizeof(T));
-  if (s != PT_OK) return s;
+  *done = sc.p != nullptr;
+  if (s != PT_OK || !*done) return s;
   return launch_layer_range<T>(op, sc.p, K, u, y, masked, 0, (int)op->lg.tiles, 0, op->lg.nodes());
 }
 
-// diag(A11), Dirichlet entries 1 when `ones`
-pt_status launch_layer_diag(pt_op *op, double *d, bool ones)
+// diag(A11), Dirichlet entries 1 when `ones`; *done as launch_layer
+pt_status launch_layer_diag(pt_op *op, double *d, bool ones, bool *done)
 {
   constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
   pt_status s = kernel_attrs((const void *)ptk::diag_layer_kernel<LNT>, smem);
   if (s != PT_OK) return s;
   LayerScratch sc(op);
-  if ((s = sc.get(sizeof(double))) != PT_OK) return s;
+  s = sc.get(sizeof(double));
+  *done = sc.p != nullptr;
+  if (s != PT_OK || !*done) return s;
   ptk::diag_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, sc.p);
   PT_LAUNCHED(op);
   return ones ? launch_layer_gather<double, ptk::LAYER_BC_ONE>(op, sc.p, 0, op->lg.nodes(), nullptr, d)
@@ -683,14 +704,15 @@ pt_status launch_a11(pt_op *op, const T *u, T *y, bool masked)
     if (op->geom_ok) {
       if (!op->full_box) PT_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * op->nvel, op->stream));
       if (op->a11_kernel == A11_LAYER || (sizeof(T) == 4 && op->a11_auto && op->nel < LAYER_F32_MAX_ELEMENTS)) {
-        if ((s = launch_layer<T>(op, op_K<T>(op), u, y, masked)) != PT_OK) return s;
+        bool done;
+        if ((s = launch_layer<T>(op, op_K<T>(op), u, y, masked, &done)) != PT_OK) return s;
         // a ghosted box's Dirichlet dofs outside the element box
-        if (masked && !op->full_box) {
+        if (done && masked && !op->full_box) {
           bc_bits_kernel<T><<<grid_stride_blocks((op->nvel + 31) / 32), 256, 0, op->stream>>>(op->d_mbits, u, y,
                                                                                              op->nvel);
           PT_LAUNCHED(op);
         }
-        return PT_OK;
+        if (done) return PT_OK;  // else on the streaming tiles, which need no scratch
       }
       if (masked) {
         // Dirichlet columns inside the kernel; rows y_k = x_k after its colour passes
@@ -741,8 +763,9 @@ pt_status diag_d(pt_op *op, double *d, bool ones = false)
     if ((s = ensure_geometry(op)) != PT_OK) return s;
     if (op->geom_ok) {
       if (!op->full_box) PT_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * op->nvel, op->stream));
-      if ((s = launch_layer_diag(op, d, ones && op->full_box)) != PT_OK) return s;
-      return ones && !op->full_box ? bc_value(op, 1.0, d) : PT_OK;
+      bool done;
+      if ((s = launch_layer_diag(op, d, ones && op->full_box, &done)) != PT_OK) return s;
+      if (done) return ones && !op->full_box ? bc_value(op, 1.0, d) : PT_OK;
     }
   }
   if (ones) {
@@ -759,7 +782,7 @@ pt_status diag_d(pt_op *op, double *d, bool ones = false)
       return PT_OK;
     }
   }
-  if (op->a11_kernel == A11_STREAM) {
+  if (op->a11_kernel == A11_STREAM || op->a11_kernel == A11_LAYER) {
     // the streaming tiles from the stored K, as the apply
     if ((s = ensure_geometry(op)) != PT_OK) return s;
     if (op->geom_ok) {
@@ -793,15 +816,16 @@ pt_status launch_div(pt_op *op)
 }
 
 // The factors, built on first use; *have = false in a capture that comes before
-// it (the colour kernels, which need nothing but the coordinates, run there).
+// it and where there is no room for them (the colour kernels, which need nothing
+// but the coordinates, run there).
 // Ghosted boxes keep them up to date from then on (finish_coords), so a graph of
 // B u or B^T p sees coordinates that are set after it was captured.
 pt_status ensure_div(pt_op *op, bool *have)
 {
-  *have = op->d_D || !capturing(op);
-  if (!*have || op->d_valid) return PT_OK;
-  if (!op->d_D) PT_CUDA(op_alloc(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel)));
-  return launch_div(op);
+  pt_status s = PT_OK;
+  if (!op->d_D && !capturing(op)) s = alloc_if_room(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel));
+  *have = op->d_D != nullptr;
+  return s != PT_OK || !*have || op->d_valid ? s : launch_div(op);
 }
 
 pt_status a21_d(pt_op *op, const double *u, double *yp, bool masked)
@@ -831,6 +855,9 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
   bool have;
   pt_status s = ensure_div(op, &have);
   if (s != PT_OK) return s;
+  LayerScratch sc(op);
+  if (have && (s = sc.get(sizeof(double))) != PT_OK) return s;
+  have = have && sc.p;
   if (!accumulate && (!op->full_box || !have)) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
   if (!have) {
     for (int c = 0; c < 8; c++) {
@@ -844,8 +871,6 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
   }
   constexpr size_t smem = ptk::layer_diag_smem_bytes<double, LNT>();
   if ((s = kernel_attrs((const void *)ptk::a12_layer_kernel<LNT>, smem)) != PT_OK) return s;
-  LayerScratch sc(op);
-  if ((s = sc.get(sizeof(double))) != PT_OK) return s;
   ptk::a12_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, p, sc.p);
   PT_LAUNCHED(op);
   const uint32_t n = op->lg.nodes();
@@ -856,9 +881,9 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
 
 // Yu = A11 u + B^T p (- x when mode is LAYER_SUB) and, unless yp is null,
 // Yp = B u, in one pass over the tiles; *done = false where the geometry does
-// not allow K, and in a capture that comes before the first use (the caller
-// then runs the blocks one by one).  masked: Dirichlet columns of u as zeros,
-// rows copied from u.
+// not allow K or the device has no room, and in a capture that comes before the
+// first use (the caller then runs the blocks one by one).  masked: Dirichlet
+// columns of u as zeros, rows copied from u.
 pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double *x, double *yu, double *yp, int mode,
                        bool *done)
 {
@@ -868,8 +893,11 @@ pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double
   if (s != PT_OK) return s;
   if (!op->geom_ok) return PT_OK;
   if (!op->d_P && capturing(op)) return PT_OK;
+  LayerScratch sc(op);
+  if ((s = sc.get(sizeof(double))) != PT_OK || !sc.p) return s;
   if (!op->d_P) {
-    PT_CUDA(op_alloc(op, (void **)&op->d_P, sizeof(double) * ptk::psize(op->nel)));
+    s = alloc_if_room(op, (void **)&op->d_P, sizeof(double) * ptk::psize(op->nel));
+    if (s != PT_OK || !op->d_P) return s;
     if ((s = launch_geometry(op)) != PT_OK) return s;  // K again with the same values, and P
   }
   constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
@@ -877,19 +905,15 @@ pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double
   if ((s = kernel_attrs((const void *)ptk::stokes_layer_kernel<LNT, false>, smem)) != PT_OK) return s;
   if (!op->full_box) PT_CUDA(cudaMemsetAsync(yu, 0, sizeof(double) * op->nvel, op->stream));
   const bool masked = mode == ptk::LAYER_BC_COPY;
-  {
-    LayerScratch sc(op);
-    if ((s = sc.get(sizeof(double))) != PT_OK) return s;
-    auto kernel = yp ? ptk::stokes_layer_kernel<LNT, true> : ptk::stokes_layer_kernel<LNT, false>;
-    kernel<<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, op->d_P, u, p,
-                                                              masked ? op->d_mbits : nullptr, sc.p, yp);
-    PT_LAUNCHED(op);
-    const uint32_t n = op->lg.nodes();
-    if (masked) s = launch_layer_gather<double, ptk::LAYER_BC_COPY>(op, sc.p, 0, n, x, yu);
-    else if (mode == ptk::LAYER_SUB) s = launch_layer_gather<double, ptk::LAYER_SUB>(op, sc.p, 0, n, x, yu);
-    else s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, n, nullptr, yu);
-    if (s != PT_OK) return s;
-  }
+  auto kernel = yp ? ptk::stokes_layer_kernel<LNT, true> : ptk::stokes_layer_kernel<LNT, false>;
+  kernel<<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_K, op->d_P, u, p,
+                                                            masked ? op->d_mbits : nullptr, sc.p, yp);
+  PT_LAUNCHED(op);
+  const uint32_t n = op->lg.nodes();
+  if (masked) s = launch_layer_gather<double, ptk::LAYER_BC_COPY>(op, sc.p, 0, n, x, yu);
+  else if (mode == ptk::LAYER_SUB) s = launch_layer_gather<double, ptk::LAYER_SUB>(op, sc.p, 0, n, x, yu);
+  else s = launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, n, nullptr, yu);
+  if (s != PT_OK) return s;
   if (!op->full_box && masked) {  // Dirichlet dofs outside the element box
     bc_bits_kernel<double><<<grid_stride_blocks((op->nvel + 31) / 32), 256, 0, op->stream>>>(op->d_mbits, x, yu,
                                                                                             op->nvel);
@@ -1008,7 +1032,7 @@ pt_status a11_host_pipelined(pt_op *op, const double *hu, double *hy, bool *done
   int tile_g = 0;            // layer tiles: next tile to run
   // a group's gather reads sums that the groups before it left in the scratch
   LayerScratch sc(op);
-  if (layer && (s = sc.get(sizeof(double))) != PT_OK) return s;
+  if (layer && ((s = sc.get(sizeof(double))) != PT_OK || !sc.p)) return s;
   PT_CUDA(cudaEventRecord(op->ev_done[0], op->stream));  // earlier work on the op's stream precedes the copies
   PT_CUDA(cudaStreamWaitEvent(op->h2d, op->ev_done[0], 0));
   for (size_t gi = 0; gi < groups.size(); gi++) {
@@ -1190,6 +1214,7 @@ static pt_status finish_coords(pt_op *op)
   op->geom_dirty = true;
   op->d_valid = false;
   op->F_valid = false;
+  op->lean = false;
   op->state++;
   return op->d_D && !op->full_box ? launch_div(op) : PT_OK;  // ensure_div
 }
@@ -1577,12 +1602,23 @@ static pt_status ensure_body_force(pt_op *op)
 {
   if (op->F_valid) return PT_OK;
   if (!op->d_F) PT_CUDA(op_alloc(op, (void **)&op->d_F, sizeof(double) * op->nvel));
-  if (!op->full_box) PT_CUDA(cudaMemsetAsync(op->d_F, 0, sizeof(double) * op->nvel, op->stream));
   constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
   pt_status s = kernel_attrs((const void *)ptk::body_force_layer_kernel<LNT>, smem);
   if (s != PT_OK) return s;
   LayerScratch sc(op);
   if ((s = sc.get(sizeof(double))) != PT_OK) return s;
+  if (!op->full_box || !sc.p) PT_CUDA(cudaMemsetAsync(op->d_F, 0, sizeof(double) * op->nvel, op->stream));
+  if (!sc.p) {  // no room for the scratch
+    for (int c = 0; c < 8; c++) {
+      ptk::ColourGrid g = ptk::colour_grid(op->box, c);
+      const int64_t n = (int64_t)g.ncx * g.ncy * g.ncz;
+      if (n == 0) continue;
+      ptk::body_force_colour_kernel<<<nblocks(n), TPB, 0, op->stream>>>(g, op->d_coords, op->d_fu, op->d_F);
+      PT_LAUNCHED(op);
+    }
+    op->F_valid = true;
+    return PT_OK;
+  }
   ptk::body_force_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_fu,
                                                                                       sc.p);
   PT_LAUNCHED(op);

@@ -1,0 +1,57 @@
+"""Calls that run without the memory of the faster routes: with the device nearly full
+the operator falls back on kernels that need no more than K."""
+import numpy as np
+import pytest
+
+from conftest import relerr
+from pt_b200 import mesh as M
+
+pytestmark = pytest.mark.gpu
+
+TOL64 = 1e-12  # the project's parity bar for FP64 operators
+TOL32 = 5e-5   # and for the FP32 apply
+MB = 1 << 20
+
+
+def _calls(op, u, p):
+    import torch
+    out = [op.MatMult_MFStokes_A11(u), op.MFStokesWrapper_A11(u), op.MatMult_MFStokes_A11(u.float()).double(),
+           op.MatGetDiagonal_MFStokes_A11(torch.empty_like(u)), op.MatMult_MFStokes_A12(p), op.MatMult_MFStokes_A21(u),
+           *op.MatMult_MFStokes_A(u, p), op.FormFunctionLocal_U(u, p)]
+    return [o.cpu().numpy() for o in out]
+
+
+# room beside K: none for B's factors; none for the tiles' sums either
+@pytest.mark.parametrize("beside_k", [130 * MB, 22 * MB])
+def test_calls_with_the_device_nearly_full(beside_k):
+    import torch
+
+    from pt_b200 import MatStokesMF
+    dims = (40, 40, 40)
+    k_bytes, b_bytes, sums = 64000 * 243 * 12, 64000 * 324 * 8, 500 * 57 * 1024
+    assert beside_k < b_bytes and (beside_k < sums or beside_k > sums + 64000 * 108 * 8)
+    m, eta, mask = M.problem("box:%d,%d,%d" % dims, seed=4)
+    u, p = (torch.from_numpy(M.uniform_vec(n, 3)).cuda() for n in (m.nvel, m.npres))
+    fu = torch.from_numpy(M.uniform_vec(81 * m.nel, 7)).cuda()
+    torch.empty(1600 * MB, dtype=torch.uint8, device="cuda")  # stays in torch's cache, for the calls' outputs
+    with MatStokesMF(*dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        op.set_body_force(fu)
+        want = _calls(op, u, p)
+    with MatStokesMF(*dims, a11_op="b200_colour") as op:  # the colour kernels' local memory is there
+        op.SetUp(m.coords, eta, mask)
+        op.MatMult_MFStokes_A11(u)
+    with MatStokesMF(*dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        op.set_body_force(fu)
+        torch.cuda.synchronize()
+        free, _ = torch.cuda.mem_get_info()
+        hog = torch.empty(free - k_bytes - beside_k, dtype=torch.uint8, device="cuda")
+        try:
+            got = _calls(op, u, p)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+    for i, (g, w) in enumerate(zip(got, want)):
+        assert relerr(g, w) < (TOL32 if i == 2 else TOL64), i
+
