@@ -898,7 +898,10 @@ pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double
   if (!op->d_P) {
     s = alloc_if_room(op, (void **)&op->d_P, sizeof(double) * ptk::psize(op->nel));
     if (s != PT_OK || !op->d_P) return s;
-    if ((s = launch_geometry(op)) != PT_OK) return s;  // K again with the same values, and P
+    if ((s = launch_geometry(op)) != PT_OK) {  // K again with the same values, and P
+      op->geom_dirty = true;                   // P is not there yet
+      return s;
+    }
   }
   constexpr size_t smem = ptk::layer_smem_bytes<double, LNT>();
   if ((s = kernel_attrs((const void *)ptk::stokes_layer_kernel<LNT, true>, smem)) != PT_OK) return s;
