@@ -82,8 +82,6 @@ constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
 constexpr int64_t LAYER_F32_MAX_ELEMENTS = 1000000;
 // layer tiles: node numbers stay below 2^31, scratch (460 B per element) below 4 GB
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
-// every box: element-node numbers stay below 2^31
-constexpr int64_t MAX_ELEMENTS = (int64_t)1 << 28;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
 constexpr int PIPE_LAYERS = 6;
@@ -166,7 +164,7 @@ void op_free(pt_op *op, void *p)
 // this kind is tried until the coordinates change.
 pt_status alloc_if_room(pt_op *op, void **p, size_t bytes)
 {
-  if (op->lean) return PT_OK;
+  if (op->lean || !op->lg.tiles) return PT_OK;
   const cudaError_t e = op_alloc(op, p, bytes);
   if (e == cudaSuccess) return PT_OK;
   *p = nullptr;
@@ -447,6 +445,7 @@ struct LayerScratch {
   explicit LayerScratch(pt_op *o) : op(o) {}
   pt_status get(size_t value_bytes)
   {
+    if (!op->lg.tiles) return PT_OK;
     if (!op->graph_own && capturing(op)) {
       PT_CUDA(cudaMallocAsync((void **)&p, value_bytes * (size_t)op->lg.tiles * ptk::LayerLayout<LNT>::TILE, op->stream));
       of_graph = true;
@@ -551,6 +550,7 @@ pt_status ensure_f32(pt_op *op)
 pt_status alloc_geometry(pt_op *op)
 {
   if (op->d_K) return PT_OK;
+  if (!op->lg.tiles) return fail(PT_ERR_OOM, "%d x %d x %d elements: no room for K", op->mx, op->my, op->mz);
   const size_t nk = (size_t)ptk::ksize(op->nel);
   PT_CUDA(op_alloc(op, (void **)&op->d_K, (sizeof(double) + sizeof(float)) * nk + sizeof(unsigned int)));
   op->d_K32 = reinterpret_cast<float *>(op->d_K + nk);
@@ -1111,11 +1111,6 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
                 desc->ox, desc->oy, desc->oz, desc->mx, desc->my, desc->mz, (long long)nx, (long long)ny, (long long)nz);
   const int64_t nnodes = nx * ny * nz;
   if (nnodes > ((int64_t)1 << 40)) return fail(PT_ERR_BAD_ARG, "mesh too large");
-  // element and element-node numbers are 32-bit in the tile kernels: past what
-  // any device holds (coordinates and viscosity alone 600 bytes per element)
-  if ((int64_t)desc->mx * desc->my * desc->mz > MAX_ELEMENTS ||
-      (2 * (int64_t)desc->mx + 1) * (2 * (int64_t)desc->my + 1) * (2 * (int64_t)desc->mz + 1) > INT32_MAX)
-    return fail(PT_ERR_OOM, "%d x %d x %d elements do not fit a device", desc->mx, desc->my, desc->mz);
   pt_op *op = (pt_op *)calloc(1, sizeof(pt_op));
   if (!op) return fail(PT_ERR_OOM, "host allocation failed");
   op->mx = desc->mx; op->my = desc->my; op->mz = desc->mz;
@@ -1133,7 +1128,10 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   op->ntx = (desc->mx + op->TX - 1) / op->TX;
   op->a11_kernel = auto_kernel(op);
   op->a11_auto = true;
-  op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
+  // element-node numbers are 32-bit in the tile kernels: a larger box (K alone
+  // would be 780 GB) has no tiles and keeps to the colour kernels
+  if ((2 * (int64_t)op->mx + 1) * (2 * (int64_t)op->my + 1) * (2 * (int64_t)op->mz + 1) <= INT32_MAX)
+    op->lg = ptk::layer_grid<LNT>(op->mx, op->my, op->mz, op->box.X, op->box.XY, op->box.off);
   pt_op_set_tiling(op, 0);
   op->geom_dirty = true;
   cudaError_t e = cudaGetDevice(&op->device);
