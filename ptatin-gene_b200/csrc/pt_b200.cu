@@ -536,14 +536,30 @@ pt_status launch_stream(pt_op *op, const T *K, const T *u, T *y)
   return launch_stream_tx<T, 128, MASKED>(op, K, u, y);
 }
 
-// FP32 copies of coordinates and viscosity for the 8-colour FP32 kernel,
-// allocated as soon as an op turns to that kernel.
+pt_status coords_to_f32(pt_op *op)
+{
+  to_f32_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_coords, op->d_coords32, op->nvel);
+  PT_LAUNCHED(op);
+  return PT_OK;
+}
+
+pt_status eta_to_f32(pt_op *op)
+{
+  to_f32_kernel<<<grid_stride_blocks(27 * op->nel), 256, 0, op->stream>>>(op->d_eta, op->d_eta32, 27 * op->nel);
+  PT_LAUNCHED(op);
+  return PT_OK;
+}
+
+// FP32 copies of coordinates and viscosity for the 8-colour FP32 kernel, made as
+// soon as an op turns to that kernel and renewed with the originals from then on
+// (finish_coords, finish_eta), never in an apply.
 pt_status ensure_f32(pt_op *op)
 {
   if (op->d_eta32) return PT_OK;
   if (!op->d_coords32) PT_CUDA(op_alloc(op, (void **)&op->d_coords32, sizeof(float) * op->nvel));
   PT_CUDA(op_alloc(op, (void **)&op->d_eta32, sizeof(float) * 27 * op->nel));
-  return PT_OK;
+  pt_status s = op->has_coords ? coords_to_f32(op) : PT_OK;
+  return s == PT_OK && op->has_eta ? eta_to_f32(op) : s;
 }
 
 // K in FP64, in FP32 and the check counter, one allocation.
@@ -734,10 +750,6 @@ pt_status launch_a11(pt_op *op, const T *u, T *y, bool masked)
     if (s != PT_OK) return s;
     coords = op->d_coords32;
     eta = op->d_eta32;
-    to_f32_kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->d_coords, op->d_coords32, op->nvel);
-    PT_LAUNCHED(op);
-    to_f32_kernel<<<grid_stride_blocks(27 * op->nel), 256, 0, op->stream>>>(op->d_eta, op->d_eta32, 27 * op->nel);
-    PT_LAUNCHED(op);
   }
   for (int c = 0; c < 8; c++) {
     ptk::ColourGrid g = ptk::colour_grid(op->box, c);
@@ -1217,7 +1229,8 @@ static pt_status finish_coords(pt_op *op)
   op->F_valid = false;
   op->lean = false;
   op->state++;
-  return op->d_D && !op->full_box ? launch_div(op) : PT_OK;  // ensure_div
+  pt_status s = op->d_eta32 ? coords_to_f32(op) : PT_OK;
+  return s == PT_OK && op->d_D && !op->full_box ? launch_div(op) : s;  // ensure_div
 }
 
 static pt_status finish_eta(pt_op *op)
@@ -1225,7 +1238,7 @@ static pt_status finish_eta(pt_op *op)
   op->has_eta = true;
   op->geom_dirty = true;
   op->state++;
-  return PT_OK;
+  return op->d_eta32 ? eta_to_f32(op) : PT_OK;
 }
 
 pt_status pt_op_set_coords_h(pt_op *op, const double *coords)
