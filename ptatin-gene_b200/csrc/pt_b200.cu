@@ -1324,7 +1324,9 @@ pt_status pt_op_set_bc_mask_h(pt_op *op, const uint8_t *mask)
 {
   if (!op) return fail(PT_ERR_BAD_ARG, "op is NULL");
   if (!mask) {
+    // the packed bits too: graphs recorded with the mask read them
     PT_CUDA(cudaMemsetAsync(op->d_mask, 0, op->nvel, op->stream));
+    if (op->d_mbits) PT_CUDA(cudaMemsetAsync(op->d_mbits, 0, sizeof(uint32_t) * ((op->nvel + 31) / 32), op->stream));
     op->has_mask = false;
     op->state++;
   } else {

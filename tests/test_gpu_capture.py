@@ -124,3 +124,38 @@ def test_graphs_of_one_op_on_two_streams():
             torch.cuda.synchronize()
             for k, (y, w) in enumerate(zip(got, want)):
                 assert torch.equal(y, w), k
+
+
+def test_graphs_follow_the_mask():
+    """Recorded with one mask, replayed with another and with none."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, eta, mask = M.problem("box:13,15,12", seed=5)
+    u, p = (torch.from_numpy(M.uniform_vec(n, 3)).cuda() for n in (m.nvel, m.npres))
+    yp, ya, yb, yu, yq = (torch.empty_like(v) for v in (p, u, u, u, p))
+
+    def calls(op):
+        op.MatMult_MFStokes_A21(u, yp)
+        op.MatMult_MFStokes_A12(p, ya)
+        op.MatMult_MFStokes_A11(u, yb)
+        op.MatMult_MFStokes_A(u, p, yu, yq)
+
+    with MatStokesMF(*m.dims) as op, MatStokesMF(*m.dims) as own:
+        op.SetUp(m.coords, eta, mask)
+        own.SetUp(m.coords, eta, mask)
+        calls(op)
+        g, st = _record(op, lambda: calls(op))
+        for mk in (mask, np.roll(mask, 3), None):
+            op.set_bc_mask(mk)
+            own.set_bc_mask(mk)
+            for y in (yp, ya, yb, yu, yq):
+                y.fill_(np.nan)
+            torch.cuda.synchronize()
+            g.replay()
+            torch.cuda.synchronize()
+            got = [y.clone() for y in (yp, ya, yb, yu, yq)]
+            calls(own)
+            torch.cuda.synchronize()
+            for k, (a, b) in enumerate(zip(got, (yp, ya, yb, yu, yq))):
+                assert torch.equal(a, b), (k, mk is None)
