@@ -67,20 +67,27 @@ pt_status fail(pt_status s, const char *fmt, ...)
 
 enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 
-// "b200" picks stored element matrices for one-rank boxes of up to
-// EBE_AUTO_MAX_ELEMENTS (FP64 / FP32 apply, matrices vs layer tiles: 10^3
-// 15.0 / 12.1 vs 25 / 23 us, 13^3 21.0 / 15.3 vs 23.6 / 23.0 us, 16^3 36.5 /
-// 19.8 vs 25.0 / 24.9 us); layer tiles above; and, in FP64, the streaming
-// kernel for boxes from STREAM_AUTO_MIN_ELEMENTS whose rows nearly fill its
-// tiles (layer tiles vs streaming: 56^3 162 vs 187 us, 80^3 398 vs 515 us,
-// 96^3 619 vs 738 us; 64^3 198 vs 205 us, 128^3 1365 vs 1427 us applied again
-// and again to one box but 1560 vs 1511 us taking turns among three).  Such a
-// box's FP32 applies use layer tiles below LAYER_F32_MAX_ELEMENTS (64^3 142 vs
-// 175 us, 128x32x64 140 vs 172 us; 128^3 1025 vs 1014 us).
+// "b200" picks a kernel for the box, in each precision.
+// - One-rank boxes of up to EBE_AUTO_MAX_ELEMENTS: stored element matrices.  The
+//   line is where their set-up comes even with the faster applies: a new
+//   viscosity costs 0.5 us per element more than layer tiles, so 12^3 (apply
+//   15.1 vs 22.7 us) pays from 110 applies on, 13^3 in FP32 (15.5 vs 22.7 us)
+//   from 146, 16^3 in FP32 (16.7 vs 22.7 us) from 320.
+// - Streaming tiles for long boxes whose rows nearly fill them.  FP64, from
+//   STREAM_AUTO_MIN_ELEMENTS and with rows of whole warps (layer tiles vs
+//   streaming: 64x60x52 159 vs 167 us, 64x64x56 180 vs 177, 32x90x80 186 vs 175,
+//   64^3 201 vs 187, 128x64x64 370 vs 374, 128^3 1399 vs 1283; other rows: 62x62x66
+//   207 vs 217, 122x60x60 333 vs 396, 120x100x100 863 vs 939).  FP32, from
+//   STREAM_AUTO_MIN_F32_ELEMENTS (64^3 140 vs 144, 64x72x72 173 vs 187, 128x64x48
+//   200 vs 196, 122x60x60 234 vs 221, 128x64x64 263 vs 229, 128^3 990 vs 825).
+// - Streaming tiles past LAYER_MAX_ELEMENTS, where the layer tiles' scratch would
+//   grow past 4.3 GB (512 bytes per element at most for rows of three elements and
+//   more, 716 for rows of two, 1,433 for rows of one).
+// - Layer tiles for the rest (80^3 381 vs 484 us, 97x70x81 408 vs 547; FP32 273 vs
+//   279, 290 vs 294).
 constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
 constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
-constexpr int64_t LAYER_F32_MAX_ELEMENTS = 1000000;
-// layer tiles: node numbers stay below 2^31, scratch (460 B per element) below 4 GB
+constexpr int64_t STREAM_AUTO_MIN_F32_ELEMENTS = 350000;
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
@@ -110,8 +117,7 @@ struct pt_op {
   bool d_valid;   // d_D matches the coordinates
   double *d_D;    // factors of B and B^T at the Gauss points (built on first use)
   double *d_P;    // factors of the whole Stokes operator beyond K (from its first use, with K)
-  int a11_kernel;
-  bool a11_auto;  // chosen by auto_kernel ("b200"), not by name
+  int a11_kernel, a11_kernel32;  // of the FP64 and the FP32 apply
   int64_t launches;
   uint64_t state;  // bumped whenever coordinates, viscosity or the mask change
   int device;
@@ -405,13 +411,18 @@ pt_status launch_diag_stream(pt_op *op, double *d)
 
 constexpr int LNT = ptk::LAYER_NT;
 
-A11Kernel auto_kernel(const pt_op *op)
+A11Kernel auto_kernel(const pt_op *op, bool fp32)
 {
   if (op->full_box && op->nel <= EBE_AUTO_MAX_ELEMENTS) return A11_EBE;
   const bool full_rows = 10 * (int64_t)op->mx >= 9 * (int64_t)op->ntx * op->TX;
-  const bool stream = op->nel > LAYER_MAX_ELEMENTS || (op->nel >= STREAM_AUTO_MIN_ELEMENTS && full_rows);
-  return stream ? A11_STREAM : A11_LAYER;
+  const bool stream = fp32 ? op->nel >= STREAM_AUTO_MIN_F32_ELEMENTS && full_rows
+                           : op->nel >= STREAM_AUTO_MIN_ELEMENTS && full_rows && op->mx % 32 == 0;
+  return stream || op->nel > LAYER_MAX_ELEMENTS ? A11_STREAM : A11_LAYER;
 }
+
+// The kernel of T's apply.
+template <typename T>
+int op_kernel(const pt_op *op) { return sizeof(T) == 4 ? op->a11_kernel32 : op->a11_kernel; }
 
 // Holds the launches of an apply together, from the first tile that writes the
 // op's scratch to the last gather that reads it: another host thread's apply of
@@ -597,7 +608,7 @@ pt_status ensure_geometry(pt_op *op)
   if (!op->geom_dirty) return PT_OK;
   pt_status ks = alloc_geometry(op);
   if (ks != PT_OK) return ks;
-  if (op->a11_kernel == A11_LAYER || (op->a11_kernel == A11_STREAM && op->a11_auto && op->nel < LAYER_F32_MAX_ELEMENTS)) {
+  if (op->a11_kernel == A11_LAYER || op->a11_kernel32 == A11_LAYER) {
     pt_status s = ensure_layer(op);
     if (s != PT_OK) return s;
   }
@@ -709,17 +720,18 @@ const float *op_K<float>(const pt_op *op) { return op->d_K32; }
 template <typename T>
 pt_status launch_a11(pt_op *op, const T *u, T *y, bool masked)
 {
-  if (op->a11_kernel == A11_EBE && op->full_box) {
+  const int kernel = op_kernel<T>(op);
+  if (kernel == A11_EBE && op->full_box) {
     pt_status s = ensure_geometry(op);
     if (s != PT_OK) return s;
     if (op->geom_ok) return launch_ebe<T>(op, u, y, masked);
   }
-  if (op->a11_kernel == A11_STREAM || op->a11_kernel == A11_LAYER) {
+  if (kernel == A11_STREAM || kernel == A11_LAYER) {
     pt_status s = ensure_geometry(op);
     if (s != PT_OK) return s;
     if (op->geom_ok) {
       if (!op->full_box) PT_CUDA(cudaMemsetAsync(y, 0, sizeof(T) * op->nvel, op->stream));
-      if (op->a11_kernel == A11_LAYER || (sizeof(T) == 4 && op->a11_auto && op->nel < LAYER_F32_MAX_ELEMENTS)) {
+      if (kernel == A11_LAYER) {
         bool done;
         if ((s = launch_layer<T>(op, op_K<T>(op), u, y, masked, &done)) != PT_OK) return s;
         // a ghosted box's Dirichlet dofs outside the element box
@@ -1138,8 +1150,8 @@ static pt_status op_create_impl(const pt_mesh_desc *desc, cudaMemPool_t pool, cu
   pthread_mutex_init(&op->layer_mu, nullptr);
   op->TX = desc->mx <= 32 ? 32 : (desc->mx <= 64 ? 64 : 128);
   op->ntx = (desc->mx + op->TX - 1) / op->TX;
-  op->a11_kernel = auto_kernel(op);
-  op->a11_auto = true;
+  op->a11_kernel = auto_kernel(op, false);
+  op->a11_kernel32 = auto_kernel(op, true);
   // element-node numbers are 32-bit in the tile kernels: a larger box (K alone
   // would be 780 GB) has no tiles and keeps to the colour kernels
   if ((2 * (int64_t)op->mx + 1) * (2 * (int64_t)op->my + 1) * (2 * (int64_t)op->mz + 1) <= INT32_MAX)
@@ -1794,7 +1806,7 @@ pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
 {
   if (!op || !name) return fail(PT_ERR_BAD_ARG, "NULL argument");
   const bool by_name = strcmp(name, "b200") != 0;
-  if (!by_name) op->a11_kernel = auto_kernel(op);
+  if (!by_name) op->a11_kernel = auto_kernel(op, false);
   else if (!strcmp(name, "b200_stream")) op->a11_kernel = A11_STREAM;
   else if (!strcmp(name, "b200_ebe")) op->a11_kernel = A11_EBE;
   else if (!strcmp(name, "b200_layer")) {
@@ -1808,7 +1820,7 @@ pt_status pt_op_set_a11_kernel(pt_op *op, const char *name)
     op->a11_kernel = A11_COLOUR;
   }
   else return fail(PT_ERR_BAD_ARG, "No -a11_op %s", name);
-  op->a11_auto = !by_name;
+  op->a11_kernel32 = by_name ? op->a11_kernel : auto_kernel(op, true);
   return PT_OK;
 }
 

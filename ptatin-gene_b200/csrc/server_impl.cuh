@@ -631,7 +631,7 @@ pt_status srv_admit(pt_server *s, SrvReq *r, int slot)
   // the batch runs layer or streaming tiles; set-up applies use the same
   if (op->a11_kernel == A11_EBE) op->a11_kernel = A11_LAYER;
   if (s->o.lz > 0) op->a11_kernel = A11_STREAM;
-  if (op->a11_kernel == A11_STREAM) op->a11_auto = false;  // one kernel for the request's set-up and batch
+  op->a11_kernel32 = op->a11_kernel;  // in both precisions: the budget counts one
   if (s->o.lz > 0) {
     op->LZ = std::min(s->o.lz, op->mz);
     op->nzc = (op->mz + op->LZ - 1) / op->LZ;

@@ -1,0 +1,86 @@
+"""The default kernel ("b200") in each precision: every route of the rule is bitwise
+the kernel of that name, and a kernel chosen by name is used in both precisions."""
+import numpy as np
+import pytest
+
+from conftest import relerr
+from pt_b200 import mesh as M
+
+pytestmark = pytest.mark.gpu
+
+TOL32 = 5e-5  # the project's bar for the FP32 apply
+
+# box, kernel of the FP64 and of the FP32 apply
+ROUTES = [((60, 60, 60), "b200_layer", "b200_layer"), ((64, 64, 64), "b200_stream", "b200_layer"),
+          ((122, 60, 60), "b200_layer", "b200_stream"), ((128, 64, 48), "b200_stream", "b200_stream")]
+
+
+@pytest.fixture(scope="module", params=ROUTES, ids=lambda r: "x".join(map(str, r[0])))
+def box(request):
+    import torch
+
+    from pt_b200 import MatStokesMF
+    dims, k64, k32 = request.param
+    m = M.make_mesh(*dims, perturb=0.05, seed=1)
+    eta, mask = M.eta_per_element(m, contrast=1e4, seed=2), M.bc_mask_freeslip(*dims)
+    with MatStokesMF(*dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        yield m, eta, mask, torch.from_numpy(M.uniform_vec(m.nvel, 3)).cuda(), op, k64, k32
+
+
+def _applies(op, u):
+    import torch
+    return [op.MatMult_MFStokes_A11(u, torch.empty_like(u)), op.MFStokesWrapper_A11(u, torch.empty_like(u))]
+
+
+def test_default_route_is_the_named_kernel(box):
+    import torch
+    m, eta, mask, u, op, k64, k32 = box
+    op.set_a11_op("b200")
+    assert op.a11_op == k64
+    got = [*_applies(op, u), *_applies(op, u.float())]
+    for name in (k64, k32):
+        op.set_a11_op(name)
+        want = [*_applies(op, u), *_applies(op, u.float())]
+        for i, (g, w) in enumerate(zip(got, want)):
+            if name == (k64 if i < 2 else k32):
+                assert torch.equal(g, w), (name, i)
+    op.set_a11_op("b200")
+
+
+def test_default_fp32_apply_matches_oracle(box, ora):
+    m, eta, mask, u, op, k64, k32 = box
+    op.set_a11_op("b200")
+    y = op.MatMult_MFStokes_A11(u.float()).double().cpu().numpy()
+    assert relerr(y, ora.matmult_a11(m.dims, m.coords, eta, mask, u.cpu().numpy())) < TOL32
+
+
+def test_default_fp32_apply_on_a_ghosted_box(ora):
+    """FP32 of a ghosted streaming box: zeros outside the element box, Dirichlet dofs
+    there copied, the inside the oracle's."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    dims, g = (64, 56, 60), 1
+    m = M.make_mesh(*dims, perturb=0.05, seed=1)
+    eta = M.eta_per_element(m, contrast=1e4, seed=2)
+    nb = tuple(2 * d + 1 + 2 * g for d in dims)
+    rng = np.random.default_rng(3)
+    sl = tuple(slice(g, g + 2 * d + 1) for d in dims[::-1])
+    c = rng.uniform(size=(nb[2], nb[1], nb[0], 3))
+    c[sl] = m.coords.reshape(c[sl].shape)
+    u = rng.uniform(-1, 1, size=c.shape)
+    mask = rng.uniform(size=c.shape) < 0.05
+    uz = np.where(mask, 0.0, u)
+    ref = np.zeros_like(u)
+    ref[sl] = ora.a11(dims, m.coords, eta, np.ascontiguousarray(uz[sl].reshape(-1))).reshape(ref[sl].shape)
+    ref[mask] = u[mask]
+    with MatStokesMF(*dims, node_box=(*nb, g, g, g)) as op:
+        op.SetUp(np.ascontiguousarray(c.reshape(-1)), eta, np.ascontiguousarray(mask.reshape(-1)).astype(np.uint8))
+        assert op.a11_op == "b200_stream"
+        ud = torch.from_numpy(np.ascontiguousarray(u.reshape(-1))).cuda().float()
+        y = op.MatMult_MFStokes_A11(ud).double().cpu().numpy()
+        assert relerr(y, ref.reshape(-1)) < TOL32
+        inside = np.zeros(c.shape, dtype=bool)
+        inside[sl] = True
+        assert not y.reshape(c.shape)[~inside & ~mask].any()
