@@ -249,21 +249,23 @@ pt_status pt_solver_destroy(pt_solver *solver);
 /* ---- batched A11 over many independent boxes ----------------------------
  *
  * No counterpart in the reference (one operator per rank there).  A work-list
- * over n ops (one-rank boxes, coords and eta set): every (problem, x-tile,
- * row, z-chunk) tile, grouped by colour and tile width; an apply is one launch
- * per non-empty class (at most 8 colours x 3 widths) over the concatenated
- * list, and each problem's result is bitwise what its own apply gives.
- * lz[i] = element layers per z-chunk for problem i (0 = the op's default);
- * the autotuner in pt_b200/batch.py picks it. */
+ * over n ops (one-rank boxes, coords and eta set), each on the tiles of its own
+ * apply in the precision applied: boxes on layer tiles (and those whose own
+ * applies use element matrices) in two launches together, boxes on streaming
+ * tiles in one launch per non-empty class of colour and tile width (at most
+ * 8 x 3).  A problem's result is bitwise what its own apply on layer or streaming
+ * tiles gives.  lz[i] > 0 = element layers per z-chunk for problem i: streaming
+ * tiles of that depth whatever its own apply uses (equal to rounding then; the
+ * autotuner in pt_b200/batch.py picks it); 0 = as its own apply. */
 typedef struct pt_batch pt_batch;
 pt_status pt_batch_create(int n, pt_op *const *ops, const int32_t *lz, pt_batch **batch);
-/* As pt_batch_create with every box tiled tile_x elements wide (32, 64 or
- * 128; 0 = each box's own width).  One width for all boxes puts the whole
- * batch in one class per colour, fewer launches per apply. */
+/* As pt_batch_create with every streaming tile tile_x elements wide (32, 64 or
+ * 128; 0 = each box's own width).  One width for all boxes puts them in one class
+ * per colour, fewer launches per apply.  Layer tiles have one width. */
 pt_status pt_batch_create_tiled(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, pt_batch **batch);
 pt_status pt_batch_destroy(pt_batch *batch);
-/* Colour-class launches of one apply (a masked apply adds one launch for the
- * Dirichlet rows of every problem). */
+/* Launches of one FP64 apply (a masked apply adds one for the Dirichlet rows of
+ * the problems on streaming tiles), and its tiles. */
 int64_t pt_batch_launches_per_apply(const pt_batch *batch);
 int64_t pt_batch_tiles(const pt_batch *batch);
 /* y_i = A11_i u_i for every problem; u, y are DEVICE arrays of n device

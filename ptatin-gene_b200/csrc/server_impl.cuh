@@ -803,14 +803,14 @@ pt_status srv_iterate(pt_server *s)
   void **tab = (void **)s->d_ptrs;
   pt_status e = batch_apply<double, true>(s->batch, (const double *const *)tab, (double *const *)(tab + n), st);
   if (e != PT_OK) return e;
-  s->launches += pt_batch_launches_per_apply(s->batch) + (s->batch->coloured ? 1 : 0);
+  s->launches += batch_launches(s->batch, false);
   chain(srv_pq_kernel, ni, SRV_THREADS, st, s->d_items, s->d_slots, s->d_scal);
   chain(srv_final_kernel<SRV_F_ALPHA>, na, SRV_THREADS, st, s->d_act, s->d_slots, s->d_scal);
   chain(srv_update_kernel, ni, SRV_THREADS, st, s->d_items, s->d_slots, s->d_scal);
   chain(srv_final_kernel<SRV_F_RR>, na, SRV_THREADS, st, s->d_act, s->d_slots, s->d_scal);
   s->launches += 4;
   e = srv_precond<T>(s, s->d_items, ni, st, [&]() {
-    s->launches += pt_batch_launches_per_apply(s->batch) + (s->batch->coloured ? 1 : 0);
+    s->launches += batch_launches(s->batch, std::is_same<T, float>::value);
     return batch_apply<T, true>(s->batch, (const T *const *)(tab + 2 * n), (T *const *)(tab + 3 * n), st);
   });
   if (e != PT_OK) return e;

@@ -1,9 +1,11 @@
 """Batched A11 over many independent boxes (pt_batch_* in the C ABI), and the
 work-list autotuner.
 
-A ``BatchA11`` is built once from a list of set-up ``MatStokesMF`` ops; an apply
-is one launch per (colour, tile width) class over the concatenated tile
-work-list, and each problem's result is bitwise what its own apply gives.
+A ``BatchA11`` is built once from a list of set-up ``MatStokesMF`` ops.  Boxes on
+layer tiles are applied in two launches together, boxes on streaming tiles in one
+launch per (colour, tile width) class; each problem's result is bitwise what its
+own apply on those tiles gives (``lz`` and ``tile_x``: streaming tiles of the
+caller's depth and width).
 """
 from __future__ import annotations
 

@@ -1,5 +1,6 @@
 """The default kernel ("b200") in each precision: every route of the rule is bitwise
-the kernel of that name, and a kernel chosen by name is used in both precisions."""
+the kernel of that name, alone and in a batch, and a kernel chosen by name is used in
+both precisions."""
 import numpy as np
 import pytest
 
@@ -53,6 +54,28 @@ def test_default_fp32_apply_matches_oracle(box, ora):
     op.set_a11_op("b200")
     y = op.MatMult_MFStokes_A11(u.float()).double().cpu().numpy()
     assert relerr(y, ora.matmult_a11(m.dims, m.coords, eta, mask, u.cpu().numpy())) < TOL32
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_batch_of_default_ops_is_bitwise_their_own_applies(box, fp32):
+    import torch
+
+    from pt_b200 import MatStokesMF
+    from pt_b200.batch import BatchA11
+    m, eta, mask, u, op, k64, k32 = box
+    op.set_a11_op("b200")
+    small = M.make_mesh(17, 13, 11, perturb=0.05, seed=4)
+    with MatStokesMF(17, 13, 11) as other:
+        other.SetUp(small.coords, M.eta_per_element(small, contrast=1e2, seed=5), M.bc_mask_freeslip(17, 13, 11))
+        us = [u, torch.from_numpy(M.uniform_vec(small.nvel, 6)).cuda()]
+        us = [v.float() for v in us] if fp32 else us
+        for masked in (True, False):
+            ys = [torch.full_like(v, float("nan")) for v in us]
+            with BatchA11([op, other]) as b:
+                b.apply(us, ys, masked=masked)
+                torch.cuda.synchronize()
+            for o, v, y in zip((op, other), us, ys):
+                assert torch.equal(y, _applies(o, v)[0 if masked else 1])
 
 
 def test_default_fp32_apply_on_a_ghosted_box(ora):
