@@ -155,7 +155,7 @@ int64_t batch_launches(const pt_batch *b, bool fp32)
   return (int64_t)l.classes.size() + (l.lay_tiles ? 2 : 0) + (l.coloured ? 1 : 0);
 }
 
-void batch_list(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, bool fp32, pt_batch::List &l)
+void batch_list(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, bool fp32, bool layers, pt_batch::List &l)
 {
   // class key: (pass, TX) -> items
   std::map<std::pair<int, int>, std::vector<int4>> cls;
@@ -173,10 +173,11 @@ void batch_list(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, boo
     d.mask = op->has_mask ? op->d_mask : nullptr;
     d.mbits = op->has_mask ? op->d_mbits : nullptr;
     d.nvel = op->nvel;
-    // layer tiles unless the caller asks for a z-chunk depth (a box whose own
-    // applies use element matrices too: they are not batched)
+    // layer tiles unless the caller asks for a z-chunk depth or there is no room
+    // for their sums (a box whose own applies use element matrices too: they are
+    // not batched)
     const int kernel = fp32 ? op->a11_kernel32 : op->a11_kernel;
-    d.layer = (kernel == A11_LAYER || kernel == A11_EBE) && !(lz && lz[i] > 0);
+    d.layer = layers && (kernel == A11_LAYER || kernel == A11_EBE) && !(lz && lz[i] > 0);
     d.lg = op->lg;
     d.lay_off = l.lay_values;
     d.K = fp32 ? (const void *)op->d_K32 : (const void *)op->d_K;
@@ -231,7 +232,7 @@ extern "C" {
 // pool == null: cudaMalloc + synchronous upload; else buffers from `pool`
 // with asynchronous uploads, both ordered on `stream`.
 static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, cudaMemPool_t pool,
-                                   cudaStream_t stream, pt_batch **out)
+                                   cudaStream_t stream, pt_batch **out, bool layers = true)
 {
   if (!out || n < 1 || !ops) return fail(PT_ERR_BAD_ARG, "need n >= 1 ops");
   if (tile_x != 0 && tile_x != 32 && tile_x != 64 && tile_x != 128)
@@ -255,7 +256,7 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
   cudaError_t e = cudaSuccess;
   for (int f = 0; f < 2; f++) {
     pt_batch::List &l = b->list[f];
-    batch_list(n, ops, lz, tile_x, f != 0, l);
+    batch_list(n, ops, lz, tile_x, f != 0, layers, l);
     if (e == cudaSuccess) e = batch_upload(b, &l.d_probs, l.h);
     if (e == cudaSuccess) e = batch_upload(b, &l.d_items, l.hitems);
     if (e == cudaSuccess) e = batch_upload(b, &l.d_lay, l.hlay);
@@ -276,6 +277,11 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
     // one apply's scratch is there before the first apply
     void *first = nullptr;
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&first, scratch, b->lay_pool, stream);
+    if (e == cudaErrorMemoryAllocation) {  // no room for the sums: all boxes on streaming tiles
+      cudaGetLastError();
+      pt_batch_destroy(b);
+      return batch_create_impl(n, ops, lz, tile_x, pool, stream, out, false);
+    }
     if (e == cudaSuccess) e = cudaFreeAsync(first, stream);
   }
   if (e != cudaSuccess) {
