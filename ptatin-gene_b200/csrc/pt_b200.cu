@@ -45,6 +45,8 @@ pt_status fail(pt_status s, const char *fmt, ...)
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
   g_err = buf;
+  // reported here: the next launch check must not find it again
+  if (s == PT_ERR_CUDA || s == PT_ERR_OOM) cudaGetLastError();
   return s;
 }
 

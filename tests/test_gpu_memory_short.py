@@ -107,3 +107,14 @@ def test_batch_with_no_room_for_the_sums(fp32):
             del hog
             torch.cuda.empty_cache()
     assert relerr(y.double().cpu(), want.double().cpu()) < (TOL32 if fp32 else TOL64)
+
+
+def test_a_failed_call_does_not_fail_the_next_one(ora):
+    from pt_b200 import MatStokesMF, _capi
+    m, eta, mask = M.problem("box:5,4,3", seed=5)
+    x = M.uniform_vec(m.nvel, 6)
+    with MatStokesMF(*m.dims) as op:
+        with pytest.raises(_capi.PtError):
+            MatStokesMF(2000, 2000, 2000)  # 1.5 TB of coordinates
+        op.SetUp(m.coords, eta, mask)
+        assert relerr(op.MatMult_MFStokes_A11(x), ora.matmult_a11(m.dims, m.coords, eta, mask, x)) < TOL64
