@@ -115,6 +115,6 @@ def test_a_failed_call_does_not_fail_the_next_one(ora):
     x = M.uniform_vec(m.nvel, 6)
     with MatStokesMF(*m.dims) as op:
         with pytest.raises(_capi.PtError):
-            MatStokesMF(2000, 2000, 2000)  # 1.5 TB of coordinates
+            MatStokesMF(2, 2, 2, node_box=(8000, 8000, 8000, 0, 0, 0))  # 12 TB of coordinates
         op.SetUp(m.coords, eta, mask)
         assert relerr(op.MatMult_MFStokes_A11(x), ora.matmult_a11(m.dims, m.coords, eta, mask, x)) < TOL64
