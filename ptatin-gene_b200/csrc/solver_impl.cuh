@@ -507,6 +507,14 @@ void mg_release(pt_solver *s, void *p)
   if (p) cudaFreeAsync(p, s->op->stream);
 }
 
+// Pool memory of one scope, given back whichever way the scope ends.
+struct MgTemp {
+  pt_solver *s;
+  double *p = nullptr;
+  explicit MgTemp(pt_solver *s_) : s(s_) {}
+  ~MgTemp() { mg_release(s, p); }
+};
+
 // Gives the hierarchy back to the pool behind the work queued on `st`.
 void mg_free(pt_solver *s, cudaStream_t st)
 {
@@ -569,16 +577,17 @@ pt_status mg_dense_inverse(pt_solver *s, pt_mg_level &L, bool fp32)
   const pt_op *op = L.op;
   const cudaStream_t st = op->stream;
   const int n = (int)L.n, nb = (n + ptk::DN_B - 1) / ptk::DN_B, np = nb * ptk::DN_B;
-  double *Ae = L.Ae64;  // Galerkin level: its own matrices; else re-discretised ones
+  MgTemp own(s), work(s);
+  const double *Ae = L.Ae64;  // Galerkin level: its own matrices; else re-discretised ones
   if (!Ae) {
-    PT_CUDA(mg_alloc(s, &Ae, sizeof(double) * ptk::EBE_LD * op->nel));
-    ptk::element_matrix_kernel<double><<<(unsigned)op->nel, 96, 0, st>>>(op->box, op->d_coords, op->d_eta, Ae);
+    PT_CUDA(mg_alloc(s, &own.p, sizeof(double) * ptk::EBE_LD * op->nel));
+    ptk::element_matrix_kernel<double><<<(unsigned)op->nel, 96, 0, st>>>(op->box, op->d_coords, op->d_eta, own.p);
+    Ae = own.p;
   }
   // the matrix, the panels, the pivot block's inverse, the check
-  double *A = nullptr;
   const size_t values = (size_t)np * np + 2 * (size_t)np * ptk::DN_B + ptk::DN_B * ptk::DN_B;
-  PT_CUDA(mg_alloc(s, &A, sizeof(double) * values + sizeof(int)));
-  double *R = A + (size_t)np * np, *C = R + (size_t)np * ptk::DN_B, *D = C + (size_t)np * ptk::DN_B;
+  PT_CUDA(mg_alloc(s, &work.p, sizeof(double) * values + sizeof(int)));
+  double *const A = work.p, *R = A + (size_t)np * np, *C = R + (size_t)np * ptk::DN_B, *D = C + (size_t)np * ptk::DN_B;
   int *bad = reinterpret_cast<int *>(A + values);
   PT_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
   ptk::dense_assemble_kernel<<<(unsigned)np, 96, 0, st>>>(op->box, Ae, op->d_mask, n, np, A);
@@ -595,8 +604,6 @@ pt_status mg_dense_inverse(pt_solver *s, pt_mg_level &L, bool fp32)
   int h_bad = 0;
   cudaError_t e = cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  mg_release(s, A);
-  if (Ae != L.Ae64) mg_release(s, Ae);
   if (e != cudaSuccess) return fail(PT_ERR_CUDA, "coarse inverse: %s", cudaGetErrorString(e));
   if (h_bad) return fail(PT_ERR_STATE, "coarse operator is not positive definite");
   return PT_OK;
