@@ -26,6 +26,7 @@
 #include "kernels_stream.cuh"
 #include "kernels_diag.cuh"
 #include "kernels_layer.cuh"
+#include "kernels_bmat.cuh"
 #include "kernels_ebe.cuh"
 #include "kernels_markers.cuh"
 #include "kernels_galerkin.cuh"
@@ -91,6 +92,13 @@ constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
 constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
 constexpr int64_t STREAM_AUTO_MIN_F32_ELEMENTS = 350000;
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
+// B and B^T of one-rank boxes from stored element blocks up to this size, on layer
+// tiles above (and on ghosted boxes).  B u and B^T p together, blocks vs layer
+// tiles, boxes taking turns: 16^3 15 vs 32 us, 28^3 33 vs 49, 36^3 66 vs 78,
+// 64x48x40 157 vs 174, 61x50x77 292 vs 304; with the set-up that new coordinates
+// need 37 vs 47, 134 vs 67, 274 vs 115, 669 vs 263 and 1248 vs 462 us.  So a mesh
+// pays for its blocks after 1, 4, 13, 24 and 70 pairs of applies.
+constexpr int64_t DIV_BLOCKS_MAX_ELEMENTS = 125000;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
 constexpr int PIPE_LAYERS = 6;
@@ -118,6 +126,7 @@ struct pt_op {
   bool geom_dirty, geom_ok, full_box, ebe_valid;
   bool d_valid;   // d_D matches the coordinates
   double *d_D;    // factors of B and B^T at the Gauss points (built on first use)
+  double *d_Be;   // behind them, for small one-rank boxes: the element blocks of B
   double *d_P;    // factors of the whole Stokes operator beyond K (from its first use, with K)
   int a11_kernel, a11_kernel32;  // of the FP64 and the FP32 apply
   int64_t launches;
@@ -837,6 +846,10 @@ pt_status launch_div(pt_op *op)
   if (s != PT_OK) return s;
   ptk::div_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_coords, op->d_D);
   PT_LAUNCHED(op);
+  if (op->d_Be) {
+    ptk::bmat_kernel<<<nblocks(op->nel, ptk::BMAT_EL), 32 * ptk::BMAT_EL, 0, op->stream>>>(op->nel, op->d_D, op->d_Be);
+    PT_LAUNCHED(op);
+  }
   op->d_valid = true;
   return PT_OK;
 }
@@ -849,7 +862,12 @@ pt_status launch_div(pt_op *op)
 pt_status ensure_div(pt_op *op, bool *have)
 {
   pt_status s = PT_OK;
-  if (!op->d_D && !capturing(op)) s = alloc_if_room(op, (void **)&op->d_D, sizeof(double) * ptk::dsize(op->nel));
+  if (!op->d_D && !capturing(op)) {
+    const int64_t nd = ptk::dsize(op->nel);
+    const bool blocks = op->full_box && op->nel <= DIV_BLOCKS_MAX_ELEMENTS;
+    s = alloc_if_room(op, (void **)&op->d_D, sizeof(double) * (nd + (blocks ? ptk::BMAT_LD * op->nel : 0)));
+    op->d_Be = op->d_D && blocks ? op->d_D + nd : nullptr;
+  }
   *have = op->d_D != nullptr;
   return s != PT_OK || !*have || op->d_valid ? s : launch_div(op);
 }
@@ -867,6 +885,12 @@ pt_status a21_d(pt_op *op, const double *u, double *yp, bool masked)
     PT_LAUNCHED(op);
     return PT_OK;
   }
+  if (op->d_Be) {
+    ptk::bmat_a21_kernel<<<nblocks(32 * op->nel), TPB, 0, op->stream>>>(op->box, op->d_Be, u,
+                                                                        masked ? op->d_mask : nullptr, yp);
+    PT_LAUNCHED(op);
+    return PT_OK;
+  }
   constexpr size_t smem = ptk::layer_geom_smem_bytes<LNT>();
   if ((s = kernel_attrs((const void *)ptk::a21_layer_kernel<LNT>, smem)) != PT_OK) return s;
   ptk::a21_layer_kernel<LNT><<<(unsigned)op->lg.tiles, LNT, smem, op->stream>>>(op->lg, op->d_D, u,
@@ -881,6 +905,14 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
   bool have;
   pt_status s = ensure_div(op, &have);
   if (s != PT_OK) return s;
+  zero = zero && op->has_mask;
+  if (have && op->d_Be) {
+    auto kernel = accumulate ? ptk::bmat_a12_kernel<ptk::LAYER_ADD>
+                             : (zero ? ptk::bmat_a12_kernel<ptk::LAYER_BC_ZERO> : ptk::bmat_a12_kernel<ptk::LAYER_PLAIN>);
+    kernel<<<grid_stride_blocks(op->nvel), 256, 0, op->stream>>>(op->box, op->d_Be, p, op->d_mask, yu);
+    PT_LAUNCHED(op);
+    return PT_OK;
+  }
   LayerScratch sc(op);
   if (have && (s = sc.get(sizeof(double))) != PT_OK) return s;
   have = have && sc.p;
@@ -901,8 +933,8 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
   PT_LAUNCHED(op);
   const uint32_t n = op->lg.nodes();
   if (accumulate) return launch_layer_gather<double, ptk::LAYER_ADD>(op, sc.p, 0, n, nullptr, yu);
-  return zero && op->has_mask ? launch_layer_gather<double, ptk::LAYER_BC_ZERO>(op, sc.p, 0, n, nullptr, yu)
-                              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, n, nullptr, yu);
+  return zero ? launch_layer_gather<double, ptk::LAYER_BC_ZERO>(op, sc.p, 0, n, nullptr, yu)
+              : launch_layer_gather<double, ptk::LAYER_PLAIN>(op, sc.p, 0, n, nullptr, yu);
 }
 
 // Yu = A11 u + B^T p (- x when mode is LAYER_SUB) and, unless yp is null,
