@@ -99,6 +99,13 @@ constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
 // need 37 vs 47, 134 vs 67, 274 vs 115, 669 vs 263 and 1248 vs 462 us.  So a mesh
 // pays for its blocks after 1, 4, 13, 24 and 70 pairs of applies.
 constexpr int64_t DIV_BLOCKS_MAX_ELEMENTS = 125000;
+// The whole operator of smaller boxes block by block, A11 from their element
+// matrices: 4^3 21.9 vs 27.0 us in one pass over the tiles, 6^3 22.9 vs 31.0, 8^3
+// 24.9 vs 29.0, 9^3 25.0 vs 29.0, 12^3 29.3 vs 28.9.  A new viscosity costs 65, 124,
+// 253, 360 and 820 us more (their matrices), which that many applies pay for: 13,
+// 15, 60, 90, none.  The residual, which comes with a new viscosity as a rule (8^3
+// together 74 vs 322 us), is always formed in one pass.
+constexpr int64_t STOKES_BLOCKS_MAX_ELEMENTS = 512;
 // pipelined host-pointer applies: groups of about PIPE_LAYERS element layers,
 // at most PIPE_GROUPS of them
 constexpr int PIPE_LAYERS = 6;
@@ -938,15 +945,16 @@ pt_status a12_d(pt_op *op, const double *p, double *yu, bool accumulate = false,
 }
 
 // Yu = A11 u + B^T p (- x when mode is LAYER_SUB) and, unless yp is null,
-// Yp = B u, in one pass over the tiles; *done = false where the geometry does
-// not allow K or the device has no room, and in a capture that comes before the
-// first use (the caller then runs the blocks one by one).  masked: Dirichlet
-// columns of u as zeros, rows copied from u.
+// Yp = B u, in one pass over the tiles; *done = false where the blocks are faster
+// one by one, the geometry does not allow K or the device has no room, and in a
+// capture that comes before the first use (the caller then runs the blocks).
+// masked: Dirichlet columns of u as zeros, rows copied from u.
 pt_status stokes_fused(pt_op *op, const double *u, const double *p, const double *x, double *yu, double *yp, int mode,
                        bool *done)
 {
   *done = false;
-  if (op->a11_kernel == A11_COLOUR) return PT_OK;
+  if (op->a11_kernel == A11_COLOUR || (op->a11_kernel == A11_EBE && yp && op->nel <= STOKES_BLOCKS_MAX_ELEMENTS))
+    return PT_OK;
   pt_status s = ensure_geometry(op);
   if (s != PT_OK) return s;
   if (!op->geom_ok) return PT_OK;

@@ -35,3 +35,27 @@ def test_b_and_bt_match_oracle(ora, workload):
         yu, yp = op.MFStokesWrapper_A(ud, pd)
         assert relerr(yu.cpu(), ora.a11(m.dims, m.coords, eta, u) + ora.a12(m.dims, m.coords, p)) < TOL64
         assert relerr(yp.cpu(), ora.a21(m.dims, m.coords, u)) < TOL64
+
+
+@pytest.mark.parametrize("workload", ["box:1,1,1", "box:8,8,8", "box:9,8,8", "box:13,13,12"])
+def test_whole_operator_matches_oracle(ora, workload):
+    """Block by block up to 512 elements, in one pass above."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m, eta, mask = M.problem(workload, seed=3)
+    u, p = M.uniform_vec(m.nvel, 4), M.uniform_vec(m.npres, 5)
+    ud, pd = torch.from_numpy(u).cuda(), torch.from_numpy(p).cuda()
+    bc = mask.astype(bool)
+    with MatStokesMF(*m.dims) as op:
+        op.SetUp(m.coords, eta, mask)
+        yu, yp = (y.cpu().numpy() for y in op.MFStokesWrapper_A(ud, pd))
+        assert relerr(yu, ora.a11(m.dims, m.coords, eta, u) + ora.a12(m.dims, m.coords, p)) < TOL64
+        assert relerr(yp, ora.a21(m.dims, m.coords, u)) < TOL64
+        yu, yp = (y.cpu().numpy() for y in op.MatMult_MFStokes_A(ud, pd))
+        ref = ora.matmult_a11(m.dims, m.coords, eta, mask, u) + ora.matmult_a12(m.dims, m.coords, mask, p)
+        assert relerr(yu, ref) < TOL64 and np.array_equal(yu[bc], u[bc])
+        assert relerr(yp, ora.matmult_a21(m.dims, m.coords, mask, u)) < TOL64
+        pa = pd.clone()  # one vector as xp and yp
+        yb, ya = op.MatMult_MFStokes_A(ud, pa, None, pa)
+        assert np.array_equal(yb.cpu(), yu) and np.array_equal(ya.cpu(), yp)
