@@ -411,7 +411,7 @@ __device__ __forceinline__ void layer_jacobian(int A, const double *xt, const La
 }
 
 // Element e's four pressure sums.
-__device__ __forceinline__ void store_p(double *__restrict__ yp, int e, const double Y[4])
+__device__ __forceinline__ void store_p(double *yp, int e, const double Y[4])
 {
   double *y = yp + 4 * (int64_t)e;
   if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
@@ -473,13 +473,15 @@ __device__ __forceinline__ void stokes_plane(int A, const double *ut, double *yt
   }
 }
 
+// pr and yp may be one vector: an element's thread reads its four entries before it
+// writes them.
 template <int NT, bool DIV>
 __global__ void __launch_bounds__(NT, 256 / NT) stokes_layer_kernel(LayerGrid g, const double *__restrict__ K,
                                                                     const double *__restrict__ P,
                                                                     const double *__restrict__ u,
-                                                                    const double *__restrict__ pr,
+                                                                    const double *pr,
                                                                     const uint32_t *__restrict__ mbits,
-                                                                    double *__restrict__ out, double *__restrict__ yp)
+                                                                    double *__restrict__ out, double *yp)
 {
   using L = LayerLayout<NT>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
