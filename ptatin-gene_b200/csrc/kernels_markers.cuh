@@ -64,8 +64,66 @@ __global__ void mk_starts_kernel(const int32_t *__restrict__ keys, int64_t n, in
 // MK_AHEAD of them loaded before they are used.  A warp per element with one
 // lane per node kept 81 sums per element, 19 times the same ones, and moved
 // every marker through ten shuffles: 64^3 with 2.1 M markers 186 us.
+//
+// A crowded element, which the others do not hide, pays two dependent round trips
+// per MK_AHEAD markers (160 ns a marker).  There lane v takes marker v of every
+// eight, an index ahead of its data and the data ahead of their sums, and the eight
+// are passed from lane to lane in order (same sums, 124 ns; 8^3 with 4096 per
+// element 1,215 -> 717 us, 100,000 in one element 16.0 -> 12.4 ms).  Where there
+// are elements enough to hide the trips the shuffles cost more than they save
+// (32^3 with 256 per element 444 vs 578 us), so a box that fills the chip (about
+// MK_FEW elements) goes that way for its outliers only.
 constexpr int MK_SUMS = 27;
 constexpr int MK_AHEAD = 4;
+constexpr int64_t MK_FEW = 16384;                      // elements
+constexpr int64_t MK_CROWDED_FEW = 256, MK_CROWDED = 1024;  // markers in an element
+
+// A crowded element's five sums of lane v, out of line so that the common loop keeps
+// its registers.
+struct MkSums {
+  double s1, s2, sb, c1, c2;
+};
+__device__ __noinline__ MkSums mk_crowded(int v, int64_t m0, int64_t m1, const int32_t *__restrict__ order,
+                                          const double *__restrict__ xi, const double *__restrict__ eta,
+                                          const double *__restrict__ rho)
+{
+  const unsigned group = 0xffu << (threadIdx.x & 24);
+  MkSums s = {};
+  double a[5] = {};  // lane v: marker v of the eight under way
+  const auto index = [&](int64_t c) { return c + v < m1 ? order[c + v] : -1; };
+  const auto load = [&](int64_t p) {
+    if (p < 0) return;
+    a[0] = xi[3 * p];
+    a[1] = xi[3 * p + 1];
+    a[2] = xi[3 * p + 2];
+    a[3] = eta[p];
+    a[4] = rho[p];
+  };
+  load(index(m0));
+  int64_t next = index(m0 + 8);
+  for (int64_t c0 = m0; c0 < m1; c0 += 8) {
+    double m[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) m[i] = a[i];
+    load(next);  // in flight while this eight is summed
+    next = index(c0 + 16);
+    const int n = (int)min((int64_t)8, m1 - c0);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (k < n) {
+        double w[5];
+#pragma unroll
+        for (int i = 0; i < 5; i++) w[i] = __shfl_sync(group, m[i], k, 8);
+        const double N = mk_q1(v, w[0], w[1], w[2]);
+        s.s1 += N * w[3];
+        s.s2 += N * w[4];
+        s.sb += N;
+        s.c1 += w[3];
+        s.c2 += w[4];
+      }
+  }
+  return s;
+}
 
 __global__ void __launch_bounds__(128) mk_element_kernel(int64_t nel, const int64_t *__restrict__ start,
                                                          const int32_t *__restrict__ order,
@@ -77,7 +135,16 @@ __global__ void __launch_bounds__(128) mk_element_kernel(int64_t nel, const int6
   if (e >= nel) return;
   double s1 = 0.0, s2 = 0.0, sb = 0.0, c1 = 0.0, c2 = 0.0;
   const int64_t m0 = start[e], m1 = start[e + 1];
-  for (int64_t c0 = m0; c0 < m1; c0 += MK_AHEAD) {
+  const bool crowded = m1 - m0 > (nel <= MK_FEW ? MK_CROWDED_FEW : MK_CROWDED);
+  if (crowded) {
+    const MkSums s = mk_crowded(v, m0, m1, order, xi, eta, rho);
+    s1 = s.s1;
+    s2 = s.s2;
+    sb = s.sb;
+    c1 = s.c1;
+    c2 = s.c2;
+  }
+  for (int64_t c0 = crowded ? m1 : m0; c0 < m1; c0 += MK_AHEAD) {
     double x[MK_AHEAD], y[MK_AHEAD], z[MK_AHEAD], ee[MK_AHEAD], rr[MK_AHEAD];
 #pragma unroll
     for (int k = 0; k < MK_AHEAD; k++)
