@@ -399,30 +399,22 @@ __device__ __forceinline__ void element_plane(int A, const T *ut, T *yt, T *side
 
   // viscous action: K of the next two points is in flight while one computes
   // (measured at 128^3: FP64 2.18 -> 2.02 ms, FP32 1.20 -> 1.12 ms)
-  constexpr bool DEEP = true;
   const T *kp = Ke + koff(9 * A, 0);
   T Kn[9], Kn2[9];
 #pragma unroll
   for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(0, r));
-  if (DEEP) {
 #pragma unroll
-    for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(1, r));
-  }
+  for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(1, r));
 #pragma unroll
   for (int p = 0; p < 9; p++) {
     T Kq[9];
 #pragma unroll
     for (int r = 0; r < 9; r++) Kq[r] = Kn[r];
-    if (DEEP) {
 #pragma unroll
-      for (int r = 0; r < 9; r++) Kn[r] = Kn2[r];
-      if (p < 7) {
+    for (int r = 0; r < 9; r++) Kn[r] = Kn2[r];
+    if (p < 7) {
 #pragma unroll
-        for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(p + 2, r));
-      }
-    } else if (p < 8) {
-#pragma unroll
-      for (int r = 0; r < 9; r++) Kn[r] = ldk(kp + koff(p + 1, r));
+      for (int r = 0; r < 9; r++) Kn2[r] = ldk(kp + koff(p + 2, r));
     }
     q2::qp_action_K(Kq, G, p);
   }
