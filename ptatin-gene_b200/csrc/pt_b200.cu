@@ -1896,7 +1896,17 @@ static double tiling_layers(const pt_op *op, int lz, int64_t slots)
   return c;
 }
 
-// Element layers per z-chunk.  Small boxes: about 2048 tiles, at least 2 layers.
+// Element layers per z-chunk of a box of txy rows of tiles: about 2048 tiles, at
+// least 2 layers.
+static int small_box_lz(int64_t txy, int mz)
+{
+  int nzc = (int)((2048 + txy - 1) / txy);
+  nzc = nzc < 1 ? 1 : (nzc > (mz + 1) / 2 ? (mz + 1) / 2 : nzc);
+  if (nzc < 1) nzc = 1;
+  return (mz + nzc - 1) / nzc;
+}
+
+// Element layers per z-chunk.  Small boxes: small_box_lz.
 // From 2048 tiles on, the depth whose colour classes take the fewest layers in
 // FP64 (256 threads per SM) and FP32 (512 with 128-wide tiles; its layers take
 // about 0.6 of the time).  128^3: classes of 1.7 waves with 8 layers (64 layers
@@ -1906,10 +1916,7 @@ static double tiling_layers(const pt_op *op, int lz, int64_t slots)
 static int default_lz(const pt_op *op)
 {
   const int64_t txy = (int64_t)op->ntx * op->my;
-  int nzc = (int)((2048 + txy - 1) / txy);
-  nzc = nzc < 1 ? 1 : (nzc > (op->mz + 1) / 2 ? (op->mz + 1) / 2 : nzc);
-  if (nzc < 1) nzc = 1;
-  const int lz0 = (op->mz + nzc - 1) / nzc;
+  const int lz0 = small_box_lz(txy, op->mz);
   if (txy * ((op->mz + 1) / 2) < 2048) return lz0;
   const int64_t slots = 148 * (256 / op->TX), slots32 = op->TX == 128 ? 2 * slots : slots;
   int best = lz0;
@@ -2078,14 +2085,8 @@ extern "C" pt_status pt_a11_apply_noalloc_d(const pt_mesh_desc *desc, const doub
   ptk::StreamGrid g;
   g.b = bx;
   g.TX = TX; g.ntx = ntx;
-  {
-    const int64_t txy = (int64_t)ntx * desc->my;
-    int nzc = (int)((2048 + txy - 1) / txy);
-    nzc = nzc < 1 ? 1 : (nzc > (desc->mz + 1) / 2 ? (desc->mz + 1) / 2 : nzc);
-    if (nzc < 1) nzc = 1;
-    g.LZ = (desc->mz + nzc - 1) / nzc;
-    g.nzc = (desc->mz + g.LZ - 1) / g.LZ;
-  }
+  g.LZ = small_box_lz((int64_t)ntx * desc->my, desc->mz);  // the scratch holds small boxes only
+  g.nzc = (desc->mz + g.LZ - 1) / g.LZ;
   if (TX == 32) s = noalloc_launch<32>(g, desc->my, K, u, y, st);
   else if (TX == 64) s = noalloc_launch<64>(g, desc->my, K, u, y, st);
   else s = noalloc_launch<128>(g, desc->my, K, u, y, st);
