@@ -50,3 +50,47 @@ def test_pinned_host_applies_beside_device_applies_of_another_thread():
         stop.set()
         t.join()
         assert not bad and seen and all(seen) and all(ok), (bad, len(seen), sum(seen), sum(ok))
+
+
+@pytest.mark.parametrize("fp32", [False, True])
+def test_one_batch_on_two_streams_and_in_a_graph(fp32):
+    """Each apply of a batch has scratch of its own: applies that overlap on two
+    streams, and a recorded one replayed beside them, are bitwise the apply alone."""
+    import torch
+
+    from pt_b200.batch import BatchA11
+    ops, us = [], []
+    try:
+        for i, dims in enumerate([(17, 13, 11), (33, 20, 9), (8, 8, 8), (41, 7, 5)]):
+            m = M.make_mesh(*dims, perturb=0.05, seed=i)
+            ops.append(_op(m, M.eta_per_element(m, contrast=1e3, seed=i), M.bc_mask_freeslip(*dims)))
+            us.append([torch.from_numpy(M.uniform_vec(m.nvel, 9 * i + k)).cuda() for k in range(3)])
+        us = [[v.float() if fp32 else v for v in row] for row in us]
+        xs = [[row[k] for row in us] for k in range(3)]  # three input sets
+        with BatchA11(ops) as b:
+            want = [[torch.empty_like(v) for v in x] for x in xs]
+            got = [[torch.empty_like(v) for v in x] for x in xs]
+            for x, w, g in zip(xs, want, got):
+                b.apply(x, w)
+                b.tables(x, g)  # pointer tables exist before the capture
+            torch.cuda.synchronize()
+            st = [torch.cuda.Stream() for _ in range(3)]
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=st[2]):
+                b.apply(xs[2], got[2], stream=st[2])
+            for _ in range(20):
+                for g in got:
+                    for y in g:
+                        y.fill_(np.nan)
+                torch.cuda.synchronize()
+                for _ in range(3):
+                    b.apply(xs[0], got[0], stream=st[0])
+                    b.apply(xs[1], got[1], stream=st[1])
+                    with torch.cuda.stream(st[2]):
+                        graph.replay()
+                torch.cuda.synchronize()
+                for k in range(3):
+                    assert all(torch.equal(a, w) for a, w in zip(got[k], want[k])), k
+    finally:
+        for op in ops:
+            op.Destroy()
