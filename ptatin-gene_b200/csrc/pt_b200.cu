@@ -869,6 +869,7 @@ pt_status launch_div(pt_op *op)
 pt_status ensure_div(pt_op *op, bool *have)
 {
   pt_status s = PT_OK;
+  LayerLock lock(op);  // two host threads' first calls share one set
   if (!op->d_D && !capturing(op)) {
     const int64_t nd = ptk::dsize(op->nel);
     const bool blocks = op->full_box && op->nel <= DIV_BLOCKS_MAX_ELEMENTS;

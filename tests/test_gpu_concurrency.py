@@ -94,3 +94,34 @@ def test_one_batch_on_two_streams_and_in_a_graph(fp32):
     finally:
         for op in ops:
             op.Destroy()
+
+
+@pytest.mark.parametrize("dims", [(9, 8, 7), (52, 50, 50)])
+def test_first_calls_of_two_threads(dims):
+    """B u, B^T p and the tiles' sums are set up by whichever thread comes first."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    m = M.make_mesh(*dims, perturb=0.05, seed=1)
+    u, p = (torch.from_numpy(M.uniform_vec(n, 3)).cuda() for n in (m.nvel, m.npres))
+    calls = [lambda op: op.MFStokesWrapper_A12(p), lambda op: op.MFStokesWrapper_A21(u)]
+    want = None
+    for _ in range(6):
+        with MatStokesMF(*dims) as op:
+            op.set_coords(m.coords)
+            op.set_stream(torch.cuda.Stream())
+            got, start = {}, threading.Barrier(4)
+
+            def run(k):
+                start.wait()
+                got[k] = calls[k % 2](op)
+
+            ts = [threading.Thread(target=run, args=(k,)) for k in range(4)]
+            for t in ts:
+                t.start()
+            for t in ts:
+                t.join()
+            torch.cuda.synchronize()
+            want = want or [c(op) for c in calls]
+            torch.cuda.synchronize()
+            assert all(torch.equal(got[k], want[k % 2]) for k in range(4))
