@@ -78,17 +78,26 @@ constexpr int MK_AHEAD = 4;
 constexpr int64_t MK_FEW = 16384;                      // elements
 constexpr int64_t MK_CROWDED_FEW = 256, MK_CROWDED = 1024;  // markers in an element
 
-// A crowded element's five sums of lane v, out of line so that the common loop keeps
-// its registers.
-struct MkSums {
-  double s1, s2, sb, c1, c2;
-};
-__device__ __noinline__ MkSums mk_crowded(int v, int64_t m0, int64_t m1, const int32_t *__restrict__ order,
-                                          const double *__restrict__ xi, const double *__restrict__ eta,
-                                          const double *__restrict__ rho)
+__device__ __forceinline__ void mk_store(double *o, int v, double s1, double s2, double sb, double c1, double c2,
+                                         int64_t n)
+{
+  o[3 * v] = s1;
+  o[3 * v + 1] = s2;
+  o[3 * v + 2] = sb;
+  if (v == 0) {
+    o[24] = c1;
+    o[25] = c2;
+    o[26] = (double)n;
+  }
+}
+
+// A crowded element, lane v; out of line so that the common loop keeps its registers.
+__device__ __noinline__ void mk_crowded(int v, int64_t m0, int64_t m1, const int32_t *__restrict__ order,
+                                        const double *__restrict__ xi, const double *__restrict__ eta,
+                                        const double *__restrict__ rho, double *__restrict__ o)
 {
   const unsigned group = 0xffu << (threadIdx.x & 24);
-  MkSums s = {};
+  double s1 = 0.0, s2 = 0.0, sb = 0.0, c1 = 0.0, c2 = 0.0;
   double a[5] = {};  // lane v: marker v of the eight under way
   const auto index = [&](int64_t c) { return c + v < m1 ? order[c + v] : -1; };
   const auto load = [&](int64_t p) {
@@ -115,14 +124,14 @@ __device__ __noinline__ MkSums mk_crowded(int v, int64_t m0, int64_t m1, const i
 #pragma unroll
         for (int i = 0; i < 5; i++) w[i] = __shfl_sync(group, m[i], k, 8);
         const double N = mk_q1(v, w[0], w[1], w[2]);
-        s.s1 += N * w[3];
-        s.s2 += N * w[4];
-        s.sb += N;
-        s.c1 += w[3];
-        s.c2 += w[4];
+        s1 += N * w[3];
+        s2 += N * w[4];
+        sb += N;
+        c1 += w[3];
+        c2 += w[4];
       }
   }
-  return s;
+  mk_store(o, v, s1, s2, sb, c1, c2, m1 - m0);
 }
 
 __global__ void __launch_bounds__(128) mk_element_kernel(int64_t nel, const int64_t *__restrict__ start,
@@ -135,16 +144,11 @@ __global__ void __launch_bounds__(128) mk_element_kernel(int64_t nel, const int6
   if (e >= nel) return;
   double s1 = 0.0, s2 = 0.0, sb = 0.0, c1 = 0.0, c2 = 0.0;
   const int64_t m0 = start[e], m1 = start[e + 1];
-  const bool crowded = m1 - m0 > (nel <= MK_FEW ? MK_CROWDED_FEW : MK_CROWDED);
-  if (crowded) {
-    const MkSums s = mk_crowded(v, m0, m1, order, xi, eta, rho);
-    s1 = s.s1;
-    s2 = s.s2;
-    sb = s.sb;
-    c1 = s.c1;
-    c2 = s.c2;
+  if (m1 - m0 > (nel <= MK_FEW ? MK_CROWDED_FEW : MK_CROWDED)) {
+    mk_crowded(v, m0, m1, order, xi, eta, rho, part + e * MK_SUMS);
+    return;
   }
-  for (int64_t c0 = crowded ? m1 : m0; c0 < m1; c0 += MK_AHEAD) {
+  for (int64_t c0 = m0; c0 < m1; c0 += MK_AHEAD) {
     double x[MK_AHEAD], y[MK_AHEAD], z[MK_AHEAD], ee[MK_AHEAD], rr[MK_AHEAD];
 #pragma unroll
     for (int k = 0; k < MK_AHEAD; k++)
@@ -167,15 +171,7 @@ __global__ void __launch_bounds__(128) mk_element_kernel(int64_t nel, const int6
         c2 += rr[k];
       }
   }
-  double *o = part + e * MK_SUMS;
-  o[3 * v] = s1;
-  o[3 * v + 1] = s2;
-  o[3 * v + 2] = sb;
-  if (v == 0) {
-    o[24] = c1;
-    o[25] = c2;
-    o[26] = (double)(m1 - m0);
-  }
+  mk_store(part + e * MK_SUMS, v, s1, s2, sb, c1, c2, m1 - m0);
 }
 
 // Per node of the element box (compact index i + j X + k X Y, X = 2mx+1):
