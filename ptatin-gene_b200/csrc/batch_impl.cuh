@@ -10,6 +10,7 @@
 // Included from pt_b200.cu after struct pt_op.
 #pragma once
 
+#include <algorithm>
 #include <map>
 #include <vector>
 
@@ -30,6 +31,7 @@ struct pt_batch {
     std::vector<Cls> classes;
     int64_t tiles, lay_tiles, lay_nodes, lay_values;
     int coloured;  // problems on coloured tiles
+    bool borrowed; // items and lay lists are the other precision's
     // host copies, kept until destroy for the pooled batches' asynchronous uploads
     std::vector<ptk::BatchProb> h;
     std::vector<int4> hitems;
@@ -254,8 +256,22 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
   b->pool = pool;
   b->stream = stream;
   cudaError_t e = cudaSuccess;
+  // one list for both precisions (but for K) where every op has one kernel for both
+  const bool one = std::all_of(ops, ops + n, [](const pt_op *op) { return op->a11_kernel == op->a11_kernel32; });
   for (int f = 0; f < 2; f++) {
     pt_batch::List &l = b->list[f];
+    if (f && one) {
+      const pt_batch::List &o = b->list[0];
+      l.d_items = o.d_items; l.d_lay = o.d_lay;
+      l.classes = o.classes;
+      l.tiles = o.tiles; l.lay_tiles = o.lay_tiles; l.lay_nodes = o.lay_nodes; l.lay_values = o.lay_values;
+      l.coloured = o.coloured;
+      l.borrowed = true;
+      l.h = o.h;
+      for (int i = 0; i < n; i++) l.h[i].K = ops[i]->d_K32;
+      if (e == cudaSuccess) e = batch_upload(b, &l.d_probs, l.h);
+      break;
+    }
     batch_list(n, ops, lz, tile_x, f != 0, layers, l);
     if (e == cudaSuccess) e = batch_upload(b, &l.d_probs, l.h);
     if (e == cudaSuccess) e = batch_upload(b, &l.d_items, l.hitems);
@@ -308,7 +324,7 @@ pt_status pt_batch_destroy(pt_batch *b)
 {
   if (!b) return PT_OK;
   for (const pt_batch::List &l : b->list) {
-    void *bufs[] = {l.d_probs, l.d_items, l.d_lay};
+    void *bufs[] = {l.d_probs, l.borrowed ? nullptr : l.d_items, l.borrowed ? nullptr : l.d_lay};
     for (void *p : bufs) {
       if (!p) continue;
       if (b->pool) cudaFreeAsync(p, b->stream);
