@@ -1,4 +1,9 @@
-// Element kernels with an 8-colour deterministic scatter.
+// Element kernels with an 8-colour deterministic scatter: A11 "b200_colour", and
+// what runs where the tile kernels cannot -- A11 and the diagonal of a geometry
+// with w eta / det <= 0, and B u, B^T p and the body-force load where there is no
+// room for their stored factors or a capture comes before those exist.  They read
+// coordinates and viscosity and store nothing, with their per-element arrays in
+// local memory.
 //
 // Elements are split by the parity of (ei, ej, ek); two elements of one
 // colour are at least two elements apart along some axis and share no node,

@@ -10,7 +10,8 @@
 // row, 8 at an x-tile edge) sums of a node in a fixed order, with the
 // Dirichlet rows in the same pass.  Two launches, deterministic, no colours.
 // The price is the scratch, about 450 B written and read per element next to
-// 1.9 KB of K, which is why large boxes keep the z-march.
+// 1.9 KB of K, which is why long boxes with full rows keep the z-march (the rule
+// and its figures: auto_kernel in pt_b200.cu).
 //
 // A tile is E consecutive elements whatever the row length (layer_grid.cuh),
 // so rows that do not divide it leave no thread idle.
@@ -755,11 +756,11 @@ __global__ void __launch_bounds__(NT, 256 / NT) body_force_layer_kernel(LayerGri
 //   (B u)_i = sum_q Np_i sum_kd D[3k+d] G'[d][k],    Np = {1, x^_0, x^_1, x^_2}
 //   dv'[d][l] = (sum_i p_i Np_i) D[3l+d]              (the transpose's input)
 // (MatMultMF_Stokes_MixedFEM3d_A21 / _A12, src/stokes_q2p1_mf_operators_def.c:
-// 423-538).  324 values per element like the 4 x 81 blocks of B itself, but
-// formed in one pass over the coordinates (the blocks took 12 transposed
-// contractions per element and scattered stores: 64x48x40 1,031 us) and
-// read in whole lines by one thread per element.  Coordinates only: a
-// viscosity update keeps them.
+// 423-538).  324 values per element like the 4 x 81 blocks of B itself (which
+// small one-rank boxes form from D, kernels_bmat.cuh), but formed in one pass
+// over the coordinates (64x48x40 70 us; the blocks straight from the coordinates
+// 1,031 us) and read in whole lines by one thread per element.  Coordinates only:
+// a viscosity update keeps them.
 constexpr int DN = 12;
 constexpr int DBLOCK = 27 * DN * KB;
 __host__ __device__ __forceinline__ int64_t delem(int64_t e) { return e / KB * DBLOCK + e % KB; }

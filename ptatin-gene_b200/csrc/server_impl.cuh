@@ -10,15 +10,15 @@
 // the batch once its set-up event has completed.  All
 // active requests advance together, one preconditioned flexible-CG iteration
 // at a time: the A11 applies of every request go through one batched
-// work-list (one launch per colour / tile-width class, batch_impl.cuh) and
-// the vector updates and dot products through chunk-list kernels over all
-// requests, so an iteration costs the same ~20 launches whatever the number
-// of requests.  Requests join between iterations as slots and memory free up
+// work-list (layer tiles and their gather, two launches; one per colour and
+// tile-width class for boxes that stream, batch_impl.cuh) and the vector updates
+// and dot products through chunk-list kernels over all requests, so an iteration
+// costs the same launches (16 at degree 3) whatever the number of requests.  Requests join between iterations as slots and memory free up
 // (admission against a byte budget; their set-up runs on a second stream
 // while the batch iterates) and leave when converged.
 //
 // Per request the arithmetic is independent of the batch: the batched apply
-// sums every node in the request's own colour order (bitwise its single-op
+// sums every node in the request's own order (bitwise its single-op
 // result), dot products reduce the request's own fixed chunks in a fixed
 // order, and scalars live per request.  A result is therefore bitwise the
 // same alone and in any mix.
