@@ -384,9 +384,9 @@ pt_status pt_residual_u_h(pt_op *op, const double *u, const double *p, double *r
 /* Select the A11 kernel by name, like the reference's -a11_op function list
  * (src/stokes_operators.c:123-154).  Names: "b200" (default: the fastest
  * measured for the box -- stored element matrices for one-rank boxes of at most
- * 2000 elements, layer tiles above, the streaming kernel for boxes whose rows
- * nearly fill its tiles -- in FP64 from 200000 elements with rows of whole warps,
- * in FP32 from 350000 -- and for boxes above 2^23),
+ * 2000 elements (in FP32 4096), layer tiles above, the streaming kernel for boxes
+ * whose rows nearly fill its tiles -- in FP64 from 200000 elements with rows of
+ * whole warps, in FP32 from 350000 -- and for boxes above 2^23),
  * "b200_layer" (single-layer tiles gathered node by node; at most 2^23
  * elements, else PT_ERR_UNSUPPORTED), "b200_stream" (the streaming kernel with
  * precomputed Gauss-point geometry), "b200_ebe" (stored 81x81 element matrices,

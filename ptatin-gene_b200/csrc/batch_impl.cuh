@@ -157,6 +157,8 @@ int64_t batch_launches(const pt_batch *b, bool fp32)
   return (int64_t)l.classes.size() + (l.lay_tiles ? 2 : 0) + (l.coloured ? 1 : 0);
 }
 
+bool batch_on_layers(int kernel) { return kernel == A11_LAYER || kernel == A11_EBE; }
+
 void batch_list(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, bool fp32, bool layers, pt_batch::List &l)
 {
   // class key: (pass, TX) -> items
@@ -179,7 +181,7 @@ void batch_list(int n, pt_op *const *ops, const int32_t *lz, int32_t tile_x, boo
     // for their sums (a box whose own applies use element matrices too: they are
     // not batched)
     const int kernel = fp32 ? op->a11_kernel32 : op->a11_kernel;
-    d.layer = layers && (kernel == A11_LAYER || kernel == A11_EBE) && !(lz && lz[i] > 0);
+    d.layer = layers && batch_on_layers(kernel) && !(lz && lz[i] > 0);
     d.lg = op->lg;
     d.lay_off = l.lay_values;
     d.K = fp32 ? (const void *)op->d_K32 : (const void *)op->d_K;
@@ -256,8 +258,10 @@ static pt_status batch_create_impl(int n, pt_op *const *ops, const int32_t *lz, 
   b->pool = pool;
   b->stream = stream;
   cudaError_t e = cudaSuccess;
-  // one list for both precisions (but for K) where every op has one kernel for both
-  const bool one = std::all_of(ops, ops + n, [](const pt_op *op) { return op->a11_kernel == op->a11_kernel32; });
+  // one list for both precisions (but for K) where every op takes the same tiles in both
+  const bool one = std::all_of(ops, ops + n, [](const pt_op *op) {
+    return batch_on_layers(op->a11_kernel) == batch_on_layers(op->a11_kernel32);
+  });
   for (int f = 0; f < 2; f++) {
     pt_batch::List &l = b->list[f];
     if (f && one) {

@@ -71,11 +71,13 @@ pt_status fail(pt_status s, const char *fmt, ...)
 enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 
 // "b200" picks a kernel for the box, in each precision.
-// - One-rank boxes of up to EBE_AUTO_MAX_ELEMENTS: stored element matrices.  The
-//   line is where their set-up comes even with the faster applies: a new
-//   viscosity costs 0.5 us per element more than layer tiles, so 12^3 (apply
-//   15.1 vs 22.7 us) pays from 110 applies on, 13^3 in FP32 (15.5 vs 22.7 us)
-//   from 146, 16^3 in FP32 (16.7 vs 22.7 us) from 320.
+// - One-rank boxes of up to EBE_AUTO_MAX_ELEMENTS (FP32 EBE_AUTO_MAX_F32_ELEMENTS):
+//   stored element matrices.  The lines are where their set-up, a quarter of a
+//   microsecond per element, viscosity and precision, comes even with the faster
+//   applies: 12^3 (15.1 vs 22.7 us on layer tiles) pays from 110 applies on, 13^3 in
+//   FP64 (20.7 vs 22.7 us) from 530; in FP32 alone 13^3 (15.5 vs 22.7 us) from 75,
+//   16^3 (16.7 vs 22.7) from 160, 18^3 (20.7 vs 22.8) from 600.  A solve makes
+//   several hundred FP32 applies per viscosity.
 // - Streaming tiles for long boxes whose rows nearly fill them.  FP64, from
 //   STREAM_AUTO_MIN_ELEMENTS and with rows of whole warps (layer tiles vs
 //   streaming: 64x60x52 159 vs 167 us, 64x64x56 180 vs 177, 32x90x80 186 vs 175,
@@ -89,6 +91,7 @@ enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 // - Layer tiles for the rest (80^3 381 vs 484 us, 97x70x81 408 vs 547; FP32 273 vs
 //   279, 290 vs 294).
 constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
+constexpr int64_t EBE_AUTO_MAX_F32_ELEMENTS = 4096;
 constexpr int64_t STREAM_AUTO_MIN_ELEMENTS = 200000;
 constexpr int64_t STREAM_AUTO_MIN_F32_ELEMENTS = 350000;
 constexpr int64_t LAYER_MAX_ELEMENTS = (int64_t)1 << 23;
@@ -431,7 +434,7 @@ constexpr int LNT = ptk::LAYER_NT;
 
 A11Kernel auto_kernel(const pt_op *op, bool fp32)
 {
-  if (op->full_box && op->nel <= EBE_AUTO_MAX_ELEMENTS) return A11_EBE;
+  if (op->full_box && op->nel <= (fp32 ? EBE_AUTO_MAX_F32_ELEMENTS : EBE_AUTO_MAX_ELEMENTS)) return A11_EBE;
   const bool full_rows = 10 * (int64_t)op->mx >= 9 * (int64_t)op->ntx * op->TX;
   const bool stream = fp32 ? op->nel >= STREAM_AUTO_MIN_F32_ELEMENTS && full_rows
                            : op->nel >= STREAM_AUTO_MIN_ELEMENTS && full_rows && op->mx % 32 == 0;
@@ -648,13 +651,16 @@ pt_status ensure_geometry(pt_op *op)
 // Element matrices of the current geometry (A11_EBE), built on first use.
 pt_status ensure_ebe(pt_op *op)
 {
-  if (op->ebe_valid) return PT_OK;
-  if (!op->d_Ae) PT_CUDA(op_alloc(op, (void **)&op->d_Ae, sizeof(double) * ptk::EBE_LD * op->nel));
+  const bool fp64 = op->a11_kernel == A11_EBE;  // else only FP32 applies use them
+  if (op->ebe_valid && (op->d_Ae || !fp64)) return PT_OK;
+  if (!op->d_Ae && fp64) PT_CUDA(op_alloc(op, (void **)&op->d_Ae, sizeof(double) * ptk::EBE_LD * op->nel));
   if (!op->d_Ae32) PT_CUDA(op_alloc(op, (void **)&op->d_Ae32, sizeof(float) * ptk::EBE_LD * op->nel));
   if (!op->d_ye) PT_CUDA(op_alloc(op, (void **)&op->d_ye, sizeof(double) * 81 * op->nel));
-  ptk::element_matrix_kernel<double><<<(unsigned)op->nel, 96, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
-                                                                               op->d_Ae);
-  PT_LAUNCHED(op);
+  if (op->d_Ae) {
+    ptk::element_matrix_kernel<double><<<(unsigned)op->nel, 96, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
+                                                                                 op->d_Ae);
+    PT_LAUNCHED(op);
+  }
   ptk::element_matrix_kernel<float><<<(unsigned)op->nel, 96, 0, op->stream>>>(op->box, op->d_coords, op->d_eta,
                                                                               op->d_Ae32);
   PT_LAUNCHED(op);
@@ -738,7 +744,11 @@ const float *op_K<float>(const pt_op *op) { return op->d_K32; }
 template <typename T>
 pt_status launch_a11(pt_op *op, const T *u, T *y, bool masked)
 {
-  const int kernel = op_kernel<T>(op);
+  int kernel = op_kernel<T>(op);
+  // Matrices that only FP32 applies use are renewed by the next of them, not by
+  // every apply: a graph records the tiles, whose K any apply renews (a solver
+  // records its graph again when the viscosity changes).
+  if (kernel == A11_EBE && op->a11_kernel == A11_LAYER && !op->graph_own && capturing(op)) kernel = A11_LAYER;
   if (kernel == A11_EBE && op->full_box) {
     pt_status s = ensure_geometry(op);
     if (s != PT_OK) return s;

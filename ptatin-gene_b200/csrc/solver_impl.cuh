@@ -550,7 +550,7 @@ pt_status mg_coarsen(pt_solver *s, const pt_op *f, const double *vf_f, double *v
   if (f->a11_kernel == A11_COLOUR) {
     c->a11_kernel = c->a11_kernel32 = A11_COLOUR;
     if ((st = ensure_f32(c)) != PT_OK) return st;
-  } else if (c->a11_kernel == A11_EBE) c->a11_kernel = c->a11_kernel32 = A11_LAYER;
+  } else if (c->a11_kernel32 == A11_EBE) c->a11_kernel = c->a11_kernel32 = A11_LAYER;
   const MgBox fb = mgbox(f), cb = mgbox(c);
   inject_coords_kernel<<<vgrid(c->nnodes), 256, 0, c->stream>>>(fb, cb, f->d_coords, c->d_coords);
   PT_LAUNCHED(c);

@@ -64,9 +64,9 @@ def test_batch_of_default_ops_is_bitwise_their_own_applies(box, fp32):
     from pt_b200.batch import BatchA11
     m, eta, mask, u, op, k64, k32 = box
     op.set_a11_op("b200")
-    small = M.make_mesh(17, 13, 11, perturb=0.05, seed=4)
-    with MatStokesMF(17, 13, 11) as other:
-        other.SetUp(small.coords, M.eta_per_element(small, contrast=1e2, seed=5), M.bc_mask_freeslip(17, 13, 11))
+    small = M.make_mesh(17, 17, 15, perturb=0.05, seed=4)
+    with MatStokesMF(17, 17, 15) as other:
+        other.SetUp(small.coords, M.eta_per_element(small, contrast=1e2, seed=5), M.bc_mask_freeslip(17, 17, 15))
         us = [u, torch.from_numpy(M.uniform_vec(small.nvel, 6)).cuda()]
         us = [v.float() for v in us] if fp32 else us
         for masked in (True, False):
@@ -107,3 +107,56 @@ def test_default_fp32_apply_on_a_ghosted_box(ora):
         inside = np.zeros(c.shape, dtype=bool)
         inside[sl] = True
         assert not y.reshape(c.shape)[~inside & ~mask].any()
+
+
+def test_fp32_alone_from_element_matrices(ora):
+    """Between the two lines of the stored matrices FP32 applies use them, FP64 ones the
+    layer tiles; graphs record the tiles, and both follow the viscosity."""
+    import torch
+
+    from pt_b200 import MatStokesMF
+    dims = (16, 16, 16)
+    m = M.make_mesh(*dims, perturb=0.05, seed=1)
+    etas = [M.eta_per_element(m, contrast=1e3, seed=s) for s in (2, 3)]
+    mask = M.bc_mask_freeslip(*dims)
+    u = torch.from_numpy(M.uniform_vec(m.nvel, 3)).cuda()
+    u32, y = u.float(), torch.empty(m.nvel, dtype=torch.float32, device="cuda")
+    want = [ora.matmult_a11(m.dims, m.coords, e, mask, u.cpu().numpy()) for e in etas]
+
+    def record(op):
+        st = torch.cuda.Stream()
+        op.set_stream(st)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            op.MatMult_MFStokes_A11(u32, y)
+        return g
+
+    with MatStokesMF(*dims) as op, MatStokesMF(*dims) as named:
+        op.SetUp(m.coords, etas[0], mask)
+        assert op.a11_op == "b200_layer"
+        op.MatMult_MFStokes_A11(u)
+        graphs = [record(op)]  # FP32 has not run yet
+        torch.cuda.synchronize()
+        for name, dtype in (("b200_layer", torch.float64), ("b200_ebe", torch.float32)):
+            named.set_a11_op(name)
+            named.SetUp(m.coords, etas[0], mask)
+            assert torch.equal(op.MatMult_MFStokes_A11(u.to(dtype)), named.MatMult_MFStokes_A11(u.to(dtype)))
+        torch.cuda.synchronize()
+        graphs.append(record(op))
+        for e, w in zip(etas, want):
+            op.set_eta(e)
+            op.MatMult_MFStokes_A11(u)  # an FP64 apply renews what the graphs read
+            for g in graphs:
+                y.fill_(float("nan"))
+                torch.cuda.synchronize()
+                g.replay()
+                torch.cuda.synchronize()
+                assert relerr(y.double().cpu(), w) < TOL32
+            y32 = op.MatMult_MFStokes_A11(u32)
+            torch.cuda.synchronize()
+            assert relerr(y32.double().cpu(), w) < TOL32
+        op.set_a11_op("b200_ebe")  # FP64 from matrices too, from here on
+        y64 = op.MatMult_MFStokes_A11(u)
+        torch.cuda.synchronize()  # the op is on the capture's stream
+        assert relerr(y64.cpu(), want[1]) < 1e-12
+        assert relerr(op.MatGetDiagonal_MFStokes_A11(), ora.getdiag_a11(m.dims, m.coords, etas[1], mask)) < 1e-12
