@@ -718,6 +718,7 @@ pt_status launch_ebe_pair(pt_op *op, const T *u, T *y)
 template <typename T>
 pt_status launch_ebe(pt_op *op, const T *u, T *y, bool masked)
 {
+  LayerLock lock(op);  // the pair shares d_ye
   pt_status s = ensure_ebe(op);
   if (s != PT_OK) return s;
   return masked ? launch_ebe_pair<T, true>(op, u, y) : launch_ebe_pair<T, false>(op, u, y);

@@ -125,3 +125,26 @@ def test_first_calls_of_two_threads(dims):
             want = want or [c(op) for c in calls]
             torch.cuda.synchronize()
             assert all(torch.equal(got[k], want[k % 2]) for k in range(4))
+
+
+@pytest.mark.parametrize("dims", [(8, 8, 8), (16, 16, 16), (20, 18, 16)])
+def test_applies_of_two_threads(dims):
+    """Both precisions of the default op from two host threads: the launches of an apply
+    stay together whatever kernel serves it."""
+    import torch
+    m = M.make_mesh(*dims, perturb=0.05, seed=1)
+    u = torch.from_numpy(M.uniform_vec(m.nvel, 3)).cuda()
+    us = [u, -2.0 * u, u.float(), (-2.0 * u).float()]
+    with _op(m, M.eta_per_element(m, contrast=1e3, seed=2), M.bc_mask_freeslip(*dims), "b200") as op:
+        want = [op.MatMult_MFStokes_A11(v) for v in us]
+        got = [[torch.empty_like(v) for _ in range(50)] for v in us]
+        torch.cuda.synchronize()
+        ts = [threading.Thread(target=lambda k=k: [op.MatMult_MFStokes_A11(us[k], y) for y in got[k]])
+              for k in range(len(us))]
+        for t in ts:
+            t.start()
+        for t in ts:
+            t.join()
+        torch.cuda.synchronize()
+        for k, w in enumerate(want):
+            assert all(torch.equal(y, w) for y in got[k]), k
