@@ -75,8 +75,8 @@ enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 //   stored element matrices.  The lines are where their set-up, a quarter of a
 //   microsecond per element, viscosity and precision, comes even with the faster
 //   applies: 12^3 (15.1 vs 22.7 us on layer tiles) pays from 110 applies on, 13^3 in
-//   FP64 (20.7 vs 22.7 us) from 530; in FP32 alone 13^3 (15.5 vs 22.7 us) from 75,
-//   16^3 (16.7 vs 22.7) from 160, 18^3 (20.7 vs 22.8) from 600.  A solve makes
+//   FP64 (20.7 vs 22.7 us) from 530; in FP32 alone 13^3 (12.5 vs 22.7 us) from 50,
+//   16^3 (16.7 vs 22.7) from 155, 18^3 (20.7 vs 22.8) from 600.  A solve makes
 //   several hundred FP32 applies per viscosity.
 // - Streaming tiles for long boxes whose rows nearly fill them.  FP64, from
 //   STREAM_AUTO_MIN_ELEMENTS and with rows of whole warps (layer tiles vs
@@ -87,7 +87,9 @@ enum A11Kernel { A11_STREAM = 0, A11_COLOUR = 1, A11_EBE = 3, A11_LAYER = 4 };
 //   200 vs 196, 122x60x60 234 vs 221, 128x64x64 263 vs 229, 128^3 990 vs 825).
 // - Streaming tiles past LAYER_MAX_ELEMENTS, where the layer tiles' scratch would
 //   grow past 4.3 GB (512 bytes per element at most for rows of three elements and
-//   more, 716 for rows of two, 1,433 for rows of one).
+//   more, 716 for rows of two, 1,433 for rows of one).  B^T p, the whole operator,
+//   the residual and the body-force load use that scratch at any size, where there
+//   is room (alloc_if_room).
 // - Layer tiles for the rest (80^3 381 vs 484 us, 97x70x81 408 vs 547; FP32 273 vs
 //   279, 290 vs 294).
 constexpr int64_t EBE_AUTO_MAX_ELEMENTS = 2000;
@@ -465,10 +467,10 @@ pt_status ensure_layer(pt_op *op)
 }
 
 // The scratch of an apply (p null where there is no room): the op's own or, in a
-// capture, memory of the graph
-// (an allocation and a free recorded with the apply), so that graphs captured
-// from one op may run at the same time on several streams.  A solver's graph
-// runs on the op's stream only and uses the op's scratch (graph_own).
+// capture, memory of the graph (an allocation and a free recorded with the apply),
+// so that graphs captured from one op may run at the same time on several streams.
+// A solver's graph runs on the op's stream only and uses the op's scratch
+// (graph_own).
 struct LayerScratch {
   pt_op *op;
   double *p = nullptr;
